@@ -117,15 +117,26 @@ __constant__ double c_yu5_pts[5][3] = { { 0.25, 0.25, 0.25 },
                                         { 1.0 / 6.0, 1.0 / 6.0, 0.5 } };
 __constant__ double c_yu5_w[5]      = { -2.0 / 15.0, 3.0 / 40.0, 3.0 / 40.0, 3.0 / 40.0, 3.0 / 40.0 };
 
+// sin and cos of 2 pi f (x + p) go through sinpi / cospi, which need no reduction by an irrational
+// period: fewer instructions than sin and cos, and no error from the rounded 2 pi f
+__device__ __forceinline__ double sin_pi( double v ) { return sinpi( v ); }
+__device__ __forceinline__ float  sin_pi( float v ) { return sinpif( v ); }
+__device__ __forceinline__ double cos_pi( double v ) { return cospi( v ); }
+__device__ __forceinline__ float  cos_pi( float v ) { return cospif( v ); }
+
+// radius: |P| where the caller has it, or a negative value
 template < typename A >
-__device__ __forceinline__ A coeff_eval( const Coefficient& k, const A* P )
+__device__ __forceinline__ A coeff_eval( const Coefficient& k, const A* P, A radius = A( -1 ) )
 {
    if ( k.kind == 0 ) return A( k.value );
    if ( k.kind == 2 )  // radial profile exp(amp (value - |x|) / freq)
-      return exp( A( k.amp ) * ( A( k.value ) - sqrt( P[0] * P[0] + P[1] * P[1] + P[2] * P[2] ) ) / A( k.freq ) );
-   const A tp = A( 2.0 * 3.14159265358979323846 * k.freq );
-   return exp( A( k.amp ) * sin( tp * ( P[0] + A( k.phase[0] ) ) ) * cos( tp * ( P[1] + A( k.phase[1] ) ) ) *
-               sin( tp * ( P[2] + A( k.phase[2] ) ) ) );
+   {
+      if ( radius < A( 0 ) ) radius = sqrt( P[0] * P[0] + P[1] * P[1] + P[2] * P[2] );
+      return exp( A( k.amp / k.freq ) * ( A( k.value ) - radius ) );
+   }
+   const A tf = A( 2.0 * k.freq );
+   return exp( A( k.amp ) * sin_pi( tf * ( P[0] + A( k.phase[0] ) ) ) * cos_pi( tf * ( P[1] + A( k.phase[1] ) ) ) *
+               sin_pi( tf * ( P[2] + A( k.phase[2] ) ) ) );
 }
 
 // IcosahedralShellMap: F(x) = x r(x)/|x|, r(x) = r_ray + lambda(x) (r_ref - r_ray) with lambda the
@@ -286,6 +297,10 @@ __constant__ int c_mc_off[6][4][3] = {
     { { 0, 0, 0 }, { 1, 0, 0 }, { 0, 1, 0 }, { 0, 0, 1 } }, { { 1, 0, 0 }, { 1, 1, 0 }, { 0, 1, 0 }, { 1, 0, 1 } },
     { { 1, 0, 0 }, { 0, 1, 0 }, { 1, 0, 1 }, { 0, 0, 1 } }, { { 1, 1, 0 }, { 1, 1, 1 }, { 0, 1, 1 }, { 1, 0, 1 } },
     { { 1, 0, 1 }, { 0, 1, 1 }, { 0, 0, 1 }, { 0, 1, 0 } }, { { 0, 1, 0 }, { 1, 1, 0 }, { 1, 0, 1 }, { 0, 1, 1 } } };
+static const int kMicroOff[6][4][3] = {
+    { { 0, 0, 0 }, { 1, 0, 0 }, { 0, 1, 0 }, { 0, 0, 1 } }, { { 1, 0, 0 }, { 1, 1, 0 }, { 0, 1, 0 }, { 1, 0, 1 } },
+    { { 1, 0, 0 }, { 0, 1, 0 }, { 1, 0, 1 }, { 0, 0, 1 } }, { { 1, 1, 0 }, { 1, 1, 1 }, { 0, 1, 1 }, { 1, 0, 1 } },
+    { { 1, 0, 1 }, { 0, 1, 1 }, { 0, 0, 1 }, { 0, 1, 0 } }, { { 0, 1, 0 }, { 1, 1, 0 }, { 1, 0, 1 }, { 0, 1, 1 } } };
 __constant__ int c_mc_shift[6] = { 0, 1, 1, 2, 1, 1 };
 // stencil direction (index into kVarDirs) from vertex i to vertex j of micro-cell type ty
 __constant__ int8_t c_mc_dir[6][4][4];
@@ -392,7 +407,9 @@ __global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const in
 // generated with; its weights are derived here from exactness for all polynomials of degree <= 4.
 // ---------------------------------------------------------------------------------------------
 __constant__ double c_xg4_pts[11][3];
+__constant__ double c_xg4_bary[11][4];
 __constant__ double c_xg4_w[11];
+__constant__ int8_t c_p2_loc[6][10];  // node of micro-cell type ty in its anchor's 3x3x3 nodes: a + 3 b + 9 c
 __constant__ double c_p2_rgrad[11][10][3];  // reference gradients of the ten basis functions per point
 __constant__ double c_p2_phi[11][10];       // values of the ten basis functions per point
 __constant__ int    c_p2_edge[6][2] = { { 2, 3 }, { 1, 3 }, { 1, 2 }, { 0, 3 }, { 0, 2 }, { 0, 1 } };
@@ -497,6 +514,22 @@ void ensure_p2_constants()
                g[q][4 + e][d] = 4.0 * ( lam[ed[e][0]] * lg[ed[e][1]][d] + lam[ed[e][1]] * lg[ed[e][0]][d] );
       }
       check_cuda( cudaMemcpyToSymbol( c_xg4_pts, pts, sizeof( pts ) ), "P2 constants (points)" );
+      double bary[11][4];
+      for ( int q = 0; q < 11; ++q )
+      {
+         bary[q][0] = 1.0 - pts[q][0] - pts[q][1] - pts[q][2];
+         for ( int d = 0; d < 3; ++d ) bary[q][d + 1] = pts[q][d];
+      }
+      check_cuda( cudaMemcpyToSymbol( c_xg4_bary, bary, sizeof( bary ) ), "P2 constants (barycentric points)" );
+      int8_t loc[6][10];
+      for ( int ty = 0; ty < 6; ++ty )
+         for ( int i = 0; i < 10; ++i )
+         {
+            const int* va = kMicroOff[ty][i < 4 ? i : ed[i - 4][0]];
+            const int* vb = kMicroOff[ty][i < 4 ? i : ed[i - 4][1]];
+            loc[ty][i]    = int8_t( ( va[0] + vb[0] ) + 3 * ( va[1] + vb[1] ) + 9 * ( va[2] + vb[2] ) );
+         }
+      check_cuda( cudaMemcpyToSymbol( c_p2_loc, loc, sizeof( loc ) ), "P2 constants (local nodes)" );
       check_cuda( cudaMemcpyToSymbol( c_xg4_w, w, sizeof( w ) ), "P2 constants (weights)" );
       check_cuda( cudaMemcpyToSymbol( c_p2_rgrad, g, sizeof( g ) ), "P2 constants (gradients)" );
       double phi[11][10];
@@ -511,6 +544,271 @@ void ensure_p2_constants()
       p2_wrap_table( wrap );
       check_cuda( cudaMemcpyToSymbol( c_p2_wrap, wrap, sizeof( wrap ) ), "P2 constants (stored order)" );
    } );
+}
+
+// ---------------------------------------------------------------------------------------------
+// Matrix-free P2 passes: what a quadrature point needs
+//
+// On a micro-cell J is constant, so only the blending map's DF varies between points.  For the shell
+// DF = s I + X g^T (s = R / |X|, g the gradient of s), a rank-one update, so
+//    det DF = s^2 m,  DF^-1 = (I - X g^T / m) / s,  DF^-T = (I - g X^T / m) / s,  m = s + g . X,
+// and m = (gradient of R . X) / |X| without cancellation.  Gradients of quadratic functions are affine,
+// so they are interpolated from the four vertices: grad u at vertex k is a combination of ten node
+// values with integer weights, and sum_q of the pairing with every basis gradient needs only
+// H_k = sum_q lambda_k(q) h(q) at the four vertices.  Per point this takes about 100 operations and the
+// coefficient, against 300 for the 3x3 inverse and two loops over ten reference gradients.
+// ---------------------------------------------------------------------------------------------
+template < typename A >
+struct ShellCell {
+   A bx[3];   // gradient of the barycentric weight t of the cell's ref vertex (up to its offset)
+   A t0;      // t at the ray vertex
+   A rad, dr; // R = rad + |t - t0| dr
+};
+
+template < typename A >
+__device__ __forceinline__ ShellCell< A > shell_cell( const CellGeom& g )
+{
+   ShellCell< A > c;
+   const double   iv = g.blend == 1 ? 1.0 / g.volT : 0.0;
+   for ( int d = 0; d < 3; ++d ) c.bx[d] = A( g.bxc[d] * iv );
+   c.t0  = A( ( g.ray[0] * g.bxc[0] + g.ray[1] * g.bxc[1] + g.ray[2] * g.bxc[2] ) * iv );
+   c.rad = A( g.rad_ray );
+   c.dr  = A( g.rad_ref - g.rad_ray );
+   return c;
+}
+
+template < typename A >
+struct ShellPoint {
+   A X[3], g[3];
+   A s, m, im, R;
+};
+
+__device__ __forceinline__ double rsqrt_of( double v ) { return rsqrt( v ); }
+__device__ __forceinline__ float  rsqrt_of( float v ) { return rsqrtf( v ); }
+
+// p.X is set by the caller
+template < typename A >
+__device__ __forceinline__ void shell_point( const ShellCell< A >& c, ShellPoint< A >& p )
+{
+   const A t   = p.X[0] * c.bx[0] + p.X[1] * c.bx[1] + p.X[2] * c.bx[2];
+   const A lam = t - c.t0;
+   p.R         = c.rad + fabs( lam ) * c.dr;
+   const A d   = lam < A( 0 ) ? -c.dr : c.dr;
+   const A ir  = rsqrt_of( p.X[0] * p.X[0] + p.X[1] * p.X[1] + p.X[2] * p.X[2] );
+   p.s         = p.R * ir;
+   const A e   = ir * d, f = p.s * ir * ir;
+   for ( int k = 0; k < 3; ++k ) p.g[k] = e * c.bx[k] - f * p.X[k];
+   p.m  = e * t;
+   p.im = A( 1 ) / p.m;
+}
+
+// one micro-cell of an anchor: first vertex, columns of J, J^-1 and |det J| (st: computational steps)
+template < typename A >
+struct MicroCell {
+   A X0[3], J[3][3], Ji[3][3], adet;
+};
+
+template < typename A >
+__device__ __forceinline__ void micro_cell( const CellGeom& g, const A st[3][3], int ty, int x, int y, int z, MicroCell< A >& c )
+{
+   const A v0[3] = { A( x + c_mc_off[ty][0][0] ), A( y + c_mc_off[ty][0][1] ), A( z + c_mc_off[ty][0][2] ) };
+   for ( int d = 0; d < 3; ++d )
+   {
+      c.X0[d] = A( g.P[0][d] ) + st[0][d] * v0[0] + st[1][d] * v0[1] + st[2][d] * v0[2];
+      for ( int k = 0; k < 3; ++k )
+         c.J[d][k] = st[0][d] * A( c_mc_off[ty][k + 1][0] - c_mc_off[ty][0][0] ) + st[1][d] * A( c_mc_off[ty][k + 1][1] - c_mc_off[ty][0][1] ) +
+                     st[2][d] * A( c_mc_off[ty][k + 1][2] - c_mc_off[ty][0][2] );
+   }
+   const A( &J )[3][3] = c.J;
+   const A c0 = J[1][1] * J[2][2] - J[1][2] * J[2][1], c1 = J[1][2] * J[2][0] - J[1][0] * J[2][2], c2 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+   const A det = J[0][0] * c0 + J[0][1] * c1 + J[0][2] * c2, id = A( 1 ) / det;
+   c.Ji[0][0] = c0 * id;
+   c.Ji[1][0] = c1 * id;
+   c.Ji[2][0] = c2 * id;
+   c.Ji[0][1] = ( J[0][2] * J[2][1] - J[0][1] * J[2][2] ) * id;
+   c.Ji[1][1] = ( J[0][0] * J[2][2] - J[0][2] * J[2][0] ) * id;
+   c.Ji[2][1] = ( J[0][1] * J[2][0] - J[0][0] * J[2][1] ) * id;
+   c.Ji[0][2] = ( J[0][1] * J[1][2] - J[0][2] * J[1][1] ) * id;
+   c.Ji[1][2] = ( J[0][2] * J[1][0] - J[0][0] * J[1][2] ) * id;
+   c.Ji[2][2] = ( J[0][0] * J[1][1] - J[0][1] * J[1][0] ) * id;
+   c.adet     = fabs( det );
+}
+
+// gradients of the quadratic function with node values u at the four vertices, with respect to X
+template < typename A >
+__device__ __forceinline__ void p2_vertex_gradients( const A u[10], const A Ji[3][3], A G[4][3] )
+{
+   // c[k][l]: coefficient of grad lambda_l at vertex k
+   const A c[4][4] = { { 3 * u[0], 4 * u[9] - u[1], 4 * u[8] - u[2], 4 * u[7] - u[3] },
+                       { 4 * u[9] - u[0], 3 * u[1], 4 * u[6] - u[2], 4 * u[5] - u[3] },
+                       { 4 * u[8] - u[0], 4 * u[6] - u[1], 3 * u[2], 4 * u[4] - u[3] },
+                       { 4 * u[7] - u[0], 4 * u[5] - u[1], 4 * u[4] - u[2], 3 * u[3] } };
+#pragma unroll
+   for ( int k = 0; k < 4; ++k )
+   {
+      const A r0 = c[k][1] - c[k][0], r1 = c[k][2] - c[k][0], r2 = c[k][3] - c[k][0];
+#pragma unroll
+      for ( int d = 0; d < 3; ++d ) G[k][d] = r0 * Ji[0][d] + r1 * Ji[1][d] + r2 * Ji[2][d];
+   }
+}
+
+// the transpose: y[i] = sum_k (gradient of basis function i at vertex k) . H[k]
+template < typename A >
+__device__ __forceinline__ void p2_pair_gradients( const A H[4][3], const A Ji[3][3], A y[10] )
+{
+   A h[4][4];
+#pragma unroll
+   for ( int k = 0; k < 4; ++k )
+   {
+#pragma unroll
+      for ( int d = 0; d < 3; ++d ) h[k][d + 1] = Ji[d][0] * H[k][0] + Ji[d][1] * H[k][1] + Ji[d][2] * H[k][2];
+      h[k][0] = -( h[k][1] + h[k][2] + h[k][3] );
+   }
+#pragma unroll
+   for ( int i = 0; i < 4; ++i ) y[i] = 4 * h[i][i] - ( ( h[0][i] + h[1][i] ) + ( h[2][i] + h[3][i] ) );
+   y[4] = 4 * ( h[2][3] + h[3][2] );
+   y[5] = 4 * ( h[1][3] + h[3][1] );
+   y[6] = 4 * ( h[1][2] + h[2][1] );
+   y[7] = 4 * ( h[0][3] + h[3][0] );
+   y[8] = 4 * ( h[0][2] + h[2][0] );
+   y[9] = 4 * ( h[0][1] + h[1][0] );
+}
+
+// y += K x of one parity pass, matrix-free (anchors of one parity share no node, see k_p2_pass).  Bound
+// by FP64 arithmetic: three quarters of it the coefficient and the map.  A thread takes one anchor and
+// keeps the 27 nodes its six micro-cells touch in shared memory (values in, sums out), so that global
+// memory sees each of them once per pass, all loads in flight together, instead of ten
+// read-modify-writes per micro-cell in a chain.  Shell of 1920 macro-cells, level 4 (7.9 M micro-cells),
+// exp/sin coefficient: 6.22 ms per apply with the 3x3 inverse per point and chained updates, 3.34 ms so;
+// three, four or five blocks per SM take the same time.
+constexpr int kP2ApplyThreads = 96;  // 41 KB of node values and sums per block, five blocks per SM
+template < typename T, typename A, bool NODAL >
+__global__ void __launch_bounds__( kP2ApplyThreads, 5 )
+    k_p2_apply_pass( int ne, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
+                     const CellGeom* __restrict__ geom, Coefficient kc, const T* __restrict__ src, A* __restrict__ acc,
+                     int64_t level_size, int* err, const double* __restrict__ kn )
+{
+   extern __shared__ __align__( 16 ) unsigned char p2_raw[];
+   A* const  xs = reinterpret_cast< A* >( p2_raw ) + threadIdx.x;  // node i of this thread: xs[i * bd], ys[i * bd]
+   const int bd = blockDim.x;
+   A* const  ys = xs + 27 * bd;
+   const int t  = blockIdx.x * bd + threadIdx.x;
+   const int c  = blockIdx.y;
+   if ( t >= nanch ) return;
+   const int       a = anch[t];
+   const int       x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
+   const CellGeom& g    = geom[c];
+   const int64_t   base = cell_off[c];
+   // nodes past the cell's slanted face do not exist; the level check guards the anchor tables
+   const int room = ns - 2 * ( x + y + z );
+   {
+      const int64_t last = base + cidx( ns, 2 * x, 2 * y, 2 * z + min( room, 2 ) );
+      if ( room < 2 || base < 0 || last >= level_size )
+      {
+         atomicExch( err, 2 );
+         return;
+      }
+   }
+#pragma unroll
+   for ( int r = 0; r < 9; ++r )
+   {
+      const int     b = r % 3, cc = r / 3;
+      const int64_t row = base + cidx( ns, 2 * x, 2 * y + b, 2 * z + cc );
+#pragma unroll
+      for ( int k = 0; k < 3; ++k )
+      {
+         xs[( 3 * r + k ) * bd] = k + b + cc <= room ? A( ld_any( src + row + k ) ) : A( 0 );
+         ys[( 3 * r + k ) * bd] = A( 0 );
+      }
+   }
+   const bool           blend = g.blend == 1;
+   const ShellCell< A > sc    = shell_cell< A >( g );
+   const A              inv_n = A( 1.0 / double( ne ) );
+   A                    st[3][3];
+   for ( int k = 0; k < 3; ++k )
+      for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
+#pragma unroll 1
+   for ( int ty = 0; ty < 6; ++ty )
+   {
+      if ( x + y + z > ne - 1 - c_mc_shift[ty] ) continue;
+      MicroCell< A > mc;
+      micro_cell( g, st, ty, x, y, z, mc );
+      A kl[NODAL ? 10 : 1];
+      A G[4][3], H[4][3];
+      {
+         A u[10];
+#pragma unroll
+         for ( int i = 0; i < 10; ++i )
+         {
+            const int l = c_p2_loc[ty][i];
+            u[i]        = xs[l * bd];
+            if constexpr ( NODAL ) kl[i] = A( kn[base + cidx( ns, 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9 )] );
+         }
+         p2_vertex_gradients( u, mc.Ji, G );
+      }
+#pragma unroll
+      for ( int k = 0; k < 4; ++k ) H[k][0] = H[k][1] = H[k][2] = A( 0 );
+#pragma unroll 1
+      for ( int q = 0; q < 11; ++q )
+      {
+         const A l0 = A( c_xg4_bary[q][0] ), l1 = A( c_xg4_bary[q][1] ), l2 = A( c_xg4_bary[q][2] ), l3 = A( c_xg4_bary[q][3] );
+         A       B[3];
+#pragma unroll
+         for ( int d = 0; d < 3; ++d ) B[d] = l0 * G[0][d] + l1 * G[1][d] + l2 * G[2][d] + l3 * G[3][d];
+         ShellPoint< A > p;
+#pragma unroll
+         for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * l1 + mc.J[d][1] * l2 + mc.J[d][2] * l3;
+         A f = A( c_xg4_w[q] ) * mc.adet, F[3] = { p.X[0], p.X[1], p.X[2] }, rad = A( -1 );
+         if ( blend )
+         {
+            // |det DF| DF^-1 DF^-T B = |m| (w - X (g . w) / m),  w = B - g (X . B) / m
+            shell_point( sc, p );
+            const A xb = ( p.X[0] * B[0] + p.X[1] * B[1] + p.X[2] * B[2] ) * p.im;
+#pragma unroll
+            for ( int d = 0; d < 3; ++d ) B[d] -= p.g[d] * xb;
+            const A gw = ( p.g[0] * B[0] + p.g[1] * B[1] + p.g[2] * B[2] ) * p.im;
+#pragma unroll
+            for ( int d = 0; d < 3; ++d )
+            {
+               B[d] -= p.X[d] * gw;
+               F[d] = p.X[d] * p.s;
+            }
+            f *= fabs( p.m );
+            rad = p.R;
+         }
+         if constexpr ( NODAL )
+         {
+            A kq = A( 0 );
+#pragma unroll
+            for ( int i = 0; i < 10; ++i ) kq += A( c_p2_phi[q][i] ) * kl[i];
+            f *= kq;
+         }
+         else
+            f *= coeff_eval( kc, F, rad );
+#pragma unroll
+         for ( int d = 0; d < 3; ++d )
+         {
+            const A h = f * B[d];
+            H[0][d] += l0 * h;
+            H[1][d] += l1 * h;
+            H[2][d] += l2 * h;
+            H[3][d] += l3 * h;
+         }
+      }
+      A yl[10];
+      p2_pair_gradients( H, mc.Ji, yl );
+#pragma unroll
+      for ( int i = 0; i < 10; ++i ) ys[c_p2_loc[ty][i] * bd] += yl[i];
+   }
+#pragma unroll
+   for ( int r = 0; r < 9; ++r )
+   {
+      const int     b = r % 3, cc = r / 3;
+      const int64_t row = base + cidx( ns, 2 * x, 2 * y + b, 2 * z + cc );
+#pragma unroll
+      for ( int k = 0; k < 3; ++k )
+         if ( k + b + cc <= room ) acc[row + k] += ys[( 3 * r + k ) * bd];
+   }
 }
 
 // mapped quantities of quadrature point q of a micro-cell: Mi = (DF J)^-1 and s = w k |det(DF J)|
@@ -659,18 +957,7 @@ __global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int nanch, const 
             {
                A Mi[3][3], s;
                p2_point( g, kc, X0, J, q, Mi, s, kn ? kl : static_cast< const A* >( nullptr ) );
-               if constexpr ( MODE == 0 )
-               {
-                  A gs[3] = { A( 0 ), A( 0 ), A( 0 ) };
-                  for ( int j = 0; j < 10; ++j )
-                     for ( int d = 0; d < 3; ++d ) gs[d] += xl[j] * A( c_p2_rgrad[q][j][d] );
-                  A gp[3], h[3];
-                  for ( int d = 0; d < 3; ++d ) gp[d] = gs[0] * Mi[0][d] + gs[1] * Mi[1][d] + gs[2] * Mi[2][d];
-                  for ( int r2 = 0; r2 < 3; ++r2 ) h[r2] = s * ( Mi[r2][0] * gp[0] + Mi[r2][1] * gp[1] + Mi[r2][2] * gp[2] );
-                  for ( int i = 0; i < 10; ++i )
-                     yl[i] += A( c_p2_rgrad[q][i][0] ) * h[0] + A( c_p2_rgrad[q][i][1] ) * h[1] + A( c_p2_rgrad[q][i][2] ) * h[2];
-               }
-               else if constexpr ( MODE == 1 )
+               if constexpr ( MODE == 1 )
                   for ( int i = 0; i < 10; ++i )
                   {
                      A G[3];
@@ -1095,29 +1382,16 @@ __global__ void __launch_bounds__( 256 ) k_p2_stored_pass( int ne, int nanch, co
 // the micro-cell's vertices on level l, the P2 nodes the ten nodes on storage level l+1; anchors of
 // one parity class share neither, so the passes are race-free.
 // ---------------------------------------------------------------------------------------------
-__constant__ double c_q2_pts[4][3];
-__constant__ double c_q2_rgrad[4][10][3];
+__constant__ double c_q2_bary[4][4];
 
 void ensure_stokes_constants()
 {
    static PerDeviceOnce once;
    once.run( [] {
       const double a = ( 5.0 - std::sqrt( 5.0 ) ) / 20.0, b = ( 5.0 + 3.0 * std::sqrt( 5.0 ) ) / 20.0;
-      const double pts[4][3] = { { a, a, a }, { b, a, a }, { a, b, a }, { a, a, b } };
-      const double lg[4][3]  = { { -1, -1, -1 }, { 1, 0, 0 }, { 0, 1, 0 }, { 0, 0, 1 } };
-      const int    ed[6][2]  = { { 2, 3 }, { 1, 3 }, { 1, 2 }, { 0, 3 }, { 0, 2 }, { 0, 1 } };
-      double       g[4][10][3];
-      for ( int q = 0; q < 4; ++q )
-      {
-         const double lam[4] = { 1.0 - pts[q][0] - pts[q][1] - pts[q][2], pts[q][0], pts[q][1], pts[q][2] };
-         for ( int i = 0; i < 4; ++i )
-            for ( int d = 0; d < 3; ++d ) g[q][i][d] = ( 4.0 * lam[i] - 1.0 ) * lg[i][d];
-         for ( int e = 0; e < 6; ++e )
-            for ( int d = 0; d < 3; ++d )
-               g[q][4 + e][d] = 4.0 * ( lam[ed[e][0]] * lg[ed[e][1]][d] + lam[ed[e][1]] * lg[ed[e][0]][d] );
-      }
-      check_cuda( cudaMemcpyToSymbol( c_q2_pts, pts, sizeof( pts ) ), "Stokes constants (points)" );
-      check_cuda( cudaMemcpyToSymbol( c_q2_rgrad, g, sizeof( g ) ), "Stokes constants (gradients)" );
+      const double c = 1.0 - 3.0 * a, e = 1.0 - 2.0 * a - b;
+      const double bary[4][4] = { { c, a, a, a }, { e, b, a, a }, { e, a, b, a }, { e, a, a, b } };
+      check_cuda( cudaMemcpyToSymbol( c_q2_bary, bary, sizeof( bary ) ), "Stokes constants (points)" );
    } );
 }
 
@@ -1165,7 +1439,7 @@ __device__ __forceinline__ void mapped_point( const CellGeom& g, const A X0[3], 
 
 // DIVT 0: p_acc[vertex i] += sum_k sum_j B_k[i][j] u_k[j];  DIVT 1: u_acc_k[node j] += sum_i B_k[i][j] p[i]
 template < typename T, typename A, int DIVT >
-__global__ void __launch_bounds__( 256 ) k_stokes_div_pass( int ne, int nanch, const int* __restrict__ anch,
+__global__ void __launch_bounds__( 128 ) k_stokes_div_pass( int ne, int nanch, const int* __restrict__ anch,
                                                              const int64_t* __restrict__ off_p, const int64_t* __restrict__ off_u,
                                                              const CellGeom* __restrict__ geom, const T* __restrict__ u0,
                                                              const T* __restrict__ u1, const T* __restrict__ u2,
@@ -1177,7 +1451,9 @@ __global__ void __launch_bounds__( 256 ) k_stokes_div_pass( int ne, int nanch, c
    if ( t >= nanch ) return;
    const int      a = anch[t];
    const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
-   const CellGeom g = geom[c];
+   const CellGeom& g = geom[c];
+   const bool           blend = g.blend == 1;
+   const ShellCell< A > sc    = shell_cell< A >( g );
    const int64_t  bp = off_p[c], bu = off_u[c];
    const A        inv_n = A( 1.0 / double( ne ) );
    A              st[3][3];
@@ -1210,64 +1486,100 @@ __global__ void __launch_bounds__( 256 ) k_stokes_div_pass( int ne, int nanch, c
             continue;
          }
       }
-      A X0[3], J[3][3];
-      for ( int d = 0; d < 3; ++d )
-      {
-         X0[d] = A( g.P[0][d] ) + st[0][d] * A( V[0][0] ) + st[1][d] * A( V[0][1] ) + st[2][d] * A( V[0][2] );
-         for ( int k = 0; k < 3; ++k )
-            J[d][k] = st[0][d] * A( V[k + 1][0] - V[0][0] ) + st[1][d] * A( V[k + 1][1] - V[0][1] ) + st[2][d] * A( V[k + 1][2] - V[0][2] );
-      }
+      MicroCell< A > mc;
+      micro_cell( g, st, ty, x, y, z, mc );
+      const A wj = -A( 1.0 / 24.0 ) * mc.adet;
       if constexpr ( DIVT == 0 )
       {
-         A ul[3][10];
-         for ( int j = 0; j < 10; ++j )
+         A G[3][4][3];
+#pragma unroll
+         for ( int k = 0; k < 3; ++k )
          {
-            ul[0][j] = A( ld_any( u0 + iu[j] ) );
-            ul[1][j] = A( ld_any( u1 + iu[j] ) );
-            ul[2][j] = A( ld_any( u2 + iu[j] ) );
+            const T* u = k == 0 ? u0 : k == 1 ? u1 : u2;
+            A        ul[10];
+#pragma unroll
+            for ( int j = 0; j < 10; ++j ) ul[j] = A( ld_any( u + iu[j] ) );
+            p2_vertex_gradients( ul, mc.Ji, G[k] );
          }
          A yl[4] = { A( 0 ), A( 0 ), A( 0 ), A( 0 ) };
+#pragma unroll 1
          for ( int q = 0; q < 4; ++q )
          {
-            A Mi[3][3], adet;
-            mapped_point( g, X0, J, c_q2_pts[q], Mi, adet );
-            // divergence of the local velocity: sum_k sum_j u_k[j] (grad_ref phi_j . Mi)_k
-            A dv = A( 0 );
-            for ( int j = 0; j < 10; ++j )
-               for ( int k = 0; k < 3; ++k )
-                  dv += ul[k][j] * ( A( c_q2_rgrad[q][j][0] ) * Mi[0][k] + A( c_q2_rgrad[q][j][1] ) * Mi[1][k] +
-                                     A( c_q2_rgrad[q][j][2] ) * Mi[2][k] );
-            const A f      = -A( 1.0 / 24.0 ) * adet * dv;
-            const A lam[4] = { A( 1.0 - c_q2_pts[q][0] - c_q2_pts[q][1] - c_q2_pts[q][2] ), A( c_q2_pts[q][0] ), A( c_q2_pts[q][1] ),
-                               A( c_q2_pts[q][2] ) };
+            const A lam[4] = { A( c_q2_bary[q][0] ), A( c_q2_bary[q][1] ), A( c_q2_bary[q][2] ), A( c_q2_bary[q][3] ) };
+            // velocity gradient B with respect to X; div = (tr B - g^T B X / m) / s and |det DF| = s^2 |m|
+            A B[3][3];
+#pragma unroll
+            for ( int k = 0; k < 3; ++k )
+#pragma unroll
+               for ( int d = 0; d < 3; ++d )
+                  B[k][d] = lam[0] * G[k][0][d] + lam[1] * G[k][1][d] + lam[2] * G[k][2][d] + lam[3] * G[k][3][d];
+            A f = B[0][0] + B[1][1] + B[2][2];
+            if ( blend )
+            {
+               ShellPoint< A > p;
+#pragma unroll
+               for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * lam[1] + mc.J[d][1] * lam[2] + mc.J[d][2] * lam[3];
+               shell_point( sc, p );
+               A gbx = A( 0 );
+#pragma unroll
+               for ( int k = 0; k < 3; ++k ) gbx += p.g[k] * ( B[k][0] * p.X[0] + B[k][1] * p.X[1] + B[k][2] * p.X[2] );
+               f = ( f - gbx * p.im ) * ( p.s * fabs( p.m ) );
+            }
+            f *= wj;
+#pragma unroll
             for ( int i = 0; i < 4; ++i ) yl[i] += f * lam[i];
          }
-         for ( int i = 0; i < 4; ++i ) accp[ip[i]] += yl[i];
+         for ( int i = 0; i < 4; ++i ) atomicAdd( accp + ip[i], yl[i] );
       }
       else
       {
          A pl[4];
          for ( int i = 0; i < 4; ++i ) pl[i] = A( ld_any( p + ip[i] ) );
-         A yl[3][10];
+         A H[3][4][3];
+#pragma unroll
          for ( int k = 0; k < 3; ++k )
-            for ( int j = 0; j < 10; ++j ) yl[k][j] = A( 0 );
+#pragma unroll
+            for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = A( 0 );
+#pragma unroll 1
          for ( int q = 0; q < 4; ++q )
          {
-            A Mi[3][3], adet;
-            mapped_point( g, X0, J, c_q2_pts[q], Mi, adet );
-            const A pq = pl[0] * A( 1.0 - c_q2_pts[q][0] - c_q2_pts[q][1] - c_q2_pts[q][2] ) + pl[1] * A( c_q2_pts[q][0] ) +
-                         pl[2] * A( c_q2_pts[q][1] ) + pl[3] * A( c_q2_pts[q][2] );
-            const A f = -A( 1.0 / 24.0 ) * adet * pq;
-            for ( int j = 0; j < 10; ++j )
+            const A lam[4] = { A( c_q2_bary[q][0] ), A( c_q2_bary[q][1] ), A( c_q2_bary[q][2] ), A( c_q2_bary[q][3] ) };
+            A       f      = wj * ( pl[0] * lam[0] + pl[1] * lam[1] + pl[2] * lam[2] + pl[3] * lam[3] );
+            // component k pairs with DF^-1 e_k |det DF| = s |m| (e_k - X g_k / m)
+            A E[3][3] = { { A( 1 ), A( 0 ), A( 0 ) }, { A( 0 ), A( 1 ), A( 0 ) }, { A( 0 ), A( 0 ), A( 1 ) } };
+            if ( blend )
+            {
+               ShellPoint< A > p;
+#pragma unroll
+               for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * lam[1] + mc.J[d][1] * lam[2] + mc.J[d][2] * lam[3];
+               shell_point( sc, p );
+#pragma unroll
                for ( int k = 0; k < 3; ++k )
-                  yl[k][j] += f * ( A( c_q2_rgrad[q][j][0] ) * Mi[0][k] + A( c_q2_rgrad[q][j][1] ) * Mi[1][k] +
-                                    A( c_q2_rgrad[q][j][2] ) * Mi[2][k] );
+               {
+                  const A gk = p.g[k] * p.im;
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d ) E[k][d] -= p.X[d] * gk;
+               }
+               f *= p.s * fabs( p.m );
+            }
+#pragma unroll
+            for ( int v = 0; v < 4; ++v )
+            {
+               const A fl = f * lam[v];
+#pragma unroll
+               for ( int k = 0; k < 3; ++k )
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d ) H[k][v][d] += fl * E[k][d];
+            }
          }
-         for ( int j = 0; j < 10; ++j )
+#pragma unroll
+         for ( int k = 0; k < 3; ++k )
          {
-            acc0[iu[j]] += yl[0][j];
-            acc1[iu[j]] += yl[1][j];
-            acc2[iu[j]] += yl[2][j];
+            A  yl[10];
+            A* o = k == 0 ? acc0 : k == 1 ? acc1 : acc2;
+            p2_pair_gradients( H[k], mc.Ji, yl );
+#pragma unroll
+            for ( int j = 0; j < 10; ++j ) atomicAdd( o + iu[j], yl[j] );
          }
       }
    }
@@ -1299,10 +1611,7 @@ static void ensure_var_tables()
 {
    static PerDeviceOnce once;
    once.run( [] {
-      static const int off[6][4][3] = {
-          { { 0, 0, 0 }, { 1, 0, 0 }, { 0, 1, 0 }, { 0, 0, 1 } }, { { 1, 0, 0 }, { 1, 1, 0 }, { 0, 1, 0 }, { 1, 0, 1 } },
-          { { 1, 0, 0 }, { 0, 1, 0 }, { 1, 0, 1 }, { 0, 0, 1 } }, { { 1, 1, 0 }, { 1, 1, 1 }, { 0, 1, 1 }, { 1, 0, 1 } },
-          { { 1, 0, 1 }, { 0, 1, 1 }, { 0, 0, 1 }, { 0, 1, 0 } }, { { 0, 1, 0 }, { 1, 1, 0 }, { 1, 0, 1 }, { 0, 1, 1 } } };
+      const int( &off )[6][4][3] = kMicroOff;
       int8_t dir[6][4][4], vd[15][3];
       for ( int d = 0; d < 15; ++d )
          for ( int k = 0; k < 3; ++k ) vd[d][k] = int8_t( kVarDirs[d][k] );
@@ -1389,6 +1698,18 @@ static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src
          const dim3 g3( ( na + 3 * wb - 1 ) / ( 3 * wb ), nC );
          k_p2_stored_pass< T, A ><<< g3, 32 * wb, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB, src,
                                                                       acc, kst, ks, kbase, P.size, ctx->d_error );
+      }
+      else if ( op->order == 2 && MODE == 0 )
+      {
+         const int    pb   = pass_block( na, kP2ApplyThreads );
+         const dim3   pg( ( na + pb - 1 ) / pb, nC );
+         const size_t smem = size_t( 54 ) * pb * sizeof( A );
+         if ( op->nodal_k )
+            k_p2_apply_pass< T, A, true ><<< pg, pb, smem, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
+                                                                            op->d_geom, op->coeff, src, acc, P.size, ctx->d_error, e.d_kn );
+         else
+            k_p2_apply_pass< T, A, false ><<< pg, pb, smem, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
+                                                                             op->d_geom, op->coeff, src, acc, P.size, ctx->d_error, nullptr );
       }
       else if ( op->order == 2 )
          k_p2_pass< T, A, MODE ><<< grid, bs, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
@@ -1669,7 +1990,7 @@ static void run_stokes( Context* ctx, Operator* op, int Lp, int divt, const void
    {
       const int na = e.aoff[pc + 1] - e.aoff[pc];
       if ( na <= 0 ) continue;
-      const int bs = pass_block( na, 256 );
+      const int bs = pass_block( na, 128 );
       dim3      grid( ( na + bs - 1 ) / bs, nC );
       const T* u0 = u ? (const T*) u[0] : nullptr;
       const T* u1 = u ? (const T*) u[1] : nullptr;
@@ -1711,7 +2032,8 @@ void launch_stokes_div( Context* ctx, Operator* op, int Lp, int dtype, int divt,
 // with mu evaluated at the blended point, Yu's 5-point degree-3 rule.  Applied matrix-free per
 // micro-cell: at each point the velocity gradient g (g_ik = d u_i / d x_k) of the ten local nodes
 // gives the stress s = w mu |det| (g + g^T - (2/3) tr(g) I), and node a of component i receives
-// grad phi_a . s_i.  The diagonal pass sums w mu |det| (|grad phi_a|^2 + (1/3) (d_i phi_a)^2).  Same
+// grad phi_a . s_i; gradients and pairings go through the four vertices as in k_p2_apply_pass, the
+// node sums leave as reductions as in k_stokes_div_pass.  The diagonal pass sums w mu |det| (|grad phi_a|^2 + (1/3) (d_i phi_a)^2).  Same
 // parity passes as the coupling blocks (anchors of one class share no P2 node).
 // ---------------------------------------------------------------------------------------------
 __constant__ double c_yu5_rgrad[5][10][3];
@@ -1752,7 +2074,9 @@ __global__ void __launch_bounds__( 128 ) k_visc_pass( int ne, int nanch, const i
    if ( t >= nanch ) return;
    const int      a  = anch[t];
    const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
-   const CellGeom g  = geom[c];
+   const CellGeom&      g     = geom[c];
+   const bool           blend = g.blend == 1;
+   const ShellCell< A > sc    = shell_cell< A >( g );
    const int64_t  bu = off_u[c];
    const A        inv_n = A( 1.0 / double( ne ) );
    A              st[3][3];
@@ -1780,55 +2104,95 @@ __global__ void __launch_bounds__( 128 ) k_visc_pass( int ne, int nanch, const i
             continue;
          }
       }
-      A X0[3], J[3][3];
-      for ( int d = 0; d < 3; ++d )
-      {
-         X0[d] = A( g.P[0][d] ) + st[0][d] * A( V[0][0] ) + st[1][d] * A( V[0][1] ) + st[2][d] * A( V[0][2] );
-         for ( int k = 0; k < 3; ++k )
-            J[d][k] = st[0][d] * A( V[k + 1][0] - V[0][0] ) + st[1][d] * A( V[k + 1][1] - V[0][1] ) + st[2][d] * A( V[k + 1][2] - V[0][2] );
-      }
-      A ul[3][10];
+      MicroCell< A > mc;
+      micro_cell( g, st, ty, x, y, z, mc );
       if constexpr ( MODE == 0 )
-         for ( int j = 0; j < 10; ++j )
-         {
-            ul[0][j] = A( ld_any( u0 + iu[j] ) );
-            ul[1][j] = A( ld_any( u1 + iu[j] ) );
-            ul[2][j] = A( ld_any( u2 + iu[j] ) );
-         }
-      A yl[3][10];
-      for ( int k = 0; k < 3; ++k )
-         for ( int j = 0; j < 10; ++j ) yl[k][j] = A( 0 );
-      for ( int q = 0; q < 5; ++q )
       {
-         A Mi[3][3], adet, Fq[3];
-         mapped_point( g, X0, J, c_yu5_pts[q], Mi, adet, Fq );
-         const A s = A( c_yu5_w[q] ) * coeff_eval( kc, Fq ) * adet;
-         if constexpr ( MODE == 0 )
+         A G[3][4][3], H[3][4][3];
+#pragma unroll
+         for ( int k = 0; k < 3; ++k )
          {
-            A gr[3][3];
-            for ( int i = 0; i < 3; ++i )
-               for ( int k = 0; k < 3; ++k ) gr[i][k] = A( 0 );
-            for ( int b = 0; b < 10; ++b )
+            const T* u = k == 0 ? u0 : k == 1 ? u1 : u2;
+            A        ul[10];
+#pragma unroll
+            for ( int j = 0; j < 10; ++j ) ul[j] = A( ld_any( u + iu[j] ) );
+            p2_vertex_gradients( ul, mc.Ji, G[k] );
+#pragma unroll
+            for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = A( 0 );
+         }
+#pragma unroll 1
+         for ( int q = 0; q < 5; ++q )
+         {
+            const A l1 = A( c_yu5_pts[q][0] ), l2 = A( c_yu5_pts[q][1] ), l3 = A( c_yu5_pts[q][2] ), l0 = A( 1 ) - l1 - l2 - l3;
+            A       D[3][3];  // velocity gradient, d u_k / d x_d
+#pragma unroll
+            for ( int k = 0; k < 3; ++k )
+#pragma unroll
+               for ( int d = 0; d < 3; ++d ) D[k][d] = l0 * G[k][0][d] + l1 * G[k][1][d] + l2 * G[k][2][d] + l3 * G[k][3][d];
+            ShellPoint< A > p;
+#pragma unroll
+            for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * l1 + mc.J[d][1] * l2 + mc.J[d][2] * l3;
+            A f = A( c_yu5_w[q] ) * mc.adet, F[3] = { p.X[0], p.X[1], p.X[2] }, rad = A( -1 );
+            if ( blend )
             {
-               A G[3];
+               // |det DF| = s^2 |m| takes the two factors 1/s of DF^-T and DF^-1
+               shell_point( sc, p );
+#pragma unroll
                for ( int k = 0; k < 3; ++k )
-                  G[k] = A( c_yu5_rgrad[q][b][0] ) * Mi[0][k] + A( c_yu5_rgrad[q][b][1] ) * Mi[1][k] + A( c_yu5_rgrad[q][b][2] ) * Mi[2][k];
-               for ( int i = 0; i < 3; ++i )
-                  for ( int k = 0; k < 3; ++k ) gr[i][k] += ul[i][b] * G[k];
+               {
+                  const A xb = ( p.X[0] * D[k][0] + p.X[1] * D[k][1] + p.X[2] * D[k][2] ) * p.im;
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d ) D[k][d] -= p.g[d] * xb;
+                  F[k] = p.X[k] * p.s;
+               }
+               f *= fabs( p.m );
+               rad = p.R;
             }
-            const A tr3 = A( 2.0 / 3.0 ) * ( gr[0][0] + gr[1][1] + gr[2][2] );
-            A       sg[3][3];
-            for ( int i = 0; i < 3; ++i )
-               for ( int k = 0; k < 3; ++k ) sg[i][k] = s * ( ( gr[i][k] + gr[k][i] ) - ( i == k ? tr3 : A( 0 ) ) );
-            for ( int b = 0; b < 10; ++b )
+            f *= coeff_eval( kc, F, rad );
+            const A tr3     = A( 2.0 / 3.0 ) * ( D[0][0] + D[1][1] + D[2][2] );
+            A       S[3][3] = { { D[0][0] + D[0][0] - tr3, D[0][1] + D[1][0], D[0][2] + D[2][0] },
+                                { D[0][1] + D[1][0], D[1][1] + D[1][1] - tr3, D[1][2] + D[2][1] },
+                                { D[0][2] + D[2][0], D[1][2] + D[2][1], D[2][2] + D[2][2] - tr3 } };
+#pragma unroll
+            for ( int k = 0; k < 3; ++k )
             {
-               A G[3];
-               for ( int k = 0; k < 3; ++k )
-                  G[k] = A( c_yu5_rgrad[q][b][0] ) * Mi[0][k] + A( c_yu5_rgrad[q][b][1] ) * Mi[1][k] + A( c_yu5_rgrad[q][b][2] ) * Mi[2][k];
-               for ( int i = 0; i < 3; ++i ) yl[i][b] += G[0] * sg[i][0] + G[1] * sg[i][1] + G[2] * sg[i][2];
+               if ( blend )
+               {
+                  const A gs = ( p.g[0] * S[k][0] + p.g[1] * S[k][1] + p.g[2] * S[k][2] ) * p.im;
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d ) S[k][d] -= p.X[d] * gs;
+               }
+#pragma unroll
+               for ( int d = 0; d < 3; ++d )
+               {
+                  const A h = f * S[k][d];
+                  H[k][0][d] += l0 * h;
+                  H[k][1][d] += l1 * h;
+                  H[k][2][d] += l2 * h;
+                  H[k][3][d] += l3 * h;
+               }
             }
          }
-         else
+#pragma unroll
+         for ( int k = 0; k < 3; ++k )
+         {
+            A  yl[10];
+            A* o = k == 0 ? acc0 : k == 1 ? acc1 : acc2;
+            p2_pair_gradients( H[k], mc.Ji, yl );
+#pragma unroll
+            for ( int j = 0; j < 10; ++j ) atomicAdd( o + iu[j], yl[j] );
+         }
+      }
+      else
+      {
+         A yl[3][10];
+         for ( int k = 0; k < 3; ++k )
+            for ( int j = 0; j < 10; ++j ) yl[k][j] = A( 0 );
+         for ( int q = 0; q < 5; ++q )
+         {
+            A Mi[3][3], adet, Fq[3];
+            mapped_point( g, mc.X0, mc.J, c_yu5_pts[q], Mi, adet, Fq );
+            const A s = A( c_yu5_w[q] ) * coeff_eval( kc, Fq ) * adet;
             for ( int b = 0; b < 10; ++b )
             {
                A G[3];
@@ -1837,12 +2201,13 @@ __global__ void __launch_bounds__( 128 ) k_visc_pass( int ne, int nanch, const i
                const A gg = G[0] * G[0] + G[1] * G[1] + G[2] * G[2];
                for ( int i = 0; i < 3; ++i ) yl[i][b] += s * ( gg + A( 1.0 / 3.0 ) * G[i] * G[i] );
             }
-      }
-      for ( int j = 0; j < 10; ++j )
-      {
-         acc0[iu[j]] += yl[0][j];
-         acc1[iu[j]] += yl[1][j];
-         acc2[iu[j]] += yl[2][j];
+         }
+         for ( int j = 0; j < 10; ++j )
+         {
+            acc0[iu[j]] += yl[0][j];
+            acc1[iu[j]] += yl[1][j];
+            acc2[iu[j]] += yl[2][j];
+         }
       }
    }
 }

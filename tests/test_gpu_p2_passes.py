@@ -1,0 +1,58 @@
+"""Matrix-free P2 passes at the sizes where their blocks and node windows end: levels 0 and 1 (one anchor
+per parity class, windows cut by the slanted face), level 4 of one tetrahedron (more anchors per class than
+a block holds), every coefficient kind, with and without the shell map, against the oracle's element
+matrices.  FP64 within 1e-12 of the largest value, the tolerance of the other P2 tests; FP32 sums about
+300 rounded terms per node, so 300 eps = 4e-5 bounds it."""
+
+import numpy as np
+import pytest
+
+import hyteg_b200 as H
+from oracle import hyteg_oracle as O
+from tests import meshes as M
+from tests.test_gpu_p2 import _rand, _relerr
+
+pytestmark = pytest.mark.gpu
+
+SPECS = {"const": (1.75, lambda P: np.full(np.asarray(P).shape[:-1], 1.75)),
+         "expsin": (("expsin", 0.5, (0.13, 0.27, 0.41)), O.k_expsin(0.5, (0.13, 0.27, 0.41))),
+         "radial": (("radial", 2.99, 1.0, 0.45), O.k_radial())}
+
+
+@pytest.mark.parametrize("case,L", [("tet", 0), ("tet", 1), ("tet", 4), ("shell", 0), ("shell", 1)])
+@pytest.mark.parametrize("kind", sorted(SPECS))
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_p2_matrix_free_apply(ctx, case, L, kind, dtype):
+    coords, tets = M.tilted_tet() if case == "tet" else O.mesh_spherical_shell(2, 2, 0.55, 1.0)
+    bl = "shell" if case == "shell" else None
+    spec, kfun = SPECS[kind]
+    op = O.P2DivKGrad(O.MacroMesh(coords, tets), L, L, kfun, blending=bl)
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    A = H.P2ElementwiseBlendingDivKGradOperator(pm, L, L, ctx, k=spec, blending=bl)
+    lev = op.levels[L]
+    x = _rand(lev, 1)
+    if dtype == "float32":
+        x = x.astype(np.float32).astype(np.float64)
+    fx, fy = (H.P2Function(n, pm, L, L, ctx, dtype) for n in "xy")
+    fx.upload(L, x)
+    A.apply(fx, fy, L, O.ALL)
+    ref = op.apply(x, np.zeros_like(x), L, O.ALL)
+    assert _relerr(fy.download(L), ref, lev.owned_mask(O.ALL)) < (1e-12 if dtype == "float64" else 4e-5)
+
+
+@pytest.mark.parametrize("kind", sorted(SPECS))
+def test_full_viscous_apply_smallest_level(ctx, kind):
+    coords, tets = O.mesh_spherical_shell(2, 2, 0.55, 1.0)
+    spec, kfun = SPECS[kind]
+    op = O.P2FullViscous(O.MacroMesh(coords, tets), 0, 0, kfun, blending="shell")
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    A = H.P2ElementwiseBlendingFullViscousOperator(pm, 0, 0, ctx, viscosity=spec, blending="shell")
+    lev = op.levels[0]
+    u = [_rand(lev, 10 + k) for k in range(3)]
+    fu, fy = ([H.P2Function(n + str(k), pm, 0, 0, ctx) for k in range(3)] for n in "uy")
+    for k in range(3):
+        fu[k].upload(0, u[k])
+    A.apply(fu, fy, 0, O.ALL)
+    ref = op.apply(u, [np.zeros_like(v) for v in u], 0, O.ALL)
+    for k in range(3):
+        assert _relerr(fy[k].download(0), ref[k], lev.owned_mask(O.ALL)) < 1e-12
