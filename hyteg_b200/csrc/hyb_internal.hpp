@@ -265,19 +265,24 @@ struct CellGeom {
 // vertices and (blending 1) the IcosahedralShellMap classification of macro-cell c
 void cell_geometry( const Topology& t, int c, int blending, CellGeom& g );
 
+struct P2StoredView;
+
 struct ElemLevel {
    void* d_acc  = nullptr;  // accumulation buffer (level size, accumulation precision)
    int   acc_dtype = -1;
    void* d_invd[3] = { nullptr, nullptr, nullptr };  // inverse diagonal per DoF, per storage dtype
    int*  d_anch     = nullptr;                         // micro-cell anchors x | y << 10 | z << 20, by parity class
    int   aoff[9]    = {};                              // class p = px | py << 1 | pz << 2 spans aoff[p]..aoff[p+1]-1
-   // stored element matrices (computeAndStoreLocalElementMatrices): the 10 upper-triangle entries
-   // of every micro-cell's 4x4 matrix, value-major, in double ([0]) and float ([1])
-   void* d_K[2] = { nullptr, nullptr };
-   // P1 operators with stored matrices keep them assembled: the 15 stencil weights of every
-   // cell-array slot (the partial stencil of that cell at copies of face/edge/vertex DoFs),
-   // weight-major over the level's slots, in double ([0]) and float ([1])
-   void* d_S[2] = { nullptr, nullptr };
+   int   akind[8][3] = {};                             // its anchors with six, five and one micro-cells, in this order
+   // operators with stored matrices (computeAndStoreLocalElementMatrices) keep them assembled, in double
+   // ([0]) and float ([1]).  P1: the 15 stencil weights of every cell-array slot (the partial stencil of
+   // that cell at copies of face/edge/vertex DoFs), weight-major over the level's slots.  P2: the class
+   // stencils of p2_stored.cuh with their tables.
+   void*                           d_S[2] = { nullptr, nullptr };
+   std::shared_ptr< P2StoredView > p2s;
+   int64_t                         p2s_count = 0;
+   void*                           d_p2s_pts = nullptr;
+   int*                            d_p2s_rank = nullptr;
    void* d_sacc = nullptr;  // Stokes coupling blocks: three velocity accumulators and one pressure accumulator
    // P2 operators with a stored coefficient function: k at every cell-array node of this storage level
    double* d_kn = nullptr;
@@ -356,6 +361,10 @@ struct StencilArgs {
 };
 
 void launch_stencil( Context* ctx, Mesh* m, Operator* A, int L, int dtype, const StencilArgs& a );
+// the sweep of a P2 operator with stored matrices over all cell-array nodes: cell interiors get the
+// operation's epilogue, nodes on a macro-cell's boundary leave their partial sums in acc
+void launch_p2_stored_sweep( Context* ctx, P1Level& P, int dtype, const P2StoredView& v, const void* S, const void* invd, void* acc,
+                             const StencilArgs* a, int ncomp );
 void launch_elementwise( Context* ctx, Mesh* m, Operator* A, int L, int dtype, const StencilArgs& a );
 // per-copy dot products and packed transfers on meshes made of disjoint copies of one mesh
 // (p1_kernels.cu; the batched solves of the serving loop)

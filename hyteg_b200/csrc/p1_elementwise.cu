@@ -16,6 +16,7 @@
 // and vertex DoFs into their owners (the additive communication of the reference).  Deterministic:
 // the order of every sum is fixed.  The path is FP64-compute-bound.
 #include "hyb_internal.hpp"
+#include "p2_stored.cuh"
 
 #include <cmath>
 #include <stdexcept>
@@ -297,10 +298,6 @@ __constant__ int c_mc_off[6][4][3] = {
     { { 0, 0, 0 }, { 1, 0, 0 }, { 0, 1, 0 }, { 0, 0, 1 } }, { { 1, 0, 0 }, { 1, 1, 0 }, { 0, 1, 0 }, { 1, 0, 1 } },
     { { 1, 0, 0 }, { 0, 1, 0 }, { 1, 0, 1 }, { 0, 0, 1 } }, { { 1, 1, 0 }, { 1, 1, 1 }, { 0, 1, 1 }, { 1, 0, 1 } },
     { { 1, 0, 1 }, { 0, 1, 1 }, { 0, 0, 1 }, { 0, 1, 0 } }, { { 0, 1, 0 }, { 1, 1, 0 }, { 1, 0, 1 }, { 0, 1, 1 } } };
-static const int kMicroOff[6][4][3] = {
-    { { 0, 0, 0 }, { 1, 0, 0 }, { 0, 1, 0 }, { 0, 0, 1 } }, { { 1, 0, 0 }, { 1, 1, 0 }, { 0, 1, 0 }, { 1, 0, 1 } },
-    { { 1, 0, 0 }, { 0, 1, 0 }, { 1, 0, 1 }, { 0, 0, 1 } }, { { 1, 1, 0 }, { 1, 1, 1 }, { 0, 1, 1 }, { 1, 0, 1 } },
-    { { 1, 0, 1 }, { 0, 1, 1 }, { 0, 0, 1 }, { 0, 1, 0 } }, { { 0, 1, 0 }, { 1, 1, 0 }, { 1, 0, 1 }, { 0, 1, 1 } } };
 __constant__ int c_mc_shift[6] = { 0, 1, 1, 2, 1, 1 };
 // stencil direction (index into kVarDirs) from vertex i to vertex j of micro-cell type ty
 __constant__ int8_t c_mc_dir[6][4][4];
@@ -319,10 +316,8 @@ __device__ __forceinline__ void   st_any( __half* p, float v ) { *p = __float2ha
 
 // One parity pass: warp per half-grid row (y, z) of anchors with y = py mod 2, z = pz mod 2, lanes
 // over x = px + 2k.  MODE 0 accumulates A src, MODE 1 the diagonal.
-// MODE 0: y += K x with K computed on the fly; 1: diagonal of K; 2: compute K and store its upper
-// triangle; 3: y += K x with K read from storage; 4: add K into the assembled stencils of the
-// cell-array slots of its vertices (kst = stencils, kstride = level size).  Stored entry v of micro-cell (cell c, type ty,
-// anchor a) sits at kst[v * kstride + (c * 6 + ty) * tet(n) + cidx(n - 1, a)].
+// MODE 0: y += K x with K computed on the fly; 1: diagonal of K; 4: add K into the assembled stencils of
+// the cell-array slots of its vertices (kst = stencils, kstride = level size).
 template < typename T, typename A, int MODE >
 __global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                                                        const CellGeom* __restrict__ geom, Coefficient kc,
@@ -352,11 +347,10 @@ __global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const in
             for ( int d = 0; d < 3; ++d ) X[m][d] = A( g.P[0][d] ) + st[0][d] * A( vx ) + st[1][d] * A( vy ) + st[2][d] * A( vz );
          }
          A K[4][4];
-         const int64_t slot = ( int64_t( c ) * 6 + ty ) * tet_size( n ) + cidx( n - 1, x, y, z );
-         // self-check: every node inside the level's vector and every stored slot inside its array;
-         // a violation is recorded (error word 2) and the micro-cell skipped
+         // self-check: every node inside the level's vector; a violation is recorded (error word 2) and
+         // the micro-cell skipped
          {
-            bool bad = ( MODE == 2 || MODE == 3 ) && ( slot < 0 || slot >= kstride );
+            bool bad = false;
             for ( int m = 0; m < 4; ++m ) bad |= idx[m] < 0 || idx[m] >= level_size;
             if ( bad )
             {
@@ -364,26 +358,10 @@ __global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const in
                continue;
             }
          }
-         if constexpr ( MODE == 3 )
-         {
-            int v = 0;
-            for ( int i = 0; i < 4; ++i )
-               for ( int j = i; j < 4; ++j, ++v ) K[i][j] = K[j][i] = kst[v * kstride + slot];
-            A xl[4];
-            for ( int m = 0; m < 4; ++m ) xl[m] = A( ld_any( src + idx[m] ) );
-            for ( int i = 0; i < 4; ++i ) acc[idx[i]] += K[i][0] * xl[0] + K[i][1] * xl[1] + K[i][2] * xl[2] + K[i][3] * xl[3];
-            continue;
-         }
          if ( kc.kind == kCoeffPSPG ) p1_pspg_element( X, K );
          else if ( kc.element == kElemLumpedMassInvK ) p1_lumped_mass_inv_k_element( g, kc, X, K );
          else p1_divkgrad_element( g, kc, X, K );
-         if constexpr ( MODE == 2 )
-         {
-            int v = 0;
-            for ( int i = 0; i < 4; ++i )
-               for ( int j = i; j < 4; ++j, ++v ) kst[v * kstride + slot] = K[i][j];
-         }
-         else if constexpr ( MODE == 0 )
+         if constexpr ( MODE == 0 )
          {
             A xl[4];
             for ( int m = 0; m < 4; ++m ) xl[m] = A( ld_any( src + idx[m] ) );
@@ -409,26 +387,13 @@ __global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const in
 __constant__ double c_xg4_pts[11][3];
 __constant__ double c_xg4_bary[11][4];
 __constant__ double c_xg4_w[11];
+__constant__ int8_t c_p2_from[60];     // micro-cell nodes 10 ty + i, grouped by the window node they are
+__constant__ int8_t c_p2_from0[28];    // window node l: entries c_p2_from0[l] .. c_p2_from0[l + 1] - 1
 __constant__ int8_t c_p2_loc[6][10];  // node of micro-cell type ty in its anchor's 3x3x3 nodes: a + 3 b + 9 c
 __constant__ double c_p2_rgrad[11][10][3];  // reference gradients of the ten basis functions per point
 __constant__ double c_p2_phi[11][10];       // values of the ten basis functions per point
 __constant__ int    c_p2_edge[6][2] = { { 2, 3 }, { 1, 3 }, { 1, 2 }, { 0, 3 }, { 0, 2 }, { 0, 1 } };
-// Stored P2 element matrices keep the 55 distinct entries of the symmetric 10x10 matrix in wrapped-
-// diagonal order: block 0 (entries 0-9) the diagonal K(i, i); block s = 1..4 (entries 10 s + e) the
-// entries K(e, (e + s) mod 10); block 5 (entries 50-54) K(e, e + 5) for e < 5.  Lane i of a ten-lane
-// group then finds its row in blocks that the group reads as whole 80-byte runs.  c_p2_wrap maps the
-// upper-triangle index r * 10 - r (r - 1) / 2 + (c - r) of (r, c), r <= c, to this order.
-__constant__ int    c_p2_wrap[55];
-
-static void p2_wrap_table( int w[55] )
-{
-   for ( int r = 0; r < 10; ++r )
-      for ( int c = r; c < 10; ++c )
-      {
-         const int ut = r * 10 - r * ( r - 1 ) / 2 + ( c - r ), d = c - r;
-         w[ut]        = d == 0 ? r : d <= 4 ? 10 * d + r : d == 5 ? 50 + r : 10 * ( 10 - d ) + c;
-      }
-}
+__constant__ int8_t c_p2s_ent[600];  // entry of node j in node i's class stencil: (10 ty + i) 10 + j
 
 // barycentric coordinates (l0, l1, l2, l3) of the rule's points (kept identical to the reference's
 // generated form: the element integrals must agree); reference coordinates are (l1, l2, l3)
@@ -524,12 +489,20 @@ void ensure_p2_constants()
       int8_t loc[6][10];
       for ( int ty = 0; ty < 6; ++ty )
          for ( int i = 0; i < 10; ++i )
-         {
-            const int* va = kMicroOff[ty][i < 4 ? i : ed[i - 4][0]];
-            const int* vb = kMicroOff[ty][i < 4 ? i : ed[i - 4][1]];
-            loc[ty][i]    = int8_t( ( va[0] + vb[0] ) + 3 * ( va[1] + vb[1] ) + 9 * ( va[2] + vb[2] ) );
-         }
+            loc[ty][i] = int8_t( p2_local( ty, i, 0 ) + 3 * p2_local( ty, i, 1 ) + 9 * p2_local( ty, i, 2 ) );
+
       check_cuda( cudaMemcpyToSymbol( c_p2_loc, loc, sizeof( loc ) ), "P2 constants (local nodes)" );
+      int8_t from[60], from0[28];
+      int    nf = 0;
+      for ( int l = 0; l < 27; ++l )
+      {
+         from0[l] = int8_t( nf );
+         for ( int v = 0; v < 60; ++v )
+            if ( loc[v / 10][v % 10] == l ) from[nf++] = int8_t( v );
+      }
+      from0[27] = int8_t( nf );
+      check_cuda( cudaMemcpyToSymbol( c_p2_from, from, sizeof( from ) ), "P2 constants (node sums)" );
+      check_cuda( cudaMemcpyToSymbol( c_p2_from0, from0, sizeof( from0 ) ), "P2 constants (node sums)" );
       check_cuda( cudaMemcpyToSymbol( c_xg4_w, w, sizeof( w ) ), "P2 constants (weights)" );
       check_cuda( cudaMemcpyToSymbol( c_p2_rgrad, g, sizeof( g ) ), "P2 constants (gradients)" );
       double phi[11][10];
@@ -540,9 +513,9 @@ void ensure_p2_constants()
          for ( int e = 0; e < 6; ++e ) phi[q][4 + e] = 4.0 * lam[ed[e][0]] * lam[ed[e][1]];
       }
       check_cuda( cudaMemcpyToSymbol( c_p2_phi, phi, sizeof( phi ) ), "P2 constants (basis values)" );
-      int wrap[55];
-      p2_wrap_table( wrap );
-      check_cuda( cudaMemcpyToSymbol( c_p2_wrap, wrap, sizeof( wrap ) ), "P2 constants (stored order)" );
+      int8_t ent[600];
+      p2_stored_entries( ent );
+      check_cuda( cudaMemcpyToSymbol( c_p2s_ent, ent, sizeof( ent ) ), "P2 constants (stencil entries)" );
    } );
 }
 
@@ -674,34 +647,117 @@ __device__ __forceinline__ void p2_pair_gradients( const A H[4][3], const A Ji[3
    y[9] = 4 * ( h[0][1] + h[1][0] );
 }
 
+// K u of one micro-cell: node values u in, sums y out (kl: the coefficient's node values, NODAL only)
+template < typename A, bool NODAL >
+__device__ __forceinline__ void p2_micro_apply( const CellGeom& g, const Coefficient& kc, A inv_n, int ty, int x, int y, int z,
+                                                const A u[10], const A* kl, A yl[10] )
+{
+   const bool           blend = g.blend == 1;
+   const ShellCell< A > sc    = shell_cell< A >( g );
+   MicroCell< A >       mc;
+   {
+      A st[3][3];
+      for ( int k = 0; k < 3; ++k )
+         for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
+      micro_cell( g, st, ty, x, y, z, mc );
+   }
+   A G[4][3], H[4][3];
+   p2_vertex_gradients( u, mc.Ji, G );
+#pragma unroll
+   for ( int k = 0; k < 4; ++k ) H[k][0] = H[k][1] = H[k][2] = A( 0 );
+   // rolled: the body is about 400 instructions, and eleven copies cost more in instruction fetches than
+   // the constants of the points save (3.18 against 2.67 ms on the shell of k_p2_apply_pass with blocks of 96)
+#pragma unroll 1
+   for ( int q = 0; q < 11; ++q )
+   {
+      const A l0 = A( c_xg4_bary[q][0] ), l1 = A( c_xg4_bary[q][1] ), l2 = A( c_xg4_bary[q][2] ), l3 = A( c_xg4_bary[q][3] );
+      A       B[3];
+#pragma unroll
+      for ( int d = 0; d < 3; ++d ) B[d] = l0 * G[0][d] + l1 * G[1][d] + l2 * G[2][d] + l3 * G[3][d];
+      ShellPoint< A > p;
+#pragma unroll
+      for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * l1 + mc.J[d][1] * l2 + mc.J[d][2] * l3;
+      A f = A( c_xg4_w[q] ) * mc.adet, F[3] = { p.X[0], p.X[1], p.X[2] }, rad = A( -1 );
+      if ( blend )
+      {
+         // |det DF| DF^-1 DF^-T B = |m| (w - X (g . w) / m),  w = B - g (X . B) / m
+         shell_point( sc, p );
+         const A xb = ( p.X[0] * B[0] + p.X[1] * B[1] + p.X[2] * B[2] ) * p.im;
+#pragma unroll
+         for ( int d = 0; d < 3; ++d ) B[d] -= p.g[d] * xb;
+         const A gw = ( p.g[0] * B[0] + p.g[1] * B[1] + p.g[2] * B[2] ) * p.im;
+#pragma unroll
+         for ( int d = 0; d < 3; ++d )
+         {
+            B[d] -= p.X[d] * gw;
+            F[d] = p.X[d] * p.s;
+         }
+         f *= fabs( p.m );
+         rad = p.R;
+      }
+      if constexpr ( NODAL )
+      {
+         A kq = A( 0 );
+#pragma unroll
+         for ( int i = 0; i < 10; ++i ) kq += A( c_p2_phi[q][i] ) * kl[i];
+         f *= kq;
+      }
+      else
+         f *= coeff_eval( kc, F, rad );
+#pragma unroll
+      for ( int d = 0; d < 3; ++d )
+      {
+         const A h = f * B[d];
+         H[0][d] += l0 * h;
+         H[1][d] += l1 * h;
+         H[2][d] += l2 * h;
+         H[3][d] += l3 * h;
+      }
+   }
+   p2_pair_gradients( H, mc.Ji, yl );
+}
+
 // y += K x of one parity pass, matrix-free (anchors of one parity share no node, see k_p2_pass).  Bound
-// by FP64 arithmetic: three quarters of it the coefficient and the map.  A thread takes one anchor and
-// keeps the 27 nodes its six micro-cells touch in shared memory (values in, sums out), so that global
-// memory sees each of them once per pass, all loads in flight together, instead of ten
-// read-modify-writes per micro-cell in a chain.  Shell of 1920 macro-cells, level 4 (7.9 M micro-cells),
-// exp/sin coefficient: 6.22 ms per apply with the 3x3 inverse per point and chained updates, 3.34 ms so;
-// three, four or five blocks per SM take the same time.
-constexpr int kP2ApplyThreads = 96;  // 41 KB of node values and sums per block, five blocks per SM
+// by the latency and rate of FP64 arithmetic, three quarters of it the coefficient and the map.
+//
+// A thread takes one anchor and keeps the 27 nodes its six micro-cells touch in shared memory (values in,
+// sums out), so that global memory sees each of them once per pass, all loads in flight together, instead
+// of ten read-modify-writes per micro-cell in a chain.  Anchors at the slanted face have one micro-cell and
+// work straight from global memory.  Blocks run over (cell, anchor) of one kind (six, five or one
+// micro-cells), so they are full whatever the number of anchors per cell and a warp's threads do the same
+// work.
+//
+// Shell of 1920 macro-cells, level 4 (7.9 M micro-cells), exp/sin coefficient, per apply: 6.22 ms with a
+// 3x3 inverse per point and chained updates, 2.27 ms so (64 threads, 168 registers; 96 threads take 2.29,
+// 128 registers 2.67, two points at a time 2.32).
+constexpr int kP2ApplyThreads = 64;
 template < typename T, typename A, bool NODAL >
-__global__ void __launch_bounds__( kP2ApplyThreads, 5 )
-    k_p2_apply_pass( int ne, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
+__global__ void __launch_bounds__( kP2ApplyThreads, 6 )
+    k_p2_apply_pass( int ne, int nC, int3 kinds, int3 blocks, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                      const CellGeom* __restrict__ geom, Coefficient kc, const T* __restrict__ src, A* __restrict__ acc,
                      int64_t level_size, int* err, const double* __restrict__ kn )
 {
    extern __shared__ __align__( 16 ) unsigned char p2_raw[];
-   A* const  xs = reinterpret_cast< A* >( p2_raw ) + threadIdx.x;  // node i of this thread: xs[i * bd], ys[i * bd]
-   const int bd = blockDim.x;
-   A* const  ys = xs + 27 * bd;
-   const int t  = blockIdx.x * bd + threadIdx.x;
-   const int c  = blockIdx.y;
-   if ( t >= nanch ) return;
-   const int       a = anch[t];
-   const int       x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
-   const CellGeom& g    = geom[c];
-   const int64_t   base = cell_off[c];
-   // nodes past the cell's slanted face do not exist; the level check guards the anchor tables
-   const int room = ns - 2 * ( x + y + z );
+   A* const  xs = reinterpret_cast< A* >( p2_raw ) + threadIdx.x;  // node l of this thread: xs[l * kP2ApplyThreads]
+   A* const  ys = xs + 27 * kP2ApplyThreads;
+   const int ns = 2 * ne;
+   const A   inv_n = A( 1.0 / double( ne ) );
+   int       bk = blockIdx.x, n = kinds.x, first = 0;
+   if ( bk >= blocks.x )
    {
+      bk -= blocks.x, first = kinds.x, n = kinds.y;
+      if ( bk >= blocks.y ) bk -= blocks.y, first += kinds.y, n = 0;
+   }
+   const bool     single = n == 0;
+   const unsigned per    = unsigned( single ? kinds.z : n );
+   const int64_t  t      = int64_t( bk ) * kP2ApplyThreads + threadIdx.x;
+   if ( t >= int64_t( nC ) * per ) return;
+   const int      c    = t < 0x7fffffff ? int( unsigned( t ) / per ) : int( t / per );
+   const int      a    = anch[first + int( t - int64_t( c ) * per )];
+   const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, room = ns - 2 * ( x + y + z );
+   const int64_t  base = cell_off[c];
+   {
+      // self-check: the window's last node inside the level's vector
       const int64_t last = base + cidx( ns, 2 * x, 2 * y, 2 * z + min( room, 2 ) );
       if ( room < 2 || base < 0 || last >= level_size )
       {
@@ -709,105 +765,164 @@ __global__ void __launch_bounds__( kP2ApplyThreads, 5 )
          return;
       }
    }
+   auto at = [&]( int l ) { return base + cidx( ns, 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9 ); };
+   if ( single )
+   {
+      A       u[10], kl[NODAL ? 10 : 1], yl[10];
+      int64_t i0[10];
+#pragma unroll
+      for ( int i = 0; i < 10; ++i )
+      {
+         i0[i] = at( c_p2_loc[0][i] );
+         u[i]  = A( ld_any( src + i0[i] ) );
+         if constexpr ( NODAL ) kl[i] = A( kn[i0[i]] );
+      }
+      p2_micro_apply< A, NODAL >( geom[c], kc, inv_n, 0, x, y, z, u, kl, yl );
+#pragma unroll
+      for ( int i = 0; i < 10; ++i ) acc[i0[i]] += yl[i];
+      return;
+   }
 #pragma unroll
    for ( int r = 0; r < 9; ++r )
    {
-      const int     b = r % 3, cc = r / 3;
-      const int64_t row = base + cidx( ns, 2 * x, 2 * y + b, 2 * z + cc );
+      const int64_t row = at( 3 * r );
 #pragma unroll
       for ( int k = 0; k < 3; ++k )
       {
-         xs[( 3 * r + k ) * bd] = k + b + cc <= room ? A( ld_any( src + row + k ) ) : A( 0 );
-         ys[( 3 * r + k ) * bd] = A( 0 );
+         xs[( 3 * r + k ) * kP2ApplyThreads] = k + r % 3 + r / 3 <= room ? A( ld_any( src + row + k ) ) : A( 0 );
+         ys[( 3 * r + k ) * kP2ApplyThreads] = A( 0 );
       }
    }
-   const bool           blend = g.blend == 1;
-   const ShellCell< A > sc    = shell_cell< A >( g );
-   const A              inv_n = A( 1.0 / double( ne ) );
-   A                    st[3][3];
-   for ( int k = 0; k < 3; ++k )
-      for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
 #pragma unroll 1
    for ( int ty = 0; ty < 6; ++ty )
    {
       if ( x + y + z > ne - 1 - c_mc_shift[ty] ) continue;
-      MicroCell< A > mc;
-      micro_cell( g, st, ty, x, y, z, mc );
-      A kl[NODAL ? 10 : 1];
-      A G[4][3], H[4][3];
+      A u[10], kl[NODAL ? 10 : 1], yl[10];
+#pragma unroll
+      for ( int i = 0; i < 10; ++i )
       {
-         A u[10];
-#pragma unroll
-         for ( int i = 0; i < 10; ++i )
-         {
-            const int l = c_p2_loc[ty][i];
-            u[i]        = xs[l * bd];
-            if constexpr ( NODAL ) kl[i] = A( kn[base + cidx( ns, 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9 )] );
-         }
-         p2_vertex_gradients( u, mc.Ji, G );
+         u[i] = xs[c_p2_loc[ty][i] * kP2ApplyThreads];
+         if constexpr ( NODAL ) kl[i] = A( kn[at( c_p2_loc[ty][i] )] );
       }
+      p2_micro_apply< A, NODAL >( geom[c], kc, inv_n, ty, x, y, z, u, kl, yl );
 #pragma unroll
-      for ( int k = 0; k < 4; ++k ) H[k][0] = H[k][1] = H[k][2] = A( 0 );
-#pragma unroll 1
-      for ( int q = 0; q < 11; ++q )
-      {
-         const A l0 = A( c_xg4_bary[q][0] ), l1 = A( c_xg4_bary[q][1] ), l2 = A( c_xg4_bary[q][2] ), l3 = A( c_xg4_bary[q][3] );
-         A       B[3];
-#pragma unroll
-         for ( int d = 0; d < 3; ++d ) B[d] = l0 * G[0][d] + l1 * G[1][d] + l2 * G[2][d] + l3 * G[3][d];
-         ShellPoint< A > p;
-#pragma unroll
-         for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * l1 + mc.J[d][1] * l2 + mc.J[d][2] * l3;
-         A f = A( c_xg4_w[q] ) * mc.adet, F[3] = { p.X[0], p.X[1], p.X[2] }, rad = A( -1 );
-         if ( blend )
-         {
-            // |det DF| DF^-1 DF^-T B = |m| (w - X (g . w) / m),  w = B - g (X . B) / m
-            shell_point( sc, p );
-            const A xb = ( p.X[0] * B[0] + p.X[1] * B[1] + p.X[2] * B[2] ) * p.im;
-#pragma unroll
-            for ( int d = 0; d < 3; ++d ) B[d] -= p.g[d] * xb;
-            const A gw = ( p.g[0] * B[0] + p.g[1] * B[1] + p.g[2] * B[2] ) * p.im;
-#pragma unroll
-            for ( int d = 0; d < 3; ++d )
-            {
-               B[d] -= p.X[d] * gw;
-               F[d] = p.X[d] * p.s;
-            }
-            f *= fabs( p.m );
-            rad = p.R;
-         }
-         if constexpr ( NODAL )
-         {
-            A kq = A( 0 );
-#pragma unroll
-            for ( int i = 0; i < 10; ++i ) kq += A( c_p2_phi[q][i] ) * kl[i];
-            f *= kq;
-         }
-         else
-            f *= coeff_eval( kc, F, rad );
-#pragma unroll
-         for ( int d = 0; d < 3; ++d )
-         {
-            const A h = f * B[d];
-            H[0][d] += l0 * h;
-            H[1][d] += l1 * h;
-            H[2][d] += l2 * h;
-            H[3][d] += l3 * h;
-         }
-      }
-      A yl[10];
-      p2_pair_gradients( H, mc.Ji, yl );
-#pragma unroll
-      for ( int i = 0; i < 10; ++i ) ys[c_p2_loc[ty][i] * bd] += yl[i];
+      for ( int i = 0; i < 10; ++i ) ys[c_p2_loc[ty][i] * kP2ApplyThreads] += yl[i];
    }
 #pragma unroll
    for ( int r = 0; r < 9; ++r )
    {
-      const int     b = r % 3, cc = r / 3;
-      const int64_t row = base + cidx( ns, 2 * x, 2 * y + b, 2 * z + cc );
+      const int64_t row = at( 3 * r );
 #pragma unroll
       for ( int k = 0; k < 3; ++k )
-         if ( k + b + cc <= room ) acc[row + k] += ys[( 3 * r + k ) * bd];
+         if ( k + r % 3 + r / 3 <= room ) acc[row + k] += ys[( 3 * r + k ) * kP2ApplyThreads];
+   }
+}
+
+// The same pass with one thread per micro-cell, for levels whose classes hold fewer anchors than the pass
+// above keeps in flight (there it takes the time of one thread's six micro-cells, 60 us a pass, however
+// small the level): warp w of a block takes type w of 32 anchors, whose nodes the block shares; their
+// sums are added in a fixed order.  Anchors with one micro-cell are taken one per thread, straight from
+// global memory (their blocks would hold one busy warp in six).
+constexpr int kP2SplitThreads = 192;
+template < typename T, typename A, bool NODAL >
+__global__ void __launch_bounds__( kP2SplitThreads, 3 )
+    k_p2_apply_split( int ne, int nC, int3 kinds, int3 blocks, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
+                     const CellGeom* __restrict__ geom, Coefficient kc, const T* __restrict__ src, A* __restrict__ acc,
+                     int64_t level_size, int* err, const double* __restrict__ kn )
+{
+   __shared__ A xs[27][32], ys[60][32], ks[NODAL ? 27 : 1][32];
+   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ns = 2 * ne;
+   const A   inv_n = A( 1.0 / double( ne ) );
+   // the block's anchors: kind, first one among (cell, anchor) of the kind
+   int bk = blockIdx.x, n = kinds.x, first = 0;
+   if ( bk >= blocks.x )
+   {
+      bk -= blocks.x, first = kinds.x, n = kinds.y;
+      if ( bk >= blocks.y ) bk -= blocks.y, first += kinds.y, n = 0;
+   }
+   const bool     single = n == 0;
+   const unsigned per    = unsigned( single ? kinds.z : n );
+   const int64_t  t      = single ? int64_t( bk ) * kP2SplitThreads + threadIdx.x : int64_t( bk ) * 32 + lane;
+   bool           live   = t < int64_t( nC ) * per;
+   const int64_t  tt     = live ? t : 0;
+   const int      c      = tt < 0x7fffffff ? int( unsigned( tt ) / per ) : int( tt / per );
+   const int      a      = anch[first + int( tt - int64_t( c ) * per )];
+   const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, room = ns - 2 * ( x + y + z );
+   const int64_t  base = cell_off[c];
+   {
+      // self-check: the window's last node inside the level's vector
+      const int64_t last = base + cidx( ns, 2 * x, 2 * y, 2 * z + min( room, 2 ) );
+      if ( live && ( room < 2 || base < 0 || last >= level_size ) )
+      {
+         atomicExch( err, 2 );
+         live = false;
+      }
+   }
+   if ( single )
+   {
+      if ( !live ) return;
+      A       u[10], kl[NODAL ? 10 : 1], yl[10];
+      int64_t at[10];
+#pragma unroll
+      for ( int i = 0; i < 10; ++i )
+      {
+         const int l = c_p2_loc[0][i];
+         at[i]       = base + cidx( ns, 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9 );
+         u[i]        = A( ld_any( src + at[i] ) );
+         if constexpr ( NODAL ) kl[i] = A( kn[at[i]] );
+      }
+      p2_micro_apply< A, NODAL >( geom[c], kc, inv_n, 0, x, y, z, u, kl, yl );
+#pragma unroll
+      for ( int i = 0; i < 10; ++i ) acc[at[i]] += yl[i];
+      return;
+   }
+   // node a + 3 b + 9 c of the window, if it exists
+   auto node = [&]( int l, int64_t& at ) -> bool {
+      const int da = l % 3, db = ( l / 3 ) % 3, dc = l / 9;
+      at           = base + cidx( ns, 2 * x + da, 2 * y + db, 2 * z + dc );
+      return live && da + db + dc <= room;
+   };
+#pragma unroll
+   for ( int r = 0; r < 5; ++r )
+   {
+      const int l = warp + 6 * r;
+      int64_t   at;
+      if ( l < 27 )
+      {
+         const bool in = node( l, at );
+         xs[l][lane]   = in ? A( ld_any( src + at ) ) : A( 0 );
+         if constexpr ( NODAL ) ks[l][lane] = in ? A( kn[at] ) : A( 0 );
+      }
+   }
+   __syncthreads();
+   if ( live && x + y + z <= ne - 1 - c_mc_shift[warp] )
+   {
+      A u[10], kl[NODAL ? 10 : 1], yl[10];
+#pragma unroll
+      for ( int i = 0; i < 10; ++i )
+      {
+         u[i] = xs[c_p2_loc[warp][i]][lane];
+         if constexpr ( NODAL ) kl[i] = ks[c_p2_loc[warp][i]][lane];
+      }
+      p2_micro_apply< A, NODAL >( geom[c], kc, inv_n, warp, x, y, z, u, kl, yl );
+#pragma unroll
+      for ( int i = 0; i < 10; ++i ) ys[10 * warp + i][lane] = yl[i];
+   }
+   else
+#pragma unroll
+      for ( int i = 0; i < 10; ++i ) ys[10 * warp + i][lane] = A( 0 );
+   __syncthreads();
+#pragma unroll
+   for ( int r = 0; r < 5; ++r )
+   {
+      const int l = warp + 6 * r;
+      int64_t   at;
+      if ( l < 27 && node( l, at ) )
+      {
+         A s = A( 0 );
+         for ( int k = c_p2_from0[l]; k < c_p2_from0[l + 1]; ++k ) s += ys[c_p2_from[k]][lane];
+         acc[at] += s;
+      }
    }
 }
 
@@ -868,19 +983,15 @@ __device__ __forceinline__ void p2_grad( int q, int i, const A Mi[3][3], A G[3] 
       G[d] = A( c_p2_rgrad[q][i][0] ) * Mi[0][d] + A( c_p2_rgrad[q][i][1] ) * Mi[1][d] + A( c_p2_rgrad[q][i][2] ) * Mi[2][d];
 }
 
-// One parity pass over the level-L micro-cells (anchors of parity (px, py, pz); ne = 2^L), nodes
-// on storage level L+1.  MODE 0: y += K x computed matrix-free (per point the gradient of the local
-// solution, then its pairing with every basis gradient); 1: diagonal of K; 2: store the 55 distinct
-// entries of K (wrapped-diagonal order, c_p2_wrap); 3: y += K x from the stored entries.  Stored entry
-// v of micro-cell (cell c, type ty, anchor t of the pass's parity class p) sits at
-// kst[55 * (6 nC aoff[p] + (c * 6 + ty) * nanch + t) + v] (kbase = 6 nC aoff[p]): the 55 entries of
-// a micro-cell are contiguous, so the lanes that read one micro-cell's rows share its 440 bytes.
-template < typename T, typename A, int MODE >
+// One parity pass over the level-L micro-cells (anchors of parity (px, py, pz); ne = 2^L), nodes on
+// storage level L+1.  MODE 1: diagonal of K into acc; 2: K added to the assembled stencils of its nodes
+// (st, layout of sv).  Anchors of one parity share no node, and the micro-cells of one anchor are taken in
+// order by one thread, so plain additions are deterministic.
+template < typename A, int MODE >
 __global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
-                                                     const CellGeom* __restrict__ geom, Coefficient kc,
-                                                     const T* __restrict__ src, A* __restrict__ acc, A* __restrict__ kst,
-                                                     int64_t kstride, int64_t kbase, int64_t level_size, int* err,
-                                                     const double* __restrict__ kn )
+                                                       const CellGeom* __restrict__ geom, Coefficient kc, A* __restrict__ acc,
+                                                       P2StoredView sv, A* __restrict__ st, int64_t level_size, int* err,
+                                                       const double* __restrict__ kn )
 {
    const int t = blockIdx.x * blockDim.x + threadIdx.x;  // one micro-cell anchor per thread
    const int c = blockIdx.y;
@@ -890,97 +1001,71 @@ __global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int nanch, const 
    const CellGeom g    = geom[c];
    const int64_t  base = cell_off[c];
    const A        inv_n = A( 1.0 / double( ne ) );
-   A              st[3][3];
+   A              step[3][3];
    for ( int k = 0; k < 3; ++k )
-      for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
-      for ( int ty = 0; ty < 6; ++ty )
+      for ( int d = 0; d < 3; ++d ) step[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
+   for ( int ty = 0; ty < 6; ++ty )
+   {
+      if ( x + y + z > ne - 1 - c_mc_shift[ty] ) continue;
+      MicroCell< A > mc;
+      micro_cell( g, step, ty, x, y, z, mc );
+      int64_t idx[10];
+      A       kl[10];
+      bool    bad = false;
+      for ( int m = 0; m < 10; ++m )
       {
-         if ( x + y + z > ne - 1 - c_mc_shift[ty] ) continue;
-         int V[4][3];
-         for ( int m = 0; m < 4; ++m )
-         {
-            V[m][0] = x + c_mc_off[ty][m][0];
-            V[m][1] = y + c_mc_off[ty][m][1];
-            V[m][2] = z + c_mc_off[ty][m][2];
-         }
-         int64_t idx[10];
-         for ( int m = 0; m < 4; ++m ) idx[m] = base + cidx( ns, 2 * V[m][0], 2 * V[m][1], 2 * V[m][2] );
-         for ( int e = 0; e < 6; ++e )
-         {
-            const int a = c_p2_edge[e][0], b = c_p2_edge[e][1];
-            idx[4 + e]  = base + cidx( ns, V[a][0] + V[b][0], V[a][1] + V[b][1], V[a][2] + V[b][2] );
-         }
-         const int64_t slot = kbase + ( int64_t( c ) * 6 + ty ) * nanch + t;
-         {
-            // self-check: nodes inside the level's vector, stored slot inside its array
-            bool bad = ( MODE >= 2 ) && ( slot < 0 || slot >= kstride );
-            for ( int m = 0; m < 10; ++m ) bad |= idx[m] < 0 || idx[m] >= level_size;
-            if ( bad )
-            {
-               atomicExch( err, 2 );
-               continue;
-            }
-         }
-         A xl[10], yl[10], kl[10];
-         if constexpr ( MODE == 0 || MODE == 3 )
-            for ( int m = 0; m < 10; ++m ) xl[m] = A( ld_any( src + idx[m] ) );
-         if constexpr ( MODE != 3 )
-            if ( kn )
-               for ( int m = 0; m < 10; ++m ) kl[m] = A( kn[idx[m]] );
-         for ( int m = 0; m < 10; ++m ) yl[m] = A( 0 );
-         if constexpr ( MODE == 3 )
-         {
-            int v = 0;
+         const int l = c_p2_loc[ty][m];
+         idx[m]      = base + cidx( ns, 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9 );
+         bad |= idx[m] < 0 || idx[m] >= level_size;
+      }
+      // self-check: nodes inside the level's vector
+      if ( bad )
+      {
+         atomicExch( err, 2 );
+         continue;
+      }
+      if ( kn )
+         for ( int m = 0; m < 10; ++m ) kl[m] = A( kn[idx[m]] );
+      A K[MODE == 2 ? 55 : 10];
+      for ( int v = 0; v < ( MODE == 2 ? 55 : 10 ); ++v ) K[v] = A( 0 );
+#pragma unroll 1
+      for ( int q = 0; q < 11; ++q )
+      {
+         A Mi[3][3], s;
+         p2_point( g, kc, mc.X0, mc.J, q, Mi, s, kn ? kl : static_cast< const A* >( nullptr ) );
+         if constexpr ( MODE == 1 )
             for ( int i = 0; i < 10; ++i )
-               for ( int j = i; j < 10; ++j, ++v )
-               {
-                  const A k = kst[slot * 55 + c_p2_wrap[v]];
-                  yl[i] += k * xl[j];
-                  if ( j != i ) yl[j] += k * xl[i];
-               }
-         }
+            {
+               A G[3];
+               p2_grad( q, i, Mi, G );
+               K[i] += s * ( G[0] * G[0] + G[1] * G[1] + G[2] * G[2] );
+            }
          else
          {
-            A X0[3], J[3][3];
-            for ( int d = 0; d < 3; ++d )
+            A G[10][3];
+            for ( int i = 0; i < 10; ++i ) p2_grad( q, i, Mi, G[i] );
+            int v = 0;
+            for ( int i = 0; i < 10; ++i )
+               for ( int j = i; j < 10; ++j, ++v ) K[v] += s * ( G[i][0] * G[j][0] + G[i][1] * G[j][1] + G[i][2] * G[j][2] );
+         }
+      }
+      if constexpr ( MODE == 1 )
+         for ( int i = 0; i < 10; ++i ) acc[idx[i]] += K[i];
+      else
+#pragma unroll
+         for ( int i = 0; i < 10; ++i )
+         {
+            const int     l = c_p2_loc[ty][i];
+            int64_t       skip;
+            const int64_t w = p2_weight_at( sv, c, 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9, skip );
+#pragma unroll
+            for ( int j = 0; j < 10; ++j )
             {
-               X0[d] = A( g.P[0][d] ) + st[0][d] * A( V[0][0] ) + st[1][d] * A( V[0][1] ) + st[2][d] * A( V[0][2] );
-               for ( int k = 0; k < 3; ++k )
-                  J[d][k] = st[0][d] * A( V[k + 1][0] - V[0][0] ) + st[1][d] * A( V[k + 1][1] - V[0][1] ) +
-                            st[2][d] * A( V[k + 1][2] - V[0][2] );
-            }
-            A K[MODE == 2 ? 55 : 1];
-            if constexpr ( MODE == 2 )
-               for ( int v = 0; v < 55; ++v ) K[v] = A( 0 );
-#pragma unroll 1
-            for ( int q = 0; q < 11; ++q )
-            {
-               A Mi[3][3], s;
-               p2_point( g, kc, X0, J, q, Mi, s, kn ? kl : static_cast< const A* >( nullptr ) );
-               if constexpr ( MODE == 1 )
-                  for ( int i = 0; i < 10; ++i )
-                  {
-                     A G[3];
-                     p2_grad( q, i, Mi, G );
-                     yl[i] += s * ( G[0] * G[0] + G[1] * G[1] + G[2] * G[2] );
-                  }
-               else
-               {
-                  A G[10][3];
-                  for ( int i = 0; i < 10; ++i ) p2_grad( q, i, Mi, G[i] );
-                  int v = 0;
-                  for ( int i = 0; i < 10; ++i )
-                     for ( int j = i; j < 10; ++j, ++v ) K[v] += s * ( G[i][0] * G[j][0] + G[i][1] * G[j][1] + G[i][2] * G[j][2] );
-               }
-            }
-            if constexpr ( MODE == 2 )
-            {
-               for ( int v = 0; v < 55; ++v ) kst[slot * 55 + c_p2_wrap[v]] = K[v];
-               continue;
+               const int lo = i < j ? i : j, hi = i < j ? j : i;
+               st[w + c_p2s_ent[( 10 * ty + i ) * 10 + j] * skip] += K[lo * 10 - lo * ( lo - 1 ) / 2 + ( hi - lo )];
             }
          }
-         for ( int i = 0; i < 10; ++i ) acc[idx[i]] += yl[i];
-      }
+   }
 }
 
 // Combine: cell interior points take s = acc, face/edge/vertex owners the sum of their copies in
@@ -1263,115 +1348,6 @@ __global__ void k_cell_invert( int n, int nrows, const int2* __restrict__ rows, 
 }
 
 // ---------------------------------------------------------------------------------------------
-// P2 apply from stored element matrices: ten lanes per micro-cell anchor (three anchors per warp,
-// lanes 30-31 idle).  Lane i owns element node i: it loads its node value, gathers the other nine
-// with shuffles, reads row i of the symmetric matrix (55 distinct entries per micro-cell in
-// wrapped-diagonal order, so each of the ten loads of a group covers one 80-byte run) and adds row i
-// times x into its node.  The ten nodes of a micro-cell are distinct, the six
-// micro-cells of an anchor are taken in turn by the same lanes, and anchors of one parity class
-// share no node, so the read-modify-writes are race-free.  One lane per anchor (the recomputing
-// pass) left most of a block idle on these levels: 10 x more lanes in flight per pass.
-// ---------------------------------------------------------------------------------------------
-template < typename T, typename A >
-__global__ void __launch_bounds__( 256 ) k_p2_stored_pass( int ne, int nanch, const int* __restrict__ anch,
-                                                            const int64_t* __restrict__ cell_off, const T* __restrict__ src,
-                                                            A* __restrict__ acc, const A* __restrict__ kst, int64_t kstride, int64_t kbase,
-                                                            int64_t level_size, int* err )
-{
-   const int lane = threadIdx.x & 31, grp = lane / 10, i = lane - 10 * grp;  // grp 3: lanes 30, 31
-   const int t    = ( blockIdx.x * ( blockDim.x >> 5 ) + ( threadIdx.x >> 5 ) ) * 3 + grp;
-   const int c    = blockIdx.y;
-   const bool live = grp < 3 && t < nanch;
-   const int  g0   = 10 * grp;  // first lane of the group
-   int        x = 0, y = 0, z = 0;
-   if ( live )
-   {
-      const int a = anch[t];
-      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20;
-   }
-   const int     ns   = 2 * ne;
-   const int64_t base = cell_off[c];
-   // row i of the symmetric matrix in the wrapped-diagonal order: term t multiplies stored entry
-   // koff[t] with the node value of lane xsrc[t] of the group (t = 0: K(i, i); t = 2s-1, 2s:
-   // K(i, i+s), K(i, i-s) from block s; t = 9: K(i, i+5) from block 5)
-   int koff[10], xsrc[10];
-   koff[0] = i;
-   xsrc[0] = i;
-#pragma unroll
-   for ( int d = 1; d <= 4; ++d )
-   {
-      koff[2 * d - 1] = 10 * d + i;
-      xsrc[2 * d - 1] = ( i + d ) % 10;
-      koff[2 * d]     = 10 * d + ( i + 10 - d ) % 10;
-      xsrc[2 * d]     = ( i + 10 - d ) % 10;
-   }
-   koff[9] = 50 + i % 5;
-   xsrc[9] = ( i + 5 ) % 10;
-   // node index, stored slot and the self-check of micro-cell type ty (all lanes of the warp take
-   // part: the check is a warp vote)
-   auto prep = [&]( int ty, int64_t& idx, int64_t& slot, bool& go ) {
-      const bool cell = live && x + y + z <= ne - 1 - c_mc_shift[ty];
-      // node i of the micro-cell: vertex i (i < 4) at 2 V_i, edge (a, b) at V_a + V_b
-      idx = 0;
-      if ( cell )
-      {
-         int P[3];
-         if ( i < 4 )
-            for ( int d = 0; d < 3; ++d ) P[d] = 2 * ( ( d == 0 ? x : d == 1 ? y : z ) + c_mc_off[ty][i][d] );
-         else
-         {
-            const int ea = c_p2_edge[i - 4][0], eb = c_p2_edge[i - 4][1];
-            for ( int d = 0; d < 3; ++d )
-               P[d] = 2 * ( d == 0 ? x : d == 1 ? y : z ) + c_mc_off[ty][ea][d] + c_mc_off[ty][eb][d];
-         }
-         idx = base + cidx( ns, P[0], P[1], P[2] );
-      }
-      slot = kbase + ( int64_t( c ) * 6 + ty ) * nanch + ( cell ? t : 0 );
-      // self-check: every node inside the level's vector and the stored slot inside its array; a
-      // violation in any lane of the group skips the micro-cell and records error word 2
-      const bool     bad  = cell && ( idx < 0 || idx >= level_size || slot < 0 || slot >= kstride );
-      const unsigned bmsk = __ballot_sync( 0xffffffffu, bad );
-      const bool     gbad = grp < 3 && ( ( bmsk >> g0 ) & 0x3ffu ) != 0u;
-      if ( bad ) atomicExch( err, 2 );
-      go = cell && !gbad;
-   };
-   // software pipeline over the six micro-cell types: the node value and matrix row of type ty+1
-   // are loaded before type ty's product and read-modify-write, which are the only steps that must
-   // stay in order (micro-cells of one anchor share nodes)
-   int64_t idx0, slot0;
-   bool    go0;
-   prep( 0, idx0, slot0, go0 );
-   A x0 = go0 ? A( ld_any( src + idx0 ) ) : A( 0 );
-   A k0[10];
-#pragma unroll
-   for ( int j = 0; j < 10; ++j ) k0[j] = go0 ? __ldg( kst + slot0 * 55 + koff[j] ) : A( 0 );
-#pragma unroll 1
-   for ( int ty = 0; ty < 6; ++ty )
-   {
-      int64_t idx1 = 0, slot1 = 0;
-      bool    go1 = false;
-      A       x1  = A( 0 ), k1[10];
-      if ( ty < 5 ) prep( ty + 1, idx1, slot1, go1 );
-      if ( go1 ) x1 = A( ld_any( src + idx1 ) );
-#pragma unroll
-      for ( int j = 0; j < 10; ++j ) k1[j] = go1 ? __ldg( kst + slot1 * 55 + koff[j] ) : A( 0 );
-      A yi = A( 0 );
-#pragma unroll
-      for ( int j = 0; j < 10; ++j )
-      {
-         const A xj = __shfl_sync( 0xffffffffu, x0, grp < 3 ? g0 + xsrc[j] : lane );
-         if ( go0 ) yi += k0[j] * xj;
-      }
-      if ( go0 ) acc[idx0] += yi;
-      idx0 = idx1;
-      go0  = go1;
-      x0   = x1;
-#pragma unroll
-      for ( int j = 0; j < 10; ++j ) k0[j] = k1[j];
-   }
-}
-
-// ---------------------------------------------------------------------------------------------
 // Stokes coupling blocks (P2P1ElementwiseBlendingStokesOperator, P2P1ElementwiseBlendingStokesOperator.hpp:
 // 113-116): div = P2ToP1ElementwiseBlendingDiv{x,y,z} (forms p2_to_p1_div_{0,1,2}_blending_q2) maps a
 // P2 velocity of level l to a P1 pressure of level l, divT (p1_to_p2_divt_{0,1,2}_blending_q2) is its
@@ -1611,7 +1587,10 @@ static void ensure_var_tables()
 {
    static PerDeviceOnce once;
    once.run( [] {
-      const int( &off )[6][4][3] = kMicroOff;
+      int off[6][4][3];
+      for ( int t = 0; t < 6; ++t )
+         for ( int i = 0; i < 4; ++i )
+            for ( int d = 0; d < 3; ++d ) off[t][i][d] = micro_vertex( t, i, d );
       int8_t dir[6][4][4], vd[15][3];
       for ( int d = 0; d < 15; ++d )
          for ( int k = 0; k < 3; ++k ) vd[d][k] = int8_t( kVarDirs[d][k] );
@@ -1638,7 +1617,6 @@ static A* assembled_stencils( Operator* op, int L ) { return reinterpret_cast< A
 // micro-cells per macro-edge of the elements living on storage level L (P2 elements of level L-1
 // have their nodes on storage level L)
 static int element_n( const Operator* op, int L ) { return op->order == 2 ? ( 1 << ( L - 1 ) ) : ( 1 << L ); }
-static int element_values( const Operator* op ) { return op->order == 2 ? 55 : 10; }
 
 // micro-cell anchors (x, y, z), x + y + z <= n - 1, grouped by coordinate parity: the micro-cells of
 // anchors of one parity class share no vertex (nor, for P2, any node), so a pass over one class
@@ -1653,21 +1631,24 @@ static void ensure_rows( Operator* op, int L )
    {
       e.aoff[p]    = int( anch.size() );
       const int px = p & 1, py = ( p >> 1 ) & 1, pz = p >> 2;
-      for ( int z = pz; z <= n - 1; z += 2 )
-         for ( int y = py; y + z <= n - 1; y += 2 )
-            for ( int x = px; x + y + z <= n - 1; x += 2 ) anch.push_back( x | ( y << 10 ) | ( z << 20 ) );
+      // by the number of micro-cells an anchor has (six; five next to the slanted face; one at it), so
+      // that the threads of a warp visit the same micro-cell types
+      for ( int k = 0; k < 3; ++k )
+      {
+         const int lo = k == 0 ? 0 : n - 3 + k, hi = n - 3 + k;
+         const int before = int( anch.size() );
+         for ( int z = pz; z <= n - 1; z += 2 )
+            for ( int y = py; y + z <= n - 1; y += 2 )
+               for ( int x = px; x + y + z <= n - 1; x += 2 )
+                  if ( x + y + z >= lo && x + y + z <= hi ) anch.push_back( x | ( y << 10 ) | ( z << 20 ) );
+         e.akind[p][k] = int( anch.size() ) - before;
+      }
    }
    e.aoff[8] = int( anch.size() );
    check_cuda( cudaMalloc( &e.d_anch, std::max< size_t >( anch.size(), 1 ) * sizeof( int ) ), "cudaMalloc(anchors)" );
    if ( !anch.empty() )
       check_cuda( cudaMemcpy( e.d_anch, anch.data(), anch.size() * sizeof( int ), cudaMemcpyHostToDevice ), "upload anchors" );
 }
-
-// entries per stored value: every (cell, micro-cell type, anchor) slot of the level
-static int64_t kstride( Mesh* m, const Operator* op, int L ) { return int64_t( m->topo.nC ) * 6 * tet_size( int64_t( element_n( op, L ) ) ); }
-
-template < typename A >
-static A* stored_matrices( Operator* op, int L ) { return reinterpret_cast< A* >( op->el[L].d_K[sizeof( A ) == 8 ? 0 : 1] ); }
 
 // threads per block of a pass over na anchors per cell (grid: blocks x cells): whole warps, at most
 // maxb, so that the small levels (a few anchors per cell) do not launch mostly idle blocks
@@ -1679,45 +1660,46 @@ static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src
    P1Level&   P = m->level( L );
    ElemLevel& e = op->el[L];
    if ( MODE != 2 && MODE != 4 ) check_cuda( cudaMemsetAsync( acc, 0, P.size * sizeof( A ), ctx->stream ), "cudaMemset(acc)" );
-   A*            kst = MODE == 4 ? assembled_stencils< A >( op, L ) : stored_matrices< A >( op, L );
-   const int64_t ks  = MODE == 4 ? P.size : kstride( m, op, L );
    const int nC = m->topo.nC;
    for ( int p = 0; p < 8; ++p )
    {
       const int na = e.aoff[p + 1] - e.aoff[p];
       if ( na <= 0 ) continue;
-      // P2 stored matrices are grouped by parity class, then cell, micro-cell type and anchor, so the
-      // anchors of one pass read consecutive slots
-      const int64_t kbase = int64_t( 6 ) * nC * e.aoff[p];
       const int bs = pass_block( na, 256 );
       dim3      grid( ( na + bs - 1 ) / bs, nC );
-      if ( op->order == 2 && MODE == 3 )
+      if ( op->order == 2 && MODE == 0 )
       {
-         // three anchors per warp (ten lanes each), at most 8 warps per block
-         const int  wb = std::min( 8, ( na + 2 ) / 3 );
-         const dim3 g3( ( na + 3 * wb - 1 ) / ( 3 * wb ), nC );
-         k_p2_stored_pass< T, A ><<< g3, 32 * wb, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB, src,
-                                                                      acc, kst, ks, kbase, P.size, ctx->d_error );
+         const int3 kinds  = make_int3( e.akind[p][0], e.akind[p][1], e.akind[p][2] );
+         // anchors that 148 SMs with six blocks of k_p2_apply_pass hold at once: below it the split pass is
+         // faster (shell of 240 cells, level 3: 183 against 494 us an apply), above it slower (2.69 against 2.27 ms on the shell named there)
+         const bool split  = int64_t( na ) * nC < 148 * 6 * kP2ApplyThreads;
+         const int  per    = split ? 32 : kP2ApplyThreads, per1 = split ? kP2SplitThreads : kP2ApplyThreads;
+         auto       blocks = [&]( int k, int b ) { return int( ( int64_t( k ) * nC + b - 1 ) / b ); };
+         const int3 bl     = make_int3( blocks( kinds.x, per ), blocks( kinds.y, per ), blocks( kinds.z, per1 ) );
+         auto       launch = [&]( auto nodal ) {
+            constexpr bool NODAL = decltype( nodal )::value;
+            const double*  kn    = NODAL ? e.d_kn : nullptr;
+            const int      pg    = bl.x + bl.y + bl.z;
+            if ( split )
+               k_p2_apply_split< T, A, NODAL ><<< pg, kP2SplitThreads, 0, ctx->stream >>>( element_n( op, L ), nC, kinds, bl, e.d_anch + e.aoff[p],
+                                                                                          P.d_off + P.nB, op->d_geom, op->coeff, src, acc,
+                                                                                          P.size, ctx->d_error, kn );
+            else
+               k_p2_apply_pass< T, A, NODAL ><<< pg, kP2ApplyThreads, 54 * kP2ApplyThreads * sizeof( A ), ctx->stream >>>(
+                   element_n( op, L ), nC, kinds, bl, e.d_anch + e.aoff[p], P.d_off + P.nB, op->d_geom, op->coeff, src, acc, P.size,
+                   ctx->d_error, kn );
+         };
+         if ( op->nodal_k ) launch( std::true_type{} );
+         else launch( std::false_type{} );
       }
-      else if ( op->order == 2 && MODE == 0 )
-      {
-         const int    pb   = pass_block( na, kP2ApplyThreads );
-         const dim3   pg( ( na + pb - 1 ) / pb, nC );
-         const size_t smem = size_t( 54 ) * pb * sizeof( A );
-         if ( op->nodal_k )
-            k_p2_apply_pass< T, A, true ><<< pg, pb, smem, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
-                                                                            op->d_geom, op->coeff, src, acc, P.size, ctx->d_error, e.d_kn );
-         else
-            k_p2_apply_pass< T, A, false ><<< pg, pb, smem, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
-                                                                             op->d_geom, op->coeff, src, acc, P.size, ctx->d_error, nullptr );
-      }
-      else if ( op->order == 2 )
-         k_p2_pass< T, A, MODE ><<< grid, bs, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
-                                                                   op->d_geom, op->coeff, src, acc, kst, ks, kbase, P.size,
-                                                                   ctx->d_error, op->nodal_k ? e.d_kn : nullptr );
-      else
-         k_elem_pass< T, A, MODE ><<< grid, bs, 0, ctx->stream >>>( P.n, na, e.d_anch + e.aoff[p], P.d_off + P.nB, op->d_geom,
-                                                                     op->coeff, src, acc, kst, ks, P.size, ctx->d_error );
+      else if ( op->order == 2 && ( MODE == 1 || MODE == 2 ) )
+         k_p2_pass< A, MODE == 2 ? 2 : 1 ><<< grid, bs, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
+                                                                            op->d_geom, op->coeff, acc, e.p2s ? *e.p2s : P2StoredView{},
+                                                                            assembled_stencils< A >( op, L ), P.size, ctx->d_error,
+                                                                            op->nodal_k ? e.d_kn : nullptr );
+      else if constexpr ( MODE != 2 )
+         k_elem_pass< T, A, MODE ><<< grid, bs, 0, ctx->stream >>>( P.n, na, e.d_anch + e.aoff[p], P.d_off + P.nB, op->d_geom, op->coeff,
+                                                                    src, acc, assembled_stencils< A >( op, L ), P.size, P.size, ctx->d_error );
       ++ctx->launches;
    }
    check_cuda( cudaGetLastError(), "elementwise pass launch" );
@@ -1781,7 +1763,6 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
    ensure_rows( op, L );
    ElemLevel& e = op->el[L];
    A*         acc = acc_buffer< A >( op, L, P.size );
-   void*&     K   = e.d_K[sizeof( A ) == 8 ? 0 : 1];
    if ( op->store_matrices && op->order == 1 )
    {
       // P1: the stored matrices are kept assembled, summed in double once and rounded for float
@@ -1799,11 +1780,41 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
          launch_convert( ctx, cnt, F32, e.d_S[1], F64, e.d_S[0] );
       }
    }
-   else if ( op->store_matrices && !K )
+   else if ( op->store_matrices && !e.d_S[sizeof( A ) == 8 ? 0 : 1] )
    {
-      check_cuda( cudaMalloc( &K, size_t( element_values( op ) ) * size_t( kstride( m, op, L ) ) * sizeof( A ) ),
-                  "cudaMalloc(element matrices)" );
-      run_passes< T, A, 2 >( ctx, m, op, L, nullptr, acc );
+      // P2: likewise; the sums in double go again where only float ones are used
+      if ( !e.p2s )
+      {
+         std::vector< ushort4 > pts;
+         std::vector< int >     rank;
+         auto                   v = std::make_shared< P2StoredView >();
+         e.p2s_count              = build_p2_stored( *v, P.n, m->topo.nC, pts, rank );
+         check_cuda( cudaMalloc( &e.d_p2s_pts, pts.size() * sizeof( ushort4 ) ), "cudaMalloc(stencil nodes)" );
+         check_cuda( cudaMemcpy( e.d_p2s_pts, pts.data(), pts.size() * sizeof( ushort4 ), cudaMemcpyHostToDevice ), "upload stencil nodes" );
+         check_cuda( cudaMalloc( &e.d_p2s_rank, rank.size() * sizeof( int ) ), "cudaMalloc(stencil ranks)" );
+         check_cuda( cudaMemcpy( e.d_p2s_rank, rank.data(), rank.size() * sizeof( int ), cudaMemcpyHostToDevice ), "upload stencil ranks" );
+         v->pts  = reinterpret_cast< const ushort4* >( e.d_p2s_pts );
+         v->rank = e.d_p2s_rank;
+         e.p2s   = v;
+      }
+      const bool had = e.d_S[0] != nullptr;
+      if ( !had )
+      {
+         check_cuda( cudaMalloc( &e.d_S[0], e.p2s_count * sizeof( double ) ), "cudaMalloc(assembled stencils)" );
+         check_cuda( cudaMemsetAsync( e.d_S[0], 0, e.p2s_count * sizeof( double ), ctx->stream ), "cudaMemset" );
+         run_passes< double, double, 2 >( ctx, m, op, L, nullptr, nullptr );
+      }
+      if ( sizeof( A ) == 4 )
+      {
+         check_cuda( cudaMalloc( &e.d_S[1], e.p2s_count * sizeof( float ) ), "cudaMalloc(assembled stencils)" );
+         launch_convert( ctx, e.p2s_count, F32, e.d_S[1], F64, e.d_S[0] );
+         if ( !had )
+         {
+            check_cuda( cudaStreamSynchronize( ctx->stream ), "assembled stencils" );
+            check_cuda( cudaFree( e.d_S[0] ), "cudaFree(assembled stencils)" );
+            e.d_S[0] = nullptr;
+         }
+      }
    }
    if ( e.d_invd[dtype] ) return;
    A* invd = nullptr;
@@ -1874,8 +1885,16 @@ static void run_elem( Context* ctx, Mesh* m, Operator* op, int L, int dtype, con
    P1Level& P   = m->level( L );
    A*       acc = acc_buffer< A >( op, L, P.size );
    const A* inv = reinterpret_cast< const A* >( op->el[L].d_invd[dtype] );
-   if ( stored_matrices< A >( op, L ) ) run_passes< T, A, 3 >( ctx, m, op, L, (const T*) a.src, acc );
-   else run_passes< T, A, 0 >( ctx, m, op, L, (const T*) a.src, acc );
+   if ( const A* S = assembled_stencils< A >( op, L ) )
+   {
+      launch_p2_stored_sweep( ctx, P, dtype, *op->el[L].p2s, S, inv, acc, &a, 1 );
+      launch_bnd_acc< T, A, OP >( ctx->stream, P, a.flag, a.copy_unflagged, acc, inv, nullptr, (const T*) a.src, (const T*) a.v1,
+                                  (T*) a.v2, (T*) a.dst, A( a.a0 ), A( a.a1 ) );
+      if ( !P.tasks.empty() ) ++ctx->launches;
+      check_cuda( cudaGetLastError(), "stored P2 combine launch" );
+      return;
+   }
+   run_passes< T, A, 0 >( ctx, m, op, L, (const T*) a.src, acc );
    const int nrows = int( P.rows.size() );
    {
       struct Join

@@ -216,9 +216,9 @@ double slot_bytes( ServeKey k )
       hyb_layout_packed_size( k.mesh, L + sh, &n );
       total += n;
       if ( k.kind == HYB_P1_ELEM_DIVKGRAD ) mats += double( n ) * 15.0;
-      // 55 values per micro-cell; P2 level l has 8^l micro-cells per macro-cell and about 8^(l+1)/6
-      // nodes, 0.75 micro-cells per node (44 values per node with the padding of the anchor rows)
-      if ( k.kind == HYB_P2_ELEM_DIVKGRAD ) mats += double( n ) * 44.0;
+      // 28.75 values per node on average (class stencils), a little more with the nodes that several
+      // macro-cells hold
+      if ( k.kind == HYB_P2_ELEM_DIVKGRAD ) mats += double( n ) * 32.0;
    }
    return double( total ) * 8.0 * ( k.mixed ? 12.0 : 10.0 ) + mats * ( k.mixed ? 12.0 : 8.0 );
 }

@@ -766,8 +766,9 @@ Operator::~Operator()
    {
       cudaFree( kv.second.d_acc );
       for ( void* p : kv.second.d_invd ) cudaFree( p );
-      for ( void* p : kv.second.d_K ) cudaFree( p );
       for ( void* p : kv.second.d_S ) cudaFree( p );
+      cudaFree( kv.second.d_p2s_pts );
+      cudaFree( kv.second.d_p2s_rank );
       cudaFree( kv.second.d_sacc );
       cudaFree( kv.second.d_kn );
       cudaFree( kv.second.d_anch );

@@ -56,3 +56,45 @@ def test_full_viscous_apply_smallest_level(ctx, kind):
     ref = op.apply(u, [np.zeros_like(v) for v in u], 0, O.ALL)
     for k in range(3):
         assert _relerr(fy[k].download(0), ref[k], lev.owned_mask(O.ALL)) < 1e-12
+
+
+def test_p2_matrix_free_apply_full_blocks(ctx):
+    """Enough anchors per class (68,640) for the one-anchor-per-thread pass, against the stencil sweep of the
+    constant operator (k = 1, no blending: the same matrix)."""
+    coords, tets = M.cube_2x1x1()
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    L = 6
+    A = H.P2ElementwiseBlendingDivKGradOperator(pm, L, L, ctx, k=1.0)
+    C = H.P2ConstantLaplaceOperator(pm, L, L, ctx)
+    fx, fy, fz = (H.P2Function(n, pm, L, L, ctx) for n in "xyz")
+    fx.fill_random(L, 7)
+    A.apply(fx, fy, L, O.INNER)
+    C.apply(fx, fz, L, O.INNER)
+    y, z = fy.download(L), fz.download(L)
+    assert np.abs(y - z).max() < 1e-12 * np.abs(z).max()
+
+
+@pytest.mark.parametrize("case,L", [("tet", 0), ("tet", 1), ("tet", 4), ("shell", 0), ("shell", 2)])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_p2_stored_apply(ctx, case, L, dtype):
+    """Stored matrices at the levels without inner nodes, with segments shorter than a block and with
+    several macro-cells in one block; FP32 sums up to 65 rounded products per macro-cell: 100 eps."""
+    coords, tets = M.tilted_tet() if case == "tet" else O.mesh_spherical_shell(2, 2, 0.55, 1.0)
+    bl = "shell" if case == "shell" else None
+    spec, kfun = SPECS["expsin"]
+    op = O.P2DivKGrad(O.MacroMesh(coords, tets), L, L, kfun, blending=bl)
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    A = H.P2ElementwiseBlendingDivKGradOperator(pm, L, L, ctx, k=spec, blending=bl)
+    A.computeAndStoreLocalElementMatrices()
+    lev = op.levels[L]
+    x = _rand(lev, 1)
+    if dtype == "float32":
+        x = x.astype(np.float32).astype(np.float64)
+    fx, fy = (H.P2Function(n, pm, L, L, ctx, dtype) for n in "xy")
+    fx.upload(L, x)
+    for flag in (O.INNER, O.ALL):
+        fy.interpolate(0.0, L, H.All)
+        A.apply(fx, fy, L, flag)
+        ref = op.apply(x, np.zeros_like(x), L, flag)
+        err = np.abs(fy.download(L) - ref)[lev.owned_mask(O.ALL)].max()
+        assert err <= (1e-12 if dtype == "float64" else 1.2e-5) * max(np.abs(ref).max(), 1e-300)
