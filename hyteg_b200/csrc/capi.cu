@@ -2744,9 +2744,57 @@ void stokes_prepare( hyb_stokes* s, hyb_fn* u0, hyb_fn* b0, int dt )
       s->dtype = dt;
       return;
    }
+   // the smoother's two work vectors of the second and third component (the first uses the solver's)
+   for ( int k = 1; k < 3; ++k )
+      for ( hyb_fn** g : { &s->vz[k], &s->vt[k] } )
+      {
+         *g               = new_fn( s->ctx, m, dt, s->p.min_level + 1, s->p.max_level + 1 );
+         ( *g )->f.lshift = 1;
+      }
    // radii of the velocity block (power iteration on D^-1 A per level, once)
    gmg_prepare( s->vel, u0, b0, s->p.max_level + 1 );
    s->dtype = dt;
+}
+
+// the velocity smoother on the three components: with stored matrices and order two or more each step is
+// one sweep that reads the matrices once for the three, else component by component
+void velocity_smooth( hyb_stokes* s, hyb_fn* const* u, hyb_fn* const* r, int Ls )
+{
+   const int   dt = u[0]->f.dtype;
+   const auto& c  = s->vel->coeff.at( Ls - s->vel->p.min_level );
+   const int   order = int( c.size() );
+   hyb_fn *    za[3] = { s->vel->z0, s->vz[1], s->vz[2] }, *zb[3] = { s->vel->z1, s->vt[1], s->vt[2] };
+   auto        step  = [&]( int op, int copy, hyb_fn* const* src, hyb_fn* const* v1, hyb_fn* const* v2, hyb_fn* const* dst, double a0, double a1 ) {
+      StencilArgs a[3]{};
+      for ( int k = 0; k < 3; ++k )
+      {
+         a[k].op             = op;
+         a[k].flag           = kSolveFlag;
+         a[k].copy_unflagged = copy;
+         a[k].src            = src[k]->f.ptr( Ls );
+         a[k].v1             = v1 ? v1[k]->f.ptr( Ls ) : nullptr;
+         a[k].v2             = v2 ? v2[k]->f.ptr( Ls ) : nullptr;
+         a[k].dst            = dst ? dst[k]->f.ptr( Ls ) : nullptr;
+         a[k].a0             = a0;
+         a[k].a1             = a1;
+      }
+      return launch_stored3( &s->ctx->c, &s->mesh->m, &s->A->o, Ls, dt, a );
+   };
+   if ( order < 2 || !s->vz[1] || !step( OP_CHEB0, 1, u, r, nullptr, za, 0, 0 ) )
+   {
+      for ( int k = 0; k < 3; ++k ) smooth( s->vel, u[k], r[k], Ls );
+      return;
+   }
+   for ( int m = 1; m < order; ++m )
+   {
+      if ( m < order - 1 )
+      {
+         step( OP_CHEBI, 1, za, nullptr, u, zb, c[m - 1], 0 );
+         for ( int k = 0; k < 3; ++k ) std::swap( za[k], zb[k] );
+      }
+      else
+         step( OP_CHEBL, 0, za, nullptr, u, nullptr, c[m - 1], c[m] );
+   }
 }
 
 // UzawaSmoother::uzawaSmooth, block-Laplace variant without stabilisation (UzawaSmoother.hpp:
@@ -2757,24 +2805,25 @@ void uzawa_smooth( hyb_stokes* s, hyb_fn* const* u, hyb_fn* p, hyb_fn* const* bu
    Context&  cx = s->ctx->c;
    const int Ls = l + 1, dt = p->f.dtype;
    void*     rr[3] = { s->ru[0]->f.ptr( Ls ), s->ru[1]->f.ptr( Ls ), s->ru[2]->f.ptr( Ls ) };
-   launch_stokes_div( &cx, &s->D->o, l, dt, 1, nullptr, p->f.ptr( l ), rr, nullptr, kSolveFlag, 0 );
-   const double sc[2] = { 1.0, -1.0 };
-   for ( int k = 0; k < 3; ++k )
-   {
-      hyb_fn* src[2] = { bu[k], s->ru[k] };
-      pointwise( s->ru[k], l, kSolveFlag, PT_LINCOMB, 2, sc, src );
-   }
+   StokesUpdate up{};
+   for ( int k = 0; k < 3; ++k ) up.b[k] = bu[k]->f.ptr( Ls );
+   launch_stokes_div( &cx, &s->D->o, l, dt, 1, nullptr, p->f.ptr( l ), rr, nullptr, kSolveFlag, 0, &up );
    for ( int it = 0; it < s->p.velocity_sweeps; ++it )
    {
-      if ( s->V )
-      {
-         visc_smooth( s, u, s->ru, l );
-         continue;
-      }
-      for ( int k = 0; k < 3; ++k ) smooth( s->vel, u[k], s->ru[k], Ls );
+      if ( s->V ) visc_smooth( s, u, s->ru, l );
+      else velocity_smooth( s, u, s->ru, Ls );
    }
    const void* uu[3] = { u[0]->f.ptr( Ls ), u[1]->f.ptr( Ls ), u[2]->f.ptr( Ls ) };
+   if ( dt != F16 )
+   {
+      up.b[0]  = bp->f.ptr( l );
+      up.sinv  = s->sinv->f.ptr( l );
+      up.omega = s->p.omega;
+      launch_stokes_div( &cx, &s->D->o, l, dt, 0, uu, nullptr, nullptr, p->f.ptr( l ), kAll, 0, &up );
+      return;
+   }
    launch_stokes_div( &cx, &s->D->o, l, dt, 0, uu, nullptr, nullptr, s->rp->f.ptr( l ), kAll, 0 );
+   const double sc[2] = { 1.0, -1.0 };
    {
       hyb_fn* src[2] = { bp, s->rp };
       pointwise( s->rp, l, kAll, PT_LINCOMB, 2, sc, src );
@@ -3058,7 +3107,7 @@ int hyb_stokes_estimate_relaxation( hyb_stokes* s, int level, int iterations, in
             visc_smooth( s, u, s->ru, l );
             continue;
          }
-         for ( int k = 0; k < 3; ++k ) smooth( s->vel, u[k], s->ru[k], Ls );
+         velocity_smooth( s, u, s->ru, Ls );
       }
       const void* uu[3] = { u[0]->f.ptr( Ls ), u[1]->f.ptr( Ls ), u[2]->f.ptr( Ls ) };
       launch_stokes_div( &cx, &s->D->o, l, dt, 0, uu, nullptr, nullptr, s->rp->f.ptr( l ), kAll, 0 );

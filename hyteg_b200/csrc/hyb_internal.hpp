@@ -275,13 +275,15 @@ struct ElemLevel {
    int   aoff[9]    = {};                              // class p = px | py << 1 | pz << 2 spans aoff[p]..aoff[p+1]-1
    int   akind[8][3] = {};                             // its anchors with six, five and one micro-cells, in this order
    // operators with stored matrices (computeAndStoreLocalElementMatrices) keep them assembled, in double
-   // ([0]) and float ([1]).  P1: the 15 stencil weights of every cell-array slot (the partial stencil of
-   // that cell at copies of face/edge/vertex DoFs), weight-major over the level's slots.  P2: the class
+   // ([0]) and float ([1]).  P1: eight stencil weights of every cell-array slot (centre and one direction of
+   // each opposite pair; the partial stencil of that cell at copies of face/edge/vertex DoFs), weight-major
+   // over the level's slots.  P2: the class
    // stencils of p2_stored.cuh with their tables.
    void*                           d_S[2] = { nullptr, nullptr };
    std::shared_ptr< P2StoredView > p2s;
    int64_t                         p2s_count = 0;
    void*                           d_p2s_pts = nullptr;
+   void*                           d_pts     = nullptr;  // P1: coordinates of a cell's points (ushort4)
    int*                            d_p2s_rank = nullptr;
    void* d_sacc = nullptr;  // Stokes coupling blocks: three velocity accumulators and one pressure accumulator
    // P2 operators with a stored coefficient function: k at every cell-array node of this storage level
@@ -389,8 +391,18 @@ void set_p2_nodal_coefficient( Context* ctx, Operator* A, int Ls, const double* 
 void ensure_stokes_constants();
 // Stokes coupling blocks on P1 level Lp / P2 level Lp (storage Lp+1): divt 0 dst_p (+)= div u,
 // divt 1 dst_u[k] (+)= divT_k p
+// (up given: the Uzawa step's updates in the combine, divt 1 dst_u[k] = b[k] - divT_k p, divt 0 in FP64 and
+// FP32 dst_p += omega sinv (b[0] - div u), in place of the plain results)
+struct StokesUpdate {
+   const void* b[3];
+   const void* sinv;
+   double      omega;
+};
 void launch_stokes_div( Context* ctx, Operator* op, int Lp, int dtype, int divt, const void* const* u, const void* p, void* const* dst_u,
-                        void* dst_p, uint32_t flag, int add );
+                        void* dst_p, uint32_t flag, int add, const StokesUpdate* up = nullptr );
+// one operation of a P2 operator with stored matrices on three vectors (a[0..2], same operation and
+// scalars): the weights are read once; false (nothing done) for other operators
+bool launch_stored3( Context* ctx, Mesh* m, Operator* op, int L, int dtype, const StencilArgs* a );
 
 // full viscous velocity block on P2 level Lp (storage Lp+1): mode 0 dst[k] (+)= sum_j A_kj u[j] on
 // flagged owners; mode 1 writes 1/diag(A_kk) into the accumulation-precision arrays dst[k] (u unused)

@@ -305,7 +305,6 @@ __constant__ int8_t c_mc_dir[6][4][4];
 static const int kVarDirs[15][3] = { { 0, 0, 0 },  { -1, 0, 0 }, { 1, 0, 0 },  { 0, -1, 0 }, { 0, 1, 0 },
                                      { 0, 0, -1 }, { 0, 0, 1 },  { -1, 1, 0 }, { 1, -1, 0 }, { -1, 0, 1 },
                                      { 1, 0, -1 }, { 0, -1, 1 }, { 0, 1, -1 }, { 1, -1, 1 }, { -1, 1, -1 } };
-__constant__ int8_t c_var_dir[15][3];
 
 __device__ __forceinline__ double ld_any( const double* p ) { return *p; }
 __device__ __forceinline__ float  ld_any( const float* p ) { return *p; }
@@ -371,7 +370,11 @@ __global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const in
             for ( int i = 0; i < 4; ++i ) acc[idx[i]] += K[i][i];
          else if constexpr ( MODE == 4 )
             for ( int i = 0; i < 4; ++i )
-               for ( int j = 0; j < 4; ++j ) kst[int64_t( c_mc_dir[ty][i][j] ) * kstride + idx[i]] += K[i][j];
+               for ( int j = 0; j < 4; ++j )
+               {
+                  const int d = c_mc_dir[ty][i][j];  // opposite directions: the one with the even number is kept
+                  if ( !( d & 1 ) ) kst[int64_t( d / 2 ) * kstride + idx[i]] += K[i][j];
+               }
       }
 }
 
@@ -1087,11 +1090,26 @@ __device__ __forceinline__ A epilogue_value( int64_t i, A s, A invd, const T* sr
    return s;
 }
 
+// the vectors of up to three components that one combine launch serves
+template < typename T, typename A >
+struct AccVecs {
+   const A* acc[3];
+   const T* src[3];
+   const T* v1[3];
+   T*       v2[3];
+   T*       dst[3];
+};
+
 template < typename T, typename A, int OP >
 __global__ void __launch_bounds__( 256 ) k_cell_acc( int n, int nrows, const int2* __restrict__ rows, const int64_t* __restrict__ cell_off,
-                                                      const uint8_t* __restrict__ cell_bc, uint32_t flag, const A* __restrict__ acc,
-                                                      const A* __restrict__ invd, const T* src, const T* v1, T* v2, T* dst, A a0, A a1 )
+                                                      const uint8_t* __restrict__ cell_bc, uint32_t flag, AccVecs< T, A > vec,
+                                                      const A* __restrict__ invd, A a0, A a1 )
 {
+   const A* __restrict__ acc = vec.acc[blockIdx.z];
+   const T* src = vec.src[blockIdx.z];
+   const T* v1  = vec.v1[blockIdx.z];
+   T*       v2  = vec.v2[blockIdx.z];
+   T*       dst = vec.dst[blockIdx.z];
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
    const int r    = blockIdx.x * 8 + warp;
    const int c    = blockIdx.y;
@@ -1167,9 +1185,13 @@ __global__ void __launch_bounds__( 256 ) k_bnd_acc( int n, int ntasks, const int
                                                      const int64_t* __restrict__ cell_off, const int8_t* __restrict__ bkind,
                                                      const uint8_t* __restrict__ bc, const int* __restrict__ inc_begin,
                                                      const Incidence* __restrict__ inc, uint32_t flag, int copy_unflagged,
-                                                     const A* __restrict__ acc, const A* __restrict__ invd, A* invd_out, const T* src,
-                                                     const T* v1, T* v2, T* dst, A a0, A a1 )
+                                                     AccVecs< T, A > vec, const A* __restrict__ invd, A* invd_out, A a0, A a1 )
 {
+   const A* __restrict__ acc = vec.acc[blockIdx.y];
+   const T* src = vec.src[blockIdx.y];
+   const T* v1  = vec.v1[blockIdx.y];
+   T*       v2  = vec.v2[blockIdx.y];
+   T*       dst = vec.dst[blockIdx.y];
    static_assert( G == 1 || G == 2 || G == 4 || G == 8 || G == 16 || G == 32, "G divides the warp" );
    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
    const int t  = gt / G, sub = gt % G;
@@ -1226,111 +1248,108 @@ __global__ void __launch_bounds__( 256 ) k_bnd_acc( int n, int ntasks, const int
 
 // launch of the owner combine over the level's tasks, lanes per task by level size
 template < typename T, typename A, int OP >
-static void launch_bnd_acc( cudaStream_t st, const P1Level& P, uint32_t flag, int copy_unflagged, const A* acc, const A* invd, A* invd_out,
-                            const T* src, const T* v1, T* v2, T* dst, A a0, A a1 )
+static void launch_bnd_acc( Context* ctx, cudaStream_t st, const P1Level& P, uint32_t flag, int copy_unflagged, const AccVecs< T, A >& vec,
+                            int ncomp, const A* invd, A* invd_out, A a0, A a1 )
 {
    const int nt = int( P.tasks.size() );
    if ( nt <= 0 ) return;
    if ( P.n <= 4 )
-      k_bnd_acc< T, A, OP, 8 ><<< ( 8 * nt + 255 ) / 256, 256, 0, st >>>( P.n, nt, P.d_tasks, P.d_off, P.d_off + P.nB, P.d_bkind, P.d_bc,
-                                                                          P.d_inc_begin, P.d_inc, flag, copy_unflagged, acc, invd, invd_out,
-                                                                          src, v1, v2, dst, a0, a1 );
+      k_bnd_acc< T, A, OP, 8 ><<< dim3( ( 8 * nt + 255 ) / 256, ncomp ), 256, 0, st >>>( P.n, nt, P.d_tasks, P.d_off, P.d_off + P.nB,
+                                                                                        P.d_bkind, P.d_bc, P.d_inc_begin, P.d_inc, flag,
+                                                                                        copy_unflagged, vec, invd, invd_out, a0, a1 );
    else
-      k_bnd_acc< T, A, OP, 1 ><<< ( nt + 255 ) / 256, 256, 0, st >>>( P.n, nt, P.d_tasks, P.d_off, P.d_off + P.nB, P.d_bkind, P.d_bc,
-                                                                      P.d_inc_begin, P.d_inc, flag, copy_unflagged, acc, invd, invd_out, src,
-                                                                      v1, v2, dst, a0, a1 );
+      k_bnd_acc< T, A, OP, 1 ><<< dim3( ( nt + 255 ) / 256, ncomp ), 256, 0, st >>>( P.n, nt, P.d_tasks, P.d_off, P.d_off + P.nB, P.d_bkind,
+                                                                                    P.d_bc, P.d_inc_begin, P.d_inc, flag, copy_unflagged, vec,
+                                                                                    invd, invd_out, a0, a1 );
+   ++ctx->launches;
+}
+
+template < typename T, typename A >
+static AccVecs< T, A > acc_vecs( const A* acc, const StencilArgs& a )
+{
+   AccVecs< T, A > v{};
+   v.acc[0] = acc;
+   v.src[0] = (const T*) a.src;
+   v.v1[0]  = (const T*) a.v1;
+   v.v2[0]  = (T*) a.v2;
+   v.dst[0] = (T*) a.dst;
+   return v;
 }
 
 // ---------------------------------------------------------------------------------------------
 // Assembled stencils (P1 operators with stored matrices): A src at cell-local (x, y, z) of a cell is
 // sum_d S_d(slot) src(x + dir_d), S_d the sum of the element-matrix entries of the cell's micro-cells
 // that couple the point with its neighbour in direction d (the same sum the elementwise apply forms,
-// P1ElementwiseOperator.cpp:169-260, taken once at setup instead of every apply).  One read of 15
-// weights per point replaces the 6 micro-cells x 10 entries an elementwise sweep reads.
+// P1ElementwiseOperator.cpp:169-260, taken once at setup instead of every apply).  The matrices are
+// symmetric, so only the centre and one direction of each opposite pair are kept, eight values per slot
+// (kVarDirs lists opposite directions next to each other: 2k - 1 is minus 2k); the other seven are the
+// neighbours' values for the direction back.
+//
+// One thread per cell-array slot, so warps are full whatever the length of the rows (a warp per row left
+// two thirds of its lanes idle at 32 points per edge).  Bound by the weights: 64 bytes per slot from
+// memory in FP64, the other 56 from cache.  Inner points finish here, points on the cell's boundary leave
+// their partial sums in acc for the owners (a gather of their weights by the owners took as long as the
+// whole interior).  V(3,3) Chebyshev(3) cycle on a shell of 240 cells, levels 0-5, FP64: 8.59 ms with a warp
+// per row, 15 stored weights and gathering owners, 3.62 ms so.
 // ---------------------------------------------------------------------------------------------
-template < typename T, typename A, bool INTERIOR >
-__device__ __forceinline__ A var_apply( const A* __restrict__ S, int64_t ssize, const T* __restrict__ src, int64_t base, int n, int x,
-                                        int y, int z )
+template < int D >
+struct VarDir {
+   static constexpr int dirs[15][3] = { { 0, 0, 0 },  { -1, 0, 0 }, { 1, 0, 0 },  { 0, -1, 0 }, { 0, 1, 0 },
+                                        { 0, 0, -1 }, { 0, 0, 1 },  { -1, 1, 0 }, { 1, -1, 0 }, { -1, 0, 1 },
+                                        { 1, 0, -1 }, { 0, -1, 1 }, { 0, 1, -1 }, { 1, -1, 1 }, { -1, 1, -1 } };
+   static constexpr int x = dirs[D][0], y = dirs[D][1], z = dirs[D][2];
+};
+
+template < int D, typename T, typename A >
+__device__ __forceinline__ void var_term( const A* S, int64_t ssize, const T* src, int n, int x, int y, int z, bool inner, A ( &s )[3] )
 {
-   const int64_t slot = base + cidx( n, x, y, z );
-   A             acc  = A( 0 );
-#pragma unroll
-   for ( int d = 0; d < 15; ++d )
-   {
-      const int dx = c_var_dir[d][0], dy = c_var_dir[d][1], dz = c_var_dir[d][2];
-      const int xx = x + dx, yy = y + dy, zz = z + dz;
-      if ( !INTERIOR && ( xx < 0 || yy < 0 || zz < 0 || xx + yy + zz > n ) ) continue;
-      acc += S[d * ssize + slot] * A( ld_any( src + base + cidx( n, xx, yy, zz ) ) );
-   }
-   return acc;
+   constexpr int dx = VarDir< D >::x, dy = VarDir< D >::y, dz = VarDir< D >::z;
+   if ( !inner && ( x + dx < 0 || y + dy < 0 || z + dz < 0 || x + y + z + ( dx + dy + dz ) > n ) ) return;
+   const int o = row_shift< dy, dz >( n, y, z ) + dx;
+   const A   w = ( D & 1 ) ? __ldg( S + ( ( D + 1 ) / 2 ) * ssize + o ) : __ldg( S + ( D / 2 ) * ssize );
+   s[D % 3] += w * A( ld_any( src + o ) );
+}
+
+template < typename T, typename A, int... D >
+__device__ __forceinline__ A var_sum( const A* S, int64_t ssize, const T* src, int n, int x, int y, int z, bool inner,
+                                      std::integer_sequence< int, D... > )
+{
+   A s[3] = { A( 0 ), A( 0 ), A( 0 ) };
+   ( var_term< D, T, A >( S, ssize, src, n, x, y, z, inner, s ), ... );
+   return ( s[0] + s[1] ) + s[2];
 }
 
 template < typename T, typename A, int OP >
-__global__ void __launch_bounds__( 256 ) k_var_cell( int n, int nrows, const int2* __restrict__ rows, const int64_t* __restrict__ cell_off,
-                                                      const uint8_t* __restrict__ cell_bc, uint32_t flag, const A* __restrict__ S,
-                                                      int64_t ssize, const A* __restrict__ invd, const T* src, const T* v1, T* v2, T* dst,
-                                                      A a0, A a1 )
+__global__ void __launch_bounds__( 256 ) k_var_sweep( int n, int nC, int np, int cell_stride, const ushort4* __restrict__ pts,
+                                                       const int64_t* __restrict__ cell_off, const uint8_t* __restrict__ cell_bc, uint32_t flag,
+                                                       const A* __restrict__ S, int64_t ssize, const A* __restrict__ invd,
+                                                       A* __restrict__ acc, const T* src, const T* v1, T* v2, T* dst, A a0, A a1 )
 {
-   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int r    = blockIdx.x * 8 + warp;
-   const int c    = blockIdx.y;
-   if ( r >= nrows || !( cell_bc[c] & flag ) ) return;
-   const int2    yz   = rows[r];
-   const int64_t cb   = cell_off[c];
-   const int64_t base = cb + cidx( n, 0, yz.x, yz.y );
-   for ( int x = 1 + lane; x <= n - 1 - yz.x - yz.y; x += 32 )
+   // threads over the slots of all macro-cells in storage order
+   const int64_t g = int64_t( blockIdx.x ) * 256 + threadIdx.x;
+   if ( g >= int64_t( nC ) * cell_stride ) return;
+   const int c = g < 0x7fffffff ? int( unsigned( g ) / unsigned( cell_stride ) ) : int( g / cell_stride );
+   const int k = int( g - int64_t( c ) * cell_stride );
+   if ( k >= np ) return;  // padding
+   const ushort4 pt    = pts[k];
+   const int     x = pt.x, y = pt.y, z = pt.z;
+   const bool    inner = x > 0 && y > 0 && z > 0 && x + y + z < n;
+   if ( inner && !( cell_bc[c] & flag ) ) return;
+   const int64_t i = cell_off[c] + k;
+   const A       s = var_sum< T, A >( S + i, ssize, src + i, n, x, y, z, inner, std::make_integer_sequence< int, 15 >() );
+   if ( !inner )
    {
-      const int64_t i = base + x;
-      A             second;
-      const A       s   = var_apply< T, A, true >( S, ssize, src, cb, n, x, yz.x, yz.y );
-      const A       val = epilogue_value< T, A, OP >( i, s, invd[i], src, v1, v2, a0, a1, &second );
-      if constexpr ( OP == OP_CHEBL ) st_any( v2 + i, val );
-      else if constexpr ( OP == OP_APPLY_ADD ) st_any( dst + i, A( ld_any( dst + i ) ) + val );
-      else
-      {
-         st_any( dst + i, val );
-         if constexpr ( OP == OP_CHEBI ) st_any( v2 + i, second );
-      }
-   }
-}
-
-template < typename T, typename A, int OP >
-__global__ void __launch_bounds__( 256 ) k_var_bnd( int n, int ntasks, const int4* __restrict__ tasks, const int64_t* __restrict__ off,
-                                                     const int64_t* __restrict__ cell_off, const int8_t* __restrict__ bkind,
-                                                     const uint8_t* __restrict__ bc, const int* __restrict__ inc_begin,
-                                                     const Incidence* __restrict__ inc, uint32_t flag, int copy_unflagged,
-                                                     const A* __restrict__ S, int64_t ssize, const A* __restrict__ invd, const T* src,
-                                                     const T* v1, T* v2, T* dst, A a0, A a1 )
-{
-   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-   if ( t >= ntasks ) return;
-   const int4    tk    = tasks[t];
-   const int     b     = tk.x;
-   const int     k     = bkind[b];
-   const int64_t owner = off[b] + ( k == 0 ? 0 : ( k == 1 ? int64_t( tk.y ) : fidx( n, tk.y, tk.z ) ) );
-   if ( !( bc[b] & flag ) )
-   {
-      if ( !copy_unflagged ) return;
-      if constexpr ( OP == OP_JAC || OP == OP_CHEB0 )
-         wt_store< T, A >( n, tk, owner, inc_begin, inc, cell_off, dst, A( ld_any( src + owner ) ) );
-      else if constexpr ( OP == OP_CHEBI ) wt_store< T, A >( n, tk, owner, inc_begin, inc, cell_off, dst, A( ld_any( v2 + owner ) ) );
+      acc[i] = s;
       return;
    }
-   const A s = inc_sum< A, 2 >( __ldg( inc_begin + b ), __ldg( inc_begin + b + 1 ), inc, [&]( const Incidence& I ) {
-      const int x = n * I.o[0] + tk.y * I.e1[0] + tk.z * I.e2[0];
-      const int y = n * I.o[1] + tk.y * I.e1[1] + tk.z * I.e2[1];
-      const int z = n * I.o[2] + tk.y * I.e1[2] + tk.z * I.e2[2];
-      return var_apply< T, A, false >( S, ssize, src, __ldg( cell_off + I.cell ), n, x, y, z );
-   } );
    A       second;
-   const A val = epilogue_value< T, A, OP >( owner, s, invd[owner], src, v1, v2, a0, a1, &second );
-   if constexpr ( OP == OP_CHEBL ) wt_store< T, A >( n, tk, owner, inc_begin, inc, cell_off, v2, val );
-   else if constexpr ( OP == OP_APPLY_ADD )
-      wt_store< T, A >( n, tk, owner, inc_begin, inc, cell_off, dst, A( ld_any( dst + owner ) ) + val );
+   const A val = epilogue_value< T, A, OP >( i, s, invd[i], src, v1, v2, a0, a1, &second );
+   if constexpr ( OP == OP_CHEBL ) st_any( v2 + i, val );
+   else if constexpr ( OP == OP_APPLY_ADD ) st_any( dst + i, A( ld_any( dst + i ) ) + val );
    else
    {
-      wt_store< T, A >( n, tk, owner, inc_begin, inc, cell_off, dst, val );
-      if constexpr ( OP == OP_CHEBI ) wt_store< T, A >( n, tk, owner, inc_begin, inc, cell_off, v2, second );
+      st_any( dst + i, val );
+      if constexpr ( OP == OP_CHEBI ) st_any( v2 + i, second );
    }
 }
 
@@ -1591,9 +1610,7 @@ static void ensure_var_tables()
       for ( int t = 0; t < 6; ++t )
          for ( int i = 0; i < 4; ++i )
             for ( int d = 0; d < 3; ++d ) off[t][i][d] = micro_vertex( t, i, d );
-      int8_t dir[6][4][4], vd[15][3];
-      for ( int d = 0; d < 15; ++d )
-         for ( int k = 0; k < 3; ++k ) vd[d][k] = int8_t( kVarDirs[d][k] );
+      int8_t dir[6][4][4];
       for ( int t = 0; t < 6; ++t )
          for ( int i = 0; i < 4; ++i )
             for ( int j = 0; j < 4; ++j )
@@ -1607,7 +1624,6 @@ static void ensure_var_tables()
                dir[t][i][j] = int8_t( found );
             }
       check_cuda( cudaMemcpyToSymbol( c_mc_dir, dir, sizeof( dir ) ), "upload stencil directions" );
-      check_cuda( cudaMemcpyToSymbol( c_var_dir, vd, sizeof( vd ) ), "upload stencil directions" );
    } );
 }
 
@@ -1753,6 +1769,19 @@ void set_p2_nodal_coefficient( Context* ctx, Operator* op, int Ls, const double*
    }
 }
 
+// coordinates of a macro-cell's points in storage order (shared by all cells of the level)
+static void ensure_cell_points( ElemLevel& e, const P1Level& P )
+{
+   if ( e.d_pts ) return;
+   std::vector< ushort4 > pts;
+   pts.reserve( size_t( tet_size( P.n + 1 ) ) );
+   for ( int z = 0; z <= P.n; ++z )
+      for ( int y = 0; y + z <= P.n; ++y )
+         for ( int x = 0; x + y + z <= P.n; ++x ) pts.push_back( make_ushort4( (unsigned short) x, (unsigned short) y, (unsigned short) z, 0 ) );
+   check_cuda( cudaMalloc( &e.d_pts, pts.size() * sizeof( ushort4 ) ), "cudaMalloc(cell points)" );
+   check_cuda( cudaMemcpy( e.d_pts, pts.data(), pts.size() * sizeof( ushort4 ), cudaMemcpyHostToDevice ), "upload cell points" );
+}
+
 template < typename T, typename A >
 static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
 {
@@ -1767,7 +1796,8 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
    {
       // P1: the stored matrices are kept assembled, summed in double once and rounded for float
       ensure_var_tables();
-      const int64_t cnt = int64_t( 15 ) * P.size;
+      const int64_t cnt = int64_t( 8 ) * P.size;
+      ensure_cell_points( e, P );
       if ( !e.d_S[0] )
       {
          check_cuda( cudaMalloc( &e.d_S[0], cnt * sizeof( double ) ), "cudaMalloc(assembled stencils)" );
@@ -1830,7 +1860,7 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
       k_cell_invert< A ><<< grid, 256, 0, ctx->stream >>>( P.n, nrows, P.d_rows, P.d_off + P.nB, acc, invd );
    }
    if ( !P.tasks.empty() )
-      launch_bnd_acc< T, A, OP_APPLY >( ctx->stream, P, kAll, 0, acc, nullptr, invd, nullptr, nullptr, nullptr, nullptr, A( 0 ), A( 0 ) );
+      launch_bnd_acc< T, A, OP_APPLY >( ctx, ctx->stream, P, kAll, 0, acc_vecs< T, A >( acc, {} ), 1, nullptr, invd, A( 0 ), A( 0 ) );
    check_cuda( cudaGetLastError(), "diagonal launch" );
 }
 
@@ -1845,36 +1875,16 @@ template < typename T, typename A, int OP >
 static void run_var( Context* ctx, Mesh* m, Operator* op, int L, int dtype, const StencilArgs& a )
 {
    P1Level& P = m->level( L );
-   const A* S   = assembled_stencils< A >( op, L );
-   const A* inv = reinterpret_cast< const A* >( op->el[L].d_invd[dtype] );
-   struct Join
-   {
-      Context* c;
-      ~Join()
-      {
-         cudaEventRecord( c->ev_join, c->aux );
-         cudaStreamWaitEvent( c->stream, c->ev_join, 0 );
-      }
-   };
-   check_cuda( cudaEventRecord( ctx->ev_fork, ctx->stream ), "fork" );
-   check_cuda( cudaStreamWaitEvent( ctx->aux, ctx->ev_fork, 0 ), "fork" );
-   Join      j{ ctx };
-   const int nrows = int( P.rows.size() );
-   if ( nrows > 0 )
-   {
-      dim3 grid( ( nrows + 7 ) / 8, m->topo.nC );
-      k_var_cell< T, A, OP ><<< grid, 256, 0, ctx->stream >>>( P.n, nrows, P.d_rows, P.d_off + P.nB, P.d_bc + P.nB, a.flag, S, P.size, inv,
-                                                                (const T*) a.src, (const T*) a.v1, (T*) a.v2, (T*) a.dst, A( a.a0 ),
-                                                                A( a.a1 ) );
-      ++ctx->launches;
-   }
-   if ( !P.tasks.empty() )
-   {
-      k_var_bnd< T, A, OP ><<< ( int( P.tasks.size() ) + 255 ) / 256, 256, 0, ctx->aux >>>(
-          P.n, int( P.tasks.size() ), P.d_tasks, P.d_off, P.d_off + P.nB, P.d_bkind, P.d_bc, P.d_inc_begin, P.d_inc, a.flag,
-          a.copy_unflagged, S, P.size, inv, (const T*) a.src, (const T*) a.v1, (T*) a.v2, (T*) a.dst, A( a.a0 ), A( a.a1 ) );
-      ++ctx->launches;
-   }
+   ElemLevel& e  = op->el[L];
+   A*         acc = acc_buffer< A >( op, L, P.size );
+   const A*   S   = assembled_stencils< A >( op, L );
+   const A*   inv = reinterpret_cast< const A* >( e.d_invd[dtype] );
+   const int  np = int( tet_size( P.n + 1 ) ), stride = ( np + 31 ) / 32 * 32, nC = m->topo.nC;
+   k_var_sweep< T, A, OP ><<< unsigned( ( int64_t( nC ) * stride + 255 ) / 256 ), 256, 0, ctx->stream >>>(
+       P.n, nC, np, stride, reinterpret_cast< const ushort4* >( e.d_pts ), P.d_off + P.nB, P.d_bc + P.nB, a.flag, S, P.size, inv, acc,
+       (const T*) a.src, (const T*) a.v1, (T*) a.v2, (T*) a.dst, A( a.a0 ), A( a.a1 ) );
+   ++ctx->launches;
+   launch_bnd_acc< T, A, OP >( ctx, ctx->stream, P, a.flag, a.copy_unflagged, acc_vecs< T, A >( acc, a ), 1, inv, nullptr, A( a.a0 ), A( a.a1 ) );
    check_cuda( cudaGetLastError(), "assembled stencil launch" );
 }
 
@@ -1888,9 +1898,8 @@ static void run_elem( Context* ctx, Mesh* m, Operator* op, int L, int dtype, con
    if ( const A* S = assembled_stencils< A >( op, L ) )
    {
       launch_p2_stored_sweep( ctx, P, dtype, *op->el[L].p2s, S, inv, acc, &a, 1 );
-      launch_bnd_acc< T, A, OP >( ctx->stream, P, a.flag, a.copy_unflagged, acc, inv, nullptr, (const T*) a.src, (const T*) a.v1,
-                                  (T*) a.v2, (T*) a.dst, A( a.a0 ), A( a.a1 ) );
-      if ( !P.tasks.empty() ) ++ctx->launches;
+      launch_bnd_acc< T, A, OP >( ctx, ctx->stream, P, a.flag, a.copy_unflagged, acc_vecs< T, A >( acc, a ), 1, inv, nullptr, A( a.a0 ),
+                                  A( a.a1 ) );
       check_cuda( cudaGetLastError(), "stored P2 combine launch" );
       return;
    }
@@ -1912,17 +1921,12 @@ static void run_elem( Context* ctx, Mesh* m, Operator* op, int L, int dtype, con
       if ( nrows > 0 )
       {
          dim3 grid( ( nrows + 7 ) / 8, m->topo.nC );
-         k_cell_acc< T, A, OP ><<< grid, 256, 0, ctx->stream >>>( P.n, nrows, P.d_rows, P.d_off + P.nB, P.d_bc + P.nB, a.flag, acc, inv,
-                                                                   (const T*) a.src, (const T*) a.v1, (T*) a.v2, (T*) a.dst, A( a.a0 ),
-                                                                   A( a.a1 ) );
+         k_cell_acc< T, A, OP ><<< grid, 256, 0, ctx->stream >>>( P.n, nrows, P.d_rows, P.d_off + P.nB, P.d_bc + P.nB, a.flag,
+                                                                   acc_vecs< T, A >( acc, a ), inv, A( a.a0 ), A( a.a1 ) );
          ++ctx->launches;
       }
-      if ( !P.tasks.empty() )
-      {
-         launch_bnd_acc< T, A, OP >( ctx->aux, P, a.flag, a.copy_unflagged, acc, inv, nullptr, (const T*) a.src, (const T*) a.v1,
-                                     (T*) a.v2, (T*) a.dst, A( a.a0 ), A( a.a1 ) );
-         ++ctx->launches;
-      }
+      launch_bnd_acc< T, A, OP >( ctx, ctx->aux, P, a.flag, a.copy_unflagged, acc_vecs< T, A >( acc, a ), 1, inv, nullptr, A( a.a0 ),
+                                  A( a.a1 ) );
    }
    check_cuda( cudaGetLastError(), "elementwise combine launch" );
 }
@@ -1944,11 +1948,11 @@ static void dispatch_elem( Context* ctx, Mesh* m, Operator* op, int L, int dtype
    }
 }
 
-// owner/copy combine of an accumulation array (cell-array slots) into dst with the apply epilogue:
-// cell interiors on the main stream, face/edge/vertex owners (sum of their cell copies, written
+// owner/copy combine of the accumulation arrays of ncomp components (cell-array slots) with the epilogue
+// of OP: cell interiors on the main stream, face/edge/vertex owners (sum of their cell copies, written
 // through) on the second stream
 template < typename T, typename A, int OP >
-static void combine_acc( Context* ctx, Mesh* m, int L, const A* acc, uint32_t flag, T* dst )
+static void combine_acc( Context* ctx, Mesh* m, int L, const AccVecs< T, A >& vec, int ncomp, uint32_t flag, const A* invd = nullptr, A a0 = A( 0 ) )
 {
    P1Level& P = m->level( L );
    struct Join
@@ -1966,22 +1970,17 @@ static void combine_acc( Context* ctx, Mesh* m, int L, const A* acc, uint32_t fl
    const int nrows = int( P.rows.size() );
    if ( nrows > 0 )
    {
-      dim3 grid( ( nrows + 7 ) / 8, m->topo.nC );
-      k_cell_acc< T, A, OP ><<< grid, 256, 0, ctx->stream >>>( P.n, nrows, P.d_rows, P.d_off + P.nB, P.d_bc + P.nB, flag, acc, nullptr,
-                                                                nullptr, nullptr, nullptr, dst, A( 0 ), A( 0 ) );
+      dim3 grid( ( nrows + 7 ) / 8, m->topo.nC, ncomp );
+      k_cell_acc< T, A, OP ><<< grid, 256, 0, ctx->stream >>>( P.n, nrows, P.d_rows, P.d_off + P.nB, P.d_bc + P.nB, flag, vec, invd, a0, A( 0 ) );
       ++ctx->launches;
    }
-   if ( !P.tasks.empty() )
-   {
-      launch_bnd_acc< T, A, OP >( ctx->aux, P, flag, 0, acc, nullptr, nullptr, nullptr, nullptr, nullptr, dst, A( 0 ), A( 0 ) );
-      ++ctx->launches;
-   }
+   launch_bnd_acc< T, A, OP >( ctx, ctx->aux, P, flag, 0, vec, ncomp, invd, nullptr, a0, A( 0 ) );
    check_cuda( cudaGetLastError(), "combine launch" );
 }
 
 template < typename T, typename A >
 static void run_stokes( Context* ctx, Operator* op, int Lp, int divt, const void* const* u, const void* p, void* const* dst_u, void* dst_p,
-                        uint32_t flag, int add )
+                        uint32_t flag, int add, const StokesUpdate* up )
 {
    Mesh*      m  = op->mesh;
    const int  Ls = Lp + 1;
@@ -2027,22 +2026,43 @@ static void run_stokes( Context* ctx, Operator* op, int Lp, int divt, const void
       ++ctx->launches;
    }
    check_cuda( cudaGetLastError(), "Stokes pass launch" );
+   AccVecs< T, A > vec{};
    if ( divt )
+   {
       for ( int k = 0; k < 3; ++k )
       {
-         if ( add ) combine_acc< T, A, OP_APPLY_ADD >( ctx, m, Ls, acc_u + k * PU.size, flag, (T*) dst_u[k] );
-         else combine_acc< T, A, OP_APPLY >( ctx, m, Ls, acc_u + k * PU.size, flag, (T*) dst_u[k] );
+         vec.acc[k] = acc_u + k * PU.size;
+         vec.dst[k] = (T*) dst_u[k];
+         vec.v1[k]  = up ? (const T*) up->b[k] : nullptr;
       }
-   else if ( add ) combine_acc< T, A, OP_APPLY_ADD >( ctx, m, Lp, acc_p, flag, (T*) dst_p );
-   else combine_acc< T, A, OP_APPLY >( ctx, m, Lp, acc_p, flag, (T*) dst_p );
+      if ( up ) combine_acc< T, A, OP_RESID >( ctx, m, Ls, vec, 3, flag );
+      else if ( add ) combine_acc< T, A, OP_APPLY_ADD >( ctx, m, Ls, vec, 3, flag );
+      else combine_acc< T, A, OP_APPLY >( ctx, m, Ls, vec, 3, flag );
+      return;
+   }
+   vec.acc[0] = acc_p;
+   vec.dst[0] = (T*) dst_p;
+   if ( up )
+   {
+      if constexpr ( std::is_same< T, A >::value )
+      {
+         vec.src[0] = vec.dst[0];
+         vec.v1[0]  = (const T*) up->b[0];
+         combine_acc< T, A, OP_JAC >( ctx, m, Lp, vec, 1, flag, (const A*) up->sinv, A( up->omega ) );
+      }
+      else
+         throw std::invalid_argument( "the fused pressure update needs FP64 or FP32 storage" );
+   }
+   else if ( add ) combine_acc< T, A, OP_APPLY_ADD >( ctx, m, Lp, vec, 1, flag );
+   else combine_acc< T, A, OP_APPLY >( ctx, m, Lp, vec, 1, flag );
 }
 
 void launch_stokes_div( Context* ctx, Operator* op, int Lp, int dtype, int divt, const void* const* u, const void* p, void* const* dst_u,
-                        void* dst_p, uint32_t flag, int add )
+                        void* dst_p, uint32_t flag, int add, const StokesUpdate* up )
 {
-   if ( dtype == F64 ) run_stokes< double, double >( ctx, op, Lp, divt, u, p, dst_u, dst_p, flag, add );
-   else if ( dtype == F32 ) run_stokes< float, float >( ctx, op, Lp, divt, u, p, dst_u, dst_p, flag, add );
-   else run_stokes< __half, float >( ctx, op, Lp, divt, u, p, dst_u, dst_p, flag, add );
+   if ( dtype == F64 ) run_stokes< double, double >( ctx, op, Lp, divt, u, p, dst_u, dst_p, flag, add, up );
+   else if ( dtype == F32 ) run_stokes< float, float >( ctx, op, Lp, divt, u, p, dst_u, dst_p, flag, add, up );
+   else run_stokes< __half, float >( ctx, op, Lp, divt, u, p, dst_u, dst_p, flag, add, up );
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -2273,11 +2293,14 @@ static void run_visc( Context* ctx, Operator* op, int Lp, int mode, const void* 
    check_cuda( cudaGetLastError(), "viscous block pass launch" );
    if ( mode == 0 )
    {
+      AccVecs< T, A > vec{};
       for ( int k = 0; k < 3; ++k )
       {
-         if ( add ) combine_acc< T, A, OP_APPLY_ADD >( ctx, m, Ls, acc + k * PU.size, flag, (T*) dst[k] );
-         else combine_acc< T, A, OP_APPLY >( ctx, m, Ls, acc + k * PU.size, flag, (T*) dst[k] );
+         vec.acc[k] = acc + k * PU.size;
+         vec.dst[k] = (T*) dst[k];
       }
+      if ( add ) combine_acc< T, A, OP_APPLY_ADD >( ctx, m, Ls, vec, 3, flag );
+      else combine_acc< T, A, OP_APPLY >( ctx, m, Ls, vec, 3, flag );
       return;
    }
    // diagonal: owners sum their copies, then 1/diag on every owned node (dst: three A arrays)
@@ -2292,8 +2315,8 @@ static void run_visc( Context* ctx, Operator* op, int Lp, int mode, const void* 
          k_cell_invert< A ><<< grid, 256, 0, ctx->stream >>>( PU.n, nrows, PU.d_rows, PU.d_off + PU.nB, acc + k * PU.size, invd );
       }
       if ( !PU.tasks.empty() )
-         launch_bnd_acc< T, A, OP_APPLY >( ctx->stream, PU, kAll, 0, acc + k * PU.size, nullptr, invd, nullptr, nullptr, nullptr, nullptr,
-                                           A( 0 ), A( 0 ) );
+         launch_bnd_acc< T, A, OP_APPLY >( ctx, ctx->stream, PU, kAll, 0, acc_vecs< T, A >( acc + k * PU.size, {} ), 1, nullptr, invd, A( 0 ),
+                                           A( 0 ) );
    }
    check_cuda( cudaGetLastError(), "viscous block diagonal launch" );
 }
@@ -2304,6 +2327,49 @@ void launch_full_viscous( Context* ctx, Operator* op, int Lp, int dtype, int mod
    if ( dtype == F64 ) run_visc< double, double >( ctx, op, Lp, mode, u, dst, flag, add );
    else if ( dtype == F32 ) run_visc< float, float >( ctx, op, Lp, mode, u, dst, flag, add );
    else run_visc< __half, float >( ctx, op, Lp, mode, u, dst, flag, add );
+}
+
+template < typename T, typename A, int OP >
+static void run_stored3( Context* ctx, Mesh* m, Operator* op, int L, int dtype, const StencilArgs* a )
+{
+   P1Level&   P = m->level( L );
+   ElemLevel& e = op->el[L];
+   const A*   S = assembled_stencils< A >( op, L );
+   const A*   inv = reinterpret_cast< const A* >( e.d_invd[dtype] );
+   if ( !e.d_sacc ) check_cuda( cudaMalloc( &e.d_sacc, size_t( 3 * P.size ) * sizeof( double ) ), "cudaMalloc(component scratch)" );
+   A* acc = reinterpret_cast< A* >( e.d_sacc );
+   launch_p2_stored_sweep( ctx, P, dtype, *e.p2s, S, inv, acc, a, 3 );
+   AccVecs< T, A > vec{};
+   for ( int k = 0; k < 3; ++k )
+   {
+      const AccVecs< T, A > v = acc_vecs< T, A >( acc + k * P.size, a[k] );
+      vec.acc[k] = v.acc[0], vec.src[k] = v.src[0], vec.v1[k] = v.v1[0], vec.v2[k] = v.v2[0], vec.dst[k] = v.dst[0];
+   }
+   launch_bnd_acc< T, A, OP >( ctx, ctx->stream, P, a[0].flag, a[0].copy_unflagged, vec, 3, inv, nullptr, A( a[0].a0 ), A( a[0].a1 ) );
+   check_cuda( cudaGetLastError(), "stored P2 combine launch" );
+}
+
+template < typename T, typename A >
+static void dispatch_stored3( Context* ctx, Mesh* m, Operator* op, int L, int dtype, const StencilArgs* a )
+{
+   switch ( a[0].op )
+   {
+   case OP_CHEB0: run_stored3< T, A, OP_CHEB0 >( ctx, m, op, L, dtype, a ); break;
+   case OP_CHEBI: run_stored3< T, A, OP_CHEBI >( ctx, m, op, L, dtype, a ); break;
+   case OP_CHEBL: run_stored3< T, A, OP_CHEBL >( ctx, m, op, L, dtype, a ); break;
+   case OP_RESID: run_stored3< T, A, OP_RESID >( ctx, m, op, L, dtype, a ); break;
+   default: throw std::invalid_argument( "operation not provided for three components" );
+   }
+}
+
+bool launch_stored3( Context* ctx, Mesh* m, Operator* op, int L, int dtype, const StencilArgs* a )
+{
+   if ( !op->elementwise || op->order != 2 || !op->store_matrices ) return false;
+   ensure_elementwise_level( ctx, op, L, dtype );
+   if ( dtype == F64 ) dispatch_stored3< double, double >( ctx, m, op, L, dtype, a );
+   else if ( dtype == F32 ) dispatch_stored3< float, float >( ctx, m, op, L, dtype, a );
+   else dispatch_stored3< __half, float >( ctx, m, op, L, dtype, a );
+   return true;
 }
 
 void launch_elementwise( Context* ctx, Mesh* m, Operator* op, int L, int dtype, const StencilArgs& a )

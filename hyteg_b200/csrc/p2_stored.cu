@@ -92,20 +92,6 @@ struct StoredVecs {
    T*       dst[NV];
 };
 
-// start of row (y + dy, z + dz) of a cell array minus the start of row (y, z)
-template < int DY, int DZ >
-__device__ __forceinline__ int row_shift( int n, int y, int z )
-{
-   const int q = n + 1 - z;  // points in the first row of slice z
-   int       s = 0;
-   if constexpr ( DZ >= 1 ) s += q * ( q + 1 ) / 2;
-   if constexpr ( DZ >= 2 ) s += ( q - 1 ) * q / 2;
-   if constexpr ( DZ <= -1 ) s -= ( q + 1 ) * ( q + 2 ) / 2;
-   if constexpr ( DZ <= -2 ) s -= ( q + 2 ) * ( q + 3 ) / 2;
-   const int w = y + DY;
-   return s + ( w * ( q - DZ ) - w * ( w - 1 ) / 2 ) - ( y * q - y * ( y - 1 ) / 2 );
-}
-
 template < int P, bool BND, int D, typename T, typename A, int NV >
 __device__ __forceinline__ void stored_term( const T* const ( &at )[NV], const A* W, int64_t step, int n, int x, int y, int z, A ( &s )[2][NV] )
 {
@@ -238,10 +224,15 @@ void run_sweep( Context* ctx, P1Level& P, const P2StoredView& v, const void* S, 
 void launch_p2_stored_sweep( Context* ctx, P1Level& P, int dtype, const P2StoredView& v, const void* S, const void* invd, void* acc,
                              const StencilArgs* a, int ncomp )
 {
-   if ( ncomp != 1 ) throw std::invalid_argument( "stored P2 sweep: one vector" );
-   if ( dtype == F64 ) run_sweep< double, double, 1 >( ctx, P, v, S, invd, acc, a );
-   else if ( dtype == F32 ) run_sweep< float, float, 1 >( ctx, P, v, S, invd, acc, a );
-   else run_sweep< __half, float, 1 >( ctx, P, v, S, invd, acc, a );
+   auto run = [&]( auto nv ) {
+      constexpr int NV = decltype( nv )::value;
+      if ( dtype == F64 ) run_sweep< double, double, NV >( ctx, P, v, S, invd, acc, a );
+      else if ( dtype == F32 ) run_sweep< float, float, NV >( ctx, P, v, S, invd, acc, a );
+      else run_sweep< __half, float, NV >( ctx, P, v, S, invd, acc, a );
+   };
+   if ( ncomp == 1 ) run( std::integral_constant< int, 1 >{} );
+   else if ( ncomp == 3 ) run( std::integral_constant< int, 3 >{} );
+   else throw std::invalid_argument( "stored P2 sweep: one or three vectors" );
 }
 
 }  // namespace hyb

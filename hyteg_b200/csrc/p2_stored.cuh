@@ -92,6 +92,20 @@ __device__ __forceinline__ int64_t p2_weight_at( const P2StoredView& v, int c, i
    return v.wbase[s] + int64_t( c ) * v.np[s] + v.rank[cidx( v.n, x, y, z )];
 }
 
+// start of row (y + dy, z + dz) of a cell array minus the start of row (y, z)
+template < int DY, int DZ >
+__device__ __forceinline__ int row_shift( int n, int y, int z )
+{
+   const int q = n + 1 - z;  // points in the first row of slice z
+   int       s = 0;
+   if constexpr ( DZ >= 1 ) s += q * ( q + 1 ) / 2;
+   if constexpr ( DZ >= 2 ) s += ( q - 1 ) * q / 2;
+   if constexpr ( DZ <= -1 ) s -= ( q + 1 ) * ( q + 2 ) / 2;
+   if constexpr ( DZ <= -2 ) s -= ( q + 2 ) * ( q + 3 ) / 2;
+   const int w = y + DY;
+   return s + ( w * ( q - DZ ) - w * ( w - 1 ) / 2 ) - ( y * q - y * ( y - 1 ) / 2 );
+}
+
 // tables of a storage level with n nodes per macro-edge; returns the number of weights
 int64_t build_p2_stored( P2StoredView& v, int n, int nC, std::vector< ushort4 >& pts, std::vector< int >& rank );
 // entry of node j in node i's stencil, every micro-cell type: ent[(10 ty + i) 10 + j]

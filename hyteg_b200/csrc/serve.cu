@@ -203,7 +203,7 @@ void make_fn( hyb_ctx* ctx, hyb_mesh* mesh, int kind, int lo, int hi, hyb_fn** f
 
 // bytes a slot holds: x, b (all levels), tmp and the solver's temporaries (about six more vectors
 // per level), plus the elementwise scratch
-// (plus, for div-k-grad, the stored matrices, kept as assembled stencils: 15 values per DoF slot and
+// (plus, for div-k-grad, the stored matrices, kept as assembled stencils: 8 values per DoF slot and
 // level, in FP64 and for mixed slots also in FP32)
 double slot_bytes( ServeKey k )
 {
@@ -215,7 +215,7 @@ double slot_bytes( ServeKey k )
       int64_t n = 0;
       hyb_layout_packed_size( k.mesh, L + sh, &n );
       total += n;
-      if ( k.kind == HYB_P1_ELEM_DIVKGRAD ) mats += double( n ) * 15.0;
+      if ( k.kind == HYB_P1_ELEM_DIVKGRAD ) mats += double( n ) * 8.0;
       // 28.75 values per node on average (class stencils), a little more with the nodes that several
       // macro-cells hold
       if ( k.kind == HYB_P2_ELEM_DIVKGRAD ) mats += double( n ) * 32.0;

@@ -768,6 +768,7 @@ Operator::~Operator()
       for ( void* p : kv.second.d_invd ) cudaFree( p );
       for ( void* p : kv.second.d_S ) cudaFree( p );
       cudaFree( kv.second.d_p2s_pts );
+      cudaFree( kv.second.d_pts );
       cudaFree( kv.second.d_p2s_rank );
       cudaFree( kv.second.d_sacc );
       cudaFree( kv.second.d_kn );

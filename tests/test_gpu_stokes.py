@@ -259,3 +259,25 @@ def test_stokes_lumped_mass_scaling_uzawa_step_and_relaxation_estimate(ctx):
         bu[k].upload(L2, bu0[k])
     hist = st2.solve(u, p, bu, bp, L2, 4)
     assert (hist[1:] / hist[:-1]).max() < 0.5, hist
+
+
+@pytest.mark.parametrize("level", [0, 2])
+def test_uzawa_step_three_components_at_once(ctx, level):
+    """The velocity components smoothed in one sweep of the stored stencils: one Uzawa step equals the step
+    of a rotated right-hand side with the components exchanged, to rounding (1e-12 of the largest value)."""
+    coords, tets = M.cube_6()
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    st = H.StokesUzawaMultigrid(ctx, pm, 0, 2)
+    st.set_velocity_radii([3.0, 3.0, 3.0])
+    res = []
+    for order in ((0, 1, 2), (2, 0, 1)):
+        u = [H.P2Function("u%d" % k, pm, 0, 2, ctx) for k in range(3)]
+        b = [H.P2Function("b%d" % k, pm, 0, 2, ctx) for k in range(3)]
+        p, bp = H.P1Function("p", pm, 0, 2, ctx), H.P1Function("bp", pm, 0, 2, ctx)
+        for k, src in enumerate(order):
+            b[k].fill_random(level, 11 + src)
+        st.uzawa_smooth(u, p, b, bp, level)
+        res.append([u[order.index(k)].download(level) for k in range(3)])
+    scale = max(np.abs(v).max() for v in res[0])
+    for a, c in zip(*res):
+        assert np.abs(a - c).max() <= 1e-12 * max(scale, 1e-300)
