@@ -61,8 +61,13 @@ struct LevelView
    int              ntasks;
    const int4*      tasks;
    const int4*      btasks;      // the same tasks grouped by their primitive's boundary type
-   const FaceRec*   frec;        // per grouped task: its two-cell face record (cell0 < 0: none)
-   int              bcount[4];   // tasks per group: Inner, Dirichlet, Neumann, Freeslip
+   const FaceRec*   frec;        // face records of all groups, in group order
+   const LowRec*    lrec;        // vertex and edge records of all groups, in group order
+   const IncRec*    irec;        // their incidences
+   int              nlow[4];     // vertex and edge tasks per group: Inner, Dirichlet, Neumann, Freeslip
+   int              nface[4];    // face tasks per group
+   int              nipts;       // interior points per macro-cell and their coordinates
+   const ushort4*   ipts;
    const int64_t*   off;       // all primitives
    const int64_t*   cell_off;  // off + nB
    const int*       inc_begin;
@@ -71,8 +76,6 @@ struct LevelView
    const uint8_t*   cell_bc;  // bc + nB
    const int8_t*    bkind;
    const float*     ncell_cls;
-   int              nmarch;
-   const int4*      march;
    int              nzblocks;  // blocks of the rolled sweep and their units (zunits/zcell from zbegin[b])
    const int4*      zunits;
    const int*       zcell;
@@ -103,7 +106,11 @@ static inline LevelView make_view( Mesh* m, int L )
    v.tasks     = P.d_tasks;
    v.btasks    = P.d_btasks;
    v.frec      = P.d_frec;
-   for ( int g = 0; g < 4; ++g ) v.bcount[g] = P.bcount[g];
+   v.lrec      = P.d_lrec;
+   v.irec      = P.d_irec;
+   for ( int g = 0; g < 4; ++g ) v.nlow[g] = P.nlow[g], v.nface[g] = P.nface[g];
+   v.nipts = P.nipts;
+   v.ipts  = reinterpret_cast< const ushort4* >( P.d_ipts );
    v.off       = P.d_off;
    v.cell_off  = P.d_off + P.nB;
    v.inc_begin = P.d_inc_begin;
@@ -112,8 +119,6 @@ static inline LevelView make_view( Mesh* m, int L )
    v.cell_bc   = P.d_bc + P.nB;
    v.bkind     = P.d_bkind;
    v.ncell_cls = P.d_ncell_cls;
-   v.nmarch     = int( P.march.size() );
-   v.march      = P.d_march;
    v.nzblocks = int( P.zbegin.size() ) - 1;
    v.zunits   = P.d_zunits;
    v.zcell    = P.d_zcell;
@@ -143,13 +148,14 @@ static inline TaskSegments task_segments( const LevelView& v, uint32_t flag, int
    int                   k = 0, at = 0;
    for ( int g = 0; g < 4; ++g )
    {
-      if ( v.bcount[g] > 0 && ( all || ( flag & type_bit[g] ) ) )
+      const int n = v.nlow[g] + v.nface[g];
+      if ( n > 0 && ( all || ( flag & type_bit[g] ) ) )
       {
          s.start[k] = at;
-         s.count[k] = v.bcount[g];
+         s.count[k] = n;
          ++k;
       }
-      at += v.bcount[g];
+      at += n;
    }
    return s;
 }
@@ -261,6 +267,29 @@ __host__ __device__ constexpr bool sweep_aux()
 {
    return OP == OP_APPLY_ADD || OP == OP_RESID || OP == OP_JAC || OP == OP_CHEB0 || OP == OP_CHEBI || OP == OP_CHEBL;
 }
+
+// start of row (y + dy, z + dz) of a cell array minus the start of row (y, z)
+template < int DY, int DZ >
+__device__ __forceinline__ int row_shift( int n, int y, int z )
+{
+   const int q = n + 1 - z;  // points in the first row of slice z
+   int       s = 0;
+   if constexpr ( DZ >= 1 ) s += q * ( q + 1 ) / 2;
+   if constexpr ( DZ >= 2 ) s += ( q - 1 ) * q / 2;
+   if constexpr ( DZ <= -1 ) s -= ( q + 1 ) * ( q + 2 ) / 2;
+   if constexpr ( DZ <= -2 ) s -= ( q + 2 ) * ( q + 3 ) / 2;
+   const int w = y + DY;
+   return s + ( w * ( q - DZ ) - w * ( w - 1 ) / 2 ) - ( y * q - y * ( y - 1 ) / 2 );
+}
+
+// direction D of the 15-point stencil (order of kDirs)
+template < int D >
+struct StencilDir {
+   static constexpr int dirs[15][3] = { { 0, 0, 0 },  { -1, 0, 0 }, { 1, 0, 0 },  { 0, -1, 0 }, { 0, 1, 0 },
+                                        { 0, 0, -1 }, { 0, 0, 1 },  { -1, 1, 0 }, { 1, -1, 0 }, { -1, 0, 1 },
+                                        { 1, 0, -1 }, { 0, -1, 1 }, { 0, 1, -1 }, { 1, -1, 1 }, { -1, 1, -1 } };
+   static constexpr int x = dirs[D][0], y = dirs[D][1], z = dirs[D][2];
+};
 
 // offset of slice z+1 minus offset of slice z in a macro-cell array (tri(n+1-z) points in slice z)
 __device__ __forceinline__ int64_t slice_step( int n, int z ) { return int64_t( n + 1 - z ) * ( n + 2 - z ) / 2; }

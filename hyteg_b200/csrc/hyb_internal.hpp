@@ -75,10 +75,11 @@ constexpr int kP2cCellStride = kP2cInterior + ( kNumClasses - 1 ) * kP2cEntries;
 extern const uint16_t kClassDirMask[kNumClasses];
 int class_of_point(int n, int x, int y, int z);  // host version
 
-// A face-interior boundary task between two macro-cells, resolved once per level for the boundary
-// stencil kernel: the owner slot, the slots of the owner's copies in the two cell arrays (the centres
+// Boundary tasks (owned face, edge and vertex DoFs), resolved once per level for the kernels that run
+// over them.
+// A face-interior DoF: the owner slot, the slots of its copies in the one or two cell arrays (the centres
 // of the cells' class stencils), their rows and slices, cells and position classes, the face's
-// boundary-primitive index and type.  cell0 < 0 marks any other task.
+// boundary-primitive index and type.  cell1 < 0: the face has one cell.
 struct FaceRec {
    int64_t owner;
    int64_t c0, c1;
@@ -90,6 +91,20 @@ struct FaceRec {
    uint8_t pad;
 };
 static_assert( sizeof( FaceRec ) == 48, "face record layout" );
+
+// An edge or vertex DoF: owner slot, its incidences begin .. begin + count - 1, boundary primitive and type.
+struct LowRec {
+   int64_t owner;
+   int     begin, count;
+   int     b, bc;
+};
+// One of its macro-cells: the slot of its copy there, row and slice, cell and position class.
+struct IncRec {
+   int64_t slot;
+   int     cell, cls;
+   int16_t x, y, z, pad;
+};
+static_assert( sizeof( LowRec ) == 24 && sizeof( IncRec ) == 24, "record layouts" );
 
 struct Incidence {
    int   cell;
@@ -133,6 +148,8 @@ struct Topology {
 // and runs one point per lane.  Each warp of a launch owns a list of units; a launch has kSwWarps
 // warps per block and BPS = 2, 3 or 4 blocks per SM (by value type and operation), one list set per
 // BPS.
+// points per macro-edge up to which cell interiors run one thread per point (k_flat_stencil)
+constexpr int kFlatMaxN    = 64;
 constexpr int kSwR         = 4;
 constexpr int kSwTX        = 64;  // 32 or 64
 constexpr int kSwWarps     = 4;
@@ -155,9 +172,6 @@ struct P1Level {
    std::vector< Incidence >     inc;
    std::vector< std::array< int, 4 > > tasks;  // {b, i, j, 0}: owned DoFs of boundary primitives
    std::vector< std::array< int, 2 > > rows;   // (y, z) of cell interior rows
-   // y-marching work items of the cell stencil sweep: (z, x0, y_first, y_last); a warp covers
-   // x0..x0+31 of slice z and marches over rows y_first..y_last
-   std::vector< std::array< int, 4 > > march;
    // rolled-register sweep: units {x0 (| kSwUnitHalf), y0, z_first, z_last} of macro-cell zcell[i];
    // block k runs units zbegin[k]..zbegin[k+1]-1
    std::vector< std::array< int, 4 > > zunits;
@@ -176,10 +190,14 @@ struct P1Level {
    Incidence* d_inc       = nullptr;
    int4*      d_tasks     = nullptr;
    int4*      d_btasks    = nullptr;  // tasks grouped by boundary type (Inner, Dirichlet, Neumann, Freeslip)
-   FaceRec*   d_frec      = nullptr;  // per grouped task: its two-cell face record, if it is one
-   int        bcount[4]   = {};
+   FaceRec*   d_frec      = nullptr;  // face tasks, edge and vertex tasks in group order
+   LowRec*    d_lrec      = nullptr;
+   IncRec*    d_irec      = nullptr;
+   int        nlow[4]     = {};       // edge and vertex tasks, face tasks per group
+   int        nface[4]    = {};
+   int        nipts       = 0;        // interior points of a macro-cell, listed for n <= kFlatMaxN
+   void*      d_ipts      = nullptr;  // their coordinates (ushort4)
    int2*      d_rows      = nullptr;
-   int4*      d_march     = nullptr;
    int4*      d_zunits            = nullptr;
    int*       d_zcell             = nullptr;
    int*       d_zbegin            = nullptr;

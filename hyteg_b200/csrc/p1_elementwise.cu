@@ -1292,18 +1292,10 @@ static AccVecs< T, A > acc_vecs( const A* acc, const StencilArgs& a )
 // whole interior).  V(3,3) Chebyshev(3) cycle on a shell of 240 cells, levels 0-5, FP64: 8.59 ms with a warp
 // per row, 15 stored weights and gathering owners, 3.62 ms so.
 // ---------------------------------------------------------------------------------------------
-template < int D >
-struct VarDir {
-   static constexpr int dirs[15][3] = { { 0, 0, 0 },  { -1, 0, 0 }, { 1, 0, 0 },  { 0, -1, 0 }, { 0, 1, 0 },
-                                        { 0, 0, -1 }, { 0, 0, 1 },  { -1, 1, 0 }, { 1, -1, 0 }, { -1, 0, 1 },
-                                        { 1, 0, -1 }, { 0, -1, 1 }, { 0, 1, -1 }, { 1, -1, 1 }, { -1, 1, -1 } };
-   static constexpr int x = dirs[D][0], y = dirs[D][1], z = dirs[D][2];
-};
-
 template < int D, typename T, typename A >
 __device__ __forceinline__ void var_term( const A* S, int64_t ssize, const T* src, int n, int x, int y, int z, bool inner, A ( &s )[3] )
 {
-   constexpr int dx = VarDir< D >::x, dy = VarDir< D >::y, dz = VarDir< D >::z;
+   constexpr int dx = StencilDir< D >::x, dy = StencilDir< D >::y, dz = StencilDir< D >::z;
    if ( !inner && ( x + dx < 0 || y + dy < 0 || z + dz < 0 || x + y + z + ( dx + dy + dz ) > n ) ) return;
    const int o = row_shift< dy, dz >( n, y, z ) + dx;
    const A   w = ( D & 1 ) ? __ldg( S + ( ( D + 1 ) / 2 ) * ssize + o ) : __ldg( S + ( D / 2 ) * ssize );

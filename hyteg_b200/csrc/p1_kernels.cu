@@ -23,6 +23,7 @@
 #include <stdexcept>
 #include <string>
 #include <type_traits>
+#include <utility>
 
 namespace hyb {
 
@@ -65,94 +66,6 @@ __device__ __forceinline__ int point_class( int n, int x, int y, int z )
 // ---------------------------------------------------------------------------------------------
 // stencil sweeps
 // ---------------------------------------------------------------------------------------------
-
-// y-marching cell sweep: a warp owns x0..x0+31 of slice z and walks the rows y_first..y_last.  The
-// rows (y-1, y, y+1) of slice z, (y-1, y) of slice z+1 and (y, y+1) of slice z-1 roll through
-// registers, so each step loads three new rows (x-1, x, x+1 per lane; neighbours hit L1) instead
-// of fifteen values per point.
-template < typename T, typename A >
-struct Row3
-{
-   A m, o, p;
-};
-
-template < typename T, typename A >
-__device__ __forceinline__ Row3< T, A > load_row( const T* s, int n, int yy, int zz, int x )
-{
-   const int64_t rb  = cidx( n, 0, yy, zz );
-   const int     len = n - yy - zz;  // last valid x of the row
-   Row3< T, A >  r;
-   r.m = ( x - 1 <= len ) ? A( ldv( s + rb + x - 1 ) ) : A( 0 );
-   r.o = ( x <= len ) ? A( ldv( s + rb + x ) ) : A( 0 );
-   r.p = ( x + 1 <= len ) ? A( ldv( s + rb + x + 1 ) ) : A( 0 );
-   return r;
-}
-
-__device__ __forceinline__ void prefetch_l2( const void* p ) { asm volatile( "prefetch.global.L2 [%0];" ::"l"( p ) ); }
-
-template < typename T, typename A, int OP >
-__global__ void __launch_bounds__( 256 ) k_cell_march( LevelView v, OpView< A > o, uint32_t flag, const T* __restrict__ src,
-                                                        const T* __restrict__ v1, T* v2, T* dst, A a0, A a1 )
-{
-   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int item = blockIdx.x * 8 + warp;
-   const int c    = blockIdx.y;
-   if ( item >= v.nmarch ) return;
-   if ( !( v.cell_bc[c] & flag ) ) return;
-   const int4    it   = v.march[item];
-   const int     z = it.x, x = it.y + lane, ya = it.z, yb = it.w, n = v.n;
-   const int64_t base = v.cell_off[c];
-   const T*      s    = src + base;
-   const A*      W    = o.W + size_t( c ) * kNumClasses * kNumDirs;
-   const A w0 = W[0], wW = W[1], wE = W[2], wS = W[3], wN = W[4], wB = W[5], wT = W[6], wNW = W[7], wSE = W[8], wTW = W[9],
-           wBE = W[10], wTS = W[11], wBN = W[12], wTSE = W[13], wBNW = W[14];
-   const A invd = o.invd_c[c];
-   Row3< T, A > cm = load_row< T, A >( s, n, ya - 1, z, x );
-   Row3< T, A > c0 = load_row< T, A >( s, n, ya, z, x );
-   Row3< T, A > tm = load_row< T, A >( s, n, ya - 1, z + 1, x );
-   Row3< T, A > b0 = load_row< T, A >( s, n, ya, z - 1, x );
-   constexpr int pd = 8;  // rows pulled into L2 ahead of the march
-#pragma unroll 2
-   for ( int y = ya; y <= yb; ++y )
-   {
-      if ( pd > 0 )
-      {
-         // pull the rows needed pd steps ahead into L2 (addresses stay inside the cell array)
-         const int yp = y + pd;
-         if ( yp + 1 + z <= n && x <= n - yp - 1 - z ) prefetch_l2( s + cidx( n, x, yp + 1, z ) );
-         if ( yp + z + 1 <= n && x <= n - yp - z - 1 ) prefetch_l2( s + cidx( n, x, yp, z + 1 ) );
-         if ( yp + 1 + z - 1 <= n && x <= n - yp - z ) prefetch_l2( s + cidx( n, x, yp + 1, z - 1 ) );
-      }
-      const Row3< T, A > cp = load_row< T, A >( s, n, y + 1, z, x );
-      const Row3< T, A > t0 = load_row< T, A >( s, n, y, z + 1, x );
-      const Row3< T, A > bp = load_row< T, A >( s, n, y + 1, z - 1, x );
-      if ( x + y + z <= n - 1 )
-      {
-         A acc = w0 * c0.o;
-         acc += wW * c0.m;
-         acc += wE * c0.p;
-         acc += wS * cm.o;
-         acc += wN * cp.o;
-         acc += wB * b0.o;
-         acc += wT * t0.o;
-         acc += wNW * cp.m;
-         acc += wSE * cm.p;
-         acc += wTW * t0.m;
-         acc += wBE * b0.p;
-         acc += wTS * tm.o;
-         acc += wBN * bp.o;
-         acc += wTSE * tm.p;
-         acc += wBNW * bp.m;
-         stencil_epilogue< T, A, OP >( base + cidx( n, x, y, z ), acc, invd, src, v1, v2, dst, a0, a1 );
-      }
-      cm = c0;
-      c0 = cp;
-      tm = t0;
-      b0 = bp;
-   }
-}
-
-
 
 // epilogue of the z-streamed sweep: the centre of src and the second vector come from the stage
 template < typename T, typename A, int OP >
@@ -887,147 +800,219 @@ __device__ __forceinline__ A class_stencil( const T* s, const A* W, uint16_t mas
    return class_stencil_at< T, A >( s, W, mask, n, x, y, z ).sum;
 }
 
-// One owned face / edge / vertex DoF (boundary task t): the sum over its neighbour cells of the
-// stencil of its position class in each cell, the operation's epilogue, and the write to the owner
-// and every copy in the neighbouring cell arrays.
-template < typename T, typename A, int OP >
-__device__ __forceinline__ void bnd_task( const LevelView& v, const OpView< A >& o, uint32_t flag, int copy_unflagged,
-                                          const T* __restrict__ src, const T* __restrict__ v1, T* v2, T* dst, A a0, A a1, int4 tk )
+// Stencil of a face's position class (1: z = 0, 2: y = 0, 3: x = 0, 4: x + y + z = n) at a slot of row y and
+// slice z: the directions that stay in the cell are known when compiling, so a term is two loads, one
+// address and one multiply-add
+template < int D, int CLS, typename T, typename A >
+__device__ __forceinline__ void face_term( const T* c, const A* W, int n, int y, int z, A ( &s )[2] )
 {
-   const int     b     = tk.x, i = tk.y, j = tk.z, n = v.n;
-   const int64_t owner = owner_slot( v, b, i, j );
-   if ( !( v.bc[b] & flag ) )
+   constexpr int dx = StencilDir< D >::x, dy = StencilDir< D >::y, dz = StencilDir< D >::z;
+   if constexpr ( ( CLS == 1 && dz < 0 ) || ( CLS == 2 && dy < 0 ) || ( CLS == 3 && dx < 0 ) || ( CLS == 4 && dx + dy + dz > 0 ) ) return;
+   else s[D & 1] += __ldg( W + D ) * A( ldv( c + ( row_shift< dy, dz >( n, y, z ) + dx ) ) );
+}
+template < int CLS, typename T, typename A, int... D >
+__device__ __forceinline__ A face_terms( const T* c, const A* W, int n, int y, int z, std::integer_sequence< int, D... > )
+{
+   A s[2] = { A( 0 ), A( 0 ) };
+   ( face_term< D, CLS, T, A >( c, W, n, y, z, s ), ... );
+   return s[0] + s[1];
+}
+template < typename T, typename A >
+__device__ __forceinline__ A face_stencil( const T* c, const A* W, int cls, int n, int y, int z )
+{
+   constexpr auto all = std::make_integer_sequence< int, kNumDirs >();
+   switch ( cls )
    {
-      if ( !copy_unflagged ) return;
-      if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) write_through( v, dst, b, i, j, owner, A( ldv( src + owner ) ) );
-      else if constexpr ( OP == OP_CHEBI ) write_through( v, dst, b, i, j, owner, A( ldc( v2 + owner ) ) );
-      return;
+   case 1: return face_terms< 1, T, A >( c, W, n, y, z, all );
+   case 2: return face_terms< 2, T, A >( c, W, n, y, z, all );
+   case 3: return face_terms< 3, T, A >( c, W, n, y, z, all );
+   default: return face_terms< 4, T, A >( c, W, n, y, z, all );
    }
-   A         acc = A( 0 );
-   const int q0 = v.inc_begin[b], q1 = v.inc_begin[b + 1];
-   if ( q1 - q0 == 2 )
-   {
-      // a face between two cells: both class stencils written out, so the loads of the two cells
-      // are in flight together (same sum, same order as the loop); the copies of the owner in the
-      // two cell arrays are the stencils' centres
-      const Incidence I0 = v.inc[q0], I1 = v.inc[q0 + 1];
-      int             x0, y0, z0, x1, y1, z1;
-      inc_point( I0, n, i, j, x0, y0, z0 );
-      inc_point( I1, n, i, j, x1, y1, z1 );
-      const int64_t         cb0 = v.cell_off[I0.cell], cb1 = v.cell_off[I1.cell];
-      const StencilAt< A >  s0  = class_stencil_at< T, A >( src + cb0, o.W + ( size_t( I0.cell ) * kNumClasses + I0.cls ) * kNumDirs,
-                                                           c_cls_mask[I0.cls], n, x0, y0, z0 );
-      const StencilAt< A >  s1  = class_stencil_at< T, A >( src + cb1, o.W + ( size_t( I1.cell ) * kNumClasses + I1.cls ) * kNumDirs,
-                                                           c_cls_mask[I1.cls], n, x1, y1, z1 );
-      const int64_t         c0 = s0.centre, c1 = s1.centre;
-      acc                       = ( acc + s0.sum ) + s1.sum;
-      const A invd = o.invd_b[b];
-      auto    put  = [&]( T* vec, A val ) {
-         stv( vec + owner, val );
-         stv( vec + cb0 + c0, val );
-         stv( vec + cb1 + c1, val );
-      };
-      if constexpr ( OP == OP_APPLY ) put( dst, acc );
-      else if constexpr ( OP == OP_APPLY_ADD ) put( dst, A( ldc( dst + owner ) ) + acc );
-      else if constexpr ( OP == OP_RESID ) put( dst, A( ldv( v1 + owner ) ) - acc );
-      else if constexpr ( OP == OP_JAC ) put( dst, A( ldv( src + owner ) ) + a0 * ( invd * ( A( ldv( v1 + owner ) ) - acc ) ) );
-      else if constexpr ( OP == OP_CHEB0 ) put( dst, invd * ( A( ldv( v1 + owner ) ) - acc ) );
-      else if constexpr ( OP == OP_CHEBI )
-      {
-         put( dst, invd * acc );
-         put( v2, A( ldc( v2 + owner ) ) + a0 * A( ldv( src + owner ) ) );
-      }
-      else if constexpr ( OP == OP_CHEBL ) put( v2, ( A( ldc( v2 + owner ) ) + a0 * A( ldv( src + owner ) ) ) + a1 * ( invd * acc ) );
-      else if constexpr ( OP == OP_DINV_APPLY ) put( dst, invd * acc );
-      return;
-   }
-   else
-      // edges and vertices: two incidences' stencils in flight, summed in incidence order
-      for ( int q = q0; q < q1; q += 2 )
-      {
-         A sq[2];
-#pragma unroll
-         for ( int u = 0; u < 2; ++u )
-         {
-            sq[u] = A( 0 );
-            if ( q + u < q1 )
-            {
-               const Incidence I = v.inc[q + u];
-               int             x, y, z;
-               inc_point( I, n, i, j, x, y, z );
-               sq[u] = class_stencil< T, A >( src + v.cell_off[I.cell], o.W + ( size_t( I.cell ) * kNumClasses + I.cls ) * kNumDirs,
-                                              c_cls_mask[I.cls], n, x, y, z );
-            }
-         }
-         acc += sq[0];
-         if ( q + 1 < q1 ) acc += sq[1];
-      }
-   const A invd = o.invd_b[b];
-   if constexpr ( OP == OP_APPLY ) write_through( v, dst, b, i, j, owner, acc );
-   else if constexpr ( OP == OP_APPLY_ADD ) write_through( v, dst, b, i, j, owner, A( ldc( dst + owner ) ) + acc );
-   else if constexpr ( OP == OP_RESID ) write_through( v, dst, b, i, j, owner, A( ldv( v1 + owner ) ) - acc );
-   else if constexpr ( OP == OP_JAC )
-      write_through( v, dst, b, i, j, owner, A( ldv( src + owner ) ) + a0 * ( invd * ( A( ldv( v1 + owner ) ) - acc ) ) );
-   else if constexpr ( OP == OP_CHEB0 ) write_through( v, dst, b, i, j, owner, invd * ( A( ldv( v1 + owner ) ) - acc ) );
+}
+
+// value of an operation at an owner from the stencil sum, and the second vector's value (Chebyshev steps)
+template < typename T, typename A, int OP >
+__device__ __forceinline__ A owner_value( int64_t o, A s, A invd, const T* src, const T* v1, const T* v2, const T* dst, A a0, A a1, A& second )
+{
+   if constexpr ( OP == OP_APPLY_ADD ) return A( ldc( dst + o ) ) + s;
+   else if constexpr ( OP == OP_RESID ) return A( ldv( v1 + o ) ) - s;
+   else if constexpr ( OP == OP_JAC ) return A( ldv( src + o ) ) + a0 * ( invd * ( A( ldv( v1 + o ) ) - s ) );
+   else if constexpr ( OP == OP_CHEB0 ) return invd * ( A( ldv( v1 + o ) ) - s );
    else if constexpr ( OP == OP_CHEBI )
    {
-      write_through( v, dst, b, i, j, owner, invd * acc );
-      write_through( v, v2, b, i, j, owner, A( ldc( v2 + owner ) ) + a0 * A( ldv( src + owner ) ) );
+      second = A( ldc( v2 + o ) ) + a0 * A( ldv( src + o ) );
+      return invd * s;
    }
-   else if constexpr ( OP == OP_CHEBL )
-      write_through( v, v2, b, i, j, owner, ( A( ldc( v2 + owner ) ) + a0 * A( ldv( src + owner ) ) ) + a1 * ( invd * acc ) );
-   else if constexpr ( OP == OP_DINV_APPLY ) write_through( v, dst, b, i, j, owner, invd * acc );
+   else if constexpr ( OP == OP_CHEBL ) return ( A( ldc( v2 + o ) ) + a0 * A( ldv( src + o ) ) ) + a1 * ( invd * s );
+   else if constexpr ( OP == OP_DINV_APPLY ) return invd * s;
+   else return s;
+}
+
+// The boundary tasks of the selected types: edges and vertices first, eight threads each (from
+// threads lat on, a multiple of 32 per type), then faces, one thread each
+struct BndSegments
+{
+   int lstart[4], lthreads[4], lcount[4];
+   int fstart[4], fcount[4];
+   int threads;
+};
+
+static inline BndSegments bnd_segments( const LevelView& v, uint32_t flag, int all )
+{
+   static const uint32_t type_bit[4] = { kInner, kDirichlet, kNeumann, kFreeslip };
+   BndSegments           s{};
+   int                   k = 0, lat = 0, fat = 0;
+   for ( int g = 0; g < 4; ++g )
+   {
+      if ( all || ( flag & type_bit[g] ) )
+      {
+         s.lstart[k]   = lat;
+         s.lcount[k]   = v.nlow[g];
+         s.lthreads[k] = ( 8 * v.nlow[g] + 31 ) / 32 * 32;
+         s.fstart[k]   = fat;
+         s.fcount[k]   = v.nface[g];
+         s.threads += s.lthreads[k] + s.fcount[k];
+         ++k;
+      }
+      lat += v.nlow[g];
+      fat += v.nface[g];
+   }
+   return s;
+}
+
+// One boundary task: the sum over its neighbour cells of the stencil of its position class in each, the
+// operation's epilogue, and the write to the owner and every copy in the neighbouring cell arrays.  Every
+// index comes from the task's records, so the values wait on one dependent load for a face and on two for
+// an edge or vertex, whose cells (6 on average, up to 30) are shared by eight threads: one thread that
+// walked them two at a time took 17 us on a level of 200 tasks.
+template < typename T, typename A, int OP >
+__device__ __forceinline__ void bnd_point( const LevelView& v, const OpView< A >& o, const BndSegments& seg, int t, uint32_t flag,
+                                           int copy_unflagged, const T* __restrict__ src, const T* __restrict__ v1, T* v2, T* dst, A a0, A a1 )
+{
+#pragma unroll
+   for ( int g = 0; g < 4; ++g )  // unrolled: the segment arrays are read with constant indices
+   {
+      if ( t < seg.lthreads[g] )
+      {
+         const int  k = t >> 3, sub = t & 7;
+         const bool live = k < seg.lcount[g];
+         LowRec     r    = v.lrec[seg.lstart[g] + ( live ? k : 0 )];
+         const bool flagged = ( r.bc & flag ) != 0;
+         if ( !live || ( !flagged && !copy_unflagged ) ) r.count = 0;
+         A val = A( 0 ), second = A( 0 ), s = A( 0 );
+         if ( flagged )
+         {
+            for ( int q = sub; q < r.count; q += 8 )
+            {
+               const IncRec I = v.irec[r.begin + q];
+               s += class_stencil_slot< T, A >( src, o.W + ( size_t( I.cell ) * kNumClasses + I.cls ) * kNumDirs, c_cls_mask[I.cls], v.n,
+                                                I.slot, I.y, I.z );
+            }
+         }
+#pragma unroll
+         for ( int m = 4; m > 0; m >>= 1 ) s += __shfl_xor_sync( 0xffffffffu, s, m, 8 );
+         if ( r.count > 0 )
+         {
+            if ( flagged ) val = owner_value< T, A, OP >( r.owner, s, o.invd_b[r.b], src, v1, v2, dst, a0, a1, second );
+            else if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) val = A( ldv( src + r.owner ) );
+            else if constexpr ( OP == OP_CHEBI ) val = A( ldc( v2 + r.owner ) );
+         }
+         __syncwarp();  // every thread of a task has read the owner before any writes it
+         auto put = [&]( T* vec, A x ) {
+            if ( r.count > 0 && sub == 0 ) stv( vec + r.owner, x );
+            for ( int q = sub; q < r.count; q += 8 ) stv( vec + v.irec[r.begin + q].slot, x );
+         };
+         if constexpr ( OP == OP_CHEBL ) put( v2, val );
+         else put( dst, val );
+         if constexpr ( OP == OP_CHEBI )
+            if ( flagged ) put( v2, second );
+         return;
+      }
+      t -= seg.lthreads[g];
+   }
+   int at = -1;
+#pragma unroll
+   for ( int g = 0; g < 4; ++g )
+   {
+      if ( at < 0 && t < seg.fcount[g] ) at = seg.fstart[g] + t;
+      if ( at < 0 ) t -= seg.fcount[g];
+   }
+   if ( at < 0 ) return;
+   const FaceRec r   = v.frec[at];
+   auto          put = [&]( T* vec, A x ) {
+      stv( vec + r.owner, x );
+      stv( vec + r.c0, x );
+      if ( r.cell1 >= 0 ) stv( vec + r.c1, x );
+   };
+   if ( !( r.bc & flag ) )
+   {
+      if ( !copy_unflagged ) return;
+      if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) put( dst, A( ldv( src + r.owner ) ) );
+      else if constexpr ( OP == OP_CHEBI ) put( dst, A( ldc( v2 + r.owner ) ) );
+      return;
+   }
+   A s = face_stencil< T, A >( src + r.c0, o.W + ( size_t( r.cell0 ) * kNumClasses + r.cls0 ) * kNumDirs, r.cls0, v.n, r.y0, r.z0 );
+   if ( r.cell1 >= 0 )
+      s += face_stencil< T, A >( src + r.c1, o.W + ( size_t( r.cell1 ) * kNumClasses + r.cls1 ) * kNumDirs, r.cls1, v.n, r.y1, r.z1 );
+   A       second = A( 0 );
+   const A val    = owner_value< T, A, OP >( r.owner, s, o.invd_b[r.b], src, v1, v2, dst, a0, a1, second );
+   if constexpr ( OP == OP_CHEBL ) put( v2, val );
+   else put( dst, val );
+   if constexpr ( OP == OP_CHEBI ) put( v2, second );
 }
 
 // threads per block of the boundary kernel
 constexpr int kBndThreads = 256;
 
 template < typename T, typename A, int OP >
-__global__ void __launch_bounds__( kBndThreads ) k_bnd_stencil( LevelView v, OpView< A > o, TaskSegments seg, uint32_t flag, int copy_unflagged,
+__global__ void __launch_bounds__( kBndThreads ) k_bnd_stencil( LevelView v, OpView< A > o, BndSegments seg, uint32_t flag, int copy_unflagged,
                                                          const T* __restrict__ src, const T* __restrict__ v1, T* v2, T* dst,
                                                          A a0, A a1 )
 {
-   // tasks of the primitives whose boundary type is flagged (or all, when unflagged owners are
-   // copied): up to four contiguous groups of the type-sorted task list
-   int t = blockIdx.x * blockDim.x + threadIdx.x, at = -1;
-#pragma unroll
-   for ( int g = 0; g < 4; ++g )  // unrolled: the segment arrays are read with constant indices
+   const int t = blockIdx.x * kBndThreads + threadIdx.x;
+   bnd_point< T, A, OP >( v, o, seg, t, flag, copy_unflagged, src, v1, v2, dst, a0, a1 );
+}
+
+// one interior point: slot i of row y, slice z of a cell with weights W (class 0) and inverse diagonal invd
+template < int D, typename T, typename A >
+__device__ __forceinline__ void point_term( const T* c, const A* W, int n, int y, int z, A ( &s )[3] )
+{
+   constexpr int dx = StencilDir< D >::x, dy = StencilDir< D >::y, dz = StencilDir< D >::z;
+   s[D % 3] += __ldg( W + D ) * A( ldv( c + ( row_shift< dy, dz >( n, y, z ) + dx ) ) );
+}
+template < typename T, typename A, int... D >
+__device__ __forceinline__ A point_stencil( const T* c, const A* W, int n, int y, int z, std::integer_sequence< int, D... > )
+{
+   A s[3] = { A( 0 ), A( 0 ), A( 0 ) };
+   ( point_term< D, T, A >( c, W, n, y, z, s ), ... );
+   return s[0] + ( s[1] + s[2] );
+}
+
+// Levels up to kFlatMaxN points per macro-edge: boundary tasks and interior points of all cells in one
+// launch, one thread per point, all 15 loads in flight.  Small levels are bound by latency: a y-marching
+// cell kernel beside a boundary kernel on a second stream took 10.3 us for a level-4 FP32 apply on 36 cells
+// where this takes 5.9, and ten V(2,2) cycles of the level-5 cube 4.55 ms where these take 2.66.  The
+// tiled sweeps are faster from 128 points on (level-7 FP32 smoothing on 12 cells 521 against 592 us; the
+// level-8 apply 90 against 283 us), this kernel up to 64 (level-8 FP64 cycle 4.51 against 4.79 ms with the
+// sweep there).
+template < typename T, typename A, int OP >
+__global__ void __launch_bounds__( kBndThreads ) k_flat_stencil( LevelView v, OpView< A > o, BndSegments seg, int nbnd, int nC, uint32_t flag,
+                                                                 int copy_unflagged, const T* __restrict__ src, const T* __restrict__ v1,
+                                                                 T* v2, T* dst, A a0, A a1 )
+{
+   if ( int( blockIdx.x ) < nbnd )
    {
-      if ( at < 0 && t < seg.count[g] ) at = seg.start[g] + t;
-      if ( at < 0 ) t -= seg.count[g];
-   }
-   if ( at < 0 ) return;
-   // a flagged face point between two cells: everything the stencil needs comes from one record,
-   // so the value loads follow a single dependent load (the same sums, in the same order, as bnd_task)
-   const FaceRec r = v.frec[at];
-   if ( r.cell0 >= 0 && ( r.bc & flag ) )
-   {
-      const A s0 = class_stencil_slot< T, A >( src, o.W + ( size_t( r.cell0 ) * kNumClasses + r.cls0 ) * kNumDirs, c_cls_mask[r.cls0], v.n,
-                                              r.c0, r.y0, r.z0 );
-      const A s1 = class_stencil_slot< T, A >( src, o.W + ( size_t( r.cell1 ) * kNumClasses + r.cls1 ) * kNumDirs, c_cls_mask[r.cls1], v.n,
-                                              r.c1, r.y1, r.z1 );
-      const A acc  = ( A( 0 ) + s0 ) + s1;
-      const A invd = o.invd_b[r.b];
-      auto    put  = [&]( T* vec, A val ) {
-         stv( vec + r.owner, val );
-         stv( vec + r.c0, val );
-         stv( vec + r.c1, val );
-      };
-      if constexpr ( OP == OP_APPLY ) put( dst, acc );
-      else if constexpr ( OP == OP_APPLY_ADD ) put( dst, A( ldc( dst + r.owner ) ) + acc );
-      else if constexpr ( OP == OP_RESID ) put( dst, A( ldv( v1 + r.owner ) ) - acc );
-      else if constexpr ( OP == OP_JAC ) put( dst, A( ldv( src + r.owner ) ) + a0 * ( invd * ( A( ldv( v1 + r.owner ) ) - acc ) ) );
-      else if constexpr ( OP == OP_CHEB0 ) put( dst, invd * ( A( ldv( v1 + r.owner ) ) - acc ) );
-      else if constexpr ( OP == OP_CHEBI )
-      {
-         put( dst, invd * acc );
-         put( v2, A( ldc( v2 + r.owner ) ) + a0 * A( ldv( src + r.owner ) ) );
-      }
-      else if constexpr ( OP == OP_CHEBL ) put( v2, ( A( ldc( v2 + r.owner ) ) + a0 * A( ldv( src + r.owner ) ) ) + a1 * ( invd * acc ) );
-      else if constexpr ( OP == OP_DINV_APPLY ) put( dst, invd * acc );
+      bnd_point< T, A, OP >( v, o, seg, blockIdx.x * kBndThreads + threadIdx.x, flag, copy_unflagged, src, v1, v2, dst, a0, a1 );
       return;
    }
-   bnd_task< T, A, OP >( v, o, flag, copy_unflagged, src, v1, v2, dst, a0, a1, v.btasks[at] );
+   const int64_t g = int64_t( blockIdx.x - nbnd ) * kBndThreads + threadIdx.x;
+   if ( g >= int64_t( nC ) * v.nipts ) return;
+   const int c = g < 0x7fffffff ? int( unsigned( g ) / unsigned( v.nipts ) ) : int( g / v.nipts );
+   if ( !( v.cell_bc[c] & flag ) ) return;
+   const ushort4 p = v.ipts[int( g - int64_t( c ) * v.nipts )];
+   const int64_t i = v.cell_off[c] + cidx( v.n, p.x, p.y, p.z );
+   const A s = point_stencil< T, A >( src + i, o.W + size_t( c ) * kNumClasses * kNumDirs, v.n, p.y, p.z, std::make_integer_sequence< int, kNumDirs >() );
+   stencil_epilogue< T, A, OP >( i, s, o.invd_c[c], src, v1, v2, dst, a0, a1 );
 }
 
 template < typename T, typename A, int OP >
@@ -1037,17 +1022,25 @@ static void run_stencil( Context* ctx, const LevelView& v, const OpView< A >& o,
    const T* v1  = (const T*) a.v1;
    T*       v2  = (T*) a.v2;
    T*       dst = (T*) a.dst;
-   // the bulk-copy sweep from n = 32 on (two 64-point tiles per row and up), the y-marching sweep on
-   // the small levels, where a slice holds too few rows to fill a ring
    using Cfg = SwCfg< T, OP >;
    // cell interiors and boundary owners write disjoint slots and read only src (and their own
    // slots of the second vector), so the two kernels may run in either order
-   const TaskSegments seg = task_segments( v, a.flag, a.copy_unflagged );
-   const int          nt  = seg.count[0] + seg.count[1] + seg.count[2] + seg.count[3];
+   const BndSegments seg = bnd_segments( v, a.flag, a.copy_unflagged );
+   const int         nt  = seg.threads, nbnd = ( nt + kBndThreads - 1 ) / kBndThreads;
+   if ( v.n <= kFlatMaxN )
+   {
+      const int blocks = nbnd + int( ( int64_t( nC ) * v.nipts + kBndThreads - 1 ) / kBndThreads );
+      if ( blocks == 0 ) return;
+      k_flat_stencil< T, A, OP ><<< blocks, kBndThreads, 0, ctx->stream >>>( v, o, seg, nbnd, nC, a.flag, a.copy_unflagged, src, v1, v2, dst,
+                                                                            A( a.a0 ), A( a.a1 ) );
+      ++ctx->launches;
+      check_cuda( cudaGetLastError(), "stencil launch" );
+      return;
+   }
    // the partial-sum sweep for the operations without a second vector, the rolled-register sweep
    // for the others (their epilogues' registers would leave the partial-sum sweep 8 warps per SM)
    constexpr bool ROLLED = sweep_aux< OP >();
-   const bool     big    = v.n >= 32 && nC > 0 && ( ROLLED ? v.nzblocks > 0 : v.nswarps[Cfg::BPS - 2] > 0 );
+   const bool     big    = nC > 0 && ( ROLLED ? v.nzblocks > 0 : v.nswarps[Cfg::BPS - 2] > 0 );
    auto           cell   = [&]() {
       if constexpr ( ROLLED )
       {
@@ -1070,7 +1063,7 @@ static void run_stencil( Context* ctx, const LevelView& v, const OpView< A >& o,
       // branches, and the boundary kernel fills the SMs the sweep's last blocks leave idle.
       if ( nt > 0 )
       {
-         k_bnd_stencil< T, A, OP ><<< ( nt + kBndThreads - 1 ) / kBndThreads, kBndThreads, 0, ctx->stream >>>( v, o, seg, a.flag, a.copy_unflagged, src, v1, v2, dst,
+         k_bnd_stencil< T, A, OP ><<< nbnd, kBndThreads, 0, ctx->stream >>>( v, o, seg, a.flag, a.copy_unflagged, src, v1, v2, dst,
                                                                                    A( a.a0 ), A( a.a1 ) );
          ++ctx->launches;
       }
@@ -1081,15 +1074,9 @@ static void run_stencil( Context* ctx, const LevelView& v, const OpView< A >& o,
    // the cell kernel and the boundary kernel side by side on two streams
    Fork fk( ctx );
    if ( big ) cell();
-   else if ( v.nmarch > 0 && nC > 0 )
-   {
-      dim3 grid( ( v.nmarch + 7 ) / 8, nC );
-      k_cell_march< T, A, OP ><<< grid, 256, 0, ctx->stream >>>( v, o, a.flag, src, v1, v2, dst, A( a.a0 ), A( a.a1 ) );
-      ++ctx->launches;
-   }
    if ( nt > 0 )
    {
-      k_bnd_stencil< T, A, OP ><<< ( nt + kBndThreads - 1 ) / kBndThreads, kBndThreads, 0, fk.aux() >>>( v, o, seg, a.flag, a.copy_unflagged, src, v1, v2, dst,
+      k_bnd_stencil< T, A, OP ><<< nbnd, kBndThreads, 0, fk.aux() >>>( v, o, seg, a.flag, a.copy_unflagged, src, v1, v2, dst,
                                                                              A( a.a0 ), A( a.a1 ) );
       ++ctx->launches;
    }

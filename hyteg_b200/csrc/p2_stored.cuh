@@ -8,7 +8,7 @@
 // macro-cells or the length of their rows.  Boundary nodes hold the partial stencil of their macro-cell.
 #pragma once
 
-#include "hyb_internal.hpp"
+#include "hyb_device.cuh"
 
 namespace hyb {
 
@@ -90,20 +90,6 @@ __device__ __forceinline__ int64_t p2_weight_at( const P2StoredView& v, int c, i
    const int  s   = ( ( x & 1 ) | ( y & 1 ) << 1 | ( z & 1 ) << 2 ) + ( bnd ? 8 : 0 );
    step           = int64_t( v.nC ) * v.np[s];
    return v.wbase[s] + int64_t( c ) * v.np[s] + v.rank[cidx( v.n, x, y, z )];
-}
-
-// start of row (y + dy, z + dz) of a cell array minus the start of row (y, z)
-template < int DY, int DZ >
-__device__ __forceinline__ int row_shift( int n, int y, int z )
-{
-   const int q = n + 1 - z;  // points in the first row of slice z
-   int       s = 0;
-   if constexpr ( DZ >= 1 ) s += q * ( q + 1 ) / 2;
-   if constexpr ( DZ >= 2 ) s += ( q - 1 ) * q / 2;
-   if constexpr ( DZ <= -1 ) s -= ( q + 1 ) * ( q + 2 ) / 2;
-   if constexpr ( DZ <= -2 ) s -= ( q + 2 ) * ( q + 3 ) / 2;
-   const int w = y + DY;
-   return s + ( w * ( q - DZ ) - w * ( w - 1 ) / 2 ) - ( y * q - y * ( y - 1 ) / 2 );
 }
 
 // tables of a storage level with n nodes per macro-edge; returns the number of weights

@@ -291,16 +291,6 @@ void build_level( Mesh* m, int L )
          for ( int j = 1; j < n; ++j )
             for ( int i = 1; i + j < n; ++i ) P.tasks.push_back( { b, i, j, 0 } );
    }
-   // y-marching work items (interior points: x, y, z >= 1, x+y+z <= n-1)
-   {
-      const int YC = 16;
-      for ( int z = 1; z <= n - 3; ++z )
-         for ( int x0 = 1; x0 <= n - 2 - z; x0 += 32 )
-         {
-            const int ylast = n - 1 - z - x0;
-            for ( int y0 = 1; y0 <= ylast; y0 += YC ) P.march.push_back( { z, x0, y0, std::min( ylast, y0 + YC - 1 ) } );
-         }
-   }
    // cell interior rows (y, z), memory order
    for ( int z = 1; z <= n - 2; ++z )
       for ( int y = 1; y + z <= n - 2; ++y )
@@ -487,51 +477,79 @@ void ensure_device( Mesh* m, P1Level& P )
       std::vector< int4 > bt;
       for ( int g = 0; g < 4; ++g )
       {
-         P.bcount[g] = 0;
          for ( const int4& q : tk )
          {
             const int      b  = q.x;
             const uint32_t ty = b < t.nV ? t.bc( t.flag_v[b] )
                                          : ( b < t.nV + t.nE ? t.bc( t.flag_e[b - t.nV] ) : t.bc( t.flag_f[b - t.nV - t.nE] ) );
-            if ( ty == type_bit[g] ) bt.push_back( q ), ++P.bcount[g];
+            if ( ty == type_bit[g] ) bt.push_back( q ), ++( b < t.nV + t.nE ? P.nlow : P.nface )[g];
          }
       }
       if ( bt.size() != tk.size() ) throw std::logic_error( "boundary task without a single boundary type" );
       up( &P.d_btasks, bt.data(), bt.size() );
-      std::vector< FaceRec > fr( bt.size() );
+      std::vector< FaceRec > fr;
+      std::vector< LowRec >  lr;
+      std::vector< IncRec >  ir;
       const int              n = P.n;
-      for ( size_t k = 0; k < bt.size(); ++k )
+      for ( const int4& q : bt )
       {
-         FaceRec&  r = fr[k];
-         const int b = bt[k].x, i = bt[k].y, j = bt[k].z;
-         r         = FaceRec{};
-         r.cell0   = -1;
-         if ( b < t.nV + t.nE || P.inc_begin[b + 1] - P.inc_begin[b] != 2 ) continue;
-         r.owner = P.off[b] + fidx( n, i, j );
-         r.b     = b;
-         r.bc    = uint8_t( t.bc( t.flag_f[b - t.nV - t.nE] ) );
-         for ( int s = 0; s < 2; ++s )
+         const int  b = q.x, i = q.y, j = q.z, q0 = P.inc_begin[b], q1 = P.inc_begin[b + 1];
+         const bool face = b >= t.nV + t.nE;
+         const auto bc   = uint8_t( b < t.nV ? t.bc( t.flag_v[b] ) : face ? t.bc( t.flag_f[b - t.nV - t.nE] ) : t.bc( t.flag_e[b - t.nV] ) );
+         FaceRec    f{};
+         f.cell1 = -1;
+         LowRec l{};
+         l.begin = int( ir.size() );
+         for ( int k = q0; k < q1; ++k )
          {
-            const Incidence& I = P.inc[P.inc_begin[b] + s];
+            const Incidence& I = P.inc[k];
             const int        x = n * I.o[0] + i * I.e1[0] + j * I.e2[0];
             const int        y = n * I.o[1] + i * I.e1[1] + j * I.e2[1];
             const int        z = n * I.o[2] + i * I.e1[2] + j * I.e2[2];
             const int64_t    c = P.off[P.nB + I.cell] + cidx( n, x, y, z );
-            ( s ? r.c1 : r.c0 )     = c;
-            ( s ? r.cell1 : r.cell0 ) = I.cell;
-            ( s ? r.y1 : r.y0 )     = int16_t( y );
-            ( s ? r.z1 : r.z0 )     = int16_t( z );
-            ( s ? r.cls1 : r.cls0 ) = int8_t( I.cls );
+            if ( face )
+            {
+               const int s = k - q0;
+               ( s ? f.c1 : f.c0 )       = c;
+               ( s ? f.cell1 : f.cell0 ) = I.cell;
+               ( s ? f.y1 : f.y0 )       = int16_t( y );
+               ( s ? f.z1 : f.z0 )       = int16_t( z );
+               ( s ? f.cls1 : f.cls0 )   = int8_t( I.cls );
+            }
+            else
+               ir.push_back( { c, I.cell, I.cls, int16_t( x ), int16_t( y ), int16_t( z ), 0 } );
+         }
+         if ( face )
+         {
+            f.owner = P.off[b] + fidx( n, i, j );
+            f.b     = b;
+            f.bc    = bc;
+            fr.push_back( f );
+         }
+         else
+         {
+            l.owner = P.off[b] + ( b < t.nV ? 0 : i );
+            l.count = q1 - q0;
+            l.b     = b;
+            l.bc    = bc;
+            lr.push_back( l );
          }
       }
       up( &P.d_frec, fr.data(), fr.size() );
+      up( &P.d_lrec, lr.data(), lr.size() );
+      up( &P.d_irec, ir.data(), ir.size() );
+      std::vector< ushort4 > ip;
+      for ( int z = 1; z < n && n <= kFlatMaxN; ++z )
+         for ( int y = 1; y + z < n; ++y )
+            for ( int x = 1; x + y + z < n; ++x ) ip.push_back( make_ushort4( (unsigned short) x, (unsigned short) y, (unsigned short) z, 0 ) );
+      P.nipts      = int( ip.size() );
+      ushort4* pts = nullptr;
+      up( &pts, ip.data(), ip.size() );
+      P.d_ipts = pts;
    }
    std::vector< int2 > rw( P.rows.size() );
    for ( size_t i = 0; i < rw.size(); ++i ) rw[i] = make_int2( P.rows[i][0], P.rows[i][1] );
    up( &P.d_rows, rw.data(), rw.size() );
-   std::vector< int4 > mi( P.march.size() );
-   for ( size_t i = 0; i < mi.size(); ++i ) mi[i] = make_int4( P.march[i][0], P.march[i][1], P.march[i][2], P.march[i][3] );
-   up( &P.d_march, mi.data(), mi.size() );
    int dev = 0, sms = 0;
    check_cuda( cudaGetDevice( &dev ), "cudaGetDevice" );
    check_cuda( cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev ), "device attribute" );
@@ -597,8 +615,10 @@ Mesh::~Mesh()
       cudaFree( P.d_tasks );
       cudaFree( P.d_btasks );
       cudaFree( P.d_frec );
+      cudaFree( P.d_lrec );
+      cudaFree( P.d_irec );
+      cudaFree( P.d_ipts );
       cudaFree( P.d_rows );
-      cudaFree( P.d_march );
       cudaFree( P.d_zunits ), cudaFree( P.d_zcell ), cudaFree( P.d_zbegin );
       for ( int b = 0; b < kSwLists; ++b ) cudaFree( P.d_swunits[b] ), cudaFree( P.d_swcell[b] ), cudaFree( P.d_swbegin[b] );
       cudaFree( P.d_bc );

@@ -1,0 +1,82 @@
+"""P1 constant-stencil operations at the levels around the change from the one-launch kernel (up to 64 points
+per macro-edge) to the tiled sweeps, and on meshes with edges and vertices of many cells: apply, residual
+via Jacobi, Chebyshev step, unflagged owners carried over, with Neumann faces (one cell).  FP64 against the
+oracle's assembled operator, 1e-12 of the largest value as in the other P1 tests."""
+
+import numpy as np
+import pytest
+
+import hyteg_b200 as H
+from oracle import hyteg_oracle as O
+from tests import meshes as M
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mesh", ["unit_tet", "pyramid_4", "octahedron_8", "cube_2x1x1"])
+@pytest.mark.parametrize("L", [0, 1, 2, 4])
+@pytest.mark.parametrize("neumann", [False, True])
+def test_p1_operations(ctx, mesh, L, neumann):
+    coords, tets = M.ALL[mesh]()
+    om = O.MacroMesh(coords, tets, bc_types={0: O.INNER, 1: O.NEUMANN} if neumann else None)
+    op = O.P1ConstantLaplace(om, L, L)
+    lev = op.levels[L]
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    if neumann:
+        pm.set_bc_type(1, H.NeumannBoundary)
+    A = H.P1ConstantLaplaceOperator(pm, L, L, ctx)
+    flag = H.Inner | H.NeumannBoundary
+    rng = np.random.default_rng(L)
+    vec = {}
+    for n in ("x", "b", "y"):
+        v = np.zeros(lev.size)
+        v[lev.owned] = rng.uniform(-1, 1, lev.owned.size)
+        vec[n] = lev.sync(v)
+    f = {n: H.P1Function(n, pm, L, L, ctx) for n in vec}
+    for n in vec:
+        f[n].upload(L, vec[n])
+    own = lev.owned_mask(O.ALL)
+
+    def check(got, ref):
+        assert np.abs(got[own] - ref[own]).max() <= 1e-12 * max(np.abs(ref[own]).max(), 1e-300)
+        d, s = lev.copy_map()
+        np.testing.assert_array_equal(got[d], got[s])
+
+    A.apply(f["x"], f["y"], L, flag)
+    ref = op.apply(vec["x"], vec["y"].copy(), L, flag)
+    check(f["y"].download(L), ref)
+    A.apply(f["x"], f["y"], L, flag, H.Add)
+    check(f["y"].download(L), op.apply(vec["x"], lev.sync(ref.copy()), L, flag, add=True))
+    A.smooth_jac(f["y"], f["b"], f["x"], 0.6, L, flag)
+    jac = op.smooth_jac(lev.sync(op.apply(vec["x"], lev.sync(ref.copy()), L, flag, add=True)), vec["b"], vec["x"], 0.6, L, flag)
+    check(f["y"].download(L), jac)
+
+
+@pytest.mark.parametrize("L", [5, 6, 7])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_p1_chebyshev_across_kernels(ctx, L, dtype):
+    """One Chebyshev(3) step equals its definition from the operator's own apply (FP64 1e-12; FP32: three
+    applies of 15 products each, values up to 10: 200 eps)."""
+    coords, tets = M.cube_6()
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    A = H.P1ConstantLaplaceOperator(pm, L - 1, L, ctx)
+    g = H.GeometricMultigridSolver(ctx, A, L - 1, L, smoother="chebyshev")
+    g.set_radii([2.0, 2.0])
+    c = H.chebyshev_coefficients(3, 0.3 * 2.0, 1.2 * 2.0)
+    f = {n: H.P1Function(n, pm, L - 1, L, ctx, dtype) for n in ("x", "b", "r", "z", "t", "d", "ref")}
+    for n in ("x", "b"):
+        f[n].fill_random(L, 5 if n == "x" else 6)
+        f[n].interpolate(0.0, L, H.DirichletBoundary)
+    A.getInverseDiagonalValues(f["d"], L, H.Inner)
+    f["ref"].copyFrom(f["x"], L)
+    A.apply(f["x"], f["t"], L, H.Inner)
+    f["r"].assign([1.0, -1.0], [f["b"], f["t"]], L, H.Inner)
+    f["z"].multElementwise([f["d"], f["r"]], L, H.Inner)
+    f["ref"].add([c[0]], [f["z"]], L, H.Inner)
+    for k in (1, 2):
+        A.apply(f["z"], f["t"], L, H.Inner)
+        f["z"].multElementwise([f["d"], f["t"]], L, H.Inner)
+        f["ref"].add([c[k]], [f["z"]], L, H.Inner)
+    g.smooth(f["x"], f["b"], L, 1)
+    x, ref = f["x"].download(L), f["ref"].download(L)
+    assert np.abs(x - ref).max() <= (1e-12 if dtype == "float64" else 2.4e-5) * np.abs(ref).max()
