@@ -1677,146 +1677,251 @@ void launch_dot_noalloc( Context* ctx, Mesh* m, int L, int dtype, uint32_t flag,
 // ---------------------------------------------------------------------------------------------
 // restriction (generated pull kernel semantics, R = P^T) and prolongation
 // ---------------------------------------------------------------------------------------------
-template < typename T, typename A >
-__global__ void __launch_bounds__( 256 ) k_restrict_cells( LevelView cv, LevelView fv, uint32_t flag, const T* __restrict__ fine,
-                                                            T* coarse )
+// sums over the neighbours of the fine point below a coarse face point: those in the face's plane, which
+// the face's cells share, and the others (interior to this cell)
+template < int D, int CLS, typename T, typename A >
+__device__ __forceinline__ void fine_face_term( const T* f, int nf, int Y, int Z, A ( &s )[2] )
 {
-   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int r    = blockIdx.x * 8 + warp;
-   const int c    = blockIdx.y;
-   if ( r >= cv.nrows ) return;
-   if ( !( cv.cell_bc[c] & flag ) ) return;
-   const int2    yz   = cv.rows[r];
-   const int     y = yz.x, z = yz.y, nf = fv.n;
-   const T*      f    = fine + fv.cell_off[c];
-   const int64_t cb   = cv.cell_off[c] + cidx( cv.n, 0, y, z );
-   const int     xmax = cv.n - 1 - y - z;
-   for ( int x = 1 + lane; x <= xmax; x += 32 )
+   constexpr int dx = StencilDir< D >::x, dy = StencilDir< D >::y, dz = StencilDir< D >::z;
+   constexpr int out = CLS == 1 ? dz : CLS == 2 ? dy : CLS == 3 ? dx : -( dx + dy + dz );  // steps away from the face
+   if constexpr ( D == 0 || out < 0 ) return;
+   else s[out == 0 ? 0 : 1] += A( ldv( f + ( row_shift< dy, dz >( nf, Y, Z ) + dx ) ) );
+}
+template < int CLS, typename T, typename A, int... D >
+__device__ __forceinline__ A fine_face_sum( const T* f, int nf, int Y, int Z, A share, std::integer_sequence< int, D... > )
+{
+   A s[2] = { A( 0 ), A( 0 ) };
+   ( fine_face_term< D, CLS, T, A >( f, nf, Y, Z, s ), ... );
+   return share * A( ldv( f ) ) + A( 0.5 ) * ( share * s[0] + s[1] );
+}
+// one cell's part at a coarse face point of slot c, row y and slice z; share: 1 / (cells of the face)
+template < typename T, typename A >
+__device__ __forceinline__ A restrict_face( const LevelView& cv, const LevelView& fv, const T* fine, int cell, int cls, int64_t c, int y, int z, A share )
+{
+   const int  x = int( c - cv.cell_off[cell] - cidx( cv.n, 0, y, z ) );
+   const T*   f = fine + fv.cell_off[cell] + cidx( fv.n, 2 * x, 2 * y, 2 * z );
+   constexpr auto all = std::make_integer_sequence< int, kNumDirs >();
+   switch ( cls )
    {
-      const int X = 2 * x, Y = 2 * y, Z = 2 * z;
-      A         leaves = A( 0 );
+   case 1: return fine_face_sum< 1, T, A >( f, fv.n, 2 * y, 2 * z, share, all );
+   case 2: return fine_face_sum< 2, T, A >( f, fv.n, 2 * y, 2 * z, share, all );
+   case 3: return fine_face_sum< 3, T, A >( f, fv.n, 2 * y, 2 * z, share, all );
+   default: return fine_face_sum< 4, T, A >( f, fv.n, 2 * y, 2 * z, share, all );
+   }
+}
+// one cell's part at a coarse edge or vertex point
+template < typename T, typename A >
+__device__ __forceinline__ A restrict_low( const LevelView& fv, const T* fine, const IncRec& I )
+{
+   const int      nf = fv.n, X = 2 * I.x, Y = 2 * I.y, Z = 2 * I.z;
+   const T*       f    = fine + fv.cell_off[I.cell];
+   const float*   ncc  = fv.ncell_cls + size_t( I.cell ) * kNumClasses;
+   const uint16_t mask = c_cls_mask[I.cls];
+   A              part = A( ldv( f + cidx( nf, X, Y, Z ) ) ) / A( ncc[I.cls] );
 #pragma unroll
-      for ( int d = 1; d < kNumDirs; ++d )
-         leaves += A( ldv( f + cidx( nf, X + c_dirs[d][0], Y + c_dirs[d][1], Z + c_dirs[d][2] ) ) );
-      stv( coarse + cb + x, A( ldv( f + cidx( nf, X, Y, Z ) ) ) + A( 0.5 ) * leaves );
-   }
+   for ( int d = 1; d < kNumDirs; ++d )
+      if ( mask & ( 1u << d ) )
+      {
+         const int px = X + c_dirs[d][0], py = Y + c_dirs[d][1], pz = Z + c_dirs[d][2];
+         part += A( 0.5 ) / A( ncc[point_class( nf, px, py, pz )] ) * A( ldv( f + cidx( nf, px, py, pz ) ) );
+      }
+   return part;
 }
 
+// the boundary task of thread t: an edge or vertex (eight threads: record and this thread's share of its
+// incidences) or a face (one thread); BND_NONE where the thread has none
+enum { BND_NONE = 0, BND_LOW, BND_FACE };
+__device__ __forceinline__ int bnd_thread( const LevelView& v, const BndSegments& seg, int t, LowRec& low, int& sub, FaceRec& face )
+{
+#pragma unroll
+   for ( int g = 0; g < 4; ++g )
+   {
+      if ( t < seg.lthreads[g] )
+      {
+         const bool live = ( t >> 3 ) < seg.lcount[g];
+         low             = v.lrec[seg.lstart[g] + ( live ? t >> 3 : 0 )];
+         if ( !live ) low.count = 0;
+         sub = t & 7;
+         return BND_LOW;  // whole warps: a thread without a task has no incidences
+      }
+      t -= seg.lthreads[g];
+   }
+#pragma unroll
+   for ( int g = 0; g < 4; ++g )
+   {
+      if ( t >= 0 && t < seg.fcount[g] )
+      {
+         face = v.frec[seg.fstart[g] + t];
+         return BND_FACE;
+      }
+      t -= seg.fcount[g];
+   }
+   return BND_NONE;
+}
 template < typename T, typename A >
-__global__ void __launch_bounds__( 256 ) k_restrict_bnd( LevelView cv, LevelView fv, uint32_t flag, const T* __restrict__ fine,
-                                                          T* coarse )
+__device__ __forceinline__ void put_low( const LevelView& v, const LowRec& r, int sub, T* vec, A val )
 {
-   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-   if ( t >= cv.ntasks ) return;
-   const int4 tk = cv.tasks[t];
-   const int  b = tk.x, i = tk.y, j = tk.z;
-   if ( !( cv.bc[b] & flag ) ) return;
-   const int nf  = fv.n;
-   A         acc = A( 0 );
-   for ( int q = cv.inc_begin[b]; q < cv.inc_begin[b + 1]; ++q )
-   {
-      const Incidence I = cv.inc[q];
-      int             x, y, z;
-      inc_point( I, cv.n, i, j, x, y, z );
-      const int      X = 2 * x, Y = 2 * y, Z = 2 * z;
-      const T*       f    = fine + fv.cell_off[I.cell];
-      const float*   ncc  = fv.ncell_cls + size_t( I.cell ) * kNumClasses;
-      const uint16_t mask = c_cls_mask[I.cls];
-      A              part = A( ldv( f + cidx( nf, X, Y, Z ) ) ) / A( ncc[I.cls] );
-      for ( int d = 1; d < kNumDirs; ++d )
-         if ( mask & ( 1u << d ) )
-         {
-            const int px = X + c_dirs[d][0], py = Y + c_dirs[d][1], pz = Z + c_dirs[d][2];
-            part += A( 0.5 ) / A( ncc[point_class( nf, px, py, pz )] ) * A( ldv( f + cidx( nf, px, py, pz ) ) );
-         }
-      acc += part;
-   }
-   write_through( cv, coarse, b, i, j, owner_slot( cv, b, i, j ), acc );
+   if ( r.count > 0 && sub == 0 ) stv( vec + r.owner, val );
+   for ( int q = sub; q < r.count; q += 8 ) stv( vec + v.irec[r.begin + q].slot, val );
+}
+template < typename T, typename A >
+__device__ __forceinline__ void put_face( const FaceRec& r, T* vec, A val )
+{
+   stv( vec + r.owner, val );
+   stv( vec + r.c0, val );
+   if ( r.cell1 >= 0 ) stv( vec + r.c1, val );
 }
 
-// coarse micro-edge through an odd fine point: direction per odd-coordinate pattern
-__device__ __forceinline__ void parity_dir( int x, int y, int z, int& dx, int& dy, int& dz )
+// Interior point of thread or warp `unit` of a cell sweep: the listed points for levels up to kFlatMaxN
+// (one thread per point), warps over rows above
+template < typename F >
+__device__ __forceinline__ void for_interior( const LevelView& v, int nC, uint32_t flag, int block, F f )
 {
-   const int p = ( x & 1 ) | ( ( y & 1 ) << 1 ) | ( ( z & 1 ) << 2 );
-   dx = dy = dz = 0;
-   switch ( p )
+   if ( v.n <= kFlatMaxN )
    {
-   case 1: dx = 1; break;
-   case 2: dy = 1; break;
-   case 4: dz = 1; break;
-   case 3: dx = 1, dy = -1; break;
-   case 5: dx = 1, dz = -1; break;
-   case 6: dy = 1, dz = -1; break;
-   case 7: dx = 1, dy = -1, dz = 1; break;
-   default: break;
+      const int64_t g = int64_t( block ) * 256 + threadIdx.x;
+      if ( g >= int64_t( nC ) * v.nipts ) return;
+      const int c = g < 0x7fffffff ? int( unsigned( g ) / unsigned( v.nipts ) ) : int( g / v.nipts );
+      if ( !( v.cell_bc[c] & flag ) ) return;
+      const ushort4 p = v.ipts[int( g - int64_t( c ) * v.nipts )];
+      f( c, int( p.x ), int( p.y ), int( p.z ), v.n );
+      return;
    }
+   const int64_t w = int64_t( block ) * 8 + ( threadIdx.x >> 5 );
+   if ( w >= int64_t( nC ) * v.nrows ) return;
+   const int c = int( unsigned( w ) / unsigned( v.nrows ) );
+   if ( !( v.cell_bc[c] & flag ) ) return;
+   const int2 yz = v.rows[int( w - int64_t( c ) * v.nrows )];
+   f( c, 1 + int( threadIdx.x & 31 ), yz.x, yz.y, 32 );
+}
+static int interior_blocks( const LevelView& v, int nC )
+{
+   return int( v.n <= kFlatMaxN ? ( int64_t( nC ) * v.nipts + 255 ) / 256 : ( int64_t( nC ) * v.nrows + 7 ) / 8 );
 }
 
+template < int D, typename T, typename A >
+__device__ __forceinline__ void fine_term( const T* f, int nf, int Y, int Z, A ( &s )[2] )
+{
+   if constexpr ( D > 0 ) s[D & 1] += A( ldv( f + ( row_shift< StencilDir< D >::y, StencilDir< D >::z >( nf, Y, Z ) + StencilDir< D >::x ) ) );
+}
+template < typename T, typename A, int... D >
+__device__ __forceinline__ A fine_sum( const T* f, int nf, int Y, int Z, std::integer_sequence< int, D... > )
+{
+   A s[2] = { A( 0 ), A( 0 ) };
+   ( fine_term< D, T, A >( f, nf, Y, Z, s ), ... );
+   return A( ldv( f ) ) + A( 0.5 ) * ( s[0] + s[1] );
+}
+
+// Restriction, boundary tasks and cell interiors in one launch.  Bound by the fine vector's read; the row
+// starts of the 14 neighbours follow from the point's own by a few integer operations each (computing every
+// neighbour's index anew was most of the work), and the cells of an edge or vertex are shared by eight
+// threads.  TRANSFER_R
+template < typename T, typename A >
+__global__ void __launch_bounds__( 256 ) k_restrict( LevelView cv, LevelView fv, BndSegments seg, int nbnd, int nC, uint32_t flag,
+                                                      const T* __restrict__ fine, T* coarse )
+{
+   if ( int( blockIdx.x ) < nbnd )
+   {
+      LowRec    low;
+      FaceRec   face;
+      int       sub;
+      const int kind = bnd_thread( cv, seg, blockIdx.x * 256 + threadIdx.x, low, sub, face );
+      if ( kind == BND_LOW )
+      {
+         A s = A( 0 );
+         for ( int q = sub; q < low.count; q += 8 ) s += restrict_low< T, A >( fv, fine, cv.irec[low.begin + q] );
+#pragma unroll
+         for ( int m = 4; m > 0; m >>= 1 ) s += __shfl_xor_sync( 0xffffffffu, s, m, 8 );
+         put_low( cv, low, sub, coarse, s );
+      }
+      else if ( kind == BND_FACE )
+      {
+         const A share = face.cell1 >= 0 ? A( 0.5 ) : A( 1 );
+         A       s     = restrict_face< T, A >( cv, fv, fine, face.cell0, face.cls0, face.c0, face.y0, face.z0, share );
+         if ( face.cell1 >= 0 ) s += restrict_face< T, A >( cv, fv, fine, face.cell1, face.cls1, face.c1, face.y1, face.z1, share );
+         put_face( face, coarse, s );
+      }
+      return;
+   }
+   for_interior( cv, nC, flag, blockIdx.x - nbnd, [&]( int c, int x0, int y, int z, int step ) {
+      const T* f  = fine + fv.cell_off[c] + cidx( fv.n, 0, 2 * y, 2 * z );
+      T*       co = coarse + cv.cell_off[c] + cidx( cv.n, 0, y, z );
+      for ( int x = x0; x < cv.n - y - z; x += step )
+         stv( co + x, fine_sum< T, A >( f + 2 * x, fv.n, 2 * y, 2 * z, std::make_integer_sequence< int, kNumDirs >() ) );
+   } );
+}
+
+// Linear interpolation at the fine point (x, y, z): the mean of the two ends of the coarse micro-edge the
+// point halves (twice the same node for a coarse one).  The ends lie at floor(x / 2) of one coarse row and
+// ceil(x / 2) of another, and the rows depend on y and z only.
+__device__ __forceinline__ void coarse_rows( int nc, int y, int z, int64_t& lo, int64_t& hi )
+{
+   const int yo = y & 1, zo = z & 1, zl = z >> 1;
+   lo = cidx( nc, 0, ( y + yo ) >> 1, zo && !yo ? zl + 1 : zl );
+   hi = cidx( nc, 0, y >> 1, zo && yo ? zl + 1 : zl );
+}
 template < typename T, typename A >
 __device__ __forceinline__ A interp( const T* c, int nc, int x, int y, int z )
 {
-   int dx, dy, dz;
-   parity_dir( x, y, z, dx, dy, dz );
-   if ( ( dx | dy | dz ) == 0 ) return A( ldv( c + cidx( nc, x >> 1, y >> 1, z >> 1 ) ) );
-   const A a = A( ldv( c + cidx( nc, ( x - dx ) >> 1, ( y - dy ) >> 1, ( z - dz ) >> 1 ) ) );
-   const A b = A( ldv( c + cidx( nc, ( x + dx ) >> 1, ( y + dy ) >> 1, ( z + dz ) >> 1 ) ) );
-   return A( 0.5 ) * a + A( 0.5 ) * b;
+   int64_t lo, hi;
+   coarse_rows( nc, y, z, lo, hi );
+   return A( 0.5 ) * ( A( ldv( c + lo + ( x >> 1 ) ) ) + A( ldv( c + hi + ( ( x + 1 ) >> 1 ) ) ) );
 }
 
+// Prolongation, boundary tasks and cell interiors in one launch: bound by the fine vector (TRANSFER_P)
 template < typename T, typename A >
-__global__ void __launch_bounds__( 256 ) k_prolong_cells( LevelView cv, LevelView fv, uint32_t flag, const T* __restrict__ coarse,
-                                                           T* fine, int add )
+__global__ void __launch_bounds__( 256 ) k_prolong( LevelView cv, LevelView fv, BndSegments seg, int nbnd, int nC, uint32_t flag,
+                                                     const T* __restrict__ coarse, T* fine, int add )
 {
-   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int r    = blockIdx.x * 8 + warp;
-   const int c    = blockIdx.y;
-   if ( r >= fv.nrows ) return;
-   if ( !( fv.cell_bc[c] & flag ) ) return;
-   const int2    yz   = fv.rows[r];
-   const int     y = yz.x, z = yz.y;
-   const T*      cc   = coarse + cv.cell_off[c];
-   const int64_t fb   = fv.cell_off[c] + cidx( fv.n, 0, y, z );
-   const int     xmax = fv.n - 1 - y - z;
-   for ( int x = 1 + lane; x <= xmax; x += 32 )
+   if ( int( blockIdx.x ) < nbnd )
    {
-      const A val = interp< T, A >( cc, cv.n, x, y, z );
-      stv( fine + fb + x, add ? A( ldc( fine + fb + x ) ) + val : val );
+      LowRec    low;
+      FaceRec   face;
+      int       sub;
+      const int kind = bnd_thread( fv, seg, blockIdx.x * 256 + threadIdx.x, low, sub, face );
+      if ( kind == BND_LOW )
+      {
+         A val = A( 0 );
+         if ( low.count > 0 )
+         {
+            const IncRec I = fv.irec[low.begin];
+            val            = interp< T, A >( coarse + cv.cell_off[I.cell], cv.n, I.x, I.y, I.z );
+            if ( add ) val += A( ldc( fine + low.owner ) );
+         }
+         __syncwarp();  // every thread of a task has read the owner before any writes it
+         put_low( fv, low, sub, fine, val );
+      }
+      else if ( kind == BND_FACE )
+      {
+         const int x   = int( face.c0 - fv.cell_off[face.cell0] - cidx( fv.n, 0, face.y0, face.z0 ) );
+         A         val = interp< T, A >( coarse + cv.cell_off[face.cell0], cv.n, x, face.y0, face.z0 );
+         if ( add ) val += A( ldc( fine + face.owner ) );
+         put_face( face, fine, val );
+      }
+      return;
    }
-}
-
-template < typename T, typename A >
-__global__ void __launch_bounds__( 256 ) k_prolong_bnd( LevelView cv, LevelView fv, uint32_t flag, const T* __restrict__ coarse,
-                                                         T* fine, int add )
-{
-   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-   if ( t >= fv.ntasks ) return;
-   const int4 tk = fv.tasks[t];
-   const int  b = tk.x, i = tk.y, j = tk.z;
-   if ( !( fv.bc[b] & flag ) ) return;
-   const Incidence I = fv.inc[fv.inc_begin[b]];
-   int             x, y, z;
-   inc_point( I, fv.n, i, j, x, y, z );
-   const A       val   = interp< T, A >( coarse + cv.cell_off[I.cell], cv.n, x, y, z );
-   const int64_t owner = owner_slot( fv, b, i, j );
-   write_through( fv, fine, b, i, j, owner, add ? A( ldc( fine + owner ) ) + val : val );
+   for_interior( fv, nC, flag, blockIdx.x - nbnd, [&]( int c, int x0, int y, int z, int step ) {
+      int64_t lo, hi;
+      coarse_rows( cv.n, y, z, lo, hi );
+      const T* cc = coarse + cv.cell_off[c];
+      T*       f  = fine + fv.cell_off[c] + cidx( fv.n, 0, y, z );
+      for ( int x = x0; x < fv.n - y - z; x += step )
+      {
+         const A val = A( 0.5 ) * ( A( ldv( cc + lo + ( x >> 1 ) ) ) + A( ldv( cc + hi + ( ( x + 1 ) >> 1 ) ) ) );
+         stv( f + x, add ? A( ldc( f + x ) ) + val : val );
+      }
+   } );
 }
 
 template < typename T, typename A >
 static void run_restrict( Context* ctx, const LevelView& cv, const LevelView& fv, int nC, uint32_t flag, const void* fine,
                           void* coarse )
 {
-   Fork fk( ctx );
-   if ( cv.nrows > 0 && nC > 0 )
-   {
-      dim3 grid( ( cv.nrows + 7 ) / 8, nC );
-      k_restrict_cells< T, A ><<< grid, 256, 0, ctx->stream >>>( cv, fv, flag, (const T*) fine, (T*) coarse );
-      ++ctx->launches;
-   }
-   if ( cv.ntasks > 0 )
-   {
-      k_restrict_bnd< T, A ><<< ( cv.ntasks + 255 ) / 256, 256, 0, fk.aux() >>>( cv, fv, flag, (const T*) fine, (T*) coarse );
-      ++ctx->launches;
-   }
+   const BndSegments seg  = bnd_segments( cv, flag, 0 );
+   const int         nbnd = ( seg.threads + 255 ) / 256, blocks = nbnd + interior_blocks( cv, nC );
+   if ( blocks == 0 ) return;
+   k_restrict< T, A ><<< blocks, 256, 0, ctx->stream >>>( cv, fv, seg, nbnd, nC, flag, (const T*) fine, (T*) coarse );
+   ++ctx->launches;
    check_cuda( cudaGetLastError(), "restrict launch" );
 }
 
@@ -1835,19 +1940,11 @@ template < typename T, typename A >
 static void run_prolong( Context* ctx, const LevelView& cv, const LevelView& fv, int nC, uint32_t flag, const void* coarse,
                          void* fine, int add )
 {
-   Fork fk( ctx );
-   if ( fv.nrows > 0 && nC > 0 )
-   {
-      dim3 grid( ( fv.nrows + 7 ) / 8, nC );
-      k_prolong_cells< T, A ><<< grid, 256, 0, ctx->stream >>>( cv, fv, flag, (const T*) coarse, (T*) fine, add );
-      ++ctx->launches;
-   }
-   if ( fv.ntasks > 0 )
-   {
-      k_prolong_bnd< T, A ><<< ( fv.ntasks + 255 ) / 256, 256, 0, fk.aux() >>>( cv, fv, flag, (const T*) coarse, (T*) fine,
-                                                                                     add );
-      ++ctx->launches;
-   }
+   const BndSegments seg  = bnd_segments( fv, flag, 0 );
+   const int         nbnd = ( seg.threads + 255 ) / 256, blocks = nbnd + interior_blocks( fv, nC );
+   if ( blocks == 0 ) return;
+   k_prolong< T, A ><<< blocks, 256, 0, ctx->stream >>>( cv, fv, seg, nbnd, nC, flag, (const T*) coarse, (T*) fine, add );
+   ++ctx->launches;
    check_cuda( cudaGetLastError(), "prolongate launch" );
 }
 
