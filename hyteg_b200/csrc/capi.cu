@@ -1660,6 +1660,8 @@ static void cycle_rec( hyb_gmg* g, hyb_fn* x, hyb_fn* b, int L, int invoked, boo
    const int dt = x->f.dtype;
    if ( L == g->p.min_level )
    {
+      // a coarse level without unknowns (found by coarse_probe): the zero guess is the solution
+      if ( !host_checks && g->coarse_cap == 0 && L < invoked ) return;
       if ( g->cgx64 )
       {
          // coarse-grid solve in FP64 for a low-precision hierarchy
@@ -1678,9 +1680,14 @@ static void cycle_rec( hyb_gmg* g, hyb_fn* x, hyb_fn* b, int L, int invoked, boo
    for ( int i = 0; i < pre; ++i ) smooth( g, x, b, L );
    // residual, restricted straight into b on level L-1 (b.assign({1},{tmp},L-1,flag) of the reference)
    stencil( op, L, dt, OP_RESID, kSolveFlag, 0, x->f.ptr( L ), b->f.ptr( L ), nullptr, g->tmp->f.ptr( L ) );
-   if ( op->o.order == 2 ) launch_p2_restrict( &cx, op->o.mesh, L, dt, kSolveFlag, g->tmp->f.ptr( L ), b->f.ptr( L - 1 ) );
-   else launch_restrict( &cx, op->o.mesh, L, dt, kSolveFlag, g->tmp->f.ptr( L ), b->f.ptr( L - 1 ) );
-   check_cuda( cudaMemsetAsync( x->f.ptr( L - 1 ), 0, x->f.bytes( L - 1 ), cx.stream ), "x.interpolate(0)" );
+   // (and x.interpolate(0) on level L-1)
+   if ( op->o.order == 2 )
+   {
+      launch_p2_restrict( &cx, op->o.mesh, L, dt, kSolveFlag, g->tmp->f.ptr( L ), b->f.ptr( L - 1 ) );
+      check_cuda( cudaMemsetAsync( x->f.ptr( L - 1 ), 0, x->f.bytes( L - 1 ), cx.stream ), "x.interpolate(0)" );
+   }
+   else
+      launch_restrict( &cx, op->o.mesh, L, dt, kSolveFlag, g->tmp->f.ptr( L ), b->f.ptr( L - 1 ), x->f.ptr( L - 1 ), x->f.bytes( L - 1 ) );
    cycle_rec( g, x, b, L - 1, invoked, host_checks );
    if ( g->p.cycle == HYB_WCYCLE ) cycle_rec( g, x, b, L - 1, invoked, host_checks );
    if ( op->o.order == 2 ) launch_p2_prolongate( &cx, op->o.mesh, L - 1, dt, kSolveFlag, x->f.ptr( L - 1 ), x->f.ptr( L ), 1 );

@@ -294,6 +294,104 @@ struct StencilDir {
 // offset of slice z+1 minus offset of slice z in a macro-cell array (tri(n+1-z) points in slice z)
 __device__ __forceinline__ int64_t slice_step( int n, int z ) { return int64_t( n + 1 - z ) * ( n + 2 - z ) / 2; }
 
+// value of an operation at an owner from the stencil sum, and the second vector's value (Chebyshev steps)
+// (op is a compile-time value after inlining where the caller has one)
+template < typename T, typename A >
+__device__ __forceinline__ A owner_value( int op, int64_t o, A s, A invd, const T* src, const T* v1, const T* v2, const T* dst, A a0, A a1, A& second )
+{
+   if ( op == OP_APPLY_ADD ) return A( ldc( dst + o ) ) + s;
+   else if ( op == OP_RESID ) return A( ldv( v1 + o ) ) - s;
+   else if ( op == OP_JAC ) return A( ldv( src + o ) ) + a0 * ( invd * ( A( ldv( v1 + o ) ) - s ) );
+   else if ( op == OP_CHEB0 ) return invd * ( A( ldv( v1 + o ) ) - s );
+   else if ( op == OP_CHEBI )
+   {
+      second = A( ldc( v2 + o ) ) + a0 * A( ldv( src + o ) );
+      return invd * s;
+   }
+   else if ( op == OP_CHEBL ) return ( A( ldc( v2 + o ) ) + a0 * A( ldv( src + o ) ) ) + a1 * ( invd * s );
+   else if ( op == OP_DINV_APPLY ) return invd * s;
+   else return s;
+}
+
+// The boundary tasks of the selected types: edges and vertices first, eight threads each (from
+// threads lat on, a multiple of 32 per type), then faces, one thread each (or per_face: one per cell)
+struct BndSegments
+{
+   int lstart[4], lthreads[4], lcount[4];
+   int fstart[4], fcount[4];
+   int threads;
+};
+
+static inline BndSegments bnd_segments( const LevelView& v, uint32_t flag, int all, int per_face = 1 )
+{
+   static const uint32_t type_bit[4] = { kInner, kDirichlet, kNeumann, kFreeslip };
+   BndSegments           s{};
+   int                   k = 0, lat = 0, fat = 0;
+   for ( int g = 0; g < 4; ++g )
+   {
+      if ( all || ( flag & type_bit[g] ) )
+      {
+         s.lstart[k]   = lat;
+         s.lcount[k]   = v.nlow[g];
+         s.lthreads[k] = ( 8 * v.nlow[g] + 31 ) / 32 * 32;
+         s.fstart[k]   = fat;
+         s.fcount[k]   = per_face * v.nface[g];
+         s.threads += s.lthreads[k] + s.fcount[k];
+         ++k;
+      }
+      lat += v.nlow[g];
+      fat += v.nface[g];
+   }
+   return s;
+}
+
+// the boundary task of thread t: an edge or vertex (eight threads: record and this thread's share of its
+// incidences) or a face (one thread); BND_NONE where the thread has none
+enum { BND_NONE = 0, BND_LOW, BND_FACE };
+// (F threads per face; a face's thread finds its number in sub)
+template < int F >
+__device__ __forceinline__ int bnd_thread( const LevelView& v, const FaceRec* frec, const BndSegments& seg, int t, LowRec& low, int& sub, FaceRec& face )
+{
+#pragma unroll
+   for ( int g = 0; g < 4; ++g )
+   {
+      if ( t < seg.lthreads[g] )
+      {
+         const bool live = ( t >> 3 ) < seg.lcount[g];
+         low             = v.lrec[seg.lstart[g] + ( live ? t >> 3 : 0 )];
+         if ( !live ) low.count = 0;
+         sub = t & 7;
+         return BND_LOW;  // whole warps: a thread without a task has no incidences
+      }
+      t -= seg.lthreads[g];
+   }
+#pragma unroll
+   for ( int g = 0; g < 4; ++g )
+   {
+      if ( t >= 0 && t < seg.fcount[g] )
+      {
+         face = frec[seg.fstart[g] + t / F];
+         sub  = t % F;
+         return BND_FACE;
+      }
+      t -= seg.fcount[g];
+   }
+   return BND_NONE;
+}
+template < typename T, typename A >
+__device__ __forceinline__ void put_low( const LevelView& v, const LowRec& r, int sub, T* vec, A val )
+{
+   if ( r.count > 0 && sub == 0 ) stv( vec + r.owner, val );
+   for ( int q = sub; q < r.count; q += 8 ) stv( vec + v.irec[r.begin + q].slot, val );
+}
+template < typename T, typename A >
+__device__ __forceinline__ void put_face( const FaceRec& r, T* vec, A val )
+{
+   stv( vec + r.owner, val );
+   stv( vec + r.c0, val );
+   if ( r.cell1 >= 0 ) stv( vec + r.c1, val );
+}
+
 // epilogue of a stencil operation at slot i: s = (A src)_i; invd the inverse diagonal at the point
 template < typename T, typename A, int OP >
 __device__ __forceinline__ void stencil_epilogue( int64_t i, A s, A invd, const T* src, const T* v1, T* v2, T* dst, A a0, A a1 )

@@ -150,6 +150,8 @@ struct Topology {
 // BPS.
 // points per macro-edge up to which cell interiors run one thread per point (k_flat_stencil)
 constexpr int kFlatMaxN    = 64;
+// the same for the P2 constant stencils
+constexpr int kP2cFlatMaxN = 64;
 constexpr int kSwR         = 4;
 constexpr int kSwTX        = 64;  // 32 or 64
 constexpr int kSwWarps     = 4;
@@ -237,10 +239,11 @@ struct Function {
 // eight interior inverse diagonals), FP64 and an FP32 copy
 struct P2cLevel {
    std::vector< double > W;      // [nC][kP2cCellStride]
-   std::vector< int4 >   tasks;  // boundary tasks grouped by boundary type, then by primitive and parity class
-   double* d_W     = nullptr;
-   float*  d_Wf    = nullptr;
-   int4*   d_tasks = nullptr;
+   double*  d_W    = nullptr;
+   float*   d_Wf   = nullptr;
+   FaceRec* d_frec = nullptr;  // the level's face records, inside a boundary type by face and parity class
+   void*    d_pts  = nullptr;  // interior points of a macro-cell by parity class (ushort4), n <= kP2cFlatMaxN
+   int      np[8]  = {};
 };
 
 struct OpLevel {
@@ -396,7 +399,7 @@ void launch_repack_map( Context* ctx, int64_t count, int np, const int64_t* poff
 void launch_p2_constant( Context* ctx, Mesh* m, Operator* A, int Ls, int dtype, const StencilArgs& a );
 void build_p2_constant_level( Operator* A, int Ls );
 void ensure_p2_constant_device();
-void ensure_p2_constant_tables( P2cLevel& pl );
+void ensure_p2_constant_tables( Operator* A, int Ls );
 void p2_constant_inverse_diagonal( const Operator* A, int Ls, uint32_t flag, std::vector< double >& padded );
 void ensure_p2_constants();
 void launch_p2_restrict( Context* ctx, Mesh* m, int Lf, int dtype, uint32_t flag, const void* fine, void* coarse );
@@ -459,7 +462,9 @@ void launch_repack( Context* ctx, Mesh* m, int L, int dtype, int to_padded, doub
 // deterministic dot over owned flagged DoFs -> *out (device)
 void launch_dot( Context* ctx, Mesh* m, int L, int dtype, uint32_t flag, const void* a, const void* b, double* out );
 void launch_dot_noalloc( Context* ctx, Mesh* m, int L, int dtype, uint32_t flag, const void* a, const void* b, double* host_out );
-void launch_restrict( Context* ctx, Mesh* m, int Lfine, int dtype, uint32_t flag, const void* fine, void* coarse );
+// zero, when given, is cleared by the same launch (a level vector: whole multiples of 16 bytes)
+void launch_restrict( Context* ctx, Mesh* m, int Lfine, int dtype, uint32_t flag, const void* fine, void* coarse, void* zero = nullptr,
+                      size_t zero_bytes = 0 );
 void launch_prolongate( Context* ctx, Mesh* m, int Lcoarse, int dtype, uint32_t flag, const void* coarse, void* fine, int add );
 void launch_axpy_to_f64( Context* ctx, int64_t count, double* x, int src_dtype, const void* c, double a );
 void prepare_device( Context* ctx, Mesh* m, Operator* op, int minL, int maxL, int dtype );

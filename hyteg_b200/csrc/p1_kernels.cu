@@ -830,56 +830,6 @@ __device__ __forceinline__ A face_stencil( const T* c, const A* W, int cls, int 
    }
 }
 
-// value of an operation at an owner from the stencil sum, and the second vector's value (Chebyshev steps)
-template < typename T, typename A, int OP >
-__device__ __forceinline__ A owner_value( int64_t o, A s, A invd, const T* src, const T* v1, const T* v2, const T* dst, A a0, A a1, A& second )
-{
-   if constexpr ( OP == OP_APPLY_ADD ) return A( ldc( dst + o ) ) + s;
-   else if constexpr ( OP == OP_RESID ) return A( ldv( v1 + o ) ) - s;
-   else if constexpr ( OP == OP_JAC ) return A( ldv( src + o ) ) + a0 * ( invd * ( A( ldv( v1 + o ) ) - s ) );
-   else if constexpr ( OP == OP_CHEB0 ) return invd * ( A( ldv( v1 + o ) ) - s );
-   else if constexpr ( OP == OP_CHEBI )
-   {
-      second = A( ldc( v2 + o ) ) + a0 * A( ldv( src + o ) );
-      return invd * s;
-   }
-   else if constexpr ( OP == OP_CHEBL ) return ( A( ldc( v2 + o ) ) + a0 * A( ldv( src + o ) ) ) + a1 * ( invd * s );
-   else if constexpr ( OP == OP_DINV_APPLY ) return invd * s;
-   else return s;
-}
-
-// The boundary tasks of the selected types: edges and vertices first, eight threads each (from
-// threads lat on, a multiple of 32 per type), then faces, one thread each
-struct BndSegments
-{
-   int lstart[4], lthreads[4], lcount[4];
-   int fstart[4], fcount[4];
-   int threads;
-};
-
-static inline BndSegments bnd_segments( const LevelView& v, uint32_t flag, int all )
-{
-   static const uint32_t type_bit[4] = { kInner, kDirichlet, kNeumann, kFreeslip };
-   BndSegments           s{};
-   int                   k = 0, lat = 0, fat = 0;
-   for ( int g = 0; g < 4; ++g )
-   {
-      if ( all || ( flag & type_bit[g] ) )
-      {
-         s.lstart[k]   = lat;
-         s.lcount[k]   = v.nlow[g];
-         s.lthreads[k] = ( 8 * v.nlow[g] + 31 ) / 32 * 32;
-         s.fstart[k]   = fat;
-         s.fcount[k]   = v.nface[g];
-         s.threads += s.lthreads[k] + s.fcount[k];
-         ++k;
-      }
-      lat += v.nlow[g];
-      fat += v.nface[g];
-   }
-   return s;
-}
-
 // One boundary task: the sum over its neighbour cells of the stencil of its position class in each, the
 // operation's epilogue, and the write to the owner and every copy in the neighbouring cell arrays.  Every
 // index comes from the task's records, so the values wait on one dependent load for a face and on two for
@@ -889,61 +839,38 @@ template < typename T, typename A, int OP >
 __device__ __forceinline__ void bnd_point( const LevelView& v, const OpView< A >& o, const BndSegments& seg, int t, uint32_t flag,
                                            int copy_unflagged, const T* __restrict__ src, const T* __restrict__ v1, T* v2, T* dst, A a0, A a1 )
 {
-#pragma unroll
-   for ( int g = 0; g < 4; ++g )  // unrolled: the segment arrays are read with constant indices
+   LowRec    low;
+   FaceRec   r;
+   int       sub;
+   const int kind = bnd_thread< 1 >( v, v.frec, seg, t, low, sub, r );
+   if ( kind == BND_NONE ) return;
+   if ( kind == BND_LOW )
    {
-      if ( t < seg.lthreads[g] )
+      const bool flagged = ( low.bc & flag ) != 0;
+      if ( !flagged && !copy_unflagged ) low.count = 0;
+      A val = A( 0 ), second = A( 0 ), s = A( 0 );
+      if ( flagged )
+         for ( int q = sub; q < low.count; q += 8 )
+         {
+            const IncRec I = v.irec[low.begin + q];
+            s += class_stencil_slot< T, A >( src, o.W + ( size_t( I.cell ) * kNumClasses + I.cls ) * kNumDirs, c_cls_mask[I.cls], v.n, I.slot,
+                                             I.y, I.z );
+         }
+#pragma unroll
+      for ( int m = 4; m > 0; m >>= 1 ) s += __shfl_xor_sync( 0xffffffffu, s, m, 8 );
+      if ( low.count > 0 )
       {
-         const int  k = t >> 3, sub = t & 7;
-         const bool live = k < seg.lcount[g];
-         LowRec     r    = v.lrec[seg.lstart[g] + ( live ? k : 0 )];
-         const bool flagged = ( r.bc & flag ) != 0;
-         if ( !live || ( !flagged && !copy_unflagged ) ) r.count = 0;
-         A val = A( 0 ), second = A( 0 ), s = A( 0 );
-         if ( flagged )
-         {
-            for ( int q = sub; q < r.count; q += 8 )
-            {
-               const IncRec I = v.irec[r.begin + q];
-               s += class_stencil_slot< T, A >( src, o.W + ( size_t( I.cell ) * kNumClasses + I.cls ) * kNumDirs, c_cls_mask[I.cls], v.n,
-                                                I.slot, I.y, I.z );
-            }
-         }
-#pragma unroll
-         for ( int m = 4; m > 0; m >>= 1 ) s += __shfl_xor_sync( 0xffffffffu, s, m, 8 );
-         if ( r.count > 0 )
-         {
-            if ( flagged ) val = owner_value< T, A, OP >( r.owner, s, o.invd_b[r.b], src, v1, v2, dst, a0, a1, second );
-            else if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) val = A( ldv( src + r.owner ) );
-            else if constexpr ( OP == OP_CHEBI ) val = A( ldc( v2 + r.owner ) );
-         }
-         __syncwarp();  // every thread of a task has read the owner before any writes it
-         auto put = [&]( T* vec, A x ) {
-            if ( r.count > 0 && sub == 0 ) stv( vec + r.owner, x );
-            for ( int q = sub; q < r.count; q += 8 ) stv( vec + v.irec[r.begin + q].slot, x );
-         };
-         if constexpr ( OP == OP_CHEBL ) put( v2, val );
-         else put( dst, val );
-         if constexpr ( OP == OP_CHEBI )
-            if ( flagged ) put( v2, second );
-         return;
+         if ( flagged ) val = owner_value< T, A >( OP, low.owner, s, o.invd_b[low.b], src, v1, v2, dst, a0, a1, second );
+         else if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) val = A( ldv( src + low.owner ) );
+         else if constexpr ( OP == OP_CHEBI ) val = A( ldc( v2 + low.owner ) );
       }
-      t -= seg.lthreads[g];
+      __syncwarp();  // every thread of a task has read the owner before any writes it
+      put_low( v, low, sub, OP == OP_CHEBL ? v2 : dst, val );
+      if constexpr ( OP == OP_CHEBI )
+         if ( flagged ) put_low( v, low, sub, v2, second );
+      return;
    }
-   int at = -1;
-#pragma unroll
-   for ( int g = 0; g < 4; ++g )
-   {
-      if ( at < 0 && t < seg.fcount[g] ) at = seg.fstart[g] + t;
-      if ( at < 0 ) t -= seg.fcount[g];
-   }
-   if ( at < 0 ) return;
-   const FaceRec r   = v.frec[at];
-   auto          put = [&]( T* vec, A x ) {
-      stv( vec + r.owner, x );
-      stv( vec + r.c0, x );
-      if ( r.cell1 >= 0 ) stv( vec + r.c1, x );
-   };
+   auto put = [&]( T* vec, A x ) { put_face( r, vec, x ); };
    if ( !( r.bc & flag ) )
    {
       if ( !copy_unflagged ) return;
@@ -955,7 +882,7 @@ __device__ __forceinline__ void bnd_point( const LevelView& v, const OpView< A >
    if ( r.cell1 >= 0 )
       s += face_stencil< T, A >( src + r.c1, o.W + ( size_t( r.cell1 ) * kNumClasses + r.cls1 ) * kNumDirs, r.cls1, v.n, r.y1, r.z1 );
    A       second = A( 0 );
-   const A val    = owner_value< T, A, OP >( r.owner, s, o.invd_b[r.b], src, v1, v2, dst, a0, a1, second );
+   const A val    = owner_value< T, A >( OP, r.owner, s, o.invd_b[r.b], src, v1, v2, dst, a0, a1, second );
    if constexpr ( OP == OP_CHEBL ) put( v2, val );
    else put( dst, val );
    if constexpr ( OP == OP_CHEBI ) put( v2, second );
@@ -1481,25 +1408,50 @@ static double* partials( Context* ctx, int count )
    return ctx->d_partials;
 }
 
+// both kernels' blocks in one launch: cell blocks first, the same partials in the same places
+template < typename T >
+__global__ void __launch_bounds__( 256 ) k_dot( LevelView v, int row_blocks, int nb_cells, uint32_t flag, const T* a, const T* b, double* partials )
+{
+   double acc = 0.0;
+   if ( int( blockIdx.x ) < nb_cells )
+   {
+      const int c = int( blockIdx.x ) / row_blocks, r = ( int( blockIdx.x ) - c * row_blocks ) * 8 + ( threadIdx.x >> 5 );
+      if ( r < v.nrows && ( v.cell_bc[c] & flag ) )
+      {
+         const int2    yz   = v.rows[r];
+         const int64_t base = v.cell_off[c] + cidx( v.n, 0, yz.x, yz.y );
+         const int     xmax = v.n - 1 - yz.x - yz.y;
+         for ( int x = 1 + ( threadIdx.x & 31 ); x <= xmax; x += 32 ) acc += double( ldv( a + base + x ) ) * double( ldv( b + base + x ) );
+      }
+   }
+   else
+   {
+      const int t = ( int( blockIdx.x ) - nb_cells ) * 256 + threadIdx.x;
+      if ( t < v.ntasks )
+      {
+         const int4 tk = v.tasks[t];
+         if ( v.bc[tk.x] & flag )
+         {
+            const int64_t o = owner_slot( v, tk.x, tk.y, tk.z );
+            acc             = double( ldv( a + o ) ) * double( ldv( b + o ) );
+         }
+      }
+   }
+   acc = block_sum( acc );
+   if ( threadIdx.x == 0 ) partials[blockIdx.x] = acc;
+}
+
 template < typename T >
 static void run_dot( Context* ctx, const LevelView& v, int nC, uint32_t flag, const void* a, const void* b, double* out )
 {
-   const int nb_cells = ( v.nrows > 0 && nC > 0 ) ? ( ( v.nrows + 7 ) / 8 ) * nC : 0;
+   const int rb       = ( v.nrows + 7 ) / 8;
+   const int nb_cells = rb * nC;
    const int nb_bnd   = v.ntasks > 0 ? ( v.ntasks + 255 ) / 256 : 0;
    double*   p        = partials( ctx, nb_cells + nb_bnd + 1 );
+   if ( nb_cells + nb_bnd > 0 )
    {
-      Fork fk( ctx );
-      if ( nb_cells )
-      {
-      dim3 grid( ( v.nrows + 7 ) / 8, nC );
-      k_dot_cells< T ><<< grid, 256, 0, ctx->stream >>>( v, flag, (const T*) a, (const T*) b, p );
+      k_dot< T ><<< nb_cells + nb_bnd, 256, 0, ctx->stream >>>( v, std::max( rb, 1 ), nb_cells, flag, (const T*) a, (const T*) b, p );
       ++ctx->launches;
-      }
-      if ( nb_bnd )
-      {
-         k_dot_bnd< T ><<< nb_bnd, 256, 0, fk.aux() >>>( v, flag, (const T*) a, (const T*) b, p + nb_cells );
-         ++ctx->launches;
-      }
    }
    k_sum_partials<<< 1, 1024, 0, ctx->stream >>>( p, nb_cells + nb_bnd, out );
    ++ctx->launches;
@@ -1728,50 +1680,6 @@ __device__ __forceinline__ A restrict_low( const LevelView& fv, const T* fine, c
    return part;
 }
 
-// the boundary task of thread t: an edge or vertex (eight threads: record and this thread's share of its
-// incidences) or a face (one thread); BND_NONE where the thread has none
-enum { BND_NONE = 0, BND_LOW, BND_FACE };
-__device__ __forceinline__ int bnd_thread( const LevelView& v, const BndSegments& seg, int t, LowRec& low, int& sub, FaceRec& face )
-{
-#pragma unroll
-   for ( int g = 0; g < 4; ++g )
-   {
-      if ( t < seg.lthreads[g] )
-      {
-         const bool live = ( t >> 3 ) < seg.lcount[g];
-         low             = v.lrec[seg.lstart[g] + ( live ? t >> 3 : 0 )];
-         if ( !live ) low.count = 0;
-         sub = t & 7;
-         return BND_LOW;  // whole warps: a thread without a task has no incidences
-      }
-      t -= seg.lthreads[g];
-   }
-#pragma unroll
-   for ( int g = 0; g < 4; ++g )
-   {
-      if ( t >= 0 && t < seg.fcount[g] )
-      {
-         face = v.frec[seg.fstart[g] + t];
-         return BND_FACE;
-      }
-      t -= seg.fcount[g];
-   }
-   return BND_NONE;
-}
-template < typename T, typename A >
-__device__ __forceinline__ void put_low( const LevelView& v, const LowRec& r, int sub, T* vec, A val )
-{
-   if ( r.count > 0 && sub == 0 ) stv( vec + r.owner, val );
-   for ( int q = sub; q < r.count; q += 8 ) stv( vec + v.irec[r.begin + q].slot, val );
-}
-template < typename T, typename A >
-__device__ __forceinline__ void put_face( const FaceRec& r, T* vec, A val )
-{
-   stv( vec + r.owner, val );
-   stv( vec + r.c0, val );
-   if ( r.cell1 >= 0 ) stv( vec + r.c1, val );
-}
-
 // Interior point of thread or warp `unit` of a cell sweep: the listed points for levels up to kFlatMaxN
 // (one thread per point), warps over rows above
 template < typename F >
@@ -1815,17 +1723,24 @@ __device__ __forceinline__ A fine_sum( const T* f, int nf, int Y, int Z, std::in
 // Restriction, boundary tasks and cell interiors in one launch.  Bound by the fine vector's read; the row
 // starts of the 14 neighbours follow from the point's own by a few integer operations each (computing every
 // neighbour's index anew was most of the work), and the cells of an edge or vertex are shared by eight
-// threads.  TRANSFER_R
+// threads.  Level 7 to 6 on 18 cells, FP64: 22 us, in two kernels that computed each index 61 + 37 us.
 template < typename T, typename A >
 __global__ void __launch_bounds__( 256 ) k_restrict( LevelView cv, LevelView fv, BndSegments seg, int nbnd, int nC, uint32_t flag,
-                                                      const T* __restrict__ fine, T* coarse )
+                                                      const T* __restrict__ fine, T* coarse, int nblocks, uint4* zero, int64_t nzero )
 {
+   if ( int( blockIdx.x ) >= nblocks )
+   {
+      // the blocks past the restriction clear the vector the caller solves for next
+      const int64_t step = int64_t( gridDim.x - nblocks ) * 256;
+      for ( int64_t i = int64_t( blockIdx.x - nblocks ) * 256 + threadIdx.x; i < nzero; i += step ) zero[i] = make_uint4( 0, 0, 0, 0 );
+      return;
+   }
    if ( int( blockIdx.x ) < nbnd )
    {
       LowRec    low;
       FaceRec   face;
       int       sub;
-      const int kind = bnd_thread( cv, seg, blockIdx.x * 256 + threadIdx.x, low, sub, face );
+      const int kind = bnd_thread< 1 >( cv, cv.frec, seg, blockIdx.x * 256 + threadIdx.x, low, sub, face );
       if ( kind == BND_LOW )
       {
          A s = A( 0 );
@@ -1868,7 +1783,8 @@ __device__ __forceinline__ A interp( const T* c, int nc, int x, int y, int z )
    return A( 0.5 ) * ( A( ldv( c + lo + ( x >> 1 ) ) ) + A( ldv( c + hi + ( ( x + 1 ) >> 1 ) ) ) );
 }
 
-// Prolongation, boundary tasks and cell interiors in one launch: bound by the fine vector (TRANSFER_P)
+// Prolongation, boundary tasks and cell interiors in one launch: bound by the fine vector (level 6 to 7 on 18
+// cells, FP64: 66 us against 84 + 10 us with a branch on the parities per lane and two kernels)
 template < typename T, typename A >
 __global__ void __launch_bounds__( 256 ) k_prolong( LevelView cv, LevelView fv, BndSegments seg, int nbnd, int nC, uint32_t flag,
                                                      const T* __restrict__ coarse, T* fine, int add )
@@ -1878,7 +1794,7 @@ __global__ void __launch_bounds__( 256 ) k_prolong( LevelView cv, LevelView fv, 
       LowRec    low;
       FaceRec   face;
       int       sub;
-      const int kind = bnd_thread( fv, seg, blockIdx.x * 256 + threadIdx.x, low, sub, face );
+      const int kind = bnd_thread< 1 >( fv, fv.frec, seg, blockIdx.x * 256 + threadIdx.x, low, sub, face );
       if ( kind == BND_LOW )
       {
          A val = A( 0 );
@@ -1915,25 +1831,29 @@ __global__ void __launch_bounds__( 256 ) k_prolong( LevelView cv, LevelView fv, 
 
 template < typename T, typename A >
 static void run_restrict( Context* ctx, const LevelView& cv, const LevelView& fv, int nC, uint32_t flag, const void* fine,
-                          void* coarse )
+                          void* coarse, void* zero, size_t zero_bytes )
 {
    const BndSegments seg  = bnd_segments( cv, flag, 0 );
    const int         nbnd = ( seg.threads + 255 ) / 256, blocks = nbnd + interior_blocks( cv, nC );
-   if ( blocks == 0 ) return;
-   k_restrict< T, A ><<< blocks, 256, 0, ctx->stream >>>( cv, fv, seg, nbnd, nC, flag, (const T*) fine, (T*) coarse );
+   // level vectors are whole multiples of 32 values, so of 16 bytes
+   const int64_t nzero = int64_t( zero_bytes / 16 );
+   const int     zb    = int( std::min< int64_t >( ( nzero + 1023 ) / 1024, 148 * 4 ) );
+   if ( blocks + zb == 0 ) return;
+   k_restrict< T, A ><<< blocks + zb, 256, 0, ctx->stream >>>( cv, fv, seg, nbnd, nC, flag, (const T*) fine, (T*) coarse, blocks,
+                                                              reinterpret_cast< uint4* >( zero ), nzero );
    ++ctx->launches;
    check_cuda( cudaGetLastError(), "restrict launch" );
 }
 
-void launch_restrict( Context* ctx, Mesh* m, int Lf, int dtype, uint32_t flag, const void* fine, void* coarse )
+void launch_restrict( Context* ctx, Mesh* m, int Lf, int dtype, uint32_t flag, const void* fine, void* coarse, void* zero, size_t zero_bytes )
 {
    ensure_constants();
    LevelView fv = make_view( m, Lf );
    LevelView cv = make_view( m, Lf - 1 );
    const int nC = m->topo.nC;
-   if ( dtype == F64 ) run_restrict< double, double >( ctx, cv, fv, nC, flag, fine, coarse );
-   else if ( dtype == F32 ) run_restrict< float, float >( ctx, cv, fv, nC, flag, fine, coarse );
-   else run_restrict< __half, float >( ctx, cv, fv, nC, flag, fine, coarse );
+   if ( dtype == F64 ) run_restrict< double, double >( ctx, cv, fv, nC, flag, fine, coarse, zero, zero_bytes );
+   else if ( dtype == F32 ) run_restrict< float, float >( ctx, cv, fv, nC, flag, fine, coarse, zero, zero_bytes );
+   else run_restrict< __half, float >( ctx, cv, fv, nC, flag, fine, coarse, zero, zero_bytes );
 }
 
 template < typename T, typename A >
@@ -2408,7 +2328,7 @@ void prepare_device( Context* ctx, Mesh* m, Operator* op, int minL, int maxL, in
       if ( op && op->kind == HYB_P2_CONST_LAPLACE )
       {
          ensure_p2_constant_device();
-         ensure_p2_constant_tables( op->p2c.at( L ) );
+         ensure_p2_constant_tables( op, L );
       }
       else if ( op && !op->elementwise ) ensure_device_op( op->lv.at( L ) );
       if ( op && op->elementwise )

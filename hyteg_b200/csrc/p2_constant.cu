@@ -19,15 +19,17 @@
 //    stencil at the same time and the weights are warp-uniform shared-memory reads.  Each slice is
 //    read once: its values are folded into running sums of the five output slices z-2..z+2 they
 //    reach (partial sums in y and z), and a slice's points are written two steps after it arrives.
-//  * k_p2c_bnd: owned face/edge/vertex nodes, one thread each: the partial stencils of every
-//    neighbouring cell, summed in incidence order, written through to all copies.
+//  * k_p2c_flat: owned face/edge/vertex nodes (the partial stencils of every neighbouring cell, summed
+//    and written through to all copies) and the cell interiors of small levels, one launch.
 // Both use the operation epilogues of the P1 path (apply, residual, Jacobi, Chebyshev steps).
 #include "hyb_internal.hpp"
 #include "hyb_device.cuh"
+#include "p2_stored.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
+#include <utility>
 
 namespace hyb {
 
@@ -247,31 +249,6 @@ void build_p2_constant_level( Operator* A, int Ls )
          }
       for ( int k = 0; k < 8; ++k ) Wc[kP2cEntries + k] = 1.0 / Wc[kP2Pat.base[k] + kP2Pat.centre[k]];
    }
-   // boundary tasks in the grouping of the P1 level (by boundary type, so that a launch covers the
-   // flagged groups), inside a group sorted by primitive and by the parity class of the node in its
-   // first cell: the lanes of a warp then walk the same stencil pattern
-   const P1Level& P = A->mesh->level( Ls );
-   const int      N = P.n;
-   const uint32_t type_bit[4] = { kInner, kDirichlet, kNeumann, kFreeslip };
-   auto           btype = [&]( int b ) {
-      return b < t.nV ? t.bc( t.flag_v[b] ) : ( b < t.nV + t.nE ? t.bc( t.flag_e[b - t.nV] ) : t.bc( t.flag_f[b - t.nV - t.nE] ) );
-   };
-   auto parity = [&]( const std::array< int, 4 >& q ) {
-      const Incidence& I = P.inc[P.inc_begin[q[0]]];
-      const int        x = N * I.o[0] + q[1] * I.e1[0] + q[2] * I.e2[0];
-      const int        y = N * I.o[1] + q[1] * I.e1[1] + q[2] * I.e2[1];
-      const int        z = N * I.o[2] + q[1] * I.e1[2] + q[2] * I.e2[2];
-      return ( x & 1 ) | ( ( y & 1 ) << 1 ) | ( ( z & 1 ) << 2 );
-   };
-   for ( int g = 0; g < 4; ++g )
-   {
-      std::vector< std::pair< int64_t, int > > key;
-      for ( size_t q = 0; q < P.tasks.size(); ++q )
-         if ( btype( P.tasks[q][0] ) == type_bit[g] ) key.push_back( { int64_t( P.tasks[q][0] ) * 8 + parity( P.tasks[q] ), int( q ) } );
-      std::stable_sort( key.begin(), key.end(), []( const auto& a, const auto& c ) { return a.first < c.first; } );
-      for ( const auto& kq : key ) pl.tasks.push_back( make_int4( P.tasks[kq.second][0], P.tasks[kq.second][1], P.tasks[kq.second][2], 0 ) );
-   }
-   if ( pl.tasks.size() != P.tasks.size() ) throw std::logic_error( "boundary task without a single boundary type" );
    A->p2c[Ls] = std::move( pl );
 }
 
@@ -293,17 +270,60 @@ void ensure_p2_constant_device()
    } );
 }
 
-void ensure_p2_constant_tables( P2cLevel& pl )
+void ensure_p2_constant_tables( Operator* A, int Ls )
 {
+   P2cLevel& pl = A->p2c.at( Ls );
    if ( pl.d_W ) return;
    std::vector< float > wf( pl.W.begin(), pl.W.end() );
    check_cuda( cudaMalloc( &pl.d_W, pl.W.size() * sizeof( double ) ), "cudaMalloc(P2 stencils)" );
    check_cuda( cudaMalloc( &pl.d_Wf, wf.size() * sizeof( float ) ), "cudaMalloc(P2 stencils)" );
    check_cuda( cudaMemcpy( pl.d_W, pl.W.data(), pl.W.size() * sizeof( double ), cudaMemcpyHostToDevice ), "upload P2 stencils" );
    check_cuda( cudaMemcpy( pl.d_Wf, wf.data(), wf.size() * sizeof( float ), cudaMemcpyHostToDevice ), "upload P2 stencils" );
-   check_cuda( cudaMalloc( &pl.d_tasks, std::max< size_t >( pl.tasks.size(), 1 ) * sizeof( int4 ) ), "cudaMalloc(P2 tasks)" );
-   if ( !pl.tasks.empty() )
-      check_cuda( cudaMemcpy( pl.d_tasks, pl.tasks.data(), pl.tasks.size() * sizeof( int4 ), cudaMemcpyHostToDevice ), "upload P2 tasks" );
+   // the level's face records, inside each boundary type's group sorted by face and by the parity class of
+   // the node in its first cell: the lanes of a warp then apply the same stencil
+   P1Level&  P  = A->mesh->level( Ls );
+   ensure_device( A->mesh, P );
+   const int n  = P.n;
+   int       nf = 0;
+   for ( int g = 0; g < 4; ++g ) nf += P.nface[g];
+   if ( nf > 0 )
+   {
+      std::vector< FaceRec > fr( nf );
+      check_cuda( cudaMemcpy( fr.data(), P.d_frec, size_t( nf ) * sizeof( FaceRec ), cudaMemcpyDeviceToHost ), "face records" );
+      // inside a type's group the records come face by face: a counting pass per face keeps their order
+      std::vector< FaceRec > sorted( nf );
+      auto                   parity = [&]( const FaceRec& r ) {
+         const int x = int( r.c0 - P.off[P.nB + r.cell0] - cidx( n, 0, r.y0, r.z0 ) );
+         return ( x & 1 ) | ( ( r.y0 & 1 ) << 1 ) | ( ( r.z0 & 1 ) << 2 );
+      };
+      for ( int i = 0; i < nf; )
+      {
+         int e = i, count[9] = {};
+         for ( ; e < nf && fr[e].b == fr[i].b; ++e ) ++count[parity( fr[e] ) + 1];
+         for ( int k = 0; k < 8; ++k ) count[k + 1] += count[k];
+         for ( int k = i; k < e; ++k ) sorted[i + count[parity( fr[k] )]++] = fr[k];
+         i = e;
+      }
+      fr.swap( sorted );
+      check_cuda( cudaMalloc( &pl.d_frec, size_t( nf ) * sizeof( FaceRec ) ), "cudaMalloc(P2 face records)" );
+      check_cuda( cudaMemcpy( pl.d_frec, fr.data(), size_t( nf ) * sizeof( FaceRec ), cudaMemcpyHostToDevice ), "upload P2 face records" );
+   }
+   if ( n <= kP2cFlatMaxN )
+   {
+      std::vector< ushort4 > pts;
+      for ( int k = 0; k < 8; ++k )
+      {
+         const size_t before = pts.size();
+         for ( int z = 1; z < n; ++z )
+            for ( int y = 1; y + z < n; ++y )
+               for ( int x = 1; x + y + z < n; ++x )
+                  if ( ( ( x & 1 ) | ( ( y & 1 ) << 1 ) | ( ( z & 1 ) << 2 ) ) == k )
+                     pts.push_back( make_ushort4( (unsigned short) x, (unsigned short) y, (unsigned short) z, 0 ) );
+         pl.np[k] = int( pts.size() - before );
+      }
+      check_cuda( cudaMalloc( &pl.d_pts, std::max< size_t >( pts.size(), 1 ) * sizeof( ushort4 ) ), "cudaMalloc(P2 points)" );
+      if ( !pts.empty() ) check_cuda( cudaMemcpy( pl.d_pts, pts.data(), pts.size() * sizeof( ushort4 ), cudaMemcpyHostToDevice ), "upload P2 points" );
+   }
 }
 
 // inverse diagonal of every owned slot flagged by `flag` (padded level layout), from the tables
@@ -658,91 +678,155 @@ __global__ void __launch_bounds__( kP2cWarps * 32, 2 )
 }
 
 // ---------------------------------------------------------------------------------------------
-// device: boundary owners
+// device: boundary owners, and cell interiors of levels up to kP2cFlatMaxN points per macro-edge
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool p2c_inside( int faces, int dx, int dy, int dz )
+// entry D of parity class K at the slot c points to (row y, slice z); BND: only if it stays in the cell, whose
+// faces through the point are `faces` (kClassFaces)
+template < int K, int D, bool BND, typename T, typename A >
+__device__ __forceinline__ void p2c_term( const T* c, const A* w, int n, int y, int z, int faces, A ( &s )[2] )
 {
-   return !( ( ( faces & 1 ) && dz < 0 ) || ( ( faces & 2 ) && dy < 0 ) || ( ( faces & 4 ) && dx < 0 ) ||
-             ( ( faces & 8 ) && dx + dy + dz > 0 ) );
+   constexpr int dx = P2Class< K >::S.off[D][0], dy = P2Class< K >::S.off[D][1], dz = P2Class< K >::S.off[D][2];
+   if constexpr ( BND )
+   {
+      constexpr int needs = ( dz < 0 ? 1 : 0 ) | ( dy < 0 ? 2 : 0 ) | ( dx < 0 ? 4 : 0 ) | ( dx + dy + dz > 0 ? 8 : 0 );
+      if ( faces & needs ) return;
+   }
+   s[D & 1] += __ldg( w + D ) * A( ldv( c + ( row_shift< dy, dz >( n, y, z ) + dx ) ) );
+}
+template < int K, bool BND, typename T, typename A, int... D >
+__device__ __forceinline__ A p2c_terms( const T* c, const A* W, int n, int y, int z, int faces, std::integer_sequence< int, D... > )
+{
+   constexpr int base = kP2Pat.base[K];
+   A             s[2] = { A( 0 ), A( 0 ) };
+   ( p2c_term< K, D, BND, T, A >( c, W + base, n, y, z, faces, s ), ... );
+   return s[0] + s[1];
+}
+template < bool BND, typename T, typename A >
+__device__ __forceinline__ A p2c_sum( int k, const T* c, const A* W, int n, int y, int z, int faces )
+{
+#define HYB_CLASS( K ) \
+   case K: return p2c_terms< K, BND, T, A >( c, W, n, y, z, faces, std::make_integer_sequence< int, P2Class< K >::S.n >() );
+   switch ( k )
+   {
+      HYB_CLASS( 0 )
+      HYB_CLASS( 1 )
+      HYB_CLASS( 2 )
+      HYB_CLASS( 3 )
+      HYB_CLASS( 4 )
+      HYB_CLASS( 5 )
+      HYB_CLASS( 6 )
+   default: return p2c_terms< 7, BND, T, A >( c, W, n, y, z, faces, std::make_integer_sequence< int, P2Class< 7 >::S.n >() );
+   }
+#undef HYB_CLASS
 }
 
-template < typename T, typename A, int OP >
-__global__ void __launch_bounds__( 256 ) k_p2c_bnd( LevelView v, const A* __restrict__ W, const int4* __restrict__ tasks, TaskSegments seg,
-                                                     uint32_t flag, int copy_unflagged, const T* __restrict__ src, const T* __restrict__ v1,
-                                                     T* v2, T* dst, A a0, A a1 )
+struct P2cPoints {
+   int            np[8];
+   const ushort4* pts;
+};
+
+// Eight threads per edge or vertex node, one per cell of a face node, one per interior node; all entries of
+// the node's class are unrolled, so its loads are independent (walking the entries of one cell after the
+// other, with the row start computed on the way, took 67 us for the 48k face nodes of the level-6 cube).
+// Apply on the cube, FP64, with that kernel and the tiled sweep and with this one: P2 levels 4 and 5 103 -> 17
+// and 21 us, level 6 118 -> 83 us, level 7 243 -> 232 us.  At 128 points per edge one thread per node for the
+// interior too takes 75 us on six cells, but 152 against 99 us on twelve: the sweep stays there.
+template < typename T, typename A >
+__global__ void __launch_bounds__( 256 )
+    k_p2c_flat( LevelView v, const FaceRec* __restrict__ frec, const A* __restrict__ W, BndSegments seg, int nbnd, P2cPoints pts, int nC, int op,
+                uint32_t flag, int copy_unflagged, const T* __restrict__ src, const T* __restrict__ v1, T* v2, T* dst, A a0, A a1 )
 {
-   int t = blockIdx.x * blockDim.x + threadIdx.x, at = -1;
+   const int n = v.n;
+   if ( int( blockIdx.x ) < nbnd )
+   {
+      LowRec    low;
+      FaceRec   r;
+      int       sub;
+      const int kind = bnd_thread< 2 >( v, frec, seg, blockIdx.x * 256 + threadIdx.x, low, sub, r );
+      // one cell's part: the stencil of the node's class in it and the weight of its centre
+      A    s = A( 0 ), d = A( 0 );
+      auto part = [&]( int64_t slot, int cell, int cls, int y, int z ) {
+         const int x = int( slot - v.cell_off[cell] - cidx( n, 0, y, z ) ), k = ( x & 1 ) | ( ( y & 1 ) << 1 ) | ( ( z & 1 ) << 2 );
+         const A*  w = W + size_t( cell ) * kP2cCellStride + ( cls == 0 ? 0 : kP2cInterior + ( cls - 1 ) * kP2cEntries );
+         s += p2c_sum< true, T, A >( k, src + slot, w, n, y, z, c_p2c_faces[cls] );
+         d += w[g_p2c_base[k] + g_p2c_base[k + 16]];
+      };
+      int64_t owner   = 0;
+      bool    flagged = false, any = false;
+      if ( kind == BND_LOW )
+      {
+         owner   = low.owner;
+         flagged = ( low.bc & flag ) != 0;
+         any     = low.count > 0;
+         if ( flagged )
+            for ( int q = sub; q < low.count; q += 8 )
+            {
+               const IncRec I = v.irec[low.begin + q];
+               part( I.slot, I.cell, I.cls, I.y, I.z );
+            }
 #pragma unroll
-   for ( int g = 0; g < 4; ++g )
-   {
-      if ( at < 0 && t < seg.count[g] ) at = seg.start[g] + t;
-      if ( at < 0 ) t -= seg.count[g];
-   }
-   if ( at < 0 ) return;
-   const int4    tk    = tasks[at];
-   const int     b     = tk.x, i = tk.y, j = tk.z, N = v.n;
-   const int64_t owner = owner_slot( v, b, i, j );
-   if ( !( v.bc[b] & flag ) )
-   {
-      if ( !copy_unflagged ) return;
-      if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) write_through( v, dst, b, i, j, owner, A( ldv( src + owner ) ) );
-      else if constexpr ( OP == OP_CHEBI ) write_through( v, dst, b, i, j, owner, A( ldc( v2 + owner ) ) );
+         for ( int m = 4; m > 0; m >>= 1 )
+         {
+            s += __shfl_xor_sync( 0xffffffffu, s, m, 8 );
+            d += __shfl_xor_sync( 0xffffffffu, d, m, 8 );
+         }
+      }
+      else
+      {
+         if ( kind == BND_FACE )
+         {
+            owner   = r.owner;
+            flagged = ( r.bc & flag ) != 0;
+            any     = true;
+            if ( flagged && sub == 0 ) part( r.c0, r.cell0, r.cls0, r.y0, r.z0 );
+            if ( flagged && sub == 1 && r.cell1 >= 0 ) part( r.c1, r.cell1, r.cls1, r.y1, r.z1 );
+         }
+         s += __shfl_xor_sync( 0xffffffffu, s, 1 );
+         d += __shfl_xor_sync( 0xffffffffu, d, 1 );
+      }
+      const bool carried = copy_unflagged && ( op == OP_JAC || op == OP_CHEB0 || op == OP_CHEBI );
+      A          val = A( 0 ), second = A( 0 );
+      if ( any )
+      {
+         if ( flagged ) val = owner_value< T, A >( op, owner, s, A( 1 ) / d, src, v1, v2, dst, a0, a1, second );
+         else if ( carried ) val = op == OP_CHEBI ? A( ldc( v2 + owner ) ) : A( ldv( src + owner ) );
+      }
+      __syncwarp();  // every thread of a node has read the owner before any writes it
+      if ( !any || ( !flagged && !carried ) ) return;
+      auto put = [&]( T* vec, A x ) {
+         if ( kind == BND_LOW ) put_low( v, low, sub, vec, x );
+         else if ( sub == 0 )
+         {
+            stv( vec + r.owner, x );
+            stv( vec + r.c0, x );
+         }
+         else if ( r.cell1 >= 0 ) stv( vec + r.c1, x );
+      };
+      put( op == OP_CHEBL ? v2 : dst, val );
+      if ( op == OP_CHEBI && flagged ) put( v2, second );
       return;
    }
-   A acc = A( 0 ), diag = A( 0 );
-   for ( int q = v.inc_begin[b]; q < v.inc_begin[b + 1]; ++q )
+   int     k  = 0, first = 0;
+   int64_t g = blockIdx.x - nbnd;
+   for ( ; k < 7; ++k )
    {
-      const Incidence I = v.inc[q];
-      int             x, y, z;
-      inc_point( I, N, i, j, x, y, z );
-      const int      k     = ( x & 1 ) | ( ( y & 1 ) << 1 ) | ( ( z & 1 ) << 2 );
-      const int      faces = c_p2c_faces[I.cls];
-      const int      e0    = g_p2c_base[k], ne = g_p2c_base[k + 8];
-      const A*       w     = W + size_t( I.cell ) * kP2cCellStride + ( I.cls == 0 ? 0 : kP2cInterior + ( I.cls - 1 ) * kP2cEntries ) + e0;
-      const T*       s     = src + v.cell_off[I.cell];
-      A              part  = A( 0 );
-      // cell-relative starts of the slices z-2 .. z+2 (32-bit: the host limits the level), from
-      // slice z by the slice sizes tri(N+1-z') = (N+1-z')(N+2-z')/2
-      const int w1 = N + 1;
-      int       S[5];
-      S[2] = int( cidx( N, 0, 0, z ) );
-      S[3] = S[2] + ( w1 - z ) * ( w1 - z + 1 ) / 2;
-      S[4] = S[3] + ( w1 - z - 1 ) * ( w1 - z ) / 2;
-      S[1] = S[2] - ( w1 - z + 1 ) * ( w1 - z + 2 ) / 2;
-      S[0] = S[1] - ( w1 - z + 2 ) * ( w1 - z + 3 ) / 2;
-      // entries are sorted by (dz, dy): the row start is recomputed only when that pair changes
-      int pr = 0x7fffffff, rb = 0;
-      for ( int e = 0; e < ne; ++e )
-      {
-         const char4 o = g_p2c_off[e0 + e];
-         if ( !p2c_inside( faces, o.x, o.y, o.z ) ) continue;
-         const int r = o.y * 8 + o.z;
-         if ( r != pr )
-         {
-            const int yy = y + o.y, zz = z + o.z;
-            rb = S[o.z + 2] + yy * ( w1 - zz ) - ( yy * ( yy - 1 ) ) / 2;  // start of row yy of slice zz
-            pr = r;
-         }
-         part += w[e] * A( ldv( s + rb + x + o.x ) );
-      }
-      acc += part;
-      diag += w[g_p2c_base[k + 16]];
+      const int64_t blocks = ( int64_t( nC ) * pts.np[k] + 255 ) / 256;
+      if ( g < blocks ) break;
+      g -= blocks;
+      first += pts.np[k];
    }
-   const A invd = A( 1 ) / diag;
-   if constexpr ( OP == OP_APPLY ) write_through( v, dst, b, i, j, owner, acc );
-   else if constexpr ( OP == OP_APPLY_ADD ) write_through( v, dst, b, i, j, owner, A( ldc( dst + owner ) ) + acc );
-   else if constexpr ( OP == OP_RESID ) write_through( v, dst, b, i, j, owner, A( ldv( v1 + owner ) ) - acc );
-   else if constexpr ( OP == OP_JAC )
-      write_through( v, dst, b, i, j, owner, A( ldv( src + owner ) ) + a0 * ( invd * ( A( ldv( v1 + owner ) ) - acc ) ) );
-   else if constexpr ( OP == OP_CHEB0 ) write_through( v, dst, b, i, j, owner, invd * ( A( ldv( v1 + owner ) ) - acc ) );
-   else if constexpr ( OP == OP_CHEBI )
-   {
-      write_through( v, dst, b, i, j, owner, invd * acc );
-      write_through( v, v2, b, i, j, owner, A( ldc( v2 + owner ) ) + a0 * A( ldv( src + owner ) ) );
-   }
-   else if constexpr ( OP == OP_CHEBL )
-      write_through( v, v2, b, i, j, owner, ( A( ldc( v2 + owner ) ) + a0 * A( ldv( src + owner ) ) ) + a1 * ( invd * acc ) );
-   else if constexpr ( OP == OP_DINV_APPLY ) write_through( v, dst, b, i, j, owner, invd * acc );
+   g = g * 256 + threadIdx.x;
+   if ( g >= int64_t( nC ) * pts.np[k] ) return;
+   const int c = g < 0x7fffffff ? int( unsigned( g ) / unsigned( pts.np[k] ) ) : int( g / pts.np[k] );
+   if ( !( v.cell_bc[c] & flag ) ) return;
+   const ushort4 p = pts.pts[first + int( g - int64_t( c ) * pts.np[k] )];
+   const int64_t i = v.cell_off[c] + cidx( n, p.x, p.y, p.z );
+   const A*      w = W + size_t( c ) * kP2cCellStride;
+   const A       s = p2c_sum< false, T, A >( k, src + i, w, n, p.y, p.z, 0 );
+   A             second = A( 0 );
+   const A       val    = owner_value< T, A >( op, i, s, w[kP2cEntries + k], src, v1, v2, dst, a0, a1, second );
+   stv( ( op == OP_CHEBL ? v2 : dst ) + i, val );
+   if ( op == OP_CHEBI ) stv( v2 + i, second );
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -776,25 +860,33 @@ static void p2c_attributes_all()
 }
 
 template < typename T, typename A, int OP >
-static void run_p2c( Context* ctx, const LevelView& v, const A* W, const int4* tasks, int nC, const StencilArgs& a )
+static void run_p2c( Context* ctx, const LevelView& v, const A* W, const P2cLevel& pl, int nC, const StencilArgs& a )
 {
    using Cfg            = P2cCfg< T, A >;
    const T*           src = (const T*) a.src;
    const T*           v1  = (const T*) a.v1;
    T*                 v2  = (T*) a.v2;
    T*                 dst = (T*) a.dst;
-   const TaskSegments seg = task_segments( v, a.flag, a.copy_unflagged );
-   const int          nt  = seg.count[0] + seg.count[1] + seg.count[2] + seg.count[3];
-   // boundary owners and cell interiors write disjoint slots and read only src and their own slots of
-   // the second vector, so the two kernels run one after the other on the context stream
-   if ( nt > 0 )
+   const BndSegments  seg  = bnd_segments( v, a.flag, a.copy_unflagged, 2 );
+   const int          nbnd = ( seg.threads + 255 ) / 256;
+   P2cPoints          pts{};
+   int                blocks = nbnd;
+   for ( int k = 0; k < 8; ++k )
    {
-      k_p2c_bnd< T, A, OP ><<< ( nt + 255 ) / 256, 256, 0, ctx->stream >>>( v, W, tasks, seg, a.flag, a.copy_unflagged, src, v1, v2, dst, A( a.a0 ),
-                                                                            A( a.a1 ) );
+      pts.np[k] = pl.np[k];
+      blocks += int( ( int64_t( nC ) * pl.np[k] + 255 ) / 256 );
+   }
+   pts.pts = reinterpret_cast< const ushort4* >( pl.d_pts );
+   // boundary owners and cell interiors write disjoint slots and read only src and their own slots of
+   // the second vector: one launch on the small levels, one after the other on the others
+   if ( blocks > 0 )
+   {
+      k_p2c_flat< T, A ><<< blocks, 256, 0, ctx->stream >>>( v, pl.d_frec, W, seg, nbnd, pts, nC, OP, a.flag, a.copy_unflagged, src, v1, v2, dst,
+                                                             A( a.a0 ), A( a.a1 ) );
       ++ctx->launches;
    }
    const int nw = v.nswarps[0];
-   if ( nw > 0 && nC > 0 && v.n >= 4 )
+   if ( nw > 0 && nC > 0 && v.n > kP2cFlatMaxN )
    {
       // the sweep keeps cell-relative row starts in 32-bit integers
       if ( tet_size( int64_t( v.n ) + 1 ) > int64_t( 0x7fffffff ) ) throw std::invalid_argument( "P2 constant operator: level too large" );
@@ -806,18 +898,18 @@ static void run_p2c( Context* ctx, const LevelView& v, const A* W, const int4* t
 }
 
 template < typename T, typename A >
-static void dispatch_p2c( Context* ctx, const LevelView& v, const A* W, const int4* tasks, int nC, const StencilArgs& a )
+static void dispatch_p2c( Context* ctx, const LevelView& v, const A* W, const P2cLevel& pl, int nC, const StencilArgs& a )
 {
    switch ( a.op )
    {
-   case OP_APPLY: return run_p2c< T, A, OP_APPLY >( ctx, v, W, tasks, nC, a );
-   case OP_APPLY_ADD: return run_p2c< T, A, OP_APPLY_ADD >( ctx, v, W, tasks, nC, a );
-   case OP_RESID: return run_p2c< T, A, OP_RESID >( ctx, v, W, tasks, nC, a );
-   case OP_JAC: return run_p2c< T, A, OP_JAC >( ctx, v, W, tasks, nC, a );
-   case OP_CHEB0: return run_p2c< T, A, OP_CHEB0 >( ctx, v, W, tasks, nC, a );
-   case OP_CHEBI: return run_p2c< T, A, OP_CHEBI >( ctx, v, W, tasks, nC, a );
-   case OP_CHEBL: return run_p2c< T, A, OP_CHEBL >( ctx, v, W, tasks, nC, a );
-   case OP_DINV_APPLY: return run_p2c< T, A, OP_DINV_APPLY >( ctx, v, W, tasks, nC, a );
+   case OP_APPLY: return run_p2c< T, A, OP_APPLY >( ctx, v, W, pl, nC, a );
+   case OP_APPLY_ADD: return run_p2c< T, A, OP_APPLY_ADD >( ctx, v, W, pl, nC, a );
+   case OP_RESID: return run_p2c< T, A, OP_RESID >( ctx, v, W, pl, nC, a );
+   case OP_JAC: return run_p2c< T, A, OP_JAC >( ctx, v, W, pl, nC, a );
+   case OP_CHEB0: return run_p2c< T, A, OP_CHEB0 >( ctx, v, W, pl, nC, a );
+   case OP_CHEBI: return run_p2c< T, A, OP_CHEBI >( ctx, v, W, pl, nC, a );
+   case OP_CHEBL: return run_p2c< T, A, OP_CHEBL >( ctx, v, W, pl, nC, a );
+   case OP_DINV_APPLY: return run_p2c< T, A, OP_DINV_APPLY >( ctx, v, W, pl, nC, a );
    default: throw std::invalid_argument( "unknown stencil operation" );
    }
 }
@@ -826,12 +918,12 @@ void launch_p2_constant( Context* ctx, Mesh* m, Operator* op, int Ls, int dtype,
 {
    ensure_p2_constant_device();
    P2cLevel& pl = op->p2c.at( Ls );
-   ensure_p2_constant_tables( pl );
+   ensure_p2_constant_tables( op, Ls );
    const LevelView v  = make_view( m, Ls );
    const int       nC = m->topo.nC;
-   if ( dtype == F64 ) dispatch_p2c< double, double >( ctx, v, pl.d_W, pl.d_tasks, nC, a );
-   else if ( dtype == F32 ) dispatch_p2c< float, float >( ctx, v, pl.d_Wf, pl.d_tasks, nC, a );
-   else dispatch_p2c< __half, float >( ctx, v, pl.d_Wf, pl.d_tasks, nC, a );
+   if ( dtype == F64 ) dispatch_p2c< double, double >( ctx, v, pl.d_W, pl, nC, a );
+   else if ( dtype == F32 ) dispatch_p2c< float, float >( ctx, v, pl.d_Wf, pl, nC, a );
+   else dispatch_p2c< __half, float >( ctx, v, pl.d_Wf, pl, nC, a );
 }
 
 }  // namespace hyb

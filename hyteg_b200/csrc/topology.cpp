@@ -473,29 +473,40 @@ void ensure_device( Mesh* m, P1Level& P )
    {
       // the tasks grouped by the boundary type of their primitive (order kept inside a group), so
       // that a stencil operation launches only the groups its flag selects
-      const uint32_t      type_bit[4] = { kInner, kDirichlet, kNeumann, kFreeslip };
-      std::vector< int4 > bt;
-      for ( int g = 0; g < 4; ++g )
+      const uint32_t         type_bit[4] = { kInner, kDirichlet, kNeumann, kFreeslip };
+      std::vector< uint8_t > btype( P.nB ), bgroup( P.nB );  // looked up once per primitive
+      for ( int b = 0; b < P.nB; ++b )
       {
-         for ( const int4& q : tk )
-         {
-            const int      b  = q.x;
-            const uint32_t ty = b < t.nV ? t.bc( t.flag_v[b] )
-                                         : ( b < t.nV + t.nE ? t.bc( t.flag_e[b - t.nV] ) : t.bc( t.flag_f[b - t.nV - t.nE] ) );
-            if ( ty == type_bit[g] ) bt.push_back( q ), ++( b < t.nV + t.nE ? P.nlow : P.nface )[g];
-         }
+         const uint32_t ty = b < t.nV ? t.bc( t.flag_v[b] ) : ( b < t.nV + t.nE ? t.bc( t.flag_e[b - t.nV] ) : t.bc( t.flag_f[b - t.nV - t.nE] ) );
+         int            g  = 0;
+         while ( g < 4 && type_bit[g] != ty ) ++g;
+         btype[b]  = uint8_t( ty );
+         bgroup[b] = uint8_t( g );
       }
-      if ( bt.size() != tk.size() ) throw std::logic_error( "boundary task without a single boundary type" );
+      size_t first[4] = {}, n_inc = 0, n_low = 0;
+      for ( const int4& q : tk )
+      {
+         const int g = bgroup[q.x];
+         if ( g == 4 ) throw std::logic_error( "boundary task without a single boundary type" );
+         ++( q.x < t.nV + t.nE ? P.nlow : P.nface )[g];
+         if ( q.x < t.nV + t.nE ) n_inc += size_t( P.inc_begin[q.x + 1] - P.inc_begin[q.x] ), ++n_low;
+      }
+      for ( int g = 1; g < 4; ++g ) first[g] = first[g - 1] + size_t( P.nlow[g - 1] + P.nface[g - 1] );
+      std::vector< int4 > bt( tk.size() );
+      for ( const int4& q : tk ) bt[first[bgroup[q.x]]++] = q;
       up( &P.d_btasks, bt.data(), bt.size() );
       std::vector< FaceRec > fr;
       std::vector< LowRec >  lr;
       std::vector< IncRec >  ir;
       const int              n = P.n;
+      fr.reserve( tk.size() - n_low );
+      lr.reserve( n_low );
+      ir.reserve( n_inc );
       for ( const int4& q : bt )
       {
          const int  b = q.x, i = q.y, j = q.z, q0 = P.inc_begin[b], q1 = P.inc_begin[b + 1];
          const bool face = b >= t.nV + t.nE;
-         const auto bc   = uint8_t( b < t.nV ? t.bc( t.flag_v[b] ) : face ? t.bc( t.flag_f[b - t.nV - t.nE] ) : t.bc( t.flag_e[b - t.nV] ) );
+         const auto bc   = btype[b];
          FaceRec    f{};
          f.cell1 = -1;
          LowRec l{};
@@ -539,6 +550,7 @@ void ensure_device( Mesh* m, P1Level& P )
       up( &P.d_lrec, lr.data(), lr.size() );
       up( &P.d_irec, ir.data(), ir.size() );
       std::vector< ushort4 > ip;
+      if ( n <= kFlatMaxN && n >= 4 ) ip.reserve( size_t( tet_size( n - 3 ) ) );
       for ( int z = 1; z < n && n <= kFlatMaxN; ++z )
          for ( int y = 1; y + z < n; ++y )
             for ( int x = 1; x + y + z < n; ++x ) ip.push_back( make_ushort4( (unsigned short) x, (unsigned short) y, (unsigned short) z, 0 ) );
@@ -780,7 +792,8 @@ Operator::~Operator()
    {
       cudaFree( kv.second.d_W );
       cudaFree( kv.second.d_Wf );
-      cudaFree( kv.second.d_tasks );
+      cudaFree( kv.second.d_frec );
+      cudaFree( kv.second.d_pts );
    }
    for ( auto& kv : el )
    {
