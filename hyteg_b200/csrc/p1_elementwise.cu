@@ -300,7 +300,7 @@ __constant__ int c_mc_off[6][4][3] = {
     { { 1, 0, 1 }, { 0, 1, 1 }, { 0, 0, 1 }, { 0, 1, 0 } }, { { 0, 1, 0 }, { 1, 1, 0 }, { 1, 0, 1 }, { 0, 1, 1 } } };
 __constant__ int c_mc_shift[6] = { 0, 1, 1, 2, 1, 1 };
 // stencil direction (index into kVarDirs) from vertex i to vertex j of micro-cell type ty
-__constant__ int8_t c_mc_dir[6][4][4];
+__constant__ __align__( 16 ) int8_t c_mc_dir[6][4][4];
 // the 15 stencil directions in the order of the constant-stencil weights
 static const int kVarDirs[15][3] = { { 0, 0, 0 },  { -1, 0, 0 }, { 1, 0, 0 },  { 0, -1, 0 }, { 0, 1, 0 },
                                      { 0, 0, -1 }, { 0, 0, 1 },  { -1, 1, 0 }, { 1, -1, 0 }, { -1, 0, 1 },
@@ -390,13 +390,13 @@ __global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const in
 __constant__ double c_xg4_pts[11][3];
 __constant__ double c_xg4_bary[11][4];
 __constant__ double c_xg4_w[11];
-__constant__ int8_t c_p2_from[60];     // micro-cell nodes 10 ty + i, grouped by the window node they are
-__constant__ int8_t c_p2_from0[28];    // window node l: entries c_p2_from0[l] .. c_p2_from0[l + 1] - 1
-__constant__ int8_t c_p2_loc[6][10];  // node of micro-cell type ty in its anchor's 3x3x3 nodes: a + 3 b + 9 c
+__constant__ __align__( 16 ) int8_t c_p2_from[60];     // micro-cell nodes 10 ty + i, grouped by the window node they are
+__constant__ __align__( 16 ) int8_t c_p2_from0[28];    // window node l: entries c_p2_from0[l] .. c_p2_from0[l + 1] - 1
+__constant__ __align__( 16 ) int8_t c_p2_loc[6][10];  // node of micro-cell type ty in its anchor's 3x3x3 nodes: a + 3 b + 9 c
 __constant__ double c_p2_rgrad[11][10][3];  // reference gradients of the ten basis functions per point
 __constant__ double c_p2_phi[11][10];       // values of the ten basis functions per point
 __constant__ int    c_p2_edge[6][2] = { { 2, 3 }, { 1, 3 }, { 1, 2 }, { 0, 3 }, { 0, 2 }, { 0, 1 } };
-__constant__ int8_t c_p2s_ent[600];  // entry of node j in node i's class stencil: (10 ty + i) 10 + j
+__constant__ __align__( 16 ) int8_t c_p2s_ent[600];  // entry of node j in node i's class stencil: (10 ty + i) 10 + j
 
 // barycentric coordinates (l0, l1, l2, l3) of the rule's points (kept identical to the reference's
 // generated form: the element integrals must agree); reference coordinates are (l1, l2, l3)
@@ -1100,27 +1100,29 @@ struct AccVecs {
    T*       dst[3];
 };
 
+// cell interiors of one component (blockIdx.y): the listed points, one thread each, on levels that list
+// them, else a warp per row
+// (the component is selected by comparison: indexing a kernel parameter with a runtime value copies it to local memory)
+template < typename P >
+__device__ __forceinline__ P component( const P ( &v )[3], unsigned k )
+{
+   return k == 0 ? v[0] : k == 1 ? v[1] : v[2];
+}
+
 template < typename T, typename A, int OP >
-__global__ void __launch_bounds__( 256 ) k_cell_acc( int n, int nrows, const int2* __restrict__ rows, const int64_t* __restrict__ cell_off,
+__global__ void __launch_bounds__( 256 ) k_cell_acc( int n, int nC, int nrows, const int2* __restrict__ rows, int nipts,
+                                                      const ushort4* __restrict__ ipts, const int64_t* __restrict__ cell_off,
                                                       const uint8_t* __restrict__ cell_bc, uint32_t flag, AccVecs< T, A > vec,
                                                       const A* __restrict__ invd, A a0, A a1 )
 {
-   const A* __restrict__ acc = vec.acc[blockIdx.z];
-   const T* src = vec.src[blockIdx.z];
-   const T* v1  = vec.v1[blockIdx.z];
-   T*       v2  = vec.v2[blockIdx.z];
-   T*       dst = vec.dst[blockIdx.z];
-   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int r    = blockIdx.x * 8 + warp;
-   const int c    = blockIdx.y;
-   if ( r >= nrows || !( cell_bc[c] & flag ) ) return;
-   const int2    yz   = rows[r];
-   const int64_t base = cell_off[c] + cidx( n, 0, yz.x, yz.y );
-   for ( int x = 1 + lane; x <= n - 1 - yz.x - yz.y; x += 32 )
-   {
-      const int64_t i = base + x;
-      A             second;
-      const A       val = epilogue_value< T, A, OP >( i, acc[i], invd ? invd[i] : A( 1 ), src, v1, v2, a0, a1, &second );
+   const A* __restrict__ acc = component( vec.acc, blockIdx.y );
+   const T* src = component( vec.src, blockIdx.y );
+   const T* v1  = component( vec.v1, blockIdx.y );
+   T*       v2  = component( vec.v2, blockIdx.y );
+   T*       dst = component( vec.dst, blockIdx.y );
+   auto point = [&]( int64_t i ) {
+      A       second;
+      const A val = epilogue_value< T, A, OP >( i, acc[i], invd ? invd[i] : A( 1 ), src, v1, v2, a0, a1, &second );
       if constexpr ( OP == OP_CHEBL ) st_any( v2 + i, val );
       else if constexpr ( OP == OP_APPLY_ADD ) st_any( dst + i, A( ld_any( dst + i ) ) + val );
       else
@@ -1128,7 +1130,37 @@ __global__ void __launch_bounds__( 256 ) k_cell_acc( int n, int nrows, const int
          st_any( dst + i, val );
          if constexpr ( OP == OP_CHEBI ) st_any( v2 + i, second );
       }
+   };
+   if ( n <= kFlatMaxN )
+   {
+      const int64_t g = int64_t( blockIdx.x ) * 256 + threadIdx.x;
+      if ( g >= int64_t( nC ) * nipts ) return;
+      const int c = g < 0x7fffffff ? int( unsigned( g ) / unsigned( nipts ) ) : int( g / nipts );
+      if ( !( cell_bc[c] & flag ) ) return;
+      const ushort4 p = ipts[int( g - int64_t( c ) * nipts )];
+      point( cell_off[c] + cidx( n, p.x, p.y, p.z ) );
+      return;
    }
+   const int64_t w = int64_t( blockIdx.x ) * 8 + ( threadIdx.x >> 5 );
+   if ( w >= int64_t( nC ) * nrows ) return;
+   const int c = int( unsigned( w ) / unsigned( nrows ) );
+   if ( !( cell_bc[c] & flag ) ) return;
+   const int2    yz   = rows[int( w - int64_t( c ) * nrows )];
+   const int64_t base = cell_off[c] + cidx( n, 0, yz.x, yz.y );
+   for ( int x = 1 + ( threadIdx.x & 31 ); x <= n - 1 - yz.x - yz.y; x += 32 ) point( base + x );
+}
+
+template < typename T, typename A, int OP >
+static void launch_cell_acc( Context* ctx, Mesh* m, const P1Level& P, uint32_t flag, const AccVecs< T, A >& vec, int ncomp, const A* invd, A a0,
+                             A a1 )
+{
+   const int     nC = m->topo.nC, nrows = int( P.rows.size() );
+   const int64_t blocks = P.n <= kFlatMaxN ? ( int64_t( nC ) * P.nipts + 255 ) / 256 : ( int64_t( nC ) * nrows + 7 ) / 8;
+   if ( blocks == 0 ) return;
+   k_cell_acc< T, A, OP ><<< dim3( unsigned( blocks ), ncomp ), 256, 0, ctx->stream >>>( P.n, nC, nrows, P.d_rows, P.nipts,
+                                                                                        reinterpret_cast< const ushort4* >( P.d_ipts ),
+                                                                                        P.d_off + P.nB, P.d_bc + P.nB, flag, vec, invd, a0, a1 );
+   ++ctx->launches;
 }
 
 // cell-array slot of the copy of task tk's point in incidence I
@@ -1187,11 +1219,11 @@ __global__ void __launch_bounds__( 256 ) k_bnd_acc( int n, int ntasks, const int
                                                      const Incidence* __restrict__ inc, uint32_t flag, int copy_unflagged,
                                                      AccVecs< T, A > vec, const A* __restrict__ invd, A* invd_out, A a0, A a1 )
 {
-   const A* __restrict__ acc = vec.acc[blockIdx.y];
-   const T* src = vec.src[blockIdx.y];
-   const T* v1  = vec.v1[blockIdx.y];
-   T*       v2  = vec.v2[blockIdx.y];
-   T*       dst = vec.dst[blockIdx.y];
+   const A* __restrict__ acc = component( vec.acc, blockIdx.y );
+   const T* src = component( vec.src, blockIdx.y );
+   const T* v1  = component( vec.v1, blockIdx.y );
+   T*       v2  = component( vec.v2, blockIdx.y );
+   T*       dst = component( vec.dst, blockIdx.y );
    static_assert( G == 1 || G == 2 || G == 4 || G == 8 || G == 16 || G == 32, "G divides the warp" );
    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
    const int t  = gt / G, sub = gt % G;
@@ -1424,152 +1456,281 @@ __device__ __forceinline__ void mapped_point( const CellGeom& g, const A X0[3], 
    adet        = fabs( det );
 }
 
-// DIVT 0: p_acc[vertex i] += sum_k sum_j B_k[i][j] u_k[j];  DIVT 1: u_acc_k[node j] += sum_i B_k[i][j] p[i]
-template < typename T, typename A, int DIVT >
-__global__ void __launch_bounds__( 128 ) k_stokes_div_pass( int ne, int nanch, const int* __restrict__ anch,
-                                                             const int64_t* __restrict__ off_p, const int64_t* __restrict__ off_u,
-                                                             const CellGeom* __restrict__ geom, const T* __restrict__ u0,
-                                                             const T* __restrict__ u1, const T* __restrict__ u2,
-                                                             const T* __restrict__ p, A* accp, A* acc0, A* acc1, A* acc2,
-                                                             int64_t size_p, int64_t size_u, int* err )
+// B u of one micro-cell: the pressure values of its vertices from the velocity's node values
+template < typename A >
+__device__ __forceinline__ void div_micro( const MicroCell< A >& mc, const ShellCell< A >& sc, bool blend, const A ( &ul )[3][10], A ( &yl )[4] )
 {
-   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-   const int c = blockIdx.y;
-   if ( t >= nanch ) return;
-   const int      a = anch[t];
-   const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
-   const CellGeom& g = geom[c];
-   const bool           blend = g.blend == 1;
-   const ShellCell< A > sc    = shell_cell< A >( g );
-   const int64_t  bp = off_p[c], bu = off_u[c];
-   const A        inv_n = A( 1.0 / double( ne ) );
-   A              st[3][3];
-   for ( int k = 0; k < 3; ++k )
-      for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
-   for ( int ty = 0; ty < 6; ++ty )
-   {
-      if ( x + y + z > ne - 1 - c_mc_shift[ty] ) continue;
-      int V[4][3];
-      for ( int m = 0; m < 4; ++m )
-         for ( int d = 0; d < 3; ++d ) V[m][d] = ( d == 0 ? x : d == 1 ? y : z ) + c_mc_off[ty][m][d];
-      int64_t ip[4], iu[10];
-      for ( int m = 0; m < 4; ++m )
-      {
-         ip[m] = bp + cidx( ne, V[m][0], V[m][1], V[m][2] );
-         iu[m] = bu + cidx( ns, 2 * V[m][0], 2 * V[m][1], 2 * V[m][2] );
-      }
-      for ( int e = 0; e < 6; ++e )
-      {
-         const int ea = c_p2_edge[e][0], eb = c_p2_edge[e][1];
-         iu[4 + e]    = bu + cidx( ns, V[ea][0] + V[eb][0], V[ea][1] + V[eb][1], V[ea][2] + V[eb][2] );
-      }
-      {
-         bool bad = false;
-         for ( int m = 0; m < 4; ++m ) bad |= ip[m] < 0 || ip[m] >= size_p;
-         for ( int m = 0; m < 10; ++m ) bad |= iu[m] < 0 || iu[m] >= size_u;
-         if ( bad )
-         {
-            atomicExch( err, 2 );
-            continue;
-         }
-      }
-      MicroCell< A > mc;
-      micro_cell( g, st, ty, x, y, z, mc );
-      const A wj = -A( 1.0 / 24.0 ) * mc.adet;
-      if constexpr ( DIVT == 0 )
-      {
-         A G[3][4][3];
+   const A wj = -A( 1.0 / 24.0 ) * mc.adet;
+            A G[3][4][3];
 #pragma unroll
-         for ( int k = 0; k < 3; ++k )
-         {
-            const T* u = k == 0 ? u0 : k == 1 ? u1 : u2;
-            A        ul[10];
-#pragma unroll
-            for ( int j = 0; j < 10; ++j ) ul[j] = A( ld_any( u + iu[j] ) );
-            p2_vertex_gradients( ul, mc.Ji, G[k] );
-         }
-         A yl[4] = { A( 0 ), A( 0 ), A( 0 ), A( 0 ) };
+            for ( int k = 0; k < 3; ++k )
+            {
+               p2_vertex_gradients( ul[k], mc.Ji, G[k] );
+            }
+            for ( int i = 0; i < 4; ++i ) yl[i] = A( 0 );
 #pragma unroll 1
-         for ( int q = 0; q < 4; ++q )
-         {
-            const A lam[4] = { A( c_q2_bary[q][0] ), A( c_q2_bary[q][1] ), A( c_q2_bary[q][2] ), A( c_q2_bary[q][3] ) };
-            // velocity gradient B with respect to X; div = (tr B - g^T B X / m) / s and |det DF| = s^2 |m|
-            A B[3][3];
+            for ( int q = 0; q < 4; ++q )
+            {
+               const A lam[4] = { A( c_q2_bary[q][0] ), A( c_q2_bary[q][1] ), A( c_q2_bary[q][2] ), A( c_q2_bary[q][3] ) };
+               // velocity gradient B with respect to X; div = (tr B - g^T B X / m) / s and |det DF| = s^2 |m|
+               A B[3][3];
+#pragma unroll
+               for ( int k = 0; k < 3; ++k )
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d )
+                     B[k][d] = lam[0] * G[k][0][d] + lam[1] * G[k][1][d] + lam[2] * G[k][2][d] + lam[3] * G[k][3][d];
+               A f = B[0][0] + B[1][1] + B[2][2];
+               if ( blend )
+               {
+                  ShellPoint< A > p;
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * lam[1] + mc.J[d][1] * lam[2] + mc.J[d][2] * lam[3];
+                  shell_point( sc, p );
+                  A gbx = A( 0 );
+#pragma unroll
+                  for ( int k = 0; k < 3; ++k ) gbx += p.g[k] * ( B[k][0] * p.X[0] + B[k][1] * p.X[1] + B[k][2] * p.X[2] );
+                  f = ( f - gbx * p.im ) * ( p.s * fabs( p.m ) );
+               }
+               f *= wj;
+#pragma unroll
+               for ( int i = 0; i < 4; ++i ) yl[i] += f * lam[i];
+            }
+}
+
+// B^T p of one micro-cell: the velocity's node values from the vertices' pressures
+template < typename A >
+__device__ __forceinline__ void divt_micro( const MicroCell< A >& mc, const ShellCell< A >& sc, bool blend, const A ( &pl )[4], A ( &yl )[3][10] )
+{
+   const A wj = -A( 1.0 / 24.0 ) * mc.adet;
+            A H[3][4][3];
 #pragma unroll
             for ( int k = 0; k < 3; ++k )
 #pragma unroll
-               for ( int d = 0; d < 3; ++d )
-                  B[k][d] = lam[0] * G[k][0][d] + lam[1] * G[k][1][d] + lam[2] * G[k][2][d] + lam[3] * G[k][3][d];
-            A f = B[0][0] + B[1][1] + B[2][2];
-            if ( blend )
-            {
-               ShellPoint< A > p;
-#pragma unroll
-               for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * lam[1] + mc.J[d][1] * lam[2] + mc.J[d][2] * lam[3];
-               shell_point( sc, p );
-               A gbx = A( 0 );
-#pragma unroll
-               for ( int k = 0; k < 3; ++k ) gbx += p.g[k] * ( B[k][0] * p.X[0] + B[k][1] * p.X[1] + B[k][2] * p.X[2] );
-               f = ( f - gbx * p.im ) * ( p.s * fabs( p.m ) );
-            }
-            f *= wj;
-#pragma unroll
-            for ( int i = 0; i < 4; ++i ) yl[i] += f * lam[i];
-         }
-         for ( int i = 0; i < 4; ++i ) atomicAdd( accp + ip[i], yl[i] );
-      }
-      else
-      {
-         A pl[4];
-         for ( int i = 0; i < 4; ++i ) pl[i] = A( ld_any( p + ip[i] ) );
-         A H[3][4][3];
-#pragma unroll
-         for ( int k = 0; k < 3; ++k )
-#pragma unroll
-            for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = A( 0 );
+               for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = A( 0 );
 #pragma unroll 1
-         for ( int q = 0; q < 4; ++q )
-         {
-            const A lam[4] = { A( c_q2_bary[q][0] ), A( c_q2_bary[q][1] ), A( c_q2_bary[q][2] ), A( c_q2_bary[q][3] ) };
-            A       f      = wj * ( pl[0] * lam[0] + pl[1] * lam[1] + pl[2] * lam[2] + pl[3] * lam[3] );
-            // component k pairs with DF^-1 e_k |det DF| = s |m| (e_k - X g_k / m)
-            A E[3][3] = { { A( 1 ), A( 0 ), A( 0 ) }, { A( 0 ), A( 1 ), A( 0 ) }, { A( 0 ), A( 0 ), A( 1 ) } };
-            if ( blend )
+            for ( int q = 0; q < 4; ++q )
             {
+               const A lam[4] = { A( c_q2_bary[q][0] ), A( c_q2_bary[q][1] ), A( c_q2_bary[q][2] ), A( c_q2_bary[q][3] ) };
+               A       f      = wj * ( pl[0] * lam[0] + pl[1] * lam[1] + pl[2] * lam[2] + pl[3] * lam[3] );
+               // component k pairs with DF^-1 e_k |det DF| = s |m| (e_k - X g_k / m)
+               A E[3][3] = { { A( 1 ), A( 0 ), A( 0 ) }, { A( 0 ), A( 1 ), A( 0 ) }, { A( 0 ), A( 0 ), A( 1 ) } };
+               if ( blend )
+               {
+                  ShellPoint< A > p;
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * lam[1] + mc.J[d][1] * lam[2] + mc.J[d][2] * lam[3];
+                  shell_point( sc, p );
+#pragma unroll
+                  for ( int k = 0; k < 3; ++k )
+                  {
+                     const A gk = p.g[k] * p.im;
+#pragma unroll
+                     for ( int d = 0; d < 3; ++d ) E[k][d] -= p.X[d] * gk;
+                  }
+                  f *= p.s * fabs( p.m );
+               }
+#pragma unroll
+               for ( int v = 0; v < 4; ++v )
+               {
+                  const A fl = f * lam[v];
+#pragma unroll
+                  for ( int k = 0; k < 3; ++k )
+#pragma unroll
+                     for ( int d = 0; d < 3; ++d ) H[k][v][d] += fl * E[k][d];
+               }
+            }
+#pragma unroll
+   for ( int k = 0; k < 3; ++k ) p2_pair_gradients( H[k], mc.Ji, yl[k] );
+}
+
+// the full viscous block of one micro-cell on its three components' node values
+template < typename A >
+__device__ __forceinline__ void visc_micro( const MicroCell< A >& mc, const ShellCell< A >& sc, bool blend, const Coefficient& kc,
+                                            const A ( &ul )[3][10], A ( &yl )[3][10] )
+{
+            A G[3][4][3], H[3][4][3];
+#pragma unroll
+            for ( int k = 0; k < 3; ++k )
+            {
+               p2_vertex_gradients( ul[k], mc.Ji, G[k] );
+#pragma unroll
+               for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = A( 0 );
+            }
+#pragma unroll 1
+            for ( int q = 0; q < 5; ++q )
+            {
+               const A l1 = A( c_yu5_pts[q][0] ), l2 = A( c_yu5_pts[q][1] ), l3 = A( c_yu5_pts[q][2] ), l0 = A( 1 ) - l1 - l2 - l3;
+               A       D[3][3];  // velocity gradient, d u_k / d x_d
+#pragma unroll
+               for ( int k = 0; k < 3; ++k )
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d ) D[k][d] = l0 * G[k][0][d] + l1 * G[k][1][d] + l2 * G[k][2][d] + l3 * G[k][3][d];
                ShellPoint< A > p;
 #pragma unroll
-               for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * lam[1] + mc.J[d][1] * lam[2] + mc.J[d][2] * lam[3];
-               shell_point( sc, p );
+               for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * l1 + mc.J[d][1] * l2 + mc.J[d][2] * l3;
+               A f = A( c_yu5_w[q] ) * mc.adet, F[3] = { p.X[0], p.X[1], p.X[2] }, rad = A( -1 );
+               if ( blend )
+               {
+                  // |det DF| = s^2 |m| takes the two factors 1/s of DF^-T and DF^-1
+                  shell_point( sc, p );
+#pragma unroll
+                  for ( int k = 0; k < 3; ++k )
+                  {
+                     const A xb = ( p.X[0] * D[k][0] + p.X[1] * D[k][1] + p.X[2] * D[k][2] ) * p.im;
+#pragma unroll
+                     for ( int d = 0; d < 3; ++d ) D[k][d] -= p.g[d] * xb;
+                     F[k] = p.X[k] * p.s;
+                  }
+                  f *= fabs( p.m );
+                  rad = p.R;
+               }
+               f *= coeff_eval( kc, F, rad );
+               const A tr3     = A( 2.0 / 3.0 ) * ( D[0][0] + D[1][1] + D[2][2] );
+               A       S[3][3] = { { D[0][0] + D[0][0] - tr3, D[0][1] + D[1][0], D[0][2] + D[2][0] },
+                                   { D[0][1] + D[1][0], D[1][1] + D[1][1] - tr3, D[1][2] + D[2][1] },
+                                   { D[0][2] + D[2][0], D[1][2] + D[2][1], D[2][2] + D[2][2] - tr3 } };
 #pragma unroll
                for ( int k = 0; k < 3; ++k )
                {
-                  const A gk = p.g[k] * p.im;
+                  if ( blend )
+                  {
+                     const A gs = ( p.g[0] * S[k][0] + p.g[1] * S[k][1] + p.g[2] * S[k][2] ) * p.im;
 #pragma unroll
-                  for ( int d = 0; d < 3; ++d ) E[k][d] -= p.X[d] * gk;
+                     for ( int d = 0; d < 3; ++d ) S[k][d] -= p.X[d] * gs;
+                  }
+#pragma unroll
+                  for ( int d = 0; d < 3; ++d )
+                  {
+                     const A h = f * S[k][d];
+                     H[k][0][d] += l0 * h;
+                     H[k][1][d] += l1 * h;
+                     H[k][2][d] += l2 * h;
+                     H[k][3][d] += l3 * h;
+                  }
                }
-               f *= p.s * fabs( p.m );
             }
 #pragma unroll
-            for ( int v = 0; v < 4; ++v )
-            {
-               const A fl = f * lam[v];
-#pragma unroll
-               for ( int k = 0; k < 3; ++k )
-#pragma unroll
-                  for ( int d = 0; d < 3; ++d ) H[k][v][d] += fl * E[k][d];
-            }
-         }
-#pragma unroll
-         for ( int k = 0; k < 3; ++k )
-         {
-            A  yl[10];
-            A* o = k == 0 ? acc0 : k == 1 ? acc1 : acc2;
-            p2_pair_gradients( H[k], mc.Ji, yl );
-#pragma unroll
-            for ( int j = 0; j < 10; ++j ) atomicAdd( o + iu[j], yl[j] );
-         }
+   for ( int k = 0; k < 3; ++k ) p2_pair_gradients( H[k], mc.Ji, yl[k] );
+}
+
+// One parity pass of a coupled operator, a thread per micro-cell: warp w takes type w of the block's 32
+// anchors.  The six micro-cells of an anchor share nodes, so their results meet in shared memory and are
+// added to the accumulators once per node, in a fixed order.  A thread per anchor walked its six
+// micro-cells one after the other, 20 to 40 us a pass on levels whose classes have a few thousand anchors.
+// Full viscous apply, shell of 480 cells, level 3: 399 -> 341 us; of 240 cells, level 2: 630 us with the
+// element loops of 10 basis gradients, 187 us so; 960 cells, level 4: 4.71 -> 2.69 ms.  At 168 registers two
+// blocks fit an SM.
+enum { CPL_VISCOUS = 0, CPL_DIVT, CPL_DIV };
+template < typename T, typename A >
+struct CoupledArgs {
+   const T* u[3];
+   const T* p;
+   A*       acc[3];  // velocity components, or the pressure in acc[0]
+};
+constexpr int kCoupledThreads = 192;
+template < typename T, typename A, int OPER >
+__global__ void __launch_bounds__( kCoupledThreads, 2 )
+    k_coupled_pass( int ne, int nC, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ off_p, const int64_t* __restrict__ off_u,
+                    const CellGeom* __restrict__ geom, Coefficient kc, CoupledArgs< T, A > v, int64_t size_p, int64_t size_u, int* err )
+{
+   constexpr int NC = OPER == CPL_DIV ? 1 : 3, NN = OPER == CPL_DIV ? 4 : 10;  // result components, nodes per micro-cell
+   __shared__ A  ys[NC][6 * NN][32];
+   const int     ty = threadIdx.x >> 5, lane = threadIdx.x & 31, ns = 2 * ne;
+   const int64_t t    = int64_t( blockIdx.x ) * 32 + lane;
+   bool          live = t < int64_t( nC ) * nanch;
+   const int64_t tt   = live ? t : 0;
+   const int     c    = tt < 0x7fffffff ? int( unsigned( tt ) / unsigned( nanch ) ) : int( tt / nanch );
+   const int     a    = anch[int( tt - int64_t( c ) * nanch )];
+   const int     x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, room = ns - 2 * ( x + y + z );
+   const int64_t bu = off_u[c], bp = off_p ? off_p[c] : 0;
+   {
+      // self-check: the window's last node inside the level's vectors
+      const int64_t lu = bu + cidx( ns, 2 * x, 2 * y, 2 * z + min( room, 2 ) ), lp = bp + cidx( ne, x, y, z + min( room / 2, 1 ) );
+      if ( live && ( room < 2 || bu < 0 || lu >= size_u || ( off_p && ( bp < 0 || lp >= size_p ) ) ) )
+      {
+         atomicExch( err, 2 );
+         live = false;
       }
    }
+   auto at_u = [&]( int l ) { return bu + cidx( ns, 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9 ); };
+   auto at_p = [&]( int l ) { return bp + cidx( ne, x + ( l & 1 ), y + ( ( l >> 1 ) & 1 ), z + ( l >> 2 ) ); };
+   // vertex i of the type: its number x + 2 y + 4 z among the anchor's eight
+   auto vert = [&]( int i ) {
+      const int l = c_p2_loc[ty][i];
+      return ( l % 3 ) / 2 + ( l / 3 ) % 3 / 2 * 2 + l / 9 / 2 * 4;
+   };
+   if ( live && x + y + z <= ne - 1 - c_mc_shift[ty] )
+   {
+      const CellGeom&      g     = geom[c];
+      const bool           blend = g.blend == 1;
+      const ShellCell< A > sc    = shell_cell< A >( g );
+      const A              inv_n = A( 1.0 / double( ne ) );
+      MicroCell< A >       mc;
+      {
+         A st[3][3];
+         for ( int k = 0; k < 3; ++k )
+            for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
+         micro_cell( g, st, ty, x, y, z, mc );
+      }
+      A yl[NC][NN];
+      if constexpr ( OPER == CPL_DIVT )
+      {
+         A pl[4];
+#pragma unroll
+         for ( int i = 0; i < 4; ++i ) pl[i] = A( ld_any( v.p + at_p( vert( i ) ) ) );
+         divt_micro( mc, sc, blend, pl, yl );
+      }
+      else
+      {
+         A ul[3][10];
+#pragma unroll
+         for ( int i = 0; i < 10; ++i )
+         {
+            const int64_t at = at_u( c_p2_loc[ty][i] );
+#pragma unroll
+            for ( int k = 0; k < 3; ++k ) ul[k][i] = A( ld_any( v.u[k] + at ) );
+         }
+         if constexpr ( OPER == CPL_VISCOUS ) visc_micro( mc, sc, blend, kc, ul, yl );
+         else div_micro( mc, sc, blend, ul, yl[0] );
+      }
+#pragma unroll
+      for ( int k = 0; k < NC; ++k )
+#pragma unroll
+         for ( int i = 0; i < NN; ++i ) ys[k][NN * ty + i][lane] = yl[k][i];
+   }
+   else
+#pragma unroll
+      for ( int k = 0; k < NC; ++k )
+#pragma unroll
+         for ( int i = 0; i < NN; ++i ) ys[k][NN * ty + i][lane] = A( 0 );
+   __syncthreads();
+   if ( !live ) return;
+   if constexpr ( OPER == CPL_DIV )
+   {
+      for ( int l = ty; l < 8; l += 6 )
+      {
+         const int dx = l & 1, dy = ( l >> 1 ) & 1, dz = l >> 2, w = 2 * dx + 6 * dy + 18 * dz;
+         if ( 2 * ( dx + dy + dz ) > room ) continue;
+         A s = A( 0 );
+         for ( int k = c_p2_from0[w]; k < c_p2_from0[w + 1]; ++k )
+            s += ys[0][4 * ( c_p2_from[k] / 10 ) + c_p2_from[k] % 10][lane];  // a vertex of the window is one of every micro-cell that has it
+         v.acc[0][at_p( l )] += s;
+      }
+   }
+   else
+      for ( int l = ty; l < 27; l += 6 )
+      {
+         if ( l % 3 + ( l / 3 ) % 3 + l / 9 > room ) continue;
+         A s[NC];
+#pragma unroll
+         for ( int j = 0; j < NC; ++j ) s[j] = A( 0 );
+         for ( int k = c_p2_from0[l]; k < c_p2_from0[l + 1]; ++k )
+#pragma unroll
+            for ( int j = 0; j < NC; ++j ) s[j] += ys[j][c_p2_from[k]][lane];
+         const int64_t at = at_u( l );
+#pragma unroll
+         for ( int j = 0; j < NC; ++j ) v.acc[j][at] += s[j];
+      }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1896,7 +2057,6 @@ static void run_elem( Context* ctx, Mesh* m, Operator* op, int L, int dtype, con
       return;
    }
    run_passes< T, A, 0 >( ctx, m, op, L, (const T*) a.src, acc );
-   const int nrows = int( P.rows.size() );
    {
       struct Join
       {
@@ -1910,13 +2070,7 @@ static void run_elem( Context* ctx, Mesh* m, Operator* op, int L, int dtype, con
       check_cuda( cudaEventRecord( ctx->ev_fork, ctx->stream ), "fork" );
       check_cuda( cudaStreamWaitEvent( ctx->aux, ctx->ev_fork, 0 ), "fork" );
       Join j{ ctx };
-      if ( nrows > 0 )
-      {
-         dim3 grid( ( nrows + 7 ) / 8, m->topo.nC );
-         k_cell_acc< T, A, OP ><<< grid, 256, 0, ctx->stream >>>( P.n, nrows, P.d_rows, P.d_off + P.nB, P.d_bc + P.nB, a.flag,
-                                                                   acc_vecs< T, A >( acc, a ), inv, A( a.a0 ), A( a.a1 ) );
-         ++ctx->launches;
-      }
+      launch_cell_acc< T, A, OP >( ctx, m, P, a.flag, acc_vecs< T, A >( acc, a ), 1, inv, A( a.a0 ), A( a.a1 ) );
       launch_bnd_acc< T, A, OP >( ctx, ctx->aux, P, a.flag, a.copy_unflagged, acc_vecs< T, A >( acc, a ), 1, inv, nullptr, A( a.a0 ),
                                   A( a.a1 ) );
    }
@@ -1959,13 +2113,7 @@ static void combine_acc( Context* ctx, Mesh* m, int L, const AccVecs< T, A >& ve
    check_cuda( cudaEventRecord( ctx->ev_fork, ctx->stream ), "fork" );
    check_cuda( cudaStreamWaitEvent( ctx->aux, ctx->ev_fork, 0 ), "fork" );
    Join      j{ ctx };
-   const int nrows = int( P.rows.size() );
-   if ( nrows > 0 )
-   {
-      dim3 grid( ( nrows + 7 ) / 8, m->topo.nC, ncomp );
-      k_cell_acc< T, A, OP ><<< grid, 256, 0, ctx->stream >>>( P.n, nrows, P.d_rows, P.d_off + P.nB, P.d_bc + P.nB, flag, vec, invd, a0, A( 0 ) );
-      ++ctx->launches;
-   }
+   launch_cell_acc< T, A, OP >( ctx, m, P, flag, vec, ncomp, invd, a0, A( 0 ) );
    launch_bnd_acc< T, A, OP >( ctx, ctx->aux, P, flag, 0, vec, ncomp, invd, nullptr, a0, A( 0 ) );
    check_cuda( cudaGetLastError(), "combine launch" );
 }
@@ -1980,6 +2128,7 @@ static void run_stokes( Context* ctx, Operator* op, int Lp, int divt, const void
    P1Level&   PU = m->level( Ls );
    ensure_device( m, PP );
    ensure_device( m, PU );
+   ensure_p2_constants();
    ensure_stokes_constants();
    if ( !op->d_geom )
    {
@@ -1996,25 +2145,27 @@ static void run_stokes( Context* ctx, Operator* op, int Lp, int divt, const void
    if ( divt ) check_cuda( cudaMemsetAsync( acc_u, 0, size_t( 3 * PU.size ) * sizeof( A ), ctx->stream ), "cudaMemset" );
    else check_cuda( cudaMemsetAsync( acc_p, 0, size_t( PP.size ) * sizeof( A ), ctx->stream ), "cudaMemset" );
    const int nC = m->topo.nC;
+   CoupledArgs< T, A > v{};
+   for ( int k = 0; k < 3; ++k )
+   {
+      v.u[k]   = u ? (const T*) u[k] : nullptr;
+      v.acc[k] = divt ? acc_u + k * PU.size : nullptr;
+   }
+   v.p = (const T*) p;
+   if ( !divt ) v.acc[0] = acc_p;
    for ( int pc = 0; pc < 8; ++pc )
    {
       const int na = e.aoff[pc + 1] - e.aoff[pc];
       if ( na <= 0 ) continue;
-      const int bs = pass_block( na, 128 );
-      dim3      grid( ( na + bs - 1 ) / bs, nC );
-      const T* u0 = u ? (const T*) u[0] : nullptr;
-      const T* u1 = u ? (const T*) u[1] : nullptr;
-      const T* u2 = u ? (const T*) u[2] : nullptr;
+      const unsigned blocks = unsigned( ( int64_t( na ) * nC + 31 ) / 32 );
       if ( divt )
-         k_stokes_div_pass< T, A, 1 ><<< grid, bs, 0, ctx->stream >>>( 1 << Lp, na, e.d_anch + e.aoff[pc], PP.d_off + PP.nB,
-                                                                         PU.d_off + PU.nB, op->d_geom, u0, u1, u2, (const T*) p, acc_p,
-                                                                         acc_u, acc_u + PU.size, acc_u + 2 * PU.size, PP.size, PU.size,
-                                                                         ctx->d_error );
+         k_coupled_pass< T, A, CPL_DIVT ><<< blocks, kCoupledThreads, 0, ctx->stream >>>( 1 << Lp, nC, na, e.d_anch + e.aoff[pc], PP.d_off + PP.nB,
+                                                                                         PU.d_off + PU.nB, op->d_geom, op->coeff, v, PP.size,
+                                                                                         PU.size, ctx->d_error );
       else
-         k_stokes_div_pass< T, A, 0 ><<< grid, bs, 0, ctx->stream >>>( 1 << Lp, na, e.d_anch + e.aoff[pc], PP.d_off + PP.nB,
-                                                                         PU.d_off + PU.nB, op->d_geom, u0, u1, u2, (const T*) p, acc_p,
-                                                                         acc_u, acc_u + PU.size, acc_u + 2 * PU.size, PP.size, PU.size,
-                                                                         ctx->d_error );
+         k_coupled_pass< T, A, CPL_DIV ><<< blocks, kCoupledThreads, 0, ctx->stream >>>( 1 << Lp, nC, na, e.d_anch + e.aoff[pc], PP.d_off + PP.nB,
+                                                                                        PU.d_off + PU.nB, op->d_geom, op->coeff, v, PP.size,
+                                                                                        PU.size, ctx->d_error );
       ++ctx->launches;
    }
    check_cuda( cudaGetLastError(), "Stokes pass launch" );
@@ -2094,10 +2245,10 @@ static void ensure_visc_constants()
    } );
 }
 
-template < typename T, typename A, int MODE >
-__global__ void __launch_bounds__( 128 ) k_visc_pass( int ne, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ off_u,
-                                                       const CellGeom* __restrict__ geom, Coefficient kc, const T* __restrict__ u0,
-                                                       const T* __restrict__ u1, const T* __restrict__ u2, A* acc0, A* acc1, A* acc2,
+// diagonal of the full viscous block, one parity pass
+template < typename A >
+__global__ void __launch_bounds__( 128 ) k_visc_diagonal( int ne, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ off_u,
+                                                       const CellGeom* __restrict__ geom, Coefficient kc, A* acc0, A* acc1, A* acc2,
                                                        int64_t size_u, int* err )
 {
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2106,8 +2257,6 @@ __global__ void __launch_bounds__( 128 ) k_visc_pass( int ne, int nanch, const i
    const int      a  = anch[t];
    const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
    const CellGeom&      g     = geom[c];
-   const bool           blend = g.blend == 1;
-   const ShellCell< A > sc    = shell_cell< A >( g );
    const int64_t  bu = off_u[c];
    const A        inv_n = A( 1.0 / double( ne ) );
    A              st[3][3];
@@ -2137,84 +2286,6 @@ __global__ void __launch_bounds__( 128 ) k_visc_pass( int ne, int nanch, const i
       }
       MicroCell< A > mc;
       micro_cell( g, st, ty, x, y, z, mc );
-      if constexpr ( MODE == 0 )
-      {
-         A G[3][4][3], H[3][4][3];
-#pragma unroll
-         for ( int k = 0; k < 3; ++k )
-         {
-            const T* u = k == 0 ? u0 : k == 1 ? u1 : u2;
-            A        ul[10];
-#pragma unroll
-            for ( int j = 0; j < 10; ++j ) ul[j] = A( ld_any( u + iu[j] ) );
-            p2_vertex_gradients( ul, mc.Ji, G[k] );
-#pragma unroll
-            for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = A( 0 );
-         }
-#pragma unroll 1
-         for ( int q = 0; q < 5; ++q )
-         {
-            const A l1 = A( c_yu5_pts[q][0] ), l2 = A( c_yu5_pts[q][1] ), l3 = A( c_yu5_pts[q][2] ), l0 = A( 1 ) - l1 - l2 - l3;
-            A       D[3][3];  // velocity gradient, d u_k / d x_d
-#pragma unroll
-            for ( int k = 0; k < 3; ++k )
-#pragma unroll
-               for ( int d = 0; d < 3; ++d ) D[k][d] = l0 * G[k][0][d] + l1 * G[k][1][d] + l2 * G[k][2][d] + l3 * G[k][3][d];
-            ShellPoint< A > p;
-#pragma unroll
-            for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * l1 + mc.J[d][1] * l2 + mc.J[d][2] * l3;
-            A f = A( c_yu5_w[q] ) * mc.adet, F[3] = { p.X[0], p.X[1], p.X[2] }, rad = A( -1 );
-            if ( blend )
-            {
-               // |det DF| = s^2 |m| takes the two factors 1/s of DF^-T and DF^-1
-               shell_point( sc, p );
-#pragma unroll
-               for ( int k = 0; k < 3; ++k )
-               {
-                  const A xb = ( p.X[0] * D[k][0] + p.X[1] * D[k][1] + p.X[2] * D[k][2] ) * p.im;
-#pragma unroll
-                  for ( int d = 0; d < 3; ++d ) D[k][d] -= p.g[d] * xb;
-                  F[k] = p.X[k] * p.s;
-               }
-               f *= fabs( p.m );
-               rad = p.R;
-            }
-            f *= coeff_eval( kc, F, rad );
-            const A tr3     = A( 2.0 / 3.0 ) * ( D[0][0] + D[1][1] + D[2][2] );
-            A       S[3][3] = { { D[0][0] + D[0][0] - tr3, D[0][1] + D[1][0], D[0][2] + D[2][0] },
-                                { D[0][1] + D[1][0], D[1][1] + D[1][1] - tr3, D[1][2] + D[2][1] },
-                                { D[0][2] + D[2][0], D[1][2] + D[2][1], D[2][2] + D[2][2] - tr3 } };
-#pragma unroll
-            for ( int k = 0; k < 3; ++k )
-            {
-               if ( blend )
-               {
-                  const A gs = ( p.g[0] * S[k][0] + p.g[1] * S[k][1] + p.g[2] * S[k][2] ) * p.im;
-#pragma unroll
-                  for ( int d = 0; d < 3; ++d ) S[k][d] -= p.X[d] * gs;
-               }
-#pragma unroll
-               for ( int d = 0; d < 3; ++d )
-               {
-                  const A h = f * S[k][d];
-                  H[k][0][d] += l0 * h;
-                  H[k][1][d] += l1 * h;
-                  H[k][2][d] += l2 * h;
-                  H[k][3][d] += l3 * h;
-               }
-            }
-         }
-#pragma unroll
-         for ( int k = 0; k < 3; ++k )
-         {
-            A  yl[10];
-            A* o = k == 0 ? acc0 : k == 1 ? acc1 : acc2;
-            p2_pair_gradients( H[k], mc.Ji, yl );
-#pragma unroll
-            for ( int j = 0; j < 10; ++j ) atomicAdd( o + iu[j], yl[j] );
-         }
-      }
-      else
       {
          A yl[3][10];
          for ( int k = 0; k < 3; ++k )
@@ -2250,6 +2321,7 @@ static void run_visc( Context* ctx, Operator* op, int Lp, int mode, const void* 
    const int Ls = Lp + 1;
    P1Level&  PU = m->level( Ls );
    ensure_device( m, PU );
+   ensure_p2_constants();
    ensure_visc_constants();
    if ( !op->d_geom )
    {
@@ -2263,23 +2335,26 @@ static void run_visc( Context* ctx, Operator* op, int Lp, int mode, const void* 
    A* acc = reinterpret_cast< A* >( e.d_sacc );
    check_cuda( cudaMemsetAsync( acc, 0, size_t( 3 * PU.size ) * sizeof( A ), ctx->stream ), "cudaMemset" );
    const int nC = m->topo.nC;
-   const T*  u0 = u ? (const T*) u[0] : nullptr;
-   const T*  u1 = u ? (const T*) u[1] : nullptr;
-   const T*  u2 = u ? (const T*) u[2] : nullptr;
+   CoupledArgs< T, A > v{};
+   for ( int k = 0; k < 3; ++k )
+   {
+      v.u[k]   = u ? (const T*) u[k] : nullptr;
+      v.acc[k] = acc + k * PU.size;
+   }
    for ( int pc = 0; pc < 8; ++pc )
    {
       const int na = e.aoff[pc + 1] - e.aoff[pc];
       if ( na <= 0 ) continue;
-      const int bs = pass_block( na, 128 );
-      dim3      grid( ( na + bs - 1 ) / bs, nC );
       if ( mode == 0 )
-         k_visc_pass< T, A, 0 ><<< grid, bs, 0, ctx->stream >>>( 1 << Lp, na, e.d_anch + e.aoff[pc], PU.d_off + PU.nB, op->d_geom, op->coeff,
-                                                                 u0, u1, u2, acc, acc + PU.size, acc + 2 * PU.size, PU.size,
-                                                                 ctx->d_error );
+         k_coupled_pass< T, A, CPL_VISCOUS ><<< unsigned( ( int64_t( na ) * nC + 31 ) / 32 ), kCoupledThreads, 0, ctx->stream >>>(
+             1 << Lp, nC, na, e.d_anch + e.aoff[pc], nullptr, PU.d_off + PU.nB, op->d_geom, op->coeff, v, 0, PU.size, ctx->d_error );
       else
-         k_visc_pass< T, A, 1 ><<< grid, bs, 0, ctx->stream >>>( 1 << Lp, na, e.d_anch + e.aoff[pc], PU.d_off + PU.nB, op->d_geom, op->coeff,
-                                                                 u0, u1, u2, acc, acc + PU.size, acc + 2 * PU.size, PU.size,
-                                                                 ctx->d_error );
+      {
+         const int bs = pass_block( na, 128 );
+         dim3      grid( ( na + bs - 1 ) / bs, nC );
+         k_visc_diagonal< A ><<< grid, bs, 0, ctx->stream >>>( 1 << Lp, na, e.d_anch + e.aoff[pc], PU.d_off + PU.nB, op->d_geom, op->coeff, acc,
+                                                               acc + PU.size, acc + 2 * PU.size, PU.size, ctx->d_error );
+      }
       ++ctx->launches;
    }
    check_cuda( cudaGetLastError(), "viscous block pass launch" );
