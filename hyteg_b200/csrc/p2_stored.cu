@@ -25,13 +25,15 @@ int64_t build_p2_stored( P2StoredView& v, int n, int nC, std::vector< ushort4 >&
             rank[size_t( cidx( n, x, y, z ) )] = int( seg[s].size() );
             seg[s].push_back( make_ushort4( (unsigned short) x, (unsigned short) y, (unsigned short) z, 0 ) );
          }
-   int64_t at = 0;
+   constexpr int entries[8] = { P2Class< 0 >::S.n, P2Class< 1 >::S.n, P2Class< 2 >::S.n, P2Class< 3 >::S.n,
+                                P2Class< 4 >::S.n, P2Class< 5 >::S.n, P2Class< 6 >::S.n, P2Class< 7 >::S.n };
+   int64_t       at         = 0;
    for ( int s = 0; s < 16; ++s )
    {
       v.np[s]    = int( seg[s].size() );
       v.pbase[s] = int( pts.size() );
       v.wbase[s] = at;
-      at += int64_t( p2_stencil( s & 7 ).n ) * nC * v.np[s];
+      at += int64_t( entries[s & 7] ) * nC * v.np[s];
       pts.insert( pts.end(), seg[s].begin(), seg[s].end() );
    }
    return at;
@@ -112,10 +114,12 @@ __device__ __forceinline__ void stored_terms( const T* const ( &at )[NV], const 
 }
 
 // One thread per node and all entries of its class unrolled, so the loads of a node are independent of
-// each other.  Bound by the weights' bytes (230 per node in FP64, read once, coalesced): element matrices
-// took 330 and eight passes of read-modify-writes over the nodes, and one launch replaces ten.  Nodes
-// inside a macro-cell finish here; those on its boundary leave their partial sums in acc, which the owners
-// then combine.
+// each other.  Bound by the weights (230 bytes per node in FP64, read once, coalesced) and by the vector's
+// rows, which every class reads from L2 again: element matrices took 330 bytes and eight passes of
+// read-modify-writes over the nodes, and one launch replaces ten.  Chebyshev(3) step on a shell of 240 cells,
+// level 4, FP64: 898 -> 430 us.  (A block per cell with the vector in shared memory: 519 us.)  Nodes inside a
+// macro-cell finish here; those on its boundary leave their partial sums in acc, which the owners then
+// combine.  With three vectors (the velocity components) the weights are read once for all.
 template < typename T, typename A, int NV >
 __global__ void __launch_bounds__( 256 )
     k_p2_stored_sweep( P2StoredView v, int op, uint32_t flag, const uint8_t* __restrict__ cell_bc, const int64_t* __restrict__ cell_off,
