@@ -562,7 +562,7 @@ def p2_leg(H, ctx, level=5, cycle_level=3):
     sec = time_apply(S, Ls, 5)
     mcs = nC * (1 << Ls) ** 3
     out["apply_stored"] = {"level": Ls, "micro_cells": mcs, "ms": sec * 1e3, "Mcells_per_s": mcs / sec / 1e6,
-                           "bytes_per_micro_cell": 55 * 8}
+                           "bytes_per_node": 28.75 * 8}
     del S
     Ac = H.P2ElementwiseBlendingDivKGradOperator(pm, 0, cycle_level, ctx, k=K, blending="shell")
     Ac.computeAndStoreLocalElementMatrices()
