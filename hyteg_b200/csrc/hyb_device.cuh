@@ -133,33 +133,6 @@ static inline LevelView make_view( Mesh* m, int L )
    return v;
 }
 
-// The contiguous groups of the type-sorted task list a boundary launch covers: every group when
-// unflagged owners are copied, else the groups whose boundary type is in `flag`.
-struct TaskSegments
-{
-   int start[4];
-   int count[4];
-};
-
-static inline TaskSegments task_segments( const LevelView& v, uint32_t flag, int all )
-{
-   static const uint32_t type_bit[4] = { kInner, kDirichlet, kNeumann, kFreeslip };
-   TaskSegments          s{};
-   int                   k = 0, at = 0;
-   for ( int g = 0; g < 4; ++g )
-   {
-      const int n = v.nlow[g] + v.nface[g];
-      if ( n > 0 && ( all || ( flag & type_bit[g] ) ) )
-      {
-         s.start[k] = at;
-         s.count[k] = n;
-         ++k;
-      }
-      at += n;
-   }
-   return s;
-}
-
 __device__ __forceinline__ int64_t owner_slot( const LevelView& v, int b, int i, int j )
 {
    const int k = v.bkind[b];
