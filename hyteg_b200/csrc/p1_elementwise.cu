@@ -390,6 +390,7 @@ __global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const in
 __constant__ double c_xg4_pts[11][3];
 __constant__ double c_xg4_bary[11][4];
 __constant__ double c_xg4_w[11];
+__constant__ double c_xg4_mass[11][10];  // w lambda_i lambda_j, i <= j
 __constant__ __align__( 16 ) int8_t c_p2_from[60];     // micro-cell nodes 10 ty + i, grouped by the window node they are
 __constant__ __align__( 16 ) int8_t c_p2_from0[28];    // window node l: entries c_p2_from0[l] .. c_p2_from0[l + 1] - 1
 __constant__ __align__( 16 ) int8_t c_p2_loc[6][10];  // node of micro-cell type ty in its anchor's 3x3x3 nodes: a + 3 b + 9 c
@@ -489,6 +490,11 @@ void ensure_p2_constants()
          for ( int d = 0; d < 3; ++d ) bary[q][d + 1] = pts[q][d];
       }
       check_cuda( cudaMemcpyToSymbol( c_xg4_bary, bary, sizeof( bary ) ), "P2 constants (barycentric points)" );
+      double mass[11][10];
+      for ( int q = 0; q < 11; ++q )
+         for ( int i = 0, v = 0; i < 4; ++i )
+            for ( int j = i; j < 4; ++j, ++v ) mass[q][v] = w[q] * bary[q][i] * bary[q][j];
+      check_cuda( cudaMemcpyToSymbol( c_xg4_mass, mass, sizeof( mass ) ), "P2 constants (products)" );
       int8_t loc[6][10];
       for ( int ty = 0; ty < 6; ++ty )
          for ( int i = 0; i < 10; ++i )
@@ -528,31 +534,17 @@ void ensure_p2_constants()
 // On a micro-cell J is constant, so only the blending map's DF varies between points.  For the shell
 // DF = s I + X g^T (s = R / |X|, g the gradient of s), a rank-one update, so
 //    det DF = s^2 m,  DF^-1 = (I - X g^T / m) / s,  DF^-T = (I - g X^T / m) / s,  m = s + g . X,
-// and m = (gradient of R . X) / |X| without cancellation.  Gradients of quadratic functions are affine,
+// and R's weight t = t0 + sum_k lambda_k(q) t_k is affine too.  Gradients of quadratic functions are affine,
 // so they are interpolated from the four vertices: grad u at vertex k is a combination of ten node
 // values with integer weights, and sum_q of the pairing with every basis gradient needs only
 // H_k = sum_q lambda_k(q) h(q) at the four vertices.  Per point this takes about 100 operations and the
 // coefficient, against 300 for the 3x3 inverse and two loops over ten reference gradients.
+//
+// What a micro-cell computes once (J, its inverse, t, the gradients at the vertices and the final pairing)
+// is computed in FP64 for every value type, and only the loop over the points in the accumulation type: the
+// vertices' gradients cancel at the points and J is a difference of coordinates, so that in FP32 the whole
+// was less exact than evaluating every point by itself.
 // ---------------------------------------------------------------------------------------------
-template < typename A >
-struct ShellCell {
-   A bx[3];   // gradient of the barycentric weight t of the cell's ref vertex (up to its offset)
-   A t0;      // t at the ray vertex
-   A rad, dr; // R = rad + |t - t0| dr
-};
-
-template < typename A >
-__device__ __forceinline__ ShellCell< A > shell_cell( const CellGeom& g )
-{
-   ShellCell< A > c;
-   const double   iv = g.blend == 1 ? 1.0 / g.volT : 0.0;
-   for ( int d = 0; d < 3; ++d ) c.bx[d] = A( g.bxc[d] * iv );
-   c.t0  = A( ( g.ray[0] * g.bxc[0] + g.ray[1] * g.bxc[1] + g.ray[2] * g.bxc[2] ) * iv );
-   c.rad = A( g.rad_ray );
-   c.dr  = A( g.rad_ref - g.rad_ray );
-   return c;
-}
-
 template < typename A >
 struct ShellPoint {
    A X[3], g[3];
@@ -562,42 +554,43 @@ struct ShellPoint {
 __device__ __forceinline__ double rsqrt_of( double v ) { return rsqrt( v ); }
 __device__ __forceinline__ float  rsqrt_of( float v ) { return rsqrtf( v ); }
 
-// p.X is set by the caller
-template < typename A >
-__device__ __forceinline__ void shell_point( const ShellCell< A >& c, ShellPoint< A >& p )
-{
-   const A t   = p.X[0] * c.bx[0] + p.X[1] * c.bx[1] + p.X[2] * c.bx[2];
-   const A lam = t - c.t0;
-   p.R         = c.rad + fabs( lam ) * c.dr;
-   const A d   = lam < A( 0 ) ? -c.dr : c.dr;
-   const A ir  = rsqrt_of( p.X[0] * p.X[0] + p.X[1] * p.X[1] + p.X[2] * p.X[2] );
-   p.s         = p.R * ir;
-   const A e   = ir * d, f = p.s * ir * ir;
-   for ( int k = 0; k < 3; ++k ) p.g[k] = e * c.bx[k] - f * p.X[k];
-   p.m  = e * t;
-   p.im = A( 1 ) / p.m;
-}
-
-// one micro-cell of an anchor: first vertex, columns of J, J^-1 and |det J| (st: computational steps)
+// one micro-cell of an anchor: first vertex, columns of J, J^-1, |det J| and the shell map's weight t at the
+// first vertex and its differences to the others (A: type of the points; J^-1 and |det J| in FP64)
 template < typename A >
 struct MicroCell {
-   A X0[3], J[3][3], Ji[3][3], adet;
+   A      X0[3], J[3][3];
+   A      t[4];
+   A      bx[3], rad, dr;  // gradient of t; R = rad + |t| dr
+   double Ji[3][3], adet;
 };
 
 template < typename A >
-__device__ __forceinline__ void micro_cell( const CellGeom& g, const A st[3][3], int ty, int x, int y, int z, MicroCell< A >& c )
+__device__ __forceinline__ void micro_cell( const CellGeom& g, int ne, int ty, int x, int y, int z, MicroCell< A >& c )
 {
-   const A v0[3] = { A( x + c_mc_off[ty][0][0] ), A( y + c_mc_off[ty][0][1] ), A( z + c_mc_off[ty][0][2] ) };
+   const double inv_n = 1.0 / double( ne ), v0[3] = { double( x + c_mc_off[ty][0][0] ), double( y + c_mc_off[ty][0][1] ), double( z + c_mc_off[ty][0][2] ) };
+   const double iv    = g.blend == 1 ? 1.0 / g.volT : 0.0;
+   double       J[3][3], t[4] = { 0, 0, 0, 0 };
    for ( int d = 0; d < 3; ++d )
    {
-      c.X0[d] = A( g.P[0][d] ) + st[0][d] * v0[0] + st[1][d] * v0[1] + st[2][d] * v0[2];
+      double st[3];  // computational steps
+      for ( int k = 0; k < 3; ++k ) st[k] = ( g.P[k + 1][d] - g.P[0][d] ) * inv_n;
+      const double X = g.P[0][d] + st[0] * v0[0] + st[1] * v0[1] + st[2] * v0[2], b = g.bxc[d] * iv;
       for ( int k = 0; k < 3; ++k )
-         c.J[d][k] = st[0][d] * A( c_mc_off[ty][k + 1][0] - c_mc_off[ty][0][0] ) + st[1][d] * A( c_mc_off[ty][k + 1][1] - c_mc_off[ty][0][1] ) +
-                     st[2][d] * A( c_mc_off[ty][k + 1][2] - c_mc_off[ty][0][2] );
+      {
+         J[d][k] = st[0] * double( c_mc_off[ty][k + 1][0] - c_mc_off[ty][0][0] ) + st[1] * double( c_mc_off[ty][k + 1][1] - c_mc_off[ty][0][1] ) +
+                   st[2] * double( c_mc_off[ty][k + 1][2] - c_mc_off[ty][0][2] );
+         c.J[d][k] = A( J[d][k] );
+         t[k + 1] += b * J[d][k];
+      }
+      t[0] += b * ( X - g.ray[d] );
+      c.X0[d] = A( X );
+      c.bx[d] = A( b );
    }
-   const A( &J )[3][3] = c.J;
-   const A c0 = J[1][1] * J[2][2] - J[1][2] * J[2][1], c1 = J[1][2] * J[2][0] - J[1][0] * J[2][2], c2 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-   const A det = J[0][0] * c0 + J[0][1] * c1 + J[0][2] * c2, id = A( 1 ) / det;
+   for ( int k = 0; k < 4; ++k ) c.t[k] = A( t[k] );
+   c.rad = A( g.rad_ray );
+   c.dr  = A( g.rad_ref - g.rad_ray );
+   const double c0 = J[1][1] * J[2][2] - J[1][2] * J[2][1], c1 = J[1][2] * J[2][0] - J[1][0] * J[2][2], c2 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+   const double det = J[0][0] * c0 + J[0][1] * c1 + J[0][2] * c2, id = 1.0 / det;
    c.Ji[0][0] = c0 * id;
    c.Ji[1][0] = c1 * id;
    c.Ji[2][0] = c2 * id;
@@ -610,59 +603,129 @@ __device__ __forceinline__ void micro_cell( const CellGeom& g, const A st[3][3],
    c.adet     = fabs( det );
 }
 
+// point of barycentric weights l1, l2, l3 and the shell map there
+template < typename A >
+__device__ __forceinline__ void cell_point( const MicroCell< A >& c, A l1, A l2, A l3, ShellPoint< A >& p )
+{
+#pragma unroll
+   for ( int d = 0; d < 3; ++d ) p.X[d] = c.X0[d] + c.J[d][0] * l1 + c.J[d][1] * l2 + c.J[d][2] * l3;
+}
+template < typename A >
+__device__ __forceinline__ void shell_point( const MicroCell< A >& c, A l1, A l2, A l3, ShellPoint< A >& p )
+{
+   const A t  = c.t[0] + c.t[1] * l1 + c.t[2] * l2 + c.t[3] * l3;
+   p.R        = c.rad + fabs( t ) * c.dr;
+   const A d  = t < A( 0 ) ? -c.dr : c.dr;
+   const A ir = rsqrt_of( p.X[0] * p.X[0] + p.X[1] * p.X[1] + p.X[2] * p.X[2] );
+   p.s        = p.R * ir;
+   const A e  = ir * d, f = p.s * ir * ir;
+   for ( int k = 0; k < 3; ++k ) p.g[k] = e * c.bx[k] - f * p.X[k];
+   p.m  = p.s + ( p.g[0] * p.X[0] + p.g[1] * p.X[1] + p.g[2] * p.X[2] );
+   p.im = A( 1 ) / p.m;
+}
+
 // gradients of the quadratic function with node values u at the four vertices, with respect to X
 template < typename A >
-__device__ __forceinline__ void p2_vertex_gradients( const A u[10], const A Ji[3][3], A G[4][3] )
+__device__ __forceinline__ void p2_vertex_gradients( const A u_[10], const double Ji[3][3], A G[4][3] )
 {
+   double u[10];
+#pragma unroll
+   for ( int i = 0; i < 10; ++i ) u[i] = double( u_[i] );
    // c[k][l]: coefficient of grad lambda_l at vertex k
-   const A c[4][4] = { { 3 * u[0], 4 * u[9] - u[1], 4 * u[8] - u[2], 4 * u[7] - u[3] },
-                       { 4 * u[9] - u[0], 3 * u[1], 4 * u[6] - u[2], 4 * u[5] - u[3] },
-                       { 4 * u[8] - u[0], 4 * u[6] - u[1], 3 * u[2], 4 * u[4] - u[3] },
-                       { 4 * u[7] - u[0], 4 * u[5] - u[1], 4 * u[4] - u[2], 3 * u[3] } };
+   const double c[4][4] = { { 3 * u[0], 4 * u[9] - u[1], 4 * u[8] - u[2], 4 * u[7] - u[3] },
+                            { 4 * u[9] - u[0], 3 * u[1], 4 * u[6] - u[2], 4 * u[5] - u[3] },
+                            { 4 * u[8] - u[0], 4 * u[6] - u[1], 3 * u[2], 4 * u[4] - u[3] },
+                            { 4 * u[7] - u[0], 4 * u[5] - u[1], 4 * u[4] - u[2], 3 * u[3] } };
 #pragma unroll
    for ( int k = 0; k < 4; ++k )
    {
-      const A r0 = c[k][1] - c[k][0], r1 = c[k][2] - c[k][0], r2 = c[k][3] - c[k][0];
+      const double r0 = c[k][1] - c[k][0], r1 = c[k][2] - c[k][0], r2 = c[k][3] - c[k][0];
 #pragma unroll
-      for ( int d = 0; d < 3; ++d ) G[k][d] = r0 * Ji[0][d] + r1 * Ji[1][d] + r2 * Ji[2][d];
+      for ( int d = 0; d < 3; ++d ) G[k][d] = A( r0 * Ji[0][d] + r1 * Ji[1][d] + r2 * Ji[2][d] );
    }
 }
 
 // the transpose: y[i] = sum_k (gradient of basis function i at vertex k) . H[k]
 template < typename A >
-__device__ __forceinline__ void p2_pair_gradients( const A H[4][3], const A Ji[3][3], A y[10] )
+__device__ __forceinline__ void p2_pair_gradients( const A H[4][3], const double Ji[3][3], A y[10] )
 {
-   A h[4][4];
+   double h[4][4];
 #pragma unroll
    for ( int k = 0; k < 4; ++k )
    {
+      const double a = double( H[k][0] ), b = double( H[k][1] ), c = double( H[k][2] );
 #pragma unroll
-      for ( int d = 0; d < 3; ++d ) h[k][d + 1] = Ji[d][0] * H[k][0] + Ji[d][1] * H[k][1] + Ji[d][2] * H[k][2];
+      for ( int d = 0; d < 3; ++d ) h[k][d + 1] = Ji[d][0] * a + Ji[d][1] * b + Ji[d][2] * c;
       h[k][0] = -( h[k][1] + h[k][2] + h[k][3] );
    }
 #pragma unroll
-   for ( int i = 0; i < 4; ++i ) y[i] = 4 * h[i][i] - ( ( h[0][i] + h[1][i] ) + ( h[2][i] + h[3][i] ) );
-   y[4] = 4 * ( h[2][3] + h[3][2] );
-   y[5] = 4 * ( h[1][3] + h[3][1] );
-   y[6] = 4 * ( h[1][2] + h[2][1] );
-   y[7] = 4 * ( h[0][3] + h[3][0] );
-   y[8] = 4 * ( h[0][2] + h[2][0] );
-   y[9] = 4 * ( h[0][1] + h[1][0] );
+   for ( int i = 0; i < 4; ++i ) y[i] = A( 4 * h[i][i] - ( ( h[0][i] + h[1][i] ) + ( h[2][i] + h[3][i] ) ) );
+   y[4] = A( 4 * ( h[2][3] + h[3][2] ) );
+   y[5] = A( 4 * ( h[1][3] + h[3][1] ) );
+   y[6] = A( 4 * ( h[1][2] + h[2][1] ) );
+   y[7] = A( 4 * ( h[0][3] + h[3][0] ) );
+   y[8] = A( 4 * ( h[0][2] + h[2][0] ) );
+   y[9] = A( 4 * ( h[0][1] + h[1][0] ) );
+}
+
+// the coefficient at point q of a micro-cell: from its node values kl (NODAL) or the closed form at F
+template < typename A, bool NODAL >
+__device__ __forceinline__ A p2_coefficient( const Coefficient& kc, int q, const A* kl, const A* F, A radius )
+{
+   if constexpr ( NODAL )
+   {
+      A kq = A( 0 );
+#pragma unroll
+      for ( int i = 0; i < 10; ++i ) kq += A( c_p2_phi[q][i] ) * kl[i];
+      return kq;
+   }
+   else
+      return coeff_eval( kc, F, radius );
 }
 
 // K u of one micro-cell: node values u in, sums y out (kl: the coefficient's node values, NODAL only)
-template < typename A, bool NODAL >
-__device__ __forceinline__ void p2_micro_apply( const CellGeom& g, const Coefficient& kc, A inv_n, int ty, int x, int y, int z,
+template < typename A, bool NODAL, bool BLEND >
+__device__ __forceinline__ void p2_micro_apply( const CellGeom& g, const Coefficient& kc, int ne, int ty, int x, int y, int z,
                                                 const A u[10], const A* kl, A yl[10] )
 {
-   const bool           blend = g.blend == 1;
-   const ShellCell< A > sc    = shell_cell< A >( g );
-   MicroCell< A >       mc;
+   MicroCell< A > mc;
+   micro_cell( g, ne, ty, x, y, z, mc );
+   if constexpr ( !BLEND )
    {
-      A st[3][3];
-      for ( int k = 0; k < 3; ++k )
-         for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
-      micro_cell( g, st, ty, x, y, z, mc );
+      // J is all there is, so H_k = sum_j M_kj G_j with M_kj = sum_q w k lambda_k lambda_j: ten sums per point
+      double M[10];
+#pragma unroll
+      for ( int v = 0; v < 10; ++v ) M[v] = 0;
+#pragma unroll 1
+      for ( int q = 0; q < 11; ++q )
+      {
+         ShellPoint< A > p;
+         cell_point( mc, A( c_xg4_bary[q][1] ), A( c_xg4_bary[q][2] ), A( c_xg4_bary[q][3] ), p );
+         const double f = double( p2_coefficient< A, NODAL >( kc, q, kl, p.X, A( -1 ) ) );
+#pragma unroll
+         for ( int v = 0; v < 10; ++v ) M[v] += f * c_xg4_mass[q][v];
+      }
+      double G[4][3], H[4][3], ud[10], yd[10];
+#pragma unroll
+      for ( int i = 0; i < 10; ++i ) ud[i] = double( u[i] );
+      p2_vertex_gradients( ud, mc.Ji, G );
+#pragma unroll
+      for ( int k = 0; k < 4; ++k )
+#pragma unroll
+         for ( int d = 0; d < 3; ++d )
+         {
+            H[k][d] = 0;
+#pragma unroll
+            for ( int j = 0; j < 4; ++j )
+            {
+               const int lo = k < j ? k : j, hi = k < j ? j : k;
+               H[k][d] += M[lo * 4 - lo * ( lo - 1 ) / 2 + ( hi - lo )] * G[j][d];
+            }
+         }
+      p2_pair_gradients( H, mc.Ji, yd );
+#pragma unroll
+      for ( int i = 0; i < 10; ++i ) yl[i] = A( yd[i] * mc.adet );
+      return;
    }
    A G[4][3], H[4][3];
    p2_vertex_gradients( u, mc.Ji, G );
@@ -674,39 +737,24 @@ __device__ __forceinline__ void p2_micro_apply( const CellGeom& g, const Coeffic
    for ( int q = 0; q < 11; ++q )
    {
       const A l0 = A( c_xg4_bary[q][0] ), l1 = A( c_xg4_bary[q][1] ), l2 = A( c_xg4_bary[q][2] ), l3 = A( c_xg4_bary[q][3] );
-      A       B[3];
+      A       B[3], F[3];
 #pragma unroll
       for ( int d = 0; d < 3; ++d ) B[d] = l0 * G[0][d] + l1 * G[1][d] + l2 * G[2][d] + l3 * G[3][d];
       ShellPoint< A > p;
+      cell_point( mc, l1, l2, l3, p );
+      // |det DF| DF^-1 DF^-T B = |m| (w - X (g . w) / m),  w = B - g (X . B) / m
+      shell_point( mc, l1, l2, l3, p );
+      const A xb = ( p.X[0] * B[0] + p.X[1] * B[1] + p.X[2] * B[2] ) * p.im;
 #pragma unroll
-      for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * l1 + mc.J[d][1] * l2 + mc.J[d][2] * l3;
-      A f = A( c_xg4_w[q] ) * mc.adet, F[3] = { p.X[0], p.X[1], p.X[2] }, rad = A( -1 );
-      if ( blend )
+      for ( int d = 0; d < 3; ++d ) B[d] -= p.g[d] * xb;
+      const A gw = ( p.g[0] * B[0] + p.g[1] * B[1] + p.g[2] * B[2] ) * p.im;
+#pragma unroll
+      for ( int d = 0; d < 3; ++d )
       {
-         // |det DF| DF^-1 DF^-T B = |m| (w - X (g . w) / m),  w = B - g (X . B) / m
-         shell_point( sc, p );
-         const A xb = ( p.X[0] * B[0] + p.X[1] * B[1] + p.X[2] * B[2] ) * p.im;
-#pragma unroll
-         for ( int d = 0; d < 3; ++d ) B[d] -= p.g[d] * xb;
-         const A gw = ( p.g[0] * B[0] + p.g[1] * B[1] + p.g[2] * B[2] ) * p.im;
-#pragma unroll
-         for ( int d = 0; d < 3; ++d )
-         {
-            B[d] -= p.X[d] * gw;
-            F[d] = p.X[d] * p.s;
-         }
-         f *= fabs( p.m );
-         rad = p.R;
+         B[d] -= p.X[d] * gw;
+         F[d] = p.X[d] * p.s;
       }
-      if constexpr ( NODAL )
-      {
-         A kq = A( 0 );
-#pragma unroll
-         for ( int i = 0; i < 10; ++i ) kq += A( c_p2_phi[q][i] ) * kl[i];
-         f *= kq;
-      }
-      else
-         f *= coeff_eval( kc, F, rad );
+      const A f = A( c_xg4_w[q] * mc.adet ) * fabs( p.m ) * p2_coefficient< A, NODAL >( kc, q, kl, F, p.R );
 #pragma unroll
       for ( int d = 0; d < 3; ++d )
       {
@@ -731,10 +779,10 @@ __device__ __forceinline__ void p2_micro_apply( const CellGeom& g, const Coeffic
 // work.
 //
 // Shell of 1920 macro-cells, level 4 (7.9 M micro-cells), exp/sin coefficient, per apply: 6.22 ms with a
-// 3x3 inverse per point and chained updates, 2.27 ms so (64 threads, 168 registers; 96 threads take 2.29,
-// 128 registers 2.67, two points at a time 2.32).
+// 3x3 inverse per point and chained updates, 2.24 ms so (64 threads, 168 registers; with 96 threads 1 %, with
+// 128 registers 18 %, with two points at a time 2 % more).
 constexpr int kP2ApplyThreads = 64;
-template < typename T, typename A, bool NODAL >
+template < typename T, typename A, bool NODAL, bool BLEND >
 __global__ void __launch_bounds__( kP2ApplyThreads, 6 )
     k_p2_apply_pass( int ne, int nC, int3 kinds, int3 blocks, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                      const CellGeom* __restrict__ geom, Coefficient kc, const T* __restrict__ src, A* __restrict__ acc,
@@ -744,7 +792,6 @@ __global__ void __launch_bounds__( kP2ApplyThreads, 6 )
    A* const  xs = reinterpret_cast< A* >( p2_raw ) + threadIdx.x;  // node l of this thread: xs[l * kP2ApplyThreads]
    A* const  ys = xs + 27 * kP2ApplyThreads;
    const int ns = 2 * ne;
-   const A   inv_n = A( 1.0 / double( ne ) );
    int       bk = blockIdx.x, n = kinds.x, first = 0;
    if ( bk >= blocks.x )
    {
@@ -780,7 +827,7 @@ __global__ void __launch_bounds__( kP2ApplyThreads, 6 )
          u[i]  = A( ld_any( src + i0[i] ) );
          if constexpr ( NODAL ) kl[i] = A( kn[i0[i]] );
       }
-      p2_micro_apply< A, NODAL >( geom[c], kc, inv_n, 0, x, y, z, u, kl, yl );
+      p2_micro_apply< A, NODAL, BLEND >( geom[c], kc, ne, 0, x, y, z, u, kl, yl );
 #pragma unroll
       for ( int i = 0; i < 10; ++i ) acc[i0[i]] += yl[i];
       return;
@@ -807,7 +854,7 @@ __global__ void __launch_bounds__( kP2ApplyThreads, 6 )
          u[i] = xs[c_p2_loc[ty][i] * kP2ApplyThreads];
          if constexpr ( NODAL ) kl[i] = A( kn[at( c_p2_loc[ty][i] )] );
       }
-      p2_micro_apply< A, NODAL >( geom[c], kc, inv_n, ty, x, y, z, u, kl, yl );
+      p2_micro_apply< A, NODAL, BLEND >( geom[c], kc, ne, ty, x, y, z, u, kl, yl );
 #pragma unroll
       for ( int i = 0; i < 10; ++i ) ys[c_p2_loc[ty][i] * kP2ApplyThreads] += yl[i];
    }
@@ -827,7 +874,7 @@ __global__ void __launch_bounds__( kP2ApplyThreads, 6 )
 // sums are added in a fixed order.  Anchors with one micro-cell are taken one per thread, straight from
 // global memory (their blocks would hold one busy warp in six).
 constexpr int kP2SplitThreads = 192;
-template < typename T, typename A, bool NODAL >
+template < typename T, typename A, bool NODAL, bool BLEND >
 __global__ void __launch_bounds__( kP2SplitThreads, 3 )
     k_p2_apply_split( int ne, int nC, int3 kinds, int3 blocks, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                      const CellGeom* __restrict__ geom, Coefficient kc, const T* __restrict__ src, A* __restrict__ acc,
@@ -835,7 +882,6 @@ __global__ void __launch_bounds__( kP2SplitThreads, 3 )
 {
    __shared__ A xs[27][32], ys[60][32], ks[NODAL ? 27 : 1][32];
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ns = 2 * ne;
-   const A   inv_n = A( 1.0 / double( ne ) );
    // the block's anchors: kind, first one among (cell, anchor) of the kind
    int bk = blockIdx.x, n = kinds.x, first = 0;
    if ( bk >= blocks.x )
@@ -874,7 +920,7 @@ __global__ void __launch_bounds__( kP2SplitThreads, 3 )
          u[i]        = A( ld_any( src + at[i] ) );
          if constexpr ( NODAL ) kl[i] = A( kn[at[i]] );
       }
-      p2_micro_apply< A, NODAL >( geom[c], kc, inv_n, 0, x, y, z, u, kl, yl );
+      p2_micro_apply< A, NODAL, BLEND >( geom[c], kc, ne, 0, x, y, z, u, kl, yl );
 #pragma unroll
       for ( int i = 0; i < 10; ++i ) acc[at[i]] += yl[i];
       return;
@@ -907,7 +953,7 @@ __global__ void __launch_bounds__( kP2SplitThreads, 3 )
          u[i] = xs[c_p2_loc[warp][i]][lane];
          if constexpr ( NODAL ) kl[i] = ks[c_p2_loc[warp][i]][lane];
       }
-      p2_micro_apply< A, NODAL >( geom[c], kc, inv_n, warp, x, y, z, u, kl, yl );
+      p2_micro_apply< A, NODAL, BLEND >( geom[c], kc, ne, warp, x, y, z, u, kl, yl );
 #pragma unroll
       for ( int i = 0; i < 10; ++i ) ys[10 * warp + i][lane] = yl[i];
    }
@@ -1003,15 +1049,11 @@ __global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int nanch, const 
    const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
    const CellGeom g    = geom[c];
    const int64_t  base = cell_off[c];
-   const A        inv_n = A( 1.0 / double( ne ) );
-   A              step[3][3];
-   for ( int k = 0; k < 3; ++k )
-      for ( int d = 0; d < 3; ++d ) step[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
    for ( int ty = 0; ty < 6; ++ty )
    {
       if ( x + y + z > ne - 1 - c_mc_shift[ty] ) continue;
       MicroCell< A > mc;
-      micro_cell( g, step, ty, x, y, z, mc );
+      micro_cell( g, ne, ty, x, y, z, mc );
       int64_t idx[10];
       A       kl[10];
       bool    bad = false;
@@ -1456,159 +1498,155 @@ __device__ __forceinline__ void mapped_point( const CellGeom& g, const A X0[3], 
    adet        = fabs( det );
 }
 
+// The coupled passes compute a micro-cell in FP64 for every value type and only the coefficient in the
+// accumulation type: their results are sums of terms of either sign (the divergence, the negative weight of
+// the five-point rule), which in FP32 lost up to 1.8 times as much as evaluating every point by itself.
+
 // B u of one micro-cell: the pressure values of its vertices from the velocity's node values
-template < typename A >
-__device__ __forceinline__ void div_micro( const MicroCell< A >& mc, const ShellCell< A >& sc, bool blend, const A ( &ul )[3][10], A ( &yl )[4] )
+__device__ __forceinline__ void div_micro( const MicroCell< double >& mc, bool blend, const double ( &ul )[3][10], double ( &yl )[4] )
 {
-   const A wj = -A( 1.0 / 24.0 ) * mc.adet;
-            A G[3][4][3];
+   const double wj = -( 1.0 / 24.0 ) * mc.adet;
+   double       G[3][4][3];
 #pragma unroll
-            for ( int k = 0; k < 3; ++k )
-            {
-               p2_vertex_gradients( ul[k], mc.Ji, G[k] );
-            }
-            for ( int i = 0; i < 4; ++i ) yl[i] = A( 0 );
+   for ( int k = 0; k < 3; ++k ) p2_vertex_gradients( ul[k], mc.Ji, G[k] );
+   for ( int i = 0; i < 4; ++i ) yl[i] = 0;
 #pragma unroll 1
-            for ( int q = 0; q < 4; ++q )
-            {
-               const A lam[4] = { A( c_q2_bary[q][0] ), A( c_q2_bary[q][1] ), A( c_q2_bary[q][2] ), A( c_q2_bary[q][3] ) };
-               // velocity gradient B with respect to X; div = (tr B - g^T B X / m) / s and |det DF| = s^2 |m|
-               A B[3][3];
+   for ( int q = 0; q < 4; ++q )
+   {
+      const double lam[4] = { c_q2_bary[q][0], c_q2_bary[q][1], c_q2_bary[q][2], c_q2_bary[q][3] };
+      // velocity gradient B with respect to X; div = (tr B - g^T B X / m) / s and |det DF| = s^2 |m|
+      double B[3][3];
 #pragma unroll
-               for ( int k = 0; k < 3; ++k )
+      for ( int k = 0; k < 3; ++k )
 #pragma unroll
-                  for ( int d = 0; d < 3; ++d )
-                     B[k][d] = lam[0] * G[k][0][d] + lam[1] * G[k][1][d] + lam[2] * G[k][2][d] + lam[3] * G[k][3][d];
-               A f = B[0][0] + B[1][1] + B[2][2];
-               if ( blend )
-               {
-                  ShellPoint< A > p;
+         for ( int d = 0; d < 3; ++d ) B[k][d] = lam[0] * G[k][0][d] + lam[1] * G[k][1][d] + lam[2] * G[k][2][d] + lam[3] * G[k][3][d];
+      double f = B[0][0] + B[1][1] + B[2][2];
+      if ( blend )
+      {
+         ShellPoint< double > p;
+         cell_point( mc, lam[1], lam[2], lam[3], p );
+         shell_point( mc, lam[1], lam[2], lam[3], p );
+         double gbx = 0;
 #pragma unroll
-                  for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * lam[1] + mc.J[d][1] * lam[2] + mc.J[d][2] * lam[3];
-                  shell_point( sc, p );
-                  A gbx = A( 0 );
+         for ( int k = 0; k < 3; ++k ) gbx += p.g[k] * ( B[k][0] * p.X[0] + B[k][1] * p.X[1] + B[k][2] * p.X[2] );
+         f = ( f - gbx * p.im ) * ( p.s * fabs( p.m ) );
+      }
+      f *= wj;
 #pragma unroll
-                  for ( int k = 0; k < 3; ++k ) gbx += p.g[k] * ( B[k][0] * p.X[0] + B[k][1] * p.X[1] + B[k][2] * p.X[2] );
-                  f = ( f - gbx * p.im ) * ( p.s * fabs( p.m ) );
-               }
-               f *= wj;
-#pragma unroll
-               for ( int i = 0; i < 4; ++i ) yl[i] += f * lam[i];
-            }
+      for ( int i = 0; i < 4; ++i ) yl[i] += f * lam[i];
+   }
 }
 
 // B^T p of one micro-cell: the velocity's node values from the vertices' pressures
-template < typename A >
-__device__ __forceinline__ void divt_micro( const MicroCell< A >& mc, const ShellCell< A >& sc, bool blend, const A ( &pl )[4], A ( &yl )[3][10] )
+__device__ __forceinline__ void divt_micro( const MicroCell< double >& mc, bool blend, const double ( &pl )[4], double ( &yl )[3][10] )
 {
-   const A wj = -A( 1.0 / 24.0 ) * mc.adet;
-            A H[3][4][3];
+   const double wj = -( 1.0 / 24.0 ) * mc.adet;
+   double       H[3][4][3];
 #pragma unroll
-            for ( int k = 0; k < 3; ++k )
+   for ( int k = 0; k < 3; ++k )
 #pragma unroll
-               for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = A( 0 );
+      for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = 0;
 #pragma unroll 1
-            for ( int q = 0; q < 4; ++q )
-            {
-               const A lam[4] = { A( c_q2_bary[q][0] ), A( c_q2_bary[q][1] ), A( c_q2_bary[q][2] ), A( c_q2_bary[q][3] ) };
-               A       f      = wj * ( pl[0] * lam[0] + pl[1] * lam[1] + pl[2] * lam[2] + pl[3] * lam[3] );
-               // component k pairs with DF^-1 e_k |det DF| = s |m| (e_k - X g_k / m)
-               A E[3][3] = { { A( 1 ), A( 0 ), A( 0 ) }, { A( 0 ), A( 1 ), A( 0 ) }, { A( 0 ), A( 0 ), A( 1 ) } };
-               if ( blend )
-               {
-                  ShellPoint< A > p;
+   for ( int q = 0; q < 4; ++q )
+   {
+      const double lam[4] = { c_q2_bary[q][0], c_q2_bary[q][1], c_q2_bary[q][2], c_q2_bary[q][3] };
+      double       f      = wj * ( pl[0] * lam[0] + pl[1] * lam[1] + pl[2] * lam[2] + pl[3] * lam[3] );
+      // component k pairs with DF^-1 e_k |det DF| = s |m| (e_k - X g_k / m)
+      double E[3][3] = { { 1, 0, 0 }, { 0, 1, 0 }, { 0, 0, 1 } };
+      if ( blend )
+      {
+         ShellPoint< double > p;
+         cell_point( mc, lam[1], lam[2], lam[3], p );
+         shell_point( mc, lam[1], lam[2], lam[3], p );
 #pragma unroll
-                  for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * lam[1] + mc.J[d][1] * lam[2] + mc.J[d][2] * lam[3];
-                  shell_point( sc, p );
+         for ( int k = 0; k < 3; ++k )
+         {
+            const double gk = p.g[k] * p.im;
 #pragma unroll
-                  for ( int k = 0; k < 3; ++k )
-                  {
-                     const A gk = p.g[k] * p.im;
+            for ( int d = 0; d < 3; ++d ) E[k][d] -= p.X[d] * gk;
+         }
+         f *= p.s * fabs( p.m );
+      }
 #pragma unroll
-                     for ( int d = 0; d < 3; ++d ) E[k][d] -= p.X[d] * gk;
-                  }
-                  f *= p.s * fabs( p.m );
-               }
+      for ( int v = 0; v < 4; ++v )
+      {
+         const double fl = f * lam[v];
 #pragma unroll
-               for ( int v = 0; v < 4; ++v )
-               {
-                  const A fl = f * lam[v];
+         for ( int k = 0; k < 3; ++k )
 #pragma unroll
-                  for ( int k = 0; k < 3; ++k )
-#pragma unroll
-                     for ( int d = 0; d < 3; ++d ) H[k][v][d] += fl * E[k][d];
-               }
-            }
+            for ( int d = 0; d < 3; ++d ) H[k][v][d] += fl * E[k][d];
+      }
+   }
 #pragma unroll
    for ( int k = 0; k < 3; ++k ) p2_pair_gradients( H[k], mc.Ji, yl[k] );
 }
 
-// the full viscous block of one micro-cell on its three components' node values
+// the full viscous block of one micro-cell on its three components' node values (the coefficient in A)
 template < typename A >
-__device__ __forceinline__ void visc_micro( const MicroCell< A >& mc, const ShellCell< A >& sc, bool blend, const Coefficient& kc,
-                                            const A ( &ul )[3][10], A ( &yl )[3][10] )
+__device__ __forceinline__ void visc_micro( const MicroCell< double >& mc, bool blend, const Coefficient& kc, const double ( &ul )[3][10],
+                                            double ( &yl )[3][10] )
 {
-            A G[3][4][3], H[3][4][3];
+   double G[3][4][3], H[3][4][3];
 #pragma unroll
-            for ( int k = 0; k < 3; ++k )
-            {
-               p2_vertex_gradients( ul[k], mc.Ji, G[k] );
+   for ( int k = 0; k < 3; ++k )
+   {
+      p2_vertex_gradients( ul[k], mc.Ji, G[k] );
 #pragma unroll
-               for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = A( 0 );
-            }
+      for ( int v = 0; v < 4; ++v ) H[k][v][0] = H[k][v][1] = H[k][v][2] = 0;
+   }
 #pragma unroll 1
-            for ( int q = 0; q < 5; ++q )
-            {
-               const A l1 = A( c_yu5_pts[q][0] ), l2 = A( c_yu5_pts[q][1] ), l3 = A( c_yu5_pts[q][2] ), l0 = A( 1 ) - l1 - l2 - l3;
-               A       D[3][3];  // velocity gradient, d u_k / d x_d
+   for ( int q = 0; q < 5; ++q )
+   {
+      const double l1 = c_yu5_pts[q][0], l2 = c_yu5_pts[q][1], l3 = c_yu5_pts[q][2], l0 = 1 - l1 - l2 - l3;
+      double       D[3][3];  // velocity gradient, d u_k / d x_d
 #pragma unroll
-               for ( int k = 0; k < 3; ++k )
+      for ( int k = 0; k < 3; ++k )
 #pragma unroll
-                  for ( int d = 0; d < 3; ++d ) D[k][d] = l0 * G[k][0][d] + l1 * G[k][1][d] + l2 * G[k][2][d] + l3 * G[k][3][d];
-               ShellPoint< A > p;
+         for ( int d = 0; d < 3; ++d ) D[k][d] = l0 * G[k][0][d] + l1 * G[k][1][d] + l2 * G[k][2][d] + l3 * G[k][3][d];
+      ShellPoint< double > p;
+      cell_point( mc, l1, l2, l3, p );
+      double f = c_yu5_w[q] * mc.adet;
+      A      F[3] = { A( p.X[0] ), A( p.X[1] ), A( p.X[2] ) }, rad = A( -1 );
+      if ( blend )
+      {
+         // |det DF| = s^2 |m| takes the two factors 1/s of DF^-T and DF^-1
+         shell_point( mc, l1, l2, l3, p );
 #pragma unroll
-               for ( int d = 0; d < 3; ++d ) p.X[d] = mc.X0[d] + mc.J[d][0] * l1 + mc.J[d][1] * l2 + mc.J[d][2] * l3;
-               A f = A( c_yu5_w[q] ) * mc.adet, F[3] = { p.X[0], p.X[1], p.X[2] }, rad = A( -1 );
-               if ( blend )
-               {
-                  // |det DF| = s^2 |m| takes the two factors 1/s of DF^-T and DF^-1
-                  shell_point( sc, p );
+         for ( int k = 0; k < 3; ++k )
+         {
+            const double xb = ( p.X[0] * D[k][0] + p.X[1] * D[k][1] + p.X[2] * D[k][2] ) * p.im;
 #pragma unroll
-                  for ( int k = 0; k < 3; ++k )
-                  {
-                     const A xb = ( p.X[0] * D[k][0] + p.X[1] * D[k][1] + p.X[2] * D[k][2] ) * p.im;
+            for ( int d = 0; d < 3; ++d ) D[k][d] -= p.g[d] * xb;
+            F[k] = A( p.X[k] * p.s );
+         }
+         f *= fabs( p.m );
+         rad = A( p.R );
+      }
+      f *= double( coeff_eval( kc, F, rad ) );
+      const double tr3     = ( 2.0 / 3.0 ) * ( D[0][0] + D[1][1] + D[2][2] );
+      double       S[3][3] = { { D[0][0] + D[0][0] - tr3, D[0][1] + D[1][0], D[0][2] + D[2][0] },
+                               { D[0][1] + D[1][0], D[1][1] + D[1][1] - tr3, D[1][2] + D[2][1] },
+                               { D[0][2] + D[2][0], D[1][2] + D[2][1], D[2][2] + D[2][2] - tr3 } };
 #pragma unroll
-                     for ( int d = 0; d < 3; ++d ) D[k][d] -= p.g[d] * xb;
-                     F[k] = p.X[k] * p.s;
-                  }
-                  f *= fabs( p.m );
-                  rad = p.R;
-               }
-               f *= coeff_eval( kc, F, rad );
-               const A tr3     = A( 2.0 / 3.0 ) * ( D[0][0] + D[1][1] + D[2][2] );
-               A       S[3][3] = { { D[0][0] + D[0][0] - tr3, D[0][1] + D[1][0], D[0][2] + D[2][0] },
-                                   { D[0][1] + D[1][0], D[1][1] + D[1][1] - tr3, D[1][2] + D[2][1] },
-                                   { D[0][2] + D[2][0], D[1][2] + D[2][1], D[2][2] + D[2][2] - tr3 } };
+      for ( int k = 0; k < 3; ++k )
+      {
+         if ( blend )
+         {
+            const double gs = ( p.g[0] * S[k][0] + p.g[1] * S[k][1] + p.g[2] * S[k][2] ) * p.im;
 #pragma unroll
-               for ( int k = 0; k < 3; ++k )
-               {
-                  if ( blend )
-                  {
-                     const A gs = ( p.g[0] * S[k][0] + p.g[1] * S[k][1] + p.g[2] * S[k][2] ) * p.im;
+            for ( int d = 0; d < 3; ++d ) S[k][d] -= p.X[d] * gs;
+         }
 #pragma unroll
-                     for ( int d = 0; d < 3; ++d ) S[k][d] -= p.X[d] * gs;
-                  }
-#pragma unroll
-                  for ( int d = 0; d < 3; ++d )
-                  {
-                     const A h = f * S[k][d];
-                     H[k][0][d] += l0 * h;
-                     H[k][1][d] += l1 * h;
-                     H[k][2][d] += l2 * h;
-                     H[k][3][d] += l3 * h;
-                  }
-               }
-            }
+         for ( int d = 0; d < 3; ++d )
+         {
+            const double h = f * S[k][d];
+            H[k][0][d] += l0 * h;
+            H[k][1][d] += l1 * h;
+            H[k][2][d] += l2 * h;
+            H[k][3][d] += l3 * h;
+         }
+      }
+   }
 #pragma unroll
    for ( int k = 0; k < 3; ++k ) p2_pair_gradients( H[k], mc.Ji, yl[k] );
 }
@@ -1661,42 +1699,35 @@ __global__ void __launch_bounds__( kCoupledThreads, 2 )
    };
    if ( live && x + y + z <= ne - 1 - c_mc_shift[ty] )
    {
-      const CellGeom&      g     = geom[c];
-      const bool           blend = g.blend == 1;
-      const ShellCell< A > sc    = shell_cell< A >( g );
-      const A              inv_n = A( 1.0 / double( ne ) );
-      MicroCell< A >       mc;
-      {
-         A st[3][3];
-         for ( int k = 0; k < 3; ++k )
-            for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
-         micro_cell( g, st, ty, x, y, z, mc );
-      }
-      A yl[NC][NN];
+      const CellGeom&     g     = geom[c];
+      const bool          blend = g.blend == 1;
+      MicroCell< double > mc;
+      micro_cell( g, ne, ty, x, y, z, mc );
+      double yl[NC][NN];
       if constexpr ( OPER == CPL_DIVT )
       {
-         A pl[4];
+         double pl[4];
 #pragma unroll
-         for ( int i = 0; i < 4; ++i ) pl[i] = A( ld_any( v.p + at_p( vert( i ) ) ) );
-         divt_micro( mc, sc, blend, pl, yl );
+         for ( int i = 0; i < 4; ++i ) pl[i] = double( ld_any( v.p + at_p( vert( i ) ) ) );
+         divt_micro( mc, blend, pl, yl );
       }
       else
       {
-         A ul[3][10];
+         double ul[3][10];
 #pragma unroll
          for ( int i = 0; i < 10; ++i )
          {
             const int64_t at = at_u( c_p2_loc[ty][i] );
 #pragma unroll
-            for ( int k = 0; k < 3; ++k ) ul[k][i] = A( ld_any( v.u[k] + at ) );
+            for ( int k = 0; k < 3; ++k ) ul[k][i] = double( ld_any( v.u[k] + at ) );
          }
-         if constexpr ( OPER == CPL_VISCOUS ) visc_micro( mc, sc, blend, kc, ul, yl );
-         else div_micro( mc, sc, blend, ul, yl[0] );
+         if constexpr ( OPER == CPL_VISCOUS ) visc_micro< A >( mc, blend, kc, ul, yl );
+         else div_micro( mc, blend, ul, yl[0] );
       }
 #pragma unroll
       for ( int k = 0; k < NC; ++k )
 #pragma unroll
-         for ( int i = 0; i < NN; ++i ) ys[k][NN * ty + i][lane] = yl[k][i];
+         for ( int i = 0; i < NN; ++i ) ys[k][NN * ty + i][lane] = A( yl[k][i] );
    }
    else
 #pragma unroll
@@ -1845,21 +1876,23 @@ static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src
          const int  per    = split ? 32 : kP2ApplyThreads, per1 = split ? kP2SplitThreads : kP2ApplyThreads;
          auto       blocks = [&]( int k, int b ) { return int( ( int64_t( k ) * nC + b - 1 ) / b ); };
          const int3 bl     = make_int3( blocks( kinds.x, per ), blocks( kinds.y, per ), blocks( kinds.z, per1 ) );
-         auto       launch = [&]( auto nodal ) {
-            constexpr bool NODAL = decltype( nodal )::value;
+         auto       launch = [&]( auto nodal, auto blend ) {
+            constexpr bool NODAL = decltype( nodal )::value, BLEND = decltype( blend )::value;
             const double*  kn    = NODAL ? e.d_kn : nullptr;
             const int      pg    = bl.x + bl.y + bl.z;
             if ( split )
-               k_p2_apply_split< T, A, NODAL ><<< pg, kP2SplitThreads, 0, ctx->stream >>>( element_n( op, L ), nC, kinds, bl, e.d_anch + e.aoff[p],
+               k_p2_apply_split< T, A, NODAL, BLEND ><<< pg, kP2SplitThreads, 0, ctx->stream >>>( element_n( op, L ), nC, kinds, bl, e.d_anch + e.aoff[p],
                                                                                           P.d_off + P.nB, op->d_geom, op->coeff, src, acc,
                                                                                           P.size, ctx->d_error, kn );
             else
-               k_p2_apply_pass< T, A, NODAL ><<< pg, kP2ApplyThreads, 54 * kP2ApplyThreads * sizeof( A ), ctx->stream >>>(
+               k_p2_apply_pass< T, A, NODAL, BLEND ><<< pg, kP2ApplyThreads, 54 * kP2ApplyThreads * sizeof( A ), ctx->stream >>>(
                    element_n( op, L ), nC, kinds, bl, e.d_anch + e.aoff[p], P.d_off + P.nB, op->d_geom, op->coeff, src, acc, P.size,
                    ctx->d_error, kn );
          };
-         if ( op->nodal_k ) launch( std::true_type{} );
-         else launch( std::false_type{} );
+         if ( op->nodal_k && op->blending == 1 ) launch( std::true_type{}, std::true_type{} );
+         else if ( op->nodal_k ) launch( std::true_type{}, std::false_type{} );
+         else if ( op->blending == 1 ) launch( std::false_type{}, std::true_type{} );
+         else launch( std::false_type{}, std::false_type{} );
       }
       else if ( op->order == 2 && ( MODE == 1 || MODE == 2 ) )
          k_p2_pass< A, MODE == 2 ? 2 : 1 ><<< grid, bs, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
@@ -2258,10 +2291,6 @@ __global__ void __launch_bounds__( 128 ) k_visc_diagonal( int ne, int nanch, con
    const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
    const CellGeom&      g     = geom[c];
    const int64_t  bu = off_u[c];
-   const A        inv_n = A( 1.0 / double( ne ) );
-   A              st[3][3];
-   for ( int k = 0; k < 3; ++k )
-      for ( int d = 0; d < 3; ++d ) st[k][d] = ( A( g.P[k + 1][d] ) - A( g.P[0][d] ) ) * inv_n;
    for ( int ty = 0; ty < 6; ++ty )
    {
       if ( x + y + z > ne - 1 - c_mc_shift[ty] ) continue;
@@ -2285,7 +2314,7 @@ __global__ void __launch_bounds__( 128 ) k_visc_diagonal( int ne, int nanch, con
          }
       }
       MicroCell< A > mc;
-      micro_cell( g, st, ty, x, y, z, mc );
+      micro_cell( g, ne, ty, x, y, z, mc );
       {
          A yl[3][10];
          for ( int k = 0; k < 3; ++k )

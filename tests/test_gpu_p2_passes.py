@@ -74,6 +74,50 @@ def test_p2_matrix_free_apply_full_blocks(ctx):
     assert np.abs(y - z).max() < 1e-12 * np.abs(z).max()
 
 
+@pytest.mark.parametrize("case,L", [("shell", 2), ("shell", 4), ("box", 2), ("box", 4)])
+@pytest.mark.parametrize("kind", ["const", "expsin"])
+def test_fp32_passes_are_as_exact_as_their_type(ctx, case, L, kind):
+    """FP32 results of the matrix-free operators against the same operators in FP64 on the same values: what a
+    micro-cell computes once is computed in FP64 and rounded, so that a result carries the rounding of its
+    terms, of the coefficient and of at most 24 partial sums: 2 unit roundoffs (1.2e-7) in the 2-norm."""
+    coords, tets = O.mesh_spherical_shell(2, 2, 0.55, 1.0) if case == "shell" else M.cube_2x1x1()
+    bl = "shell" if case == "shell" else None
+    spec = SPECS[kind][0]
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    out = {}
+    start = {}
+    for dtype in ("float32", "float64"):
+        u, du = ([H.P2Function(n + str(k), pm, L, L, ctx, dtype) for k in range(3)] for n in ("u", "du"))
+        p, dp = (H.P1Function(n, pm, L, L, ctx, dtype) for n in ("p", "dp"))
+        for i, f in enumerate(u + [p]):
+            if dtype == "float32":
+                f.fill_random(L, 3 + i)
+                start[i] = f.download(L)
+            else:
+                f.upload(L, start[i].astype(np.float64))
+        A = H.P2ElementwiseBlendingDivKGradOperator(pm, L, L, ctx, k=spec, blending=bl)
+        V = H.P2ElementwiseBlendingFullViscousOperator(pm, L, L, ctx, viscosity=spec, blending=bl)
+        S = H.StokesUzawaMultigrid(ctx, pm, L, L, viscosity=spec, blending=bl)
+        zero = [H.P2Function("z%d" % k, pm, L, L, ctx, dtype) for k in range(3)]
+        zp = H.P1Function("zp", pm, L, L, ctx, dtype)
+
+        def result(name, fns):
+            out.setdefault(name, []).append(np.concatenate([f.download(L).astype(np.float64) for f in fns]))
+
+        for f in zero + [zp] + du + [dp]:
+            f.interpolate(0.0, L, H.All)
+        A.apply(u[0], du[0], L, H.All)
+        result("div k grad", du[:1])
+        V.apply(u, du, L, H.All)
+        result("full viscous", du)
+        S.apply(zero, p, du, dp, L)
+        result("divT", du)
+        S.apply(u, zp, du, dp, L)
+        result("div", [dp])
+    for name, (low, ref) in out.items():
+        assert np.linalg.norm(low - ref) <= 2 * 2.0**-24 * np.linalg.norm(ref), name
+
+
 @pytest.mark.parametrize("case,L", [("tet", 0), ("tet", 1), ("tet", 4), ("shell", 0), ("shell", 2)])
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
 def test_p2_stored_apply(ctx, case, L, dtype):
