@@ -728,8 +728,8 @@ struct P2cPoints {
 // Eight threads per edge or vertex node, one per cell of a face node, one per interior node; all entries of
 // the node's class are unrolled, so its loads are independent (walking the entries of one cell after the
 // other, with the row start computed on the way, took 67 us for the 48k face nodes of the level-6 cube).
-// Apply on the cube, FP64, with that kernel and the tiled sweep and with this one: P2 levels 4 and 5 103 -> 17
-// and 21 us, level 6 118 -> 83 us, level 7 243 -> 232 us.  At 128 points per edge one thread per node for the
+// Apply on the cube, FP64, with that kernel and the tiled sweep and with this one: P2 levels 4 and 5 103 -> 11
+// and 17 us, level 6 118 -> 83 us, level 7 243 -> 232 us.  At 128 points per edge one thread per node for the
 // interior too takes 75 us on six cells, but 152 against 99 us on twelve: the sweep stays there.
 template < typename T, typename A >
 __global__ void __launch_bounds__( 256 )
@@ -743,44 +743,39 @@ __global__ void __launch_bounds__( 256 )
       FaceRec   r;
       int       sub;
       const int kind = bnd_thread< 2 >( v, frec, seg, blockIdx.x * 256 + threadIdx.x, low, sub, r );
-      // one cell's part: the stencil of the node's class in it and the weight of its centre
-      A    s = A( 0 ), d = A( 0 );
-      auto part = [&]( int64_t slot, int cell, int cls, int y, int z ) {
-         const int x = int( slot - v.cell_off[cell] - cidx( n, 0, y, z ) ), k = ( x & 1 ) | ( ( y & 1 ) << 1 ) | ( ( z & 1 ) << 2 );
-         const A*  w = W + size_t( cell ) * kP2cCellStride + ( cls == 0 ? 0 : kP2cInterior + ( cls - 1 ) * kP2cEntries );
-         s += p2c_sum< true, T, A >( k, src + slot, w, n, y, z, c_p2c_faces[cls] );
-         d += w[g_p2c_base[k] + g_p2c_base[k + 16]];
-      };
-      int64_t owner   = 0;
-      bool    flagged = false, any = false;
-      if ( kind == BND_LOW )
+      // this thread's cells: every eighth incidence of an edge or vertex, one of a face's; one copy of the
+      // unrolled classes serves both (called from three places it became a function that worked from the
+      // stack: FP32 apply on 960 cells, 32 points per edge, 517 us, so 206; FP64 409 and 269)
+      const bool    lowk  = kind == BND_LOW;
+      const int64_t owner = lowk ? low.owner : r.owner;
+      const bool    any   = lowk ? low.count > 0 : kind == BND_FACE, flagged = any && ( ( lowk ? low.bc : r.bc ) & flag ) != 0;
+      A             s = A( 0 ), d = A( 0 );
+      for ( int q = lowk ? sub : 0, end = !flagged ? 0 : lowk ? low.count : sub == 0 || r.cell1 >= 0 ? 1 : 0; q < end; q += 8 )
       {
-         owner   = low.owner;
-         flagged = ( low.bc & flag ) != 0;
-         any     = low.count > 0;
-         if ( flagged )
-            for ( int q = sub; q < low.count; q += 8 )
-            {
-               const IncRec I = v.irec[low.begin + q];
-               part( I.slot, I.cell, I.cls, I.y, I.z );
-            }
+         IncRec I;
+         if ( lowk ) I = v.irec[low.begin + q];
+         else
+         {
+            I.slot = sub ? r.c1 : r.c0;
+            I.cell = sub ? r.cell1 : r.cell0;
+            I.cls  = sub ? r.cls1 : r.cls0;
+            I.y    = sub ? r.y1 : r.y0;
+            I.z    = sub ? r.z1 : r.z0;
+         }
+         const int x = int( I.slot - v.cell_off[I.cell] - cidx( n, 0, I.y, I.z ) ), k = ( x & 1 ) | ( ( I.y & 1 ) << 1 ) | ( ( I.z & 1 ) << 2 );
+         const A*  w = W + size_t( I.cell ) * kP2cCellStride + ( I.cls == 0 ? 0 : kP2cInterior + ( I.cls - 1 ) * kP2cEntries );
+         s += p2c_sum< true, T, A >( k, src + I.slot, w, n, I.y, I.z, c_p2c_faces[I.cls] );
+         d += w[g_p2c_base[k] + g_p2c_base[k + 16]];  // the centre's weight
+      }
+      if ( lowk )
 #pragma unroll
          for ( int m = 4; m > 0; m >>= 1 )
          {
             s += __shfl_xor_sync( 0xffffffffu, s, m, 8 );
             d += __shfl_xor_sync( 0xffffffffu, d, m, 8 );
          }
-      }
       else
       {
-         if ( kind == BND_FACE )
-         {
-            owner   = r.owner;
-            flagged = ( r.bc & flag ) != 0;
-            any     = true;
-            if ( flagged && sub == 0 ) part( r.c0, r.cell0, r.cls0, r.y0, r.z0 );
-            if ( flagged && sub == 1 && r.cell1 >= 0 ) part( r.c1, r.cell1, r.cls1, r.y1, r.z1 );
-         }
          s += __shfl_xor_sync( 0xffffffffu, s, 1 );
          d += __shfl_xor_sync( 0xffffffffu, d, 1 );
       }
@@ -806,20 +801,20 @@ __global__ void __launch_bounds__( 256 )
       if ( op == OP_CHEBI && flagged ) put( v2, second );
       return;
    }
-   int     k  = 0, first = 0;
+   int     k = 0, np = 0, first = 0;
    int64_t g = blockIdx.x - nbnd;
-   for ( ; k < 7; ++k )
+#pragma unroll
+   for ( int j = 0; j < 8; ++j )  // unrolled: the counts are read with constant indices
    {
-      const int64_t blocks = ( int64_t( nC ) * pts.np[k] + 255 ) / 256;
-      if ( g < blocks ) break;
-      g -= blocks;
-      first += pts.np[k];
+      const int64_t blocks = ( int64_t( nC ) * pts.np[j] + 255 ) / 256;
+      if ( np == 0 && g < blocks ) k = j, np = pts.np[j];
+      if ( np == 0 ) g -= blocks, first += pts.np[j];
    }
    g = g * 256 + threadIdx.x;
-   if ( g >= int64_t( nC ) * pts.np[k] ) return;
-   const int c = g < 0x7fffffff ? int( unsigned( g ) / unsigned( pts.np[k] ) ) : int( g / pts.np[k] );
+   if ( g >= int64_t( nC ) * np ) return;
+   const int c = g < 0x7fffffff ? int( unsigned( g ) / unsigned( np ) ) : int( g / np );
    if ( !( v.cell_bc[c] & flag ) ) return;
-   const ushort4 p = pts.pts[first + int( g - int64_t( c ) * pts.np[k] )];
+   const ushort4 p = pts.pts[first + int( g - int64_t( c ) * np )];
    const int64_t i = v.cell_off[c] + cidx( n, p.x, p.y, p.z );
    const A*      w = W + size_t( c ) * kP2cCellStride;
    const A       s = p2c_sum< false, T, A >( k, src + i, w, n, p.y, p.z, 0 );
