@@ -1231,6 +1231,25 @@ static void stencil( hyb_op* op, int L, int dtype, int code, uint32_t flag, int 
    launch_stencil( &op->ctx->c, op->o.mesh, &op->o, L, dtype, a );
 }
 
+// one stencil operation (OP_*) as the smoothers launch it; a test reaches every operation and flag through it
+int hyb_internal_op_stencil( hyb_op* op, int level, int code, uint32_t flag, int copy_unflagged, hyb_fn* src, hyb_fn* v1, hyb_fn* v2, hyb_fn* dst,
+                             double a0, double a1 )
+{
+   HYB_TRY
+   require( op, "op is NULL" );
+   level += op->o.order - 1;
+   for ( hyb_fn* f : { src, v1, v2, dst } )
+   {
+      check_op_fn( op, f, level );
+      require( f->f.dtype == src->f.dtype, "value types differ" );
+   }
+   require( src != dst && src != v2 && dst != v2, "src, v2 and dst must differ" );
+   require( code >= OP_APPLY && code <= OP_DINV_APPLY, "unknown operation" );
+   stencil( op, level, src->f.dtype, code, flag, copy_unflagged, src->f.ptr( level ), v1->f.ptr( level ), v2->f.ptr( level ), dst->f.ptr( level ),
+            a0, a1 );
+   HYB_CATCH
+}
+
 int hyb_op_apply( hyb_op* op, hyb_fn* src, hyb_fn* dst, int level, uint32_t flag, int update )
 {
    HYB_TRY

@@ -844,10 +844,11 @@ __device__ __forceinline__ void bnd_point( const LevelView& v, const OpView< A >
    int       sub;
    const int kind = bnd_thread< 1 >( v, v.frec, seg, t, low, sub, r );
    if ( kind == BND_NONE ) return;
+   constexpr bool CARRIES = OP == OP_JAC || OP == OP_CHEB0 || OP == OP_CHEBI;  // only these write unflagged owners
    if ( kind == BND_LOW )
    {
       const bool flagged = ( low.bc & flag ) != 0;
-      if ( !flagged && !copy_unflagged ) low.count = 0;
+      if ( !flagged && !( CARRIES && copy_unflagged ) ) low.count = 0;
       A val = A( 0 ), second = A( 0 ), s = A( 0 );
       if ( flagged )
          for ( int q = sub; q < low.count; q += 8 )
@@ -873,7 +874,7 @@ __device__ __forceinline__ void bnd_point( const LevelView& v, const OpView< A >
    auto put = [&]( T* vec, A x ) { put_face( r, vec, x ); };
    if ( !( r.bc & flag ) )
    {
-      if ( !copy_unflagged ) return;
+      if ( !CARRIES || !copy_unflagged ) return;
       if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) put( dst, A( ldv( src + r.owner ) ) );
       else if constexpr ( OP == OP_CHEBI ) put( dst, A( ldc( v2 + r.owner ) ) );
       return;

@@ -1,7 +1,9 @@
 """P1 constant-stencil operations at the levels around the change from the one-launch kernel (up to 64 points
-per macro-edge) to the tiled sweeps, and on meshes with edges and vertices of many cells: apply, residual
-via Jacobi, Chebyshev step, unflagged owners carried over, with Neumann faces (one cell).  FP64 against the
-oracle's assembled operator, 1e-12 of the largest value as in the other P1 tests."""
+per macro-edge) to the tiled sweeps, and on meshes with edges and vertices of many cells: apply, add, Jacobi
+step and Chebyshev step, with Neumann faces (one cell), against the oracle's assembled operator in FP64 (1e-12
+of the largest value as in the other P1 tests); what every operation does to unflagged owners."""
+
+import ctypes
 
 import numpy as np
 import pytest
@@ -80,3 +82,59 @@ def test_p1_chebyshev_across_kernels(ctx, L, dtype):
     g.smooth(f["x"], f["b"], L, 1)
     x, ref = f["x"].download(L), f["ref"].download(L)
     assert np.abs(x - ref).max() <= (1e-12 if dtype == "float64" else 2.4e-5) * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("L", [1, 4, 7])
+@pytest.mark.parametrize("p2", [False, True])
+def test_unflagged_owners_are_carried_or_left(ctx, L, p2):
+    """Dirichlet owners and their copies under flag Inner, all with nonzero values: Jacobi and the first Chebyshev
+    step carry src over, the middle step the iterate; every other operation leaves its target as it was, whether
+    or not the caller asks for a copy."""
+    coords, tets = M.octahedron_8() if L < 7 else M.cube_6()
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    L -= 1 if p2 else 0  # the same points per macro-edge
+    A = (H.P2ConstantLaplaceOperator if p2 else H.P1ConstantLaplaceOperator)(pm, L, L, ctx)
+    kind = H.P2Function if p2 else H.P1Function
+    f = {n: kind(n, pm, L, L, ctx) for n in ("src", "v1", "v2", "dst", "mask")}
+    f["mask"].interpolate(0.0, L, H.All)
+    f["mask"].interpolate(1.0, L, H.DirichletBoundary)
+    dirichlet = f["mask"].download(L) == 1.0
+    assert dirichlet.any()
+    raw = H.lib().hyb_internal_op_stencil
+    raw.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_uint32, ctypes.c_int] + [ctypes.c_void_p] * 4 + [ctypes.c_double] * 2
+    carried = {3: "src", 4: "src", 5: "v2"}  # Jacobi, first and middle Chebyshev step
+    for code in range(8):
+        for copy in (0, 1):
+            before = {}
+            for i, n in enumerate(("src", "v1", "v2", "dst")):
+                f[n].fill_random(L, 10 * code + i)
+                f[n].add([1.0 if n != "dst" else 3.0], [f["mask"]], L, H.DirichletBoundary)
+                before[n] = f[n].download(L)
+            assert raw(A.h, L, code, H.Inner, copy, *(f[n].h for n in ("src", "v1", "v2", "dst")), 0.5, 0.25) == 0
+            want = before[carried[code]] if copy and code in carried else before["dst"]
+            np.testing.assert_array_equal(f["dst"].download(L)[dirichlet], want[dirichlet], err_msg=f"dst of operation {code}, copy {copy}")
+            np.testing.assert_array_equal(f["v2"].download(L)[dirichlet], before["v2"][dirichlet], err_msg=f"v2 of operation {code}, copy {copy}")
+
+
+@pytest.mark.parametrize("L", [3, 6, 7])
+@pytest.mark.parametrize("smoother", ["jacobi", "chebyshev"])
+def test_smoothers_keep_boundary_values(ctx, L, smoother):
+    """A smoothing step returns nonzero Dirichlet values unchanged at owners and copies."""
+    coords, tets = M.cube_6()
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    A = H.P1ConstantLaplaceOperator(pm, L - 1, L, ctx)
+    g = H.GeometricMultigridSolver(ctx, A, L - 1, L, smoother=smoother)
+    if smoother == "chebyshev":
+        g.set_radii([2.0, 2.0])
+    x, b, mask = (H.P1Function(n, pm, L - 1, L, ctx) for n in ("x", "b", "mask"))
+    x.fill_random(L, 1)
+    b.fill_random(L, 2)
+    mask.interpolate(0.0, L, H.All)
+    mask.interpolate(1.0, L, H.DirichletBoundary)
+    x.add([2.0], [mask], L, H.DirichletBoundary)
+    dirichlet, before = mask.download(L) == 1.0, x.download(L)
+    for _ in range(2):
+        g.smooth(x, b, L, 1)
+    after = x.download(L)
+    np.testing.assert_array_equal(after[dirichlet], before[dirichlet])
+    assert (after != before).any()
