@@ -1768,7 +1768,7 @@ __global__ void __launch_bounds__( 256 ) k_restrict( LevelView cv, LevelView fv,
 }
 
 // Linear interpolation at the fine point (x, y, z): the mean of the two ends of the coarse micro-edge the
-// point halves (twice the same node for a coarse one).  The ends lie at floor(x / 2) of one coarse row and
+// point halves, or the value of the coarse node it is.  The ends lie at floor(x / 2) of one coarse row and
 // ceil(x / 2) of another, and the rows depend on y and z only.
 __device__ __forceinline__ void coarse_rows( int nc, int y, int z, int64_t& lo, int64_t& hi )
 {
@@ -1777,11 +1777,17 @@ __device__ __forceinline__ void coarse_rows( int nc, int y, int z, int64_t& lo, 
    hi = cidx( nc, 0, y >> 1, zo && yo ? zl + 1 : zl );
 }
 template < typename T, typename A >
+__device__ __forceinline__ A edge_mean( const T* lo, const T* hi, bool node )
+{
+   const A a = A( ldv( lo ) ), b = A( ldv( hi ) );
+   return node ? a : A( 0.5 ) * a + A( 0.5 ) * b;  // halved first: the sum of two large values would overflow
+}
+template < typename T, typename A >
 __device__ __forceinline__ A interp( const T* c, int nc, int x, int y, int z )
 {
    int64_t lo, hi;
    coarse_rows( nc, y, z, lo, hi );
-   return A( 0.5 ) * ( A( ldv( c + lo + ( x >> 1 ) ) ) + A( ldv( c + hi + ( ( x + 1 ) >> 1 ) ) ) );
+   return edge_mean< T, A >( c + lo + ( x >> 1 ), c + hi + ( ( x + 1 ) >> 1 ), lo == hi && !( x & 1 ) );
 }
 
 // Prolongation, boundary tasks and cell interiors in one launch: bound by the fine vector (level 6 to 7 on 18
@@ -1820,11 +1826,12 @@ __global__ void __launch_bounds__( 256 ) k_prolong( LevelView cv, LevelView fv, 
    for_interior( fv, nC, flag, blockIdx.x - nbnd, [&]( int c, int x0, int y, int z, int step ) {
       int64_t lo, hi;
       coarse_rows( cv.n, y, z, lo, hi );
-      const T* cc = coarse + cv.cell_off[c];
-      T*       f  = fine + fv.cell_off[c] + cidx( fv.n, 0, y, z );
+      const T*   cc   = coarse + cv.cell_off[c];
+      T*         f    = fine + fv.cell_off[c] + cidx( fv.n, 0, y, z );
+      const bool node = lo == hi && !( x0 & 1 );  // a thread's points have one parity: step is 32, or passes the row's end
       for ( int x = x0; x < fv.n - y - z; x += step )
       {
-         const A val = A( 0.5 ) * ( A( ldv( cc + lo + ( x >> 1 ) ) ) + A( ldv( cc + hi + ( ( x + 1 ) >> 1 ) ) ) );
+         const A val = edge_mean< T, A >( cc + lo + ( x >> 1 ), cc + hi + ( ( x + 1 ) >> 1 ), node );
          stv( f + x, add ? A( ldc( f + x ) ) + val : val );
       }
    } );

@@ -66,3 +66,22 @@ def test_restriction_is_the_transpose(ctx, L):
     left, right = a.dotGlobal(b, L - 1, H.Inner), a.dotGlobal(b, L, H.Inner)
     # both sums have up to 1.7e7 terms of size one: rounding grows like their square root
     assert abs(left - right) <= 1e-12 * np.sqrt(a.dotGlobal(a, L, H.Inner) * b.dotGlobal(b, L, H.Inner))
+
+
+@pytest.mark.parametrize("L", [4, 7])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_prolongation_of_large_values(ctx, L, dtype):
+    """Values above half of the largest number interpolate to themselves: copied at coarse nodes, and the halves
+    summed at the others."""
+    coords, tets = M.cube_6()
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    f = H.P1Function("f", pm, L - 1, L, ctx, dtype)
+    got = {}
+    for value in (1.0, 0.9 * float(np.finfo(dtype).max)):
+        f.upload(L - 1, np.full(f.download(L - 1).shape, value, dtype=dtype))
+        f.upload(L, np.zeros(f.download(L).shape, dtype=dtype))
+        H.P1toP1LinearProlongation().prolongate(f, L - 1, H.All)
+        got[value] = f.download(L)
+    ones, big = got.values()
+    np.testing.assert_array_equal(big, np.where(ones == 1.0, np.asarray(value, dtype=dtype), np.asarray(0.0, dtype=dtype)))
+    assert np.count_nonzero(ones) > (2 ** L - 1) ** 3
