@@ -243,7 +243,7 @@ __host__ __device__ constexpr bool sweep_aux()
 
 // start of row (y + dy, z + dz) of a cell array minus the start of row (y, z)
 template < int DY, int DZ >
-__device__ __forceinline__ int row_shift( int n, int y, int z )
+__host__ __device__ __forceinline__ int row_shift( int n, int y, int z )
 {
    const int q = n + 1 - z;  // points in the first row of slice z
    int       s = 0;

@@ -46,6 +46,14 @@ __host__ __device__ inline int64_t cidx(int n, int x, int y, int z)
    return tet_size(w) - tet_size(wz) + (int64_t) y * (wz + 1) - ((int64_t) y * (y + 1)) / 2 + x;
 }
 
+// last index of the nodes (x + a, y + b, z + c), 0 <= a, b, c <= span and a + b + c <= room, of a cell array:
+// z grows slowest and x fastest, so it has the largest c, then the largest b, then the largest a
+__host__ __device__ inline int64_t window_last(int n, int x, int y, int z, int span, int room)
+{
+   const int c = room < span ? room : span, b = room - c < span ? room - c : span, a = room - c - b < span ? room - c - b : span;
+   return cidx(n, x + a, y + b, z + c);
+}
+
 // face-local (i, j) with i+j <= n  ->  offset inside the face array (width n+1)
 __host__ __device__ inline int64_t fidx(int n, int i, int j)
 {

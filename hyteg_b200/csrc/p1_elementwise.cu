@@ -807,8 +807,8 @@ __global__ void __launch_bounds__( kP2ApplyThreads, 6 )
    const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, room = ns - 2 * ( x + y + z );
    const int64_t  base = cell_off[c];
    {
-      // self-check: the window's last node inside the level's vector
-      const int64_t last = base + cidx( ns, 2 * x, 2 * y, 2 * z + min( room, 2 ) );
+      // self-check: every node of the window inside the level's vector
+      const int64_t last = base + window_last( ns, 2 * x, 2 * y, 2 * z, 2, room );
       if ( room < 2 || base < 0 || last >= level_size )
       {
          atomicExch( err, 2 );
@@ -899,8 +899,8 @@ __global__ void __launch_bounds__( kP2SplitThreads, 3 )
    const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, room = ns - 2 * ( x + y + z );
    const int64_t  base = cell_off[c];
    {
-      // self-check: the window's last node inside the level's vector
-      const int64_t last = base + cidx( ns, 2 * x, 2 * y, 2 * z + min( room, 2 ) );
+      // self-check: every node of the window inside the level's vector
+      const int64_t last = base + window_last( ns, 2 * x, 2 * y, 2 * z, 2, room );
       if ( live && ( room < 2 || base < 0 || last >= level_size ) )
       {
          atomicExch( err, 2 );
@@ -1039,7 +1039,7 @@ __device__ __forceinline__ void p2_grad( int q, int i, const A Mi[3][3], A G[3] 
 template < typename A, int MODE >
 __global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                                                        const CellGeom* __restrict__ geom, Coefficient kc, A* __restrict__ acc,
-                                                       P2StoredView sv, A* __restrict__ st, int64_t level_size, int* err,
+                                                       P2StoredView sv, A* __restrict__ st, int64_t st_size, int64_t level_size, int* err,
                                                        const double* __restrict__ kn )
 {
    const int t = blockIdx.x * blockDim.x + threadIdx.x;  // one micro-cell anchor per thread
@@ -1106,8 +1106,11 @@ __global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int nanch, const 
 #pragma unroll
             for ( int j = 0; j < 10; ++j )
             {
-               const int lo = i < j ? i : j, hi = i < j ? j : i;
-               st[w + c_p2s_ent[( 10 * ty + i ) * 10 + j] * skip] += K[lo * 10 - lo * ( lo - 1 ) / 2 + ( hi - lo )];
+               const int     lo = i < j ? i : j, hi = i < j ? j : i;
+               const int64_t at = w + c_p2s_ent[( 10 * ty + i ) * 10 + j] * skip;
+               // self-check: stored weights inside their array
+               if ( at < 0 || at >= st_size ) atomicExch( err, 2 );
+               else st[at] += K[lo * 10 - lo * ( lo - 1 ) / 2 + ( hi - lo )];
             }
          }
    }
@@ -1682,8 +1685,8 @@ __global__ void __launch_bounds__( kCoupledThreads, 2 )
    const int     x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, room = ns - 2 * ( x + y + z );
    const int64_t bu = off_u[c], bp = off_p ? off_p[c] : 0;
    {
-      // self-check: the window's last node inside the level's vectors
-      const int64_t lu = bu + cidx( ns, 2 * x, 2 * y, 2 * z + min( room, 2 ) ), lp = bp + cidx( ne, x, y, z + min( room / 2, 1 ) );
+      // self-check: every node of the windows inside the level's vectors
+      const int64_t lu = bu + window_last( ns, 2 * x, 2 * y, 2 * z, 2, room ), lp = bp + window_last( ne, x, y, z, 1, room / 2 );
       if ( live && ( room < 2 || bu < 0 || lu >= size_u || ( off_p && ( bp < 0 || lp >= size_p ) ) ) )
       {
          atomicExch( err, 2 );
@@ -1897,7 +1900,7 @@ static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src
       else if ( op->order == 2 && ( MODE == 1 || MODE == 2 ) )
          k_p2_pass< A, MODE == 2 ? 2 : 1 ><<< grid, bs, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
                                                                             op->d_geom, op->coeff, acc, e.p2s ? *e.p2s : P2StoredView{},
-                                                                            assembled_stencils< A >( op, L ), P.size, ctx->d_error,
+                                                                            assembled_stencils< A >( op, L ), e.p2s_count, P.size, ctx->d_error,
                                                                             op->nodal_k ? e.d_kn : nullptr );
       else if constexpr ( MODE != 2 )
          k_elem_pass< T, A, MODE ><<< grid, bs, 0, ctx->stream >>>( P.n, na, e.d_anch + e.aoff[p], P.d_off + P.nB, op->d_geom, op->coeff,
