@@ -487,6 +487,40 @@ void launch_cg_scalar( Context* ctx, double* state, int stage, double rtol, doub
 // host helpers
 void check_cuda( cudaError_t e, const char* what );
 
+// Device arrays of tables that are built together and published together: what is not kept is freed again, so
+// that a failure on the way (out of memory) leaves the level as it was and a later call builds it anew.
+void* table_malloc( size_t bytes, const char* what );
+class TableArrays
+{
+ public:
+   TableArrays() = default;
+   TableArrays( const TableArrays& ) = delete;
+   TableArrays& operator=( const TableArrays& ) = delete;
+   template < typename T >
+   T* get( size_t count, const char* what )
+   {
+      owned_.reserve( owned_.size() + 1 );
+      T* p = static_cast< T* >( table_malloc( ( count ? count : 1 ) * sizeof( T ), what ) );
+      owned_.push_back( p );
+      return p;
+   }
+   template < typename T >
+   T* upload( const T* host, size_t count, const char* what )
+   {
+      T* p = get< T >( count, what );
+      if ( count ) check_cuda( cudaMemcpy( p, host, count * sizeof( T ), cudaMemcpyHostToDevice ), what );
+      return p;
+   }
+   void keep() { owned_.clear(); }
+   ~TableArrays()
+   {
+      for ( void* p : owned_ ) cudaFree( p );
+   }
+
+ private:
+   std::vector< void* > owned_;
+};
+
 // One-time set-up per CUDA device: __constant__ tables and kernel attributes exist once per device,
 // so a process that uses several devices must run each set-up on every one of them.  run(f) calls f
 // once for the current device (thread-safe; later calls return at the cost of one atomic load).

@@ -1830,6 +1830,7 @@ static void ensure_rows( Operator* op, int L )
    if ( e.d_anch ) return;
    const int          n = element_n( op, L );
    std::vector< int > anch;
+   TableArrays        arrays;
    for ( int p = 0; p < 8; ++p )
    {
       e.aoff[p]    = int( anch.size() );
@@ -1848,17 +1849,18 @@ static void ensure_rows( Operator* op, int L )
       }
    }
    e.aoff[8] = int( anch.size() );
-   check_cuda( cudaMalloc( &e.d_anch, std::max< size_t >( anch.size(), 1 ) * sizeof( int ) ), "cudaMalloc(anchors)" );
-   if ( !anch.empty() )
-      check_cuda( cudaMemcpy( e.d_anch, anch.data(), anch.size() * sizeof( int ), cudaMemcpyHostToDevice ), "upload anchors" );
+   e.d_anch  = arrays.upload( anch.data(), anch.size(), "anchors" );
+   arrays.keep();
 }
 
 // threads per block of a pass over na anchors per cell (grid: blocks x cells): whole warps, at most
 // maxb, so that the small levels (a few anchors per cell) do not launch mostly idle blocks
 static int pass_block( int na, int maxb ) { return std::min( maxb, ( na + 31 ) / 32 * 32 ); }
 
+// (MODE 2 and 4: the stencils st, for P2 of the layout sv and st_size values, which a failure leaves unpublished)
 template < typename T, typename A, int MODE >
-static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src, A* acc )
+static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src, A* acc, A* st = nullptr, const P2StoredView* sv = nullptr,
+                        int64_t st_size = 0 )
 {
    P1Level&   P = m->level( L );
    ElemLevel& e = op->el[L];
@@ -1899,12 +1901,11 @@ static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src
       }
       else if ( op->order == 2 && ( MODE == 1 || MODE == 2 ) )
          k_p2_pass< A, MODE == 2 ? 2 : 1 ><<< grid, bs, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
-                                                                            op->d_geom, op->coeff, acc, e.p2s ? *e.p2s : P2StoredView{},
-                                                                            assembled_stencils< A >( op, L ), e.p2s_count, P.size, ctx->d_error,
-                                                                            op->nodal_k ? e.d_kn : nullptr );
+                                                                            op->d_geom, op->coeff, acc, sv ? *sv : P2StoredView{}, st, st_size, P.size,
+                                                                            ctx->d_error, op->nodal_k ? e.d_kn : nullptr );
       else if constexpr ( MODE != 2 )
          k_elem_pass< T, A, MODE ><<< grid, bs, 0, ctx->stream >>>( P.n, na, e.d_anch + e.aoff[p], P.d_off + P.nB, op->d_geom, op->coeff,
-                                                                    src, acc, assembled_stencils< A >( op, L ), P.size, P.size, ctx->d_error );
+                                                                    src, acc, st, P.size, P.size, ctx->d_error );
       ++ctx->launches;
    }
    check_cuda( cudaGetLastError(), "elementwise pass launch" );
@@ -1967,8 +1968,9 @@ static void ensure_cell_points( ElemLevel& e, const P1Level& P )
    for ( int z = 0; z <= P.n; ++z )
       for ( int y = 0; y + z <= P.n; ++y )
          for ( int x = 0; x + y + z <= P.n; ++x ) pts.push_back( make_ushort4( (unsigned short) x, (unsigned short) y, (unsigned short) z, 0 ) );
-   check_cuda( cudaMalloc( &e.d_pts, pts.size() * sizeof( ushort4 ) ), "cudaMalloc(cell points)" );
-   check_cuda( cudaMemcpy( e.d_pts, pts.data(), pts.size() * sizeof( ushort4 ), cudaMemcpyHostToDevice ), "upload cell points" );
+   TableArrays arrays;
+   e.d_pts = arrays.upload( pts.data(), pts.size(), "cell points" );
+   arrays.keep();
 }
 
 template < typename T, typename A >
@@ -1989,14 +1991,20 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
       ensure_cell_points( e, P );
       if ( !e.d_S[0] )
       {
-         check_cuda( cudaMalloc( &e.d_S[0], cnt * sizeof( double ) ), "cudaMalloc(assembled stencils)" );
-         check_cuda( cudaMemsetAsync( e.d_S[0], 0, cnt * sizeof( double ), ctx->stream ), "cudaMemset" );
-         run_passes< double, double, 4 >( ctx, m, op, L, nullptr, nullptr );
+         TableArrays arrays;
+         double*     S = arrays.get< double >( cnt, "assembled stencils" );
+         check_cuda( cudaMemsetAsync( S, 0, cnt * sizeof( double ), ctx->stream ), "cudaMemset" );
+         run_passes< double, double, 4 >( ctx, m, op, L, nullptr, nullptr, S );
+         arrays.keep();
+         e.d_S[0] = S;
       }
       if ( sizeof( A ) == 4 && !e.d_S[1] )
       {
-         check_cuda( cudaMalloc( &e.d_S[1], cnt * sizeof( float ) ), "cudaMalloc(assembled stencils)" );
-         launch_convert( ctx, cnt, F32, e.d_S[1], F64, e.d_S[0] );
+         TableArrays arrays;
+         float*      S = arrays.get< float >( cnt, "assembled stencils" );
+         launch_convert( ctx, cnt, F32, S, F64, e.d_S[0] );
+         arrays.keep();
+         e.d_S[1] = S;
       }
    }
    else if ( op->store_matrices && !e.d_S[sizeof( A ) == 8 ? 0 : 1] )
@@ -2006,40 +2014,46 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
       {
          std::vector< ushort4 > pts;
          std::vector< int >     rank;
-         auto                   v = std::make_shared< P2StoredView >();
-         e.p2s_count              = build_p2_stored( *v, P.n, m->topo.nC, pts, rank );
-         check_cuda( cudaMalloc( &e.d_p2s_pts, pts.size() * sizeof( ushort4 ) ), "cudaMalloc(stencil nodes)" );
-         check_cuda( cudaMemcpy( e.d_p2s_pts, pts.data(), pts.size() * sizeof( ushort4 ), cudaMemcpyHostToDevice ), "upload stencil nodes" );
-         check_cuda( cudaMalloc( &e.d_p2s_rank, rank.size() * sizeof( int ) ), "cudaMalloc(stencil ranks)" );
-         check_cuda( cudaMemcpy( e.d_p2s_rank, rank.data(), rank.size() * sizeof( int ), cudaMemcpyHostToDevice ), "upload stencil ranks" );
-         v->pts  = reinterpret_cast< const ushort4* >( e.d_p2s_pts );
-         v->rank = e.d_p2s_rank;
-         e.p2s   = v;
+         TableArrays            arrays;
+         auto                   v     = std::make_shared< P2StoredView >();
+         const int64_t          count = build_p2_stored( *v, P.n, m->topo.nC, pts, rank );
+         ushort4*               d_pts  = arrays.upload( pts.data(), pts.size(), "stencil nodes" );
+         int*                   d_rank = arrays.upload( rank.data(), rank.size(), "stencil ranks" );
+         arrays.keep();
+         v->pts       = d_pts;
+         v->rank      = d_rank;
+         e.d_p2s_pts  = d_pts;
+         e.d_p2s_rank = d_rank;
+         e.p2s_count  = count;
+         e.p2s        = v;
       }
-      const bool had = e.d_S[0] != nullptr;
-      if ( !had )
+      TableArrays arrays;
+      double*     S = static_cast< double* >( e.d_S[0] );
+      if ( !S )
       {
-         check_cuda( cudaMalloc( &e.d_S[0], e.p2s_count * sizeof( double ) ), "cudaMalloc(assembled stencils)" );
-         check_cuda( cudaMemsetAsync( e.d_S[0], 0, e.p2s_count * sizeof( double ), ctx->stream ), "cudaMemset" );
-         run_passes< double, double, 2 >( ctx, m, op, L, nullptr, nullptr );
+         S = arrays.get< double >( e.p2s_count, "assembled stencils" );
+         check_cuda( cudaMemsetAsync( S, 0, e.p2s_count * sizeof( double ), ctx->stream ), "cudaMemset" );
+         run_passes< double, double, 2 >( ctx, m, op, L, nullptr, nullptr, S, e.p2s.get(), e.p2s_count );
       }
       if ( sizeof( A ) == 4 )
       {
-         check_cuda( cudaMalloc( &e.d_S[1], e.p2s_count * sizeof( float ) ), "cudaMalloc(assembled stencils)" );
-         launch_convert( ctx, e.p2s_count, F32, e.d_S[1], F64, e.d_S[0] );
-         if ( !had )
-         {
-            check_cuda( cudaStreamSynchronize( ctx->stream ), "assembled stencils" );
-            check_cuda( cudaFree( e.d_S[0] ), "cudaFree(assembled stencils)" );
-            e.d_S[0] = nullptr;
-         }
+         TableArrays low;
+         float*      Sf = low.get< float >( e.p2s_count, "assembled stencils" );
+         launch_convert( ctx, e.p2s_count, F32, Sf, F64, S );
+         check_cuda( cudaStreamSynchronize( ctx->stream ), "assembled stencils" );
+         low.keep();
+         e.d_S[1] = Sf;
+      }
+      else
+      {
+         arrays.keep();
+         e.d_S[0] = S;
       }
    }
    if ( e.d_invd[dtype] ) return;
-   A* invd = nullptr;
-   check_cuda( cudaMalloc( &invd, P.size * sizeof( A ) ), "cudaMalloc(inverse diagonal)" );
+   TableArrays arrays;
+   A*          invd = arrays.get< A >( P.size, "inverse diagonal" );
    check_cuda( cudaMemsetAsync( invd, 0, P.size * sizeof( A ), ctx->stream ), "cudaMemset" );
-   e.d_invd[dtype] = invd;
    // diagonal: sum of element-matrix diagonals, owners summing their cell copies
    run_passes< T, A, 1 >( ctx, m, op, L, nullptr, acc );
    const int nrows = int( P.rows.size() );
@@ -2051,6 +2065,8 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
    if ( !P.tasks.empty() )
       launch_bnd_acc< T, A, OP_APPLY >( ctx, ctx->stream, P, kAll, 0, acc_vecs< T, A >( acc, {} ), 1, nullptr, invd, A( 0 ), A( 0 ) );
    check_cuda( cudaGetLastError(), "diagonal launch" );
+   arrays.keep();
+   e.d_invd[dtype] = invd;
 }
 
 void ensure_elementwise_level( Context* ctx, Operator* op, int L, int dtype )

@@ -274,11 +274,13 @@ void ensure_p2_constant_tables( Operator* A, int Ls )
 {
    P2cLevel& pl = A->p2c.at( Ls );
    if ( pl.d_W ) return;
+   TableArrays          arrays;
    std::vector< float > wf( pl.W.begin(), pl.W.end() );
-   check_cuda( cudaMalloc( &pl.d_W, pl.W.size() * sizeof( double ) ), "cudaMalloc(P2 stencils)" );
-   check_cuda( cudaMalloc( &pl.d_Wf, wf.size() * sizeof( float ) ), "cudaMalloc(P2 stencils)" );
-   check_cuda( cudaMemcpy( pl.d_W, pl.W.data(), pl.W.size() * sizeof( double ), cudaMemcpyHostToDevice ), "upload P2 stencils" );
-   check_cuda( cudaMemcpy( pl.d_Wf, wf.data(), wf.size() * sizeof( float ), cudaMemcpyHostToDevice ), "upload P2 stencils" );
+   double*              d_W    = arrays.upload( pl.W.data(), pl.W.size(), "P2 stencils" );
+   float*               d_Wf   = arrays.upload( wf.data(), wf.size(), "P2 stencils" );
+   FaceRec*             d_frec = nullptr;
+   ushort4*             d_pts  = nullptr;
+   int                  np[8]  = {};
    // the level's face records, inside each boundary type's group sorted by face and by the parity class of
    // the node in its first cell: the lanes of a warp then apply the same stencil
    P1Level&  P  = A->mesh->level( Ls );
@@ -305,8 +307,7 @@ void ensure_p2_constant_tables( Operator* A, int Ls )
          i = e;
       }
       fr.swap( sorted );
-      check_cuda( cudaMalloc( &pl.d_frec, size_t( nf ) * sizeof( FaceRec ) ), "cudaMalloc(P2 face records)" );
-      check_cuda( cudaMemcpy( pl.d_frec, fr.data(), size_t( nf ) * sizeof( FaceRec ), cudaMemcpyHostToDevice ), "upload P2 face records" );
+      d_frec = arrays.upload( fr.data(), fr.size(), "P2 face records" );
    }
    if ( n <= kP2cFlatMaxN )
    {
@@ -319,11 +320,16 @@ void ensure_p2_constant_tables( Operator* A, int Ls )
                for ( int x = 1; x + y + z < n; ++x )
                   if ( ( ( x & 1 ) | ( ( y & 1 ) << 1 ) | ( ( z & 1 ) << 2 ) ) == k )
                      pts.push_back( make_ushort4( (unsigned short) x, (unsigned short) y, (unsigned short) z, 0 ) );
-         pl.np[k] = int( pts.size() - before );
+         np[k] = int( pts.size() - before );
       }
-      check_cuda( cudaMalloc( &pl.d_pts, std::max< size_t >( pts.size(), 1 ) * sizeof( ushort4 ) ), "cudaMalloc(P2 points)" );
-      if ( !pts.empty() ) check_cuda( cudaMemcpy( pl.d_pts, pts.data(), pts.size() * sizeof( ushort4 ), cudaMemcpyHostToDevice ), "upload P2 points" );
+      d_pts = arrays.upload( pts.data(), pts.size(), "P2 points" );
    }
+   arrays.keep();
+   for ( int k = 0; k < 8; ++k ) pl.np[k] = np[k];
+   pl.d_Wf   = d_Wf;
+   pl.d_frec = d_frec;
+   pl.d_pts  = d_pts;
+   pl.d_W    = d_W;
 }
 
 // inverse diagonal of every owned slot flagged by `flag` (padded level layout), from the tables

@@ -448,17 +448,55 @@ void build_sweep_units( P1Level& P, int b, int nwarps, int ncells )
    }
 }
 
+// the n-th table allocation of this thread from now on fails (a test of what a failure leaves behind); 0: none
+static thread_local int fail_in = 0;
+extern "C" void hyb_internal_fail_table_allocation( int n ) { fail_in = n; }
+
+void* table_malloc( size_t bytes, const char* what )
+{
+   if ( fail_in > 0 && --fail_in == 0 ) throw std::runtime_error( std::string( what ) + ": allocation failed on request" );
+   void* p = nullptr;
+   check_cuda( cudaMalloc( &p, bytes ), what );
+   return p;
+}
+
+// without the device tables; owned: free them (else whoever allocated them does)
+static void drop_device( P1Level& P, bool owned )
+{
+   auto drop = [&]( auto*& p ) {
+      if ( owned ) cudaFree( p );
+      p = nullptr;
+   };
+   drop( P.d_off ), drop( P.d_poff ), drop( P.d_inc_begin ), drop( P.d_inc ), drop( P.d_tasks ), drop( P.d_btasks ), drop( P.d_frec );
+   drop( P.d_lrec ), drop( P.d_irec ), drop( P.d_ipts ), drop( P.d_rows ), drop( P.d_zunits ), drop( P.d_zcell ), drop( P.d_zbegin );
+   for ( int b = 0; b < kSwLists; ++b ) drop( P.d_swunits[b] ), drop( P.d_swcell[b] ), drop( P.d_swbegin[b] );
+   drop( P.d_bc ), drop( P.d_bkind ), drop( P.d_ncell_cls );
+   for ( int g = 0; g < 4; ++g ) P.nlow[g] = P.nface[g] = 0;
+   P.nipts = 0;
+}
+
+static void build_device( Mesh* m, P1Level& P, TableArrays& arrays );
+
 void ensure_device( Mesh* m, P1Level& P )
 {
    if ( P.d_off ) return;
+   TableArrays arrays;
+   try
+   {
+      build_device( m, P, arrays );
+      arrays.keep();
+   } catch ( ... )
+   {
+      drop_device( P, false );
+      throw;
+   }
+}
+
+static void build_device( Mesh* m, P1Level& P, TableArrays& arrays )
+{
    const Topology& t  = m->topo;
    const int       nP = t.nV + t.nE + t.nF + t.nC;
-   auto up = [&]( auto** dptr, const auto* host, size_t count ) {
-      using T = std::remove_pointer_t< std::remove_reference_t< decltype( *dptr ) > >;
-      size_t bytes = std::max< size_t >( count, 1 ) * sizeof( T );
-      check_cuda( cudaMalloc( (void**) dptr, bytes ), "cudaMalloc(level tables)" );
-      if ( count ) check_cuda( cudaMemcpy( *dptr, host, count * sizeof( T ), cudaMemcpyHostToDevice ), "upload level tables" );
-   };
+   auto up = [&]( auto** dptr, const auto* host, size_t count ) { *dptr = arrays.upload( host, count, "level tables" ); };
    up( &P.d_off, P.off.data(), P.off.size() );
    {
       std::vector< int64_t > po( P.packed_off.begin(), P.packed_off.end() );
@@ -617,26 +655,7 @@ P1Level& Mesh::level( int L )
 
 Mesh::~Mesh()
 {
-   for ( auto& kv : levels )
-   {
-      P1Level& P = *kv.second;
-      cudaFree( P.d_off );
-      cudaFree( P.d_poff );
-      cudaFree( P.d_inc_begin );
-      cudaFree( P.d_inc );
-      cudaFree( P.d_tasks );
-      cudaFree( P.d_btasks );
-      cudaFree( P.d_frec );
-      cudaFree( P.d_lrec );
-      cudaFree( P.d_irec );
-      cudaFree( P.d_ipts );
-      cudaFree( P.d_rows );
-      cudaFree( P.d_zunits ), cudaFree( P.d_zcell ), cudaFree( P.d_zbegin );
-      for ( int b = 0; b < kSwLists; ++b ) cudaFree( P.d_swunits[b] ), cudaFree( P.d_swcell[b] ), cudaFree( P.d_swbegin[b] );
-      cudaFree( P.d_bc );
-      cudaFree( P.d_bkind );
-      cudaFree( P.d_ncell_cls );
-   }
+   for ( auto& kv : levels ) drop_device( *kv.second, true );
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -763,18 +782,17 @@ void ensure_device_op( OpLevel& ol )
    if ( ol.d_W ) return;
    std::vector< float > Wf( ol.W.begin(), ol.W.end() ), ibf( ol.invd_b.begin(), ol.invd_b.end() ),
        icf( ol.invd_c.begin(), ol.invd_c.end() );
-   auto up = [&]( auto** dptr, const auto& vec ) {
-      using T = typename std::decay_t< decltype( vec ) >::value_type;
-      check_cuda( cudaMalloc( (void**) dptr, std::max< size_t >( vec.size(), 1 ) * sizeof( T ) ), "cudaMalloc(stencils)" );
-      if ( !vec.empty() )
-         check_cuda( cudaMemcpy( *dptr, vec.data(), vec.size() * sizeof( T ), cudaMemcpyHostToDevice ), "upload stencils" );
-   };
-   up( &ol.d_W, ol.W );
-   up( &ol.d_Wf, Wf );
-   up( &ol.d_invd_b, ol.invd_b );
-   up( &ol.d_invd_c, ol.invd_c );
-   up( &ol.d_invd_bf, ibf );
-   up( &ol.d_invd_cf, icf );
+   TableArrays arrays;
+   auto        up = [&]( const auto& vec ) { return arrays.upload( vec.data(), vec.size(), "stencils" ); };
+   double *    d_W = up( ol.W ), *d_b = up( ol.invd_b ), *d_c = up( ol.invd_c );
+   float *     d_Wf = up( Wf ), *d_bf = up( ibf ), *d_cf = up( icf );
+   arrays.keep();
+   ol.d_invd_b  = d_b;
+   ol.d_invd_c  = d_c;
+   ol.d_Wf      = d_Wf;
+   ol.d_invd_bf = d_bf;
+   ol.d_invd_cf = d_cf;
+   ol.d_W       = d_W;
 }
 
 Operator::~Operator()
