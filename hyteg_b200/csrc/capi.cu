@@ -176,7 +176,7 @@ int hyb_ctx_create( int device, void* stream, hyb_ctx** out )
    check_cuda( cudaMalloc( &h->c.d_scalars, 64 * sizeof( double ) ), "cudaMalloc(scalars)" );
    check_cuda( cudaStreamCreateWithFlags( &h->c.aux, cudaStreamNonBlocking ), "cudaStreamCreate(aux)" );
    check_cuda( cudaMalloc( &h->c.d_error, sizeof( int ) ), "cudaMalloc(error word)" );
-   check_cuda( cudaMemset( h->c.d_error, 0, sizeof( int ) ), "cudaMemset(error word)" );
+   check_cuda( cudaMemsetAsync( h->c.d_error, 0, sizeof( int ), h->c.stream ), "cudaMemset(error word)" );
    check_cuda( cudaEventCreateWithFlags( &h->c.ev_fork, cudaEventDisableTiming ), "cudaEventCreate" );
    check_cuda( cudaEventCreateWithFlags( &h->c.ev_join, cudaEventDisableTiming ), "cudaEventCreate" );
    *out = h;
@@ -199,7 +199,7 @@ int hyb_ctx_synchronize( hyb_ctx* ctx )
    check_cuda( cudaMemcpy( &e, ctx->c.d_error, sizeof( int ), cudaMemcpyDeviceToHost ), "error word readback" );
    if ( e )
    {
-      cudaMemset( ctx->c.d_error, 0, sizeof( int ) );
+      cudaMemsetAsync( ctx->c.d_error, 0, sizeof( int ), ctx->c.stream );
       if ( e == 2 )
       {
          g_err = "a kernel's index self-check failed (an access outside its buffers was skipped)";
@@ -2304,13 +2304,13 @@ extern "C" int hyb_internal_replica_maps( hyb_mesh* orig, hyb_mesh* uni, int R, 
    const int tpad = int( std::max< size_t >( 256, ( tmax + 255 ) / 256 * 256 ) );
    std::vector< int4 > tasks( size_t( R ) * tpad, make_int4( -1, 0, 0, 0 ) );
    for ( int r = 0; r < R; ++r ) std::copy( per[r].begin(), per[r].end(), tasks.begin() + size_t( r ) * tpad );
-   auto up = [&]( void** dst, const void* src, size_t bytes ) {
-      check_cuda( cudaMalloc( dst, std::max< size_t >( bytes, 16 ) ), "cudaMalloc(replica maps)" );
-      check_cuda( cudaMemcpy( *dst, src, bytes, cudaMemcpyHostToDevice ), "upload replica maps" );
-   };
-   up( d_poff, poff.data(), poff.size() * sizeof( int64_t ) );
-   up( d_off, off.data(), off.size() * sizeof( int64_t ) );
-   up( d_tasks, tasks.data(), tasks.size() * sizeof( int4 ) );
+   TableArrays arrays;
+   int64_t *   a_poff = arrays.upload( poff.data(), poff.size(), "replica maps" ), *a_off = arrays.upload( off.data(), off.size(), "replica maps" );
+   int4*       a_tasks = arrays.upload( tasks.data(), tasks.size(), "replica maps" );
+   arrays.keep();
+   *d_poff   = a_poff;
+   *d_off    = a_off;
+   *d_tasks  = a_tasks;
    *np_out   = np;
    *count    = Po.packed_size;
    *tpad_out = tpad;

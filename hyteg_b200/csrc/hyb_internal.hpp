@@ -487,6 +487,11 @@ void launch_cg_scalar( Context* ctx, double* state, int stage, double rtol, doub
 // host helpers
 void check_cuda( cudaError_t e, const char* what );
 
+// Tables are copied from pageable memory on the legacy stream.  Such a copy may return once the data is staged,
+// before it is in place on the device, and the contexts' streams are non-blocking: a kernel launched there does not
+// wait for the legacy stream.  So whoever publishes a table waits here first.
+inline void finish_uploads() { check_cuda( cudaStreamSynchronize( cudaStreamLegacy ), "table upload" ); }
+
 // Device arrays of tables that are built together and published together: what is not kept is freed again, so
 // that a failure on the way (out of memory) leaves the level as it was and a later call builds it anew.
 void* table_malloc( size_t bytes, const char* what );
@@ -509,9 +514,14 @@ class TableArrays
    {
       T* p = get< T >( count, what );
       if ( count ) check_cuda( cudaMemcpy( p, host, count * sizeof( T ), cudaMemcpyHostToDevice ), what );
+      uploads_ = true;
       return p;
    }
-   void keep() { owned_.clear(); }
+   void keep()
+   {
+      if ( uploads_ ) finish_uploads();
+      owned_.clear();
+   }
    ~TableArrays()
    {
       for ( void* p : owned_ ) cudaFree( p );
@@ -519,6 +529,7 @@ class TableArrays
 
  private:
    std::vector< void* > owned_;
+   bool                 uploads_ = false;
 };
 
 // One-time set-up per CUDA device: __constant__ tables and kernel attributes exist once per device,
@@ -538,6 +549,7 @@ class PerDeviceOnce
       std::lock_guard< std::mutex > lock( mu_ );
       if ( done_.load( std::memory_order_relaxed ) & bit ) return;
       f();
+      finish_uploads();
       done_.fetch_or( bit, std::memory_order_release );
    }
    // whether the set-up has run on the current device

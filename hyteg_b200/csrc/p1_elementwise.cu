@@ -1849,8 +1849,9 @@ static void ensure_rows( Operator* op, int L )
       }
    }
    e.aoff[8] = int( anch.size() );
-   e.d_anch  = arrays.upload( anch.data(), anch.size(), "anchors" );
+   int* d_anch = arrays.upload( anch.data(), anch.size(), "anchors" );
    arrays.keep();
+   e.d_anch = d_anch;
 }
 
 // threads per block of a pass over na anchors per cell (grid: blocks x cells): whole warps, at most
@@ -1935,8 +1936,10 @@ __global__ void __launch_bounds__( 128 ) k_p2_nodal_coeff( int ns, const int64_t
 static void upload_geometry( Operator* op )
 {
    if ( op->d_geom ) return;
-   check_cuda( cudaMalloc( &op->d_geom, op->geom.size() * sizeof( CellGeom ) ), "cudaMalloc(geometry)" );
-   check_cuda( cudaMemcpy( op->d_geom, op->geom.data(), op->geom.size() * sizeof( CellGeom ), cudaMemcpyHostToDevice ), "upload geometry" );
+   TableArrays arrays;
+   CellGeom*   d_geom = arrays.upload( op->geom.data(), op->geom.size(), "geometry" );
+   arrays.keep();
+   op->d_geom = d_geom;
 }
 
 void set_p2_nodal_coefficient( Context* ctx, Operator* op, int Ls, const double* src )
@@ -1969,8 +1972,9 @@ static void ensure_cell_points( ElemLevel& e, const P1Level& P )
       for ( int y = 0; y + z <= P.n; ++y )
          for ( int x = 0; x + y + z <= P.n; ++x ) pts.push_back( make_ushort4( (unsigned short) x, (unsigned short) y, (unsigned short) z, 0 ) );
    TableArrays arrays;
-   e.d_pts = arrays.upload( pts.data(), pts.size(), "cell points" );
+   ushort4*    d_pts = arrays.upload( pts.data(), pts.size(), "cell points" );
    arrays.keep();
+   e.d_pts = d_pts;
 }
 
 template < typename T, typename A >
@@ -2182,12 +2186,7 @@ static void run_stokes( Context* ctx, Operator* op, int Lp, int divt, const void
    ensure_device( m, PU );
    ensure_p2_constants();
    ensure_stokes_constants();
-   if ( !op->d_geom )
-   {
-      check_cuda( cudaMalloc( &op->d_geom, op->geom.size() * sizeof( CellGeom ) ), "cudaMalloc(geometry)" );
-      check_cuda( cudaMemcpy( op->d_geom, op->geom.data(), op->geom.size() * sizeof( CellGeom ), cudaMemcpyHostToDevice ),
-                  "upload geometry" );
-   }
+   upload_geometry( op );
    ensure_rows( op, Ls );
    ElemLevel& e = op->el[Ls];
    if ( !e.d_sacc )
@@ -2371,12 +2370,7 @@ static void run_visc( Context* ctx, Operator* op, int Lp, int mode, const void* 
    ensure_device( m, PU );
    ensure_p2_constants();
    ensure_visc_constants();
-   if ( !op->d_geom )
-   {
-      check_cuda( cudaMalloc( &op->d_geom, op->geom.size() * sizeof( CellGeom ) ), "cudaMalloc(geometry)" );
-      check_cuda( cudaMemcpy( op->d_geom, op->geom.data(), op->geom.size() * sizeof( CellGeom ), cudaMemcpyHostToDevice ),
-                  "upload geometry" );
-   }
+   upload_geometry( op );
    ensure_rows( op, Ls );
    ElemLevel& e = op->el[Ls];
    if ( !e.d_sacc ) check_cuda( cudaMalloc( &e.d_sacc, size_t( 3 * PU.size ) * sizeof( double ) ), "cudaMalloc(viscous block scratch)" );
