@@ -1034,16 +1034,16 @@ __device__ __forceinline__ void p2_grad( int q, int i, const A Mi[3][3], A G[3] 
 
 // One parity pass over the level-L micro-cells (anchors of parity (px, py, pz); ne = 2^L), nodes on
 // storage level L+1.  MODE 1: diagonal of K into acc; 2: K added to the assembled stencils of its nodes
-// (st, layout of sv).  Anchors of one parity share no node, and the micro-cells of one anchor are taken in
+// (st, layout of sv, whose macro-cells are the launch's: first_cell and those after it).  Anchors of one parity share no node, and the micro-cells of one anchor are taken in
 // order by one thread, so plain additions are deterministic.
 template < typename A, int MODE >
-__global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
+__global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int first_cell, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                                                        const CellGeom* __restrict__ geom, Coefficient kc, A* __restrict__ acc,
                                                        P2StoredView sv, A* __restrict__ st, int64_t st_size, int64_t level_size, int* err,
                                                        const double* __restrict__ kn )
 {
    const int t = blockIdx.x * blockDim.x + threadIdx.x;  // one micro-cell anchor per thread
-   const int c = blockIdx.y;
+   const int c = first_cell + int( blockIdx.y );
    if ( t >= nanch ) return;
    const int      a = anch[t];
    const int      x = a & 1023, y = ( a >> 10 ) & 1023, z = a >> 20, ns = 2 * ne;
@@ -1102,7 +1102,7 @@ __global__ void __launch_bounds__( 256, 2 ) k_p2_pass( int ne, int nanch, const 
          {
             const int     l = c_p2_loc[ty][i];
             int64_t       skip;
-            const int64_t w = p2_weight_at( sv, c, 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9, skip );
+            const int64_t w = p2_weight_at( sv, int( blockIdx.y ), 2 * x + l % 3, 2 * y + ( l / 3 ) % 3, 2 * z + l / 9, skip );
 #pragma unroll
             for ( int j = 0; j < 10; ++j )
             {
@@ -1858,15 +1858,16 @@ static void ensure_rows( Operator* op, int L )
 // maxb, so that the small levels (a few anchors per cell) do not launch mostly idle blocks
 static int pass_block( int na, int maxb ) { return std::min( maxb, ( na + 31 ) / 32 * 32 ); }
 
-// (MODE 2 and 4: the stencils st, for P2 of the layout sv and st_size values, which a failure leaves unpublished)
+// (MODE 2 and 4: the stencils st, for P2 of the layout sv and st_size values, which a failure leaves unpublished;
+// MODE 2: the cells first_cell .. first_cell + sv->nC - 1)
 template < typename T, typename A, int MODE >
 static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src, A* acc, A* st = nullptr, const P2StoredView* sv = nullptr,
-                        int64_t st_size = 0 )
+                        int64_t st_size = 0, int first_cell = 0 )
 {
    P1Level&   P = m->level( L );
    ElemLevel& e = op->el[L];
    if ( MODE != 2 && MODE != 4 ) check_cuda( cudaMemsetAsync( acc, 0, P.size * sizeof( A ), ctx->stream ), "cudaMemset(acc)" );
-   const int nC = m->topo.nC;
+   const int nC = MODE == 2 ? sv->nC : m->topo.nC;
    for ( int p = 0; p < 8; ++p )
    {
       const int na = e.aoff[p + 1] - e.aoff[p];
@@ -1901,7 +1902,7 @@ static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src
          else launch( std::false_type{}, std::false_type{} );
       }
       else if ( op->order == 2 && ( MODE == 1 || MODE == 2 ) )
-         k_p2_pass< A, MODE == 2 ? 2 : 1 ><<< grid, bs, 0, ctx->stream >>>( element_n( op, L ), na, e.d_anch + e.aoff[p], P.d_off + P.nB,
+         k_p2_pass< A, MODE == 2 ? 2 : 1 ><<< grid, bs, 0, ctx->stream >>>( element_n( op, L ), first_cell, na, e.d_anch + e.aoff[p], P.d_off + P.nB,
                                                                             op->d_geom, op->coeff, acc, sv ? *sv : P2StoredView{}, st, st_size, P.size,
                                                                             ctx->d_error, op->nodal_k ? e.d_kn : nullptr );
       else if constexpr ( MODE != 2 )
@@ -1977,6 +1978,47 @@ static void ensure_cell_points( ElemLevel& e, const P1Level& P )
    e.d_pts = d_pts;
 }
 
+// out[i + (i / block) (stride - block)] = in[i], rounded: one entry after the other of a slab of macro-cells into
+// the level's weights
+__global__ void __launch_bounds__( 256 ) k_slab_weights( int64_t count, int64_t block, int64_t stride, const double* __restrict__ in,
+                                                          float* __restrict__ out )
+{
+   const int64_t i = int64_t( blockIdx.x ) * 256 + threadIdx.x;
+   if ( i < count ) out[i + i / block * ( stride - block )] = float( in[i] );
+}
+
+// FP64 weights that the FP32 ones of a level are rounded from, at a time: with all of them beside the FP32 ones
+// (230 + 115 bytes per node) the set-up needed twice the memory of FP32 element matrices, and levels that had
+// fitted did not
+constexpr int64_t kSlabBytes = int64_t( 256 ) << 20;
+
+// FP32 weights of a P2 level, macro-cells in slabs of kSlabBytes (one cell at least)
+static void fill_low_weights( Context* ctx, Mesh* m, Operator* op, int L, const P2StoredView& v, int64_t count, float* out )
+{
+   const int64_t per   = count / v.nC;  // weights of a macro-cell
+   const int     cells = int( std::max< int64_t >( 1, std::min< int64_t >( v.nC, kSlabBytes / ( 8 * per ) ) ) );
+   TableArrays   arrays;
+   double*       slab = arrays.get< double >( per * cells, "stencil slab" );
+   for ( int c0 = 0; c0 < v.nC; c0 += cells )
+   {
+      P2StoredView w = v;
+      w.nC           = std::min( cells, v.nC - c0 );
+      for ( int s = 0; s < 16; ++s ) w.wbase[s] = v.wbase[s] / v.nC * w.nC;
+      check_cuda( cudaMemsetAsync( slab, 0, per * w.nC * sizeof( double ), ctx->stream ), "cudaMemset" );
+      run_passes< double, double, 2 >( ctx, m, op, L, nullptr, nullptr, slab, &w, per * w.nC, c0 );
+      for ( int s = 0; s < 16; ++s )
+      {
+         const int64_t n = ( s < 15 ? w.wbase[s + 1] : per * w.nC ) - w.wbase[s], block = int64_t( w.nC ) * v.np[s];
+         if ( n == 0 ) continue;
+         k_slab_weights<<< unsigned( ( n + 255 ) / 256 ), 256, 0, ctx->stream >>>( n, block, int64_t( v.nC ) * v.np[s], slab + w.wbase[s],
+                                                                                   out + v.wbase[s] + int64_t( c0 ) * v.np[s] );
+         ++ctx->launches;
+      }
+   }
+   check_cuda( cudaGetLastError(), "stencil slab launch" );
+   check_cuda( cudaStreamSynchronize( ctx->stream ), "stencil slabs" );
+}
+
 template < typename T, typename A >
 static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
 {
@@ -2013,7 +2055,7 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
    }
    else if ( op->store_matrices && !e.d_S[sizeof( A ) == 8 ? 0 : 1] )
    {
-      // P2: likewise; the sums in double go again where only float ones are used
+      // P2: likewise; float weights alone are rounded from slabs of sums in double
       if ( !e.p2s )
       {
          std::vector< ushort4 > pts;
@@ -2032,26 +2074,21 @@ static void ensure_level_t( Context* ctx, Operator* op, int L, int dtype )
          e.p2s        = v;
       }
       TableArrays arrays;
-      double*     S = static_cast< double* >( e.d_S[0] );
-      if ( !S )
+      if ( sizeof( A ) == 8 )
       {
-         S = arrays.get< double >( e.p2s_count, "assembled stencils" );
+         double* S = arrays.get< double >( e.p2s_count, "assembled stencils" );
          check_cuda( cudaMemsetAsync( S, 0, e.p2s_count * sizeof( double ), ctx->stream ), "cudaMemset" );
          run_passes< double, double, 2 >( ctx, m, op, L, nullptr, nullptr, S, e.p2s.get(), e.p2s_count );
-      }
-      if ( sizeof( A ) == 4 )
-      {
-         TableArrays low;
-         float*      Sf = low.get< float >( e.p2s_count, "assembled stencils" );
-         launch_convert( ctx, e.p2s_count, F32, Sf, F64, S );
-         check_cuda( cudaStreamSynchronize( ctx->stream ), "assembled stencils" );
-         low.keep();
-         e.d_S[1] = Sf;
+         arrays.keep();
+         e.d_S[0] = S;
       }
       else
       {
+         float* S = arrays.get< float >( e.p2s_count, "assembled stencils" );
+         if ( e.d_S[0] ) launch_convert( ctx, e.p2s_count, F32, S, F64, e.d_S[0] );
+         else fill_low_weights( ctx, m, op, L, *e.p2s, e.p2s_count, S );
          arrays.keep();
-         e.d_S[0] = S;
+         e.d_S[1] = S;
       }
    }
    if ( e.d_invd[dtype] ) return;

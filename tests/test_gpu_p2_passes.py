@@ -142,3 +142,40 @@ def test_p2_stored_apply(ctx, case, L, dtype):
         ref = op.apply(x, np.zeros_like(x), L, flag)
         err = np.abs(fy.download(L) - ref)[lev.owned_mask(O.ALL)].max()
         assert err <= (1e-12 if dtype == "float64" else 1.2e-5) * max(np.abs(ref).max(), 1e-300)
+
+
+def test_fp32_stored_weights_in_slabs(ctx):
+    """FP32 weights of a level whose FP64 weights (2.5 GB) do not fit beside them (1.3 GB): built from slabs of
+    macro-cells, with the same bits as weights rounded from all FP64 ones at once."""
+    import torch
+
+    coords, tets = O.mesh_spherical_shell(3, 2, 0.55, 1.0)
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    L = 5
+    fx, fy = (H.P2Function(n, pm, L, L, ctx, "float32") for n in "xy")
+    fx.fill_random(L, 1)
+
+    def operator():
+        A = H.P2ElementwiseBlendingDivKGradOperator(pm, L, L, ctx, k=SPECS["expsin"][0], blending="shell")
+        A.computeAndStoreLocalElementMatrices()
+        return A
+
+    A = operator()
+    ctx.synchronize()
+    torch.cuda.empty_cache()
+    room = int(2.4e9)
+    filler = [torch.empty(max(torch.cuda.mem_get_info()[0] - room, 1), dtype=torch.uint8, device="cuda")]
+    assert torch.cuda.mem_get_info()[0] < 1.1 * room
+    A.apply(fx, fy, L, H.All)
+    low = fy.download(L)
+    filler.clear()
+    torch.cuda.empty_cache()
+    B = operator()
+    dx, dy = (H.P2Function(n, pm, L, L, ctx) for n in ("dx", "dy"))
+    dx.upload(L, fx.download(L).astype(np.float64))
+    B.apply(dx, dy, L, H.All)
+    fy.interpolate(0.0, L, H.All)
+    B.apply(fx, fy, L, H.All)
+    np.testing.assert_array_equal(fy.download(L), low)
+    ref = dy.download(L)
+    assert np.abs(low - ref).max() <= 1.2e-5 * np.abs(ref).max()
