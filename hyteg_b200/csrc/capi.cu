@@ -167,6 +167,7 @@ int hyb_ctx_create( int device, void* stream, hyb_ctx** out )
    auto* h     = new hyb_ctx();
    h->c.device = device;
    set_device( h->c );
+   check_cuda( cudaDeviceGetAttribute( &h->c.sms, cudaDevAttrMultiProcessorCount, device ), "device attribute" );
    if ( stream ) h->c.stream = (cudaStream_t) stream;
    else
    {

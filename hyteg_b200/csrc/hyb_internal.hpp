@@ -344,6 +344,7 @@ struct Operator {
 
 struct Context {
    int          device = 0;
+   int          sms    = 0;  // streaming multiprocessors of the device
    cudaStream_t stream = nullptr;
    bool         own_stream = false;
    cudaStream_t aux     = nullptr;  // second stream for the boundary half of each operation

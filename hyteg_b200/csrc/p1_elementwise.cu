@@ -1877,9 +1877,10 @@ static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src
       if ( op->order == 2 && MODE == 0 )
       {
          const int3 kinds  = make_int3( e.akind[p][0], e.akind[p][1], e.akind[p][2] );
-         // anchors that 148 SMs with six blocks of k_p2_apply_pass hold at once: below it the split pass is
-         // faster (shell of 240 cells, level 3: 183 against 494 us an apply), above it slower (2.69 against 2.27 ms on the shell named there)
-         const bool split  = int64_t( na ) * nC < 148 * 6 * kP2ApplyThreads;
+         // anchors that the SMs with six blocks of k_p2_apply_pass each hold at once (56,832 on 148 SMs): below it
+         // the split pass is faster (shell of 240 cells, level 3: 183 against 494 us an apply), above it slower
+         // (2.69 against 2.27 ms on the shell named there)
+         const bool split  = int64_t( na ) * nC < int64_t( ctx->sms ) * 6 * kP2ApplyThreads;
          const int  per    = split ? 32 : kP2ApplyThreads, per1 = split ? kP2SplitThreads : kP2ApplyThreads;
          auto       blocks = [&]( int k, int b ) { return int( ( int64_t( k ) * nC + b - 1 ) / b ); };
          const int3 bl     = make_int3( blocks( kinds.x, per ), blocks( kinds.y, per ), blocks( kinds.z, per1 ) );

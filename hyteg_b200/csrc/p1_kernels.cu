@@ -1845,7 +1845,7 @@ static void run_restrict( Context* ctx, const LevelView& cv, const LevelView& fv
    const int         nbnd = ( seg.threads + 255 ) / 256, blocks = nbnd + interior_blocks( cv, nC );
    // level vectors are whole multiples of 32 values, so of 16 bytes
    const int64_t nzero = int64_t( zero_bytes / 16 );
-   const int     zb    = int( std::min< int64_t >( ( nzero + 1023 ) / 1024, 148 * 4 ) );
+   const int     zb    = int( std::min< int64_t >( ( nzero + 1023 ) / 1024, ctx->sms * 4 ) );
    if ( blocks + zb == 0 ) return;
    k_restrict< T, A ><<< blocks + zb, 256, 0, ctx->stream >>>( cv, fv, seg, nbnd, nC, flag, (const T*) fine, (T*) coarse, blocks,
                                                               reinterpret_cast< uint4* >( zero ), nzero );
