@@ -7,6 +7,8 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 namespace hyb {
 
 // Cell-interior and boundary-primitive kernels of one operation write disjoint slots, so the
@@ -119,13 +121,13 @@ static inline LevelView make_view( Mesh* m, int L )
    v.cell_bc   = P.d_bc + P.nB;
    v.bkind     = P.d_bkind;
    v.ncell_cls = P.d_ncell_cls;
-   v.nzblocks = int( P.zbegin.size() ) - 1;
+   v.nzblocks = std::max( int( P.zbegin.size() ) - 1, 0 );
    v.zunits   = P.d_zunits;
    v.zcell    = P.d_zcell;
    v.zbegin   = P.d_zbegin;
    for ( int b = 0; b < kSwLists; ++b )
    {
-      v.nswarps[b] = int( P.swbegin[b].size() ) - 1;
+      v.nswarps[b] = std::max( int( P.swbegin[b].size() ) - 1, 0 );
       v.swunits[b] = P.d_swunits[b];
       v.swcell[b]  = P.d_swcell[b];
       v.swbegin[b] = P.d_swbegin[b];

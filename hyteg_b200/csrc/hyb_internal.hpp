@@ -156,10 +156,12 @@ struct Topology {
 // and runs one point per lane.  Each warp of a launch owns a list of units; a launch has kSwWarps
 // warps per block and BPS = 2, 3 or 4 blocks per SM (by value type and operation), one list set per
 // BPS.
-// points per macro-edge up to which cell interiors run one thread per point (k_flat_stencil)
+// points per macro-edge up to which a level lists its interior points, for kernels with one thread per point
 constexpr int kFlatMaxN    = 64;
 // the same for the P2 constant stencils
 constexpr int kP2cFlatMaxN = 64;
+// interior points (all cells) from which such a level may still take the tiled sweeps, and so has their units
+constexpr int64_t kTiledMinPoints = 2500000;
 constexpr int kSwR         = 4;
 constexpr int kSwTX        = 64;  // 32 or 64
 constexpr int kSwWarps     = 4;

@@ -86,7 +86,7 @@ __device__ __forceinline__ void sweep_epilogue( int64_t i, A s, A invd, A centre
 }
 
 // ---------------------------------------------------------------------------------------------
-// Cell-interior sweep for levels with n >= 32 (every stencil operation, every value type).
+// Cell-interior sweep of the levels that flat_cells leaves to the tiles (operations without a second vector).
 //
 // Work unit: the rows y0..y0+kSwR-1 and the x-points x0..x0+63 (x0..x0+31 for a half-width unit)
 // of the slices z_first..z_last of one macro-cell, interior points only (x, y, z >= 1,
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__( kSwWarps * 32, SwCfg< T, OP >::BPS )
 
 // ---------------------------------------------------------------------------------------------
 // Rolled-register z-streamed cell sweep, for the operations with a second vector (residual, Jacobi,
-// Chebyshev steps, apply-add) on levels with n >= 32.
+// Chebyshev steps, apply-add) on the same levels.
 //
 // A unit is the tile x0..x0+63, y0..y0+7 of slices z_first..z_last of one macro-cell.  Two producer
 // warps stream the tile's rows of every slice (one-point halo in x and y, plus the tile rows of the
@@ -921,8 +921,7 @@ __device__ __forceinline__ A point_stencil( const T* c, const A* W, int n, int y
 // cell kernel beside a boundary kernel on a second stream took 10.3 us for a level-4 FP32 apply on 36 cells
 // where this takes 5.9, and ten V(2,2) cycles of the level-5 cube 4.55 ms where these take 2.66.  The
 // tiled sweeps are faster from 128 points on (level-7 FP32 smoothing on 12 cells 521 against 592 us; the
-// level-8 apply 90 against 283 us), this kernel up to 64 (level-8 FP64 cycle 4.51 against 4.79 ms with the
-// sweep there).
+// level-8 apply 96 against 283 us), below that by the number of points (flat_cells).
 template < typename T, typename A, int OP >
 __global__ void __launch_bounds__( kBndThreads ) k_flat_stencil( LevelView v, OpView< A > o, BndSegments seg, int nbnd, int nC, uint32_t flag,
                                                                  int copy_unflagged, const T* __restrict__ src, const T* __restrict__ v1,
@@ -943,6 +942,25 @@ __global__ void __launch_bounds__( kBndThreads ) k_flat_stencil( LevelView v, Op
    stencil_epilogue< T, A, OP >( i, s, o.invd_c[c], src, v1, v2, dst, a0, a1 );
 }
 
+// Whether a level's cell interiors run one thread per point.  Us per operation on box and shell meshes, one thread
+// per point / tiled sweep (million interior points, all cells):
+//    apply, FP64, 64 points per edge   32 / 42 (1.4)   80 / 56 (3.8)   203 / 131 (9.5)   787 / 457 (38)
+//    apply, FP32, 64                   26 / 37 (1.4)   62 / 51 (3.8)   155 / 102 (9.5)   605 / 370 (38)
+//    apply, FP64, 32                   46 / 50 (1.7)  117 / 115 (4.3)  240 / 225 (8.6)
+//    apply, FP32, 32                   36 / 42 (1.7)   83 / 88 (4.3)   173 / 179 (8.6)
+//    Chebyshev(3) step, FP64, 64      105 / 127 (1.4) 284 / 288 (3.8)  709 / 654 (9.5)  2796 / 2389 (38)
+//    Chebyshev(3) step, FP32, 64       84 / 119 (1.4) 208 / 252 (3.8)  533 / 596 (9.5)  2092 / 2169 (38)
+//    Chebyshev(3) step, FP64, 32      162 / 247 (1.7) 419 / 604 (4.3)  845 / 1182 (8.6)
+// FP16 goes with FP32; at 16 points per edge the tiles are nearly empty, at 128 see k_flat_stencil.
+template < typename T, bool AUX >
+static bool flat_cells( int n, int64_t points )
+{
+   if ( n > kFlatMaxN ) return false;
+   if ( n < 32 ) return true;
+   if ( AUX ) return sizeof( T ) < 8 || n < 64 || points < 6000000;
+   return n < 64 ? sizeof( T ) < 8 || points < 4000000 : points < kTiledMinPoints;
+}
+
 template < typename T, typename A, int OP >
 static void run_stencil( Context* ctx, const LevelView& v, const OpView< A >& o, int nC, const StencilArgs& a )
 {
@@ -955,7 +973,7 @@ static void run_stencil( Context* ctx, const LevelView& v, const OpView< A >& o,
    // slots of the second vector), so the two kernels may run in either order
    const BndSegments seg = bnd_segments( v, a.flag, a.copy_unflagged );
    const int         nt  = seg.threads, nbnd = ( nt + kBndThreads - 1 ) / kBndThreads;
-   if ( v.n <= kFlatMaxN )
+   if ( flat_cells< T, sweep_aux< OP >() >( v.n, int64_t( nC ) * v.nipts ) )
    {
       const int blocks = nbnd + int( ( int64_t( nC ) * v.nipts + kBndThreads - 1 ) / kBndThreads );
       if ( blocks == 0 ) return;

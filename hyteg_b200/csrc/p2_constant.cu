@@ -872,7 +872,12 @@ static void run_p2c( Context* ctx, const LevelView& v, const A* W, const P2cLeve
    const int          nbnd = ( seg.threads + 255 ) / 256;
    P2cPoints          pts{};
    int                blocks = nbnd;
-   for ( int k = 0; k < 8; ++k )
+   // At 64 points per edge the tiled sweep is faster without a second vector from four million points on: us per
+   // apply, one thread per point / tiled sweep (million points), FP64 60 / 79 (1.4), 159 / 155 (3.8), 429 / 336
+   // (9.5), FP32 47 / 66, 120 / 123, 305 / 271; a Chebyshev(3) step of the last size takes 1445 / 1713 and
+   // 1051 / 1377, and an apply at 32 points 598 / 694 and 447 / 566 (8.6).
+   const bool tiled = v.n > kP2cFlatMaxN || ( v.n == 64 && !sweep_aux< OP >() && int64_t( nC ) * v.nipts >= 4000000 );
+   for ( int k = 0; k < 8 && !tiled; ++k )
    {
       pts.np[k] = pl.np[k];
       blocks += int( ( int64_t( nC ) * pl.np[k] + 255 ) / 256 );
@@ -887,7 +892,7 @@ static void run_p2c( Context* ctx, const LevelView& v, const A* W, const P2cLeve
       ++ctx->launches;
    }
    const int nw = v.nswarps[0];
-   if ( nw > 0 && nC > 0 && v.n > kP2cFlatMaxN )
+   if ( nw > 0 && nC > 0 && tiled )
    {
       // the sweep keeps cell-relative row starts in 32-bit integers
       if ( tet_size( int64_t( v.n ) + 1 ) > int64_t( 0x7fffffff ) ) throw std::invalid_argument( "P2 constant operator: level too large" );

@@ -603,6 +603,8 @@ static void build_device( Mesh* m, P1Level& P, TableArrays& arrays )
    int dev = 0, sms = 0;
    check_cuda( cudaGetDevice( &dev ), "cudaGetDevice" );
    check_cuda( cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev ), "device attribute" );
+   const bool tiled = P.n > kFlatMaxN || int64_t( t.nC ) * P.nipts >= kTiledMinPoints;  // work units only where a sweep runs
+   if ( tiled )
    {
       build_zunits( P, 2 * std::max( sms, 1 ), t.nC );
       std::vector< int4 > zu( P.zunits.size() );
@@ -611,7 +613,7 @@ static void build_device( Mesh* m, P1Level& P, TableArrays& arrays )
       up( &P.d_zcell, P.zcell.data(), P.zcell.size() );
       up( &P.d_zbegin, P.zbegin.data(), P.zbegin.size() );
    }
-   for ( int b = 0; b < kSwLists; ++b )
+   for ( int b = 0; b < kSwLists && tiled; ++b )
    {
       // one list set per blocks-per-SM count (b + 2) of the sweep's instantiations
       build_sweep_units( P, b, sms * ( b + 2 ) * kSwWarps, t.nC );

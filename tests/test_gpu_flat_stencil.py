@@ -54,12 +54,44 @@ def test_p1_operations(ctx, mesh, L, neumann):
     check(f["y"].download(L), jac)
 
 
-@pytest.mark.parametrize("L", [5, 6, 7])
+def _shell(ntan, nrad):
+    return lambda: O.mesh_spherical_shell(ntan, nrad, 0.55, 1.0)
+
+
+# both sides of the changes between one thread per point and the tiles, by points per edge (64 and 128) and at 32
+# and 64 by the level's points: 60, 120 and 240 cells of 64 points have 2.4, 4.8 and 9.5 million, 960 of 32 have 4.3
+SIZES = {"cube 5": (M.cube_6, 5), "cube 6": (M.cube_6, 6), "cube 7": (M.cube_6, 7), "60 cells 6": (_shell(2, 2), 6),
+         "120 cells 6": (_shell(2, 3), 6), "240 cells 6": (_shell(3, 2), 6), "960 cells 5": (_shell(5, 2), 5)}
+
+
+@pytest.mark.parametrize("size", sorted(SIZES))
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
-def test_p1_chebyshev_across_kernels(ctx, L, dtype):
+def test_p1_apply_across_kernels(ctx, size, dtype):
+    """The constant stencils against the elementwise operator with k = 1 in FP64 (the same matrix; 1e-12 of the
+    largest value, FP32 15 products per cell and up to 30 cells: 64 eps)."""
+    make, L = SIZES[size]
+    coords, tets = make()
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    C = H.P1ConstantLaplaceOperator(pm, L, L, ctx)
+    E = H.P1ElementwiseBlendingDivKGradOperator(pm, L, L, ctx, k=1.0)
+    x, y = (H.P1Function(n, pm, L, L, ctx, dtype) for n in "xy")
+    u, z = (H.P1Function(n, pm, L, L, ctx) for n in "uz")
+    x.fill_random(L, 7)
+    u.upload(L, x.download(L).astype(np.float64))
+    for update in (H.Replace, H.Add):
+        C.apply(x, y, L, H.Inner, update)
+        E.apply(u, z, L, H.Inner, update)
+        a, b = y.download(L), z.download(L)
+        assert np.abs(a - b).max() <= (1e-12 if dtype == "float64" else 8e-6) * np.abs(b).max()
+
+
+@pytest.mark.parametrize("size", sorted(SIZES))
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_p1_chebyshev_across_kernels(ctx, size, dtype):
     """One Chebyshev(3) step equals its definition from the operator's own apply (FP64 1e-12; FP32: three
     applies of 15 products each, values up to 10: 200 eps)."""
-    coords, tets = M.cube_6()
+    make, L = SIZES[size]
+    coords, tets = make()
     pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
     A = H.P1ConstantLaplaceOperator(pm, L - 1, L, ctx)
     g = H.GeometricMultigridSolver(ctx, A, L - 1, L, smoother="chebyshev")

@@ -51,11 +51,12 @@ def test_p2_constant_matches_oracle(ctx, mesh, L, neumann):
     check(op.smooth_jac(ref.copy(), vec["b"], vec["x"], 0.6, L, flag))
 
 
-@pytest.mark.parametrize("L", [5, 6, 7])
+@pytest.mark.parametrize("cells,L", [(6, 5), (6, 6), (6, 7), (60, 5), (120, 5), (120, 4)])
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
-def test_p2_constant_equals_elementwise(ctx, L, dtype):
-    """FP32: 65 products of values up to one and weights of either sign, 100 eps."""
-    coords, tets = M.cube_6()
+def test_p2_constant_equals_elementwise(ctx, cells, L, dtype):
+    """Both sides of the changes of kernel: 64 and 128 nodes per edge, and 2.4 and 4.8 million nodes at 64.  FP32: 65
+    products of values up to one and weights of either sign, 100 eps."""
+    coords, tets = M.cube_6() if cells == 6 else O.mesh_spherical_shell(2, 1 + cells // 60, 0.55, 1.0)
     pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
     C = H.P2ConstantLaplaceOperator(pm, L, L, ctx)
     A = H.P2ElementwiseBlendingDivKGradOperator(pm, L, L, ctx, k=1.0)
