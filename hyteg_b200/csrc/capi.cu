@@ -2771,10 +2771,12 @@ void stokes_prepare( hyb_stokes* s, hyb_fn* u0, hyb_fn* b0, int dt )
       s->dtype = dt;
       return;
    }
-   // the smoother's two work vectors of the second and third component (the first uses the solver's)
-   for ( int k = 1; k < 3; ++k )
+   // the smoother's work vectors of the second and third component (the first uses the solver's): two, of which
+   // order two needs one and order one, smoothed component by component, none
+   for ( int k = 1; k < 3 && s->p.cheb_order >= 2; ++k )
       for ( hyb_fn** g : { &s->vz[k], &s->vt[k] } )
       {
+         if ( g == &s->vt[k] && s->p.cheb_order == 2 ) continue;
          *g               = new_fn( s->ctx, m, dt, s->p.min_level + 1, s->p.max_level + 1 );
          ( *g )->f.lshift = 1;
       }

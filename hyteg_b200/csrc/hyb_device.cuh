@@ -62,7 +62,6 @@ struct LevelView
    const int2*      rows;
    int              ntasks;
    const int4*      tasks;
-   const int4*      btasks;      // the same tasks grouped by their primitive's boundary type
    const FaceRec*   frec;        // face records of all groups, in group order
    const LowRec*    lrec;        // vertex and edge records of all groups, in group order
    const IncRec*    irec;        // their incidences
@@ -106,7 +105,6 @@ static inline LevelView make_view( Mesh* m, int L )
    v.rows      = P.d_rows;
    v.ntasks    = int( P.tasks.size() );
    v.tasks     = P.d_tasks;
-   v.btasks    = P.d_btasks;
    v.frec      = P.d_frec;
    v.lrec      = P.d_lrec;
    v.irec      = P.d_irec;

@@ -201,8 +201,7 @@ struct P1Level {
    int*       d_inc_begin = nullptr;
    Incidence* d_inc       = nullptr;
    int4*      d_tasks     = nullptr;
-   int4*      d_btasks    = nullptr;  // tasks grouped by boundary type (Inner, Dirichlet, Neumann, Freeslip)
-   FaceRec*   d_frec      = nullptr;  // face tasks, edge and vertex tasks in group order
+   FaceRec*   d_frec      = nullptr;  // face tasks, edge and vertex tasks by boundary type (Inner, Dirichlet, Neumann, Freeslip)
    LowRec*    d_lrec      = nullptr;
    IncRec*    d_irec      = nullptr;
    int        nlow[4]     = {};       // edge and vertex tasks, face tasks per group

@@ -117,10 +117,8 @@ static_assert( kP2Pat.base[8] <= kP2cEntries, "entry block too small" );
 static_assert( kSwR == 4 && kSwTX == 64, "the P2 sweep reuses the cell-sweep units: 4 rows by 64 x-points, x0 and y0 odd" );
 
 __constant__ int c_p2c_faces[kNumClasses];  // kClassFaces
-// the pattern for lanes that read different classes (boundary owners): offsets (dx, dy, dz) of every
-// entry, and per class its first entry, entry count and centre entry
-__device__ char4 g_p2c_off[kP2cEntries];
-__device__ int   g_p2c_base[24];
+// for lanes of different classes (boundary owners): per class its first entry, entry count and centre entry
+__device__ int g_p2c_base[24];
 
 // ---------------------------------------------------------------------------------------------
 // host: tables
@@ -259,11 +257,8 @@ static void          p2c_attributes_all();
 void ensure_p2_constant_device()
 {
    g_p2c_once.run( [] {
-      char4 off[kP2cEntries] = {};
-      for ( int e = 0; e < kP2cEntries; ++e ) off[e] = make_char4( kP2Pat.off[e][0], kP2Pat.off[e][1], kP2Pat.off[e][2], 0 );
       int base[24];
       for ( int k = 0; k < 8; ++k ) base[k] = kP2Pat.base[k], base[k + 8] = kP2Pat.cnt[k], base[k + 16] = kP2Pat.centre[k];
-      check_cuda( cudaMemcpyToSymbol( g_p2c_off, off, sizeof( off ) ), "constants(P2 pattern)" );
       check_cuda( cudaMemcpyToSymbol( g_p2c_base, base, sizeof( base ) ), "constants(P2 pattern)" );
       check_cuda( cudaMemcpyToSymbol( c_p2c_faces, kClassFaces, sizeof( kClassFaces ) ), "constants(P2 classes)" );
       p2c_attributes_all();

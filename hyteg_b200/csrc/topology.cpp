@@ -467,7 +467,7 @@ static void drop_device( P1Level& P, bool owned )
       if ( owned ) cudaFree( p );
       p = nullptr;
    };
-   drop( P.d_off ), drop( P.d_poff ), drop( P.d_inc_begin ), drop( P.d_inc ), drop( P.d_tasks ), drop( P.d_btasks ), drop( P.d_frec );
+   drop( P.d_off ), drop( P.d_poff ), drop( P.d_inc_begin ), drop( P.d_inc ), drop( P.d_tasks ), drop( P.d_frec );
    drop( P.d_lrec ), drop( P.d_irec ), drop( P.d_ipts ), drop( P.d_rows ), drop( P.d_zunits ), drop( P.d_zcell ), drop( P.d_zbegin );
    for ( int b = 0; b < kSwLists; ++b ) drop( P.d_swunits[b] ), drop( P.d_swcell[b] ), drop( P.d_swbegin[b] );
    drop( P.d_bc ), drop( P.d_bkind ), drop( P.d_ncell_cls );
@@ -532,7 +532,6 @@ static void build_device( Mesh* m, P1Level& P, TableArrays& arrays )
       for ( int g = 1; g < 4; ++g ) first[g] = first[g - 1] + size_t( P.nlow[g - 1] + P.nface[g - 1] );
       std::vector< int4 > bt( tk.size() );
       for ( const int4& q : tk ) bt[first[bgroup[q.x]]++] = q;
-      up( &P.d_btasks, bt.data(), bt.size() );
       std::vector< FaceRec > fr;
       std::vector< LowRec >  lr;
       std::vector< IncRec >  ir;
