@@ -58,12 +58,32 @@ def test_full_viscous_apply_smallest_level(ctx, kind):
         assert _relerr(fy[k].download(0), ref[k], lev.owned_mask(O.ALL)) < 1e-12
 
 
+def _anchors_per_class(L):
+    """The fewest micro-cell anchors (x, y, z), x + y + z < 2^L, of one coordinate parity."""
+    n = 1 << L
+    count = [0] * 8
+    for z in range(n):
+        for y in range(n - z):
+            for x0 in (0, 1):
+                count[(z & 1) * 4 + (y & 1) * 2 + x0] += len(range(x0, n - y - z, 2))
+    return min(count)
+
+
+def _full_blocks(cells, L):
+    """Anchors per class on both sides of the change from the split pass to one anchor per thread, as the library
+    counts them: the SMs with six blocks of 64 threads each."""
+    import torch
+
+    return cells * _anchors_per_class(L) >= torch.cuda.get_device_properties(0).multi_processor_count * 6 * 64
+
+
 def test_p2_matrix_free_apply_full_blocks(ctx):
-    """Enough anchors per class (68,640) for the one-anchor-per-thread pass, against the stencil sweep of the
-    constant operator (k = 1, no blending: the same matrix)."""
+    """The one-anchor-per-thread pass against the stencil sweep of the constant operator (k = 1, no blending: the
+    same matrix)."""
     coords, tets = M.cube_2x1x1()
     pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
     L = 6
+    assert _full_blocks(len(tets), L)
     A = H.P2ElementwiseBlendingDivKGradOperator(pm, L, L, ctx, k=1.0)
     C = H.P2ConstantLaplaceOperator(pm, L, L, ctx)
     fx, fy, fz = (H.P2Function(n, pm, L, L, ctx) for n in "xyz")
@@ -72,6 +92,29 @@ def test_p2_matrix_free_apply_full_blocks(ctx):
     C.apply(fx, fz, L, O.INNER)
     y, z = fy.download(L), fz.download(L)
     assert np.abs(y - z).max() < 1e-12 * np.abs(z).max()
+
+
+@pytest.mark.parametrize("nodal", [False, True])
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_p2_full_blocks_on_the_shell(ctx, nodal, dtype):
+    """The same pass with the shell map and a variable coefficient, closed form or node values, against the stored
+    matrices of the same operator (FP64 sums of every pair; 1e-12 of the largest value, FP32 4e-5 as above)."""
+    coords, tets = O.mesh_spherical_shell(5, 2, 0.55, 1.0)
+    pm = H.PrimitiveStorage.from_tets(coords, tets, ctx)
+    L = 4
+    assert _full_blocks(len(tets), L) and not _full_blocks(len(tets), L - 1)
+    kind = H.P2ElementwiseDivKGradOperator if nodal else H.P2ElementwiseBlendingDivKGradOperator
+    spec = SPECS["expsin"][0]
+    A, S = (kind(pm, L, L, ctx, k=spec, blending="shell") for _ in range(2))
+    S.computeAndStoreLocalElementMatrices()
+    fx, fy = (H.P2Function(n, pm, L, L, ctx, dtype) for n in "xy")
+    gx, gy = (H.P2Function(n, pm, L, L, ctx) for n in ("gx", "gy"))
+    fx.fill_random(L, 7)
+    gx.upload(L, fx.download(L).astype(np.float64))
+    A.apply(fx, fy, L, O.ALL)
+    S.apply(gx, gy, L, O.ALL)
+    y, z = fy.download(L), gy.download(L)
+    assert np.abs(y - z).max() < (1e-12 if dtype == "float64" else 4e-5) * np.abs(z).max()
 
 
 @pytest.mark.parametrize("case,L", [("shell", 2), ("shell", 4), ("box", 2), ("box", 4)])
@@ -119,10 +162,11 @@ def test_fp32_passes_are_as_exact_as_their_type(ctx, case, L, kind):
 
 
 @pytest.mark.parametrize("case,L", [("tet", 0), ("tet", 1), ("tet", 4), ("shell", 0), ("shell", 2)])
-@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("dtype", ["float64", "float32", "float16"])
 def test_p2_stored_apply(ctx, case, L, dtype):
     """Stored matrices at the levels without inner nodes, with segments shorter than a block and with
-    several macro-cells in one block; FP32 sums up to 65 rounded products per macro-cell: 100 eps."""
+    several macro-cells in one block; FP32 sums up to 65 rounded products per macro-cell: 100 eps; FP16 holds the
+    vectors only, so its result differs by their rounding, half of 2^-10, and that of the FP32 sum."""
     coords, tets = M.tilted_tet() if case == "tet" else O.mesh_spherical_shell(2, 2, 0.55, 1.0)
     bl = "shell" if case == "shell" else None
     spec, kfun = SPECS["expsin"]
@@ -132,16 +176,16 @@ def test_p2_stored_apply(ctx, case, L, dtype):
     A.computeAndStoreLocalElementMatrices()
     lev = op.levels[L]
     x = _rand(lev, 1)
-    if dtype == "float32":
-        x = x.astype(np.float32).astype(np.float64)
+    x = x.astype(dtype).astype(np.float64)
     fx, fy = (H.P2Function(n, pm, L, L, ctx, dtype) for n in "xy")
     fx.upload(L, x)
     for flag in (O.INNER, O.ALL):
         fy.interpolate(0.0, L, H.All)
         A.apply(fx, fy, L, flag)
         ref = op.apply(x, np.zeros_like(x), L, flag)
-        err = np.abs(fy.download(L) - ref)[lev.owned_mask(O.ALL)].max()
-        assert err <= (1e-12 if dtype == "float64" else 1.2e-5) * max(np.abs(ref).max(), 1e-300)
+        err = np.abs(fy.download(L).astype(np.float64) - ref)[lev.owned_mask(O.ALL)].max()
+        tol = {"float64": 1e-12, "float32": 1.2e-5, "float16": 2.0**-11 + 1.2e-5}[dtype]
+        assert err <= tol * max(np.abs(ref).max(), 1e-300)
 
 
 def test_fp32_stored_weights_in_slabs(ctx):
