@@ -313,12 +313,13 @@ __device__ __forceinline__ void   st_any( double* p, double v ) { *p = v; }
 __device__ __forceinline__ void   st_any( float* p, float v ) { *p = v; }
 __device__ __forceinline__ void   st_any( __half* p, float v ) { *p = __float2half_rn( v ); }
 
-// One parity pass: warp per half-grid row (y, z) of anchors with y = py mod 2, z = pz mod 2, lanes
-// over x = px + 2k.  MODE 0 accumulates A src, MODE 1 the diagonal.
+// One parity pass: a thread per micro-cell anchor of the class (blocks of one macro-cell) and its micro-cells in
+// order.  FP64: 168 registers, so that three blocks of 128 fit an SM; at 170 two did (shell of 1920 cells, level 4,
+// exp/sin coefficient: 2.45 ms at 155 registers with sin and cos, 3.15 with sinpi at 170, 2.23 so).
 // MODE 0: y += K x with K computed on the fly; 1: diagonal of K; 4: add K into the assembled stencils of
 // the cell-array slots of its vertices (kst = stencils, kstride = level size).
 template < typename T, typename A, int MODE >
-__global__ void __launch_bounds__( 256 ) k_elem_pass( int n, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
+__global__ void __launch_bounds__( 128, sizeof( A ) == 8 ? 3 : 6 ) k_elem_pass( int n, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                                                        const CellGeom* __restrict__ geom, Coefficient kc,
                                                        const T* __restrict__ src, A* __restrict__ acc, A* __restrict__ kst,
                                                        int64_t kstride, int64_t level_size, int* err )
@@ -1872,7 +1873,7 @@ static void run_passes( Context* ctx, Mesh* m, Operator* op, int L, const T* src
    {
       const int na = e.aoff[p + 1] - e.aoff[p];
       if ( na <= 0 ) continue;
-      const int bs = pass_block( na, 256 );
+      const int bs = pass_block( na, op->order == 1 ? 128 : 256 );
       dim3      grid( ( na + bs - 1 ) / bs, nC );
       if ( op->order == 2 && MODE == 0 )
       {
@@ -2304,7 +2305,7 @@ void launch_stokes_div( Context* ctx, Operator* op, int Lp, int dtype, int divt,
 // micro-cell: at each point the velocity gradient g (g_ik = d u_i / d x_k) of the ten local nodes
 // gives the stress s = w mu |det| (g + g^T - (2/3) tr(g) I), and node a of component i receives
 // grad phi_a . s_i; gradients and pairings go through the four vertices as in k_p2_apply_pass, the
-// node sums leave as reductions as in k_stokes_div_pass.  The diagonal pass sums w mu |det| (|grad phi_a|^2 + (1/3) (d_i phi_a)^2).  Same
+// node sums meet in shared memory (k_coupled_pass).  The diagonal pass sums w mu |det| (|grad phi_a|^2 + (1/3) (d_i phi_a)^2).  Same
 // parity passes as the coupling blocks (anchors of one class share no P2 node).
 // ---------------------------------------------------------------------------------------------
 __constant__ double c_yu5_rgrad[5][10][3];
@@ -2504,7 +2505,6 @@ static void dispatch_stored3( Context* ctx, Mesh* m, Operator* op, int L, int dt
    case OP_CHEB0: run_stored3< T, A, OP_CHEB0 >( ctx, m, op, L, dtype, a ); break;
    case OP_CHEBI: run_stored3< T, A, OP_CHEBI >( ctx, m, op, L, dtype, a ); break;
    case OP_CHEBL: run_stored3< T, A, OP_CHEBL >( ctx, m, op, L, dtype, a ); break;
-   case OP_RESID: run_stored3< T, A, OP_RESID >( ctx, m, op, L, dtype, a ); break;
    default: throw std::invalid_argument( "operation not provided for three components" );
    }
 }
