@@ -319,7 +319,7 @@ __device__ __forceinline__ void   st_any( __half* p, float v ) { *p = __float2ha
 // MODE 0: y += K x with K computed on the fly; 1: diagonal of K; 4: add K into the assembled stencils of
 // the cell-array slots of its vertices (kst = stencils, kstride = level size).
 template < typename T, typename A, int MODE >
-__global__ void __launch_bounds__( 128, sizeof( A ) == 8 ? 3 : 6 ) k_elem_pass( int n, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
+__global__ void __launch_bounds__( 128, sizeof( A ) == 8 ? 3 : 1 ) k_elem_pass( int n, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                                                        const CellGeom* __restrict__ geom, Coefficient kc,
                                                        const T* __restrict__ src, A* __restrict__ acc, A* __restrict__ kst,
                                                        int64_t kstride, int64_t level_size, int* err )
@@ -1836,11 +1836,13 @@ static void ensure_rows( Operator* op, int L )
    {
       e.aoff[p]    = int( anch.size() );
       const int px = p & 1, py = ( p >> 1 ) & 1, pz = p >> 2;
-      // by the number of micro-cells an anchor has (six; five next to the slanted face; one at it), so
-      // that the threads of a warp visit the same micro-cell types
+      // P2: by the number of micro-cells an anchor has (six; five next to the slanted face; one at it), so
+      // that the threads of a warp visit the same micro-cell types.  P1: in storage order, whose warps touch fewer
+      // sectors (level 4, FP32: 17 to 19 us a pass, 18 to 22 by kind).
       for ( int k = 0; k < 3; ++k )
       {
-         const int lo = k == 0 ? 0 : n - 3 + k, hi = n - 3 + k;
+         int lo = k == 0 ? 0 : n - 3 + k, hi = n - 3 + k;
+         if ( op->order == 1 ) lo = k == 0 ? 0 : n, hi = n - 1;
          const int before = int( anch.size() );
          for ( int z = pz; z <= n - 1; z += 2 )
             for ( int y = py; y + z <= n - 1; y += 2 )
