@@ -315,11 +315,12 @@ __device__ __forceinline__ void   st_any( __half* p, float v ) { *p = __float2ha
 
 // One parity pass: a thread per micro-cell anchor of the class (blocks of one macro-cell) and its micro-cells in
 // order.  FP64: 168 registers, so that three blocks of 128 fit an SM; at 170 two did (shell of 1920 cells, level 4,
-// exp/sin coefficient: 2.45 ms at 155 registers with sin and cos, 3.15 with sinpi at 170, 2.23 so).
+// exp/sin coefficient: 2.45 ms at 155 registers with sin and cos, 3.15 with sinpi at 170, 2.26 so).  FP32: six blocks
+// (1.09 ms there; without the bound the compiler takes more registers: 1.21).
 // MODE 0: y += K x with K computed on the fly; 1: diagonal of K; 4: add K into the assembled stencils of
 // the cell-array slots of its vertices (kst = stencils, kstride = level size).
 template < typename T, typename A, int MODE >
-__global__ void __launch_bounds__( 128, sizeof( A ) == 8 ? 3 : 1 ) k_elem_pass( int n, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
+__global__ void __launch_bounds__( 128, sizeof( A ) == 8 ? 3 : 6 ) k_elem_pass( int n, int nanch, const int* __restrict__ anch, const int64_t* __restrict__ cell_off,
                                                        const CellGeom* __restrict__ geom, Coefficient kc,
                                                        const T* __restrict__ src, A* __restrict__ acc, A* __restrict__ kst,
                                                        int64_t kstride, int64_t level_size, int* err )
