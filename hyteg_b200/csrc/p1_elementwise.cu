@@ -399,6 +399,7 @@ __constant__ __align__( 16 ) int8_t c_p2_loc[6][10];  // node of micro-cell type
 __constant__ double c_p2_rgrad[11][10][3];  // reference gradients of the ten basis functions per point
 __constant__ double c_p2_phi[11][10];       // values of the ten basis functions per point
 __constant__ int    c_p2_edge[6][2] = { { 2, 3 }, { 1, 3 }, { 1, 2 }, { 0, 3 }, { 0, 2 }, { 0, 1 } };
+__constant__ __align__( 16 ) int8_t c_p2_node0[27];   // node of micro-cell type 0 at a window node, or -1
 __constant__ __align__( 16 ) int8_t c_p2s_ent[600];  // entry of node j in node i's class stencil: (10 ty + i) 10 + j
 
 // barycentric coordinates (l0, l1, l2, l3) of the rule's points (kept identical to the reference's
@@ -503,6 +504,10 @@ void ensure_p2_constants()
             loc[ty][i] = int8_t( p2_local( ty, i, 0 ) + 3 * p2_local( ty, i, 1 ) + 9 * p2_local( ty, i, 2 ) );
 
       check_cuda( cudaMemcpyToSymbol( c_p2_loc, loc, sizeof( loc ) ), "P2 constants (local nodes)" );
+      int8_t node0[27];
+      for ( int l = 0; l < 27; ++l ) node0[l] = -1;
+      for ( int i = 0; i < 10; ++i ) node0[loc[0][i]] = int8_t( i );
+      check_cuda( cudaMemcpyToSymbol( c_p2_node0, node0, sizeof( node0 ) ), "P2 constants (local nodes)" );
       int8_t from[60], from0[28];
       int    nf = 0;
       for ( int l = 0; l < 27; ++l )
@@ -1424,6 +1429,72 @@ __global__ void __launch_bounds__( 256 ) k_var_sweep( int n, int nC, int np, int
    }
 }
 
+// Stored stencils on levels whose tasks are edges and vertices alone: P1 levels 0 and 1, P2 level 0 (two
+// storage points per edge).  A sweep would only fill partial sums, and its launch and the wait for it are most of
+// the time there (shell of 240 cells: P1 apply, level 1 12.7 us with a sweep and the owners' combine and 8.8 us so,
+// P2 level 0 19.3 and 8.8), so the owners gather from their cells at once, eight threads each.  part( I ): the sum of incidence I's cell.
+template < typename T, typename A, int OP, typename F >
+__device__ __forceinline__ void low_owner( const LevelView& v, const BndSegments& seg, uint32_t flag, int copy_unflagged, const A* invd,
+                                           const T* src, const T* v1, T* v2, T* dst, A a0, A a1, F part )
+{
+   LowRec    low;
+   FaceRec   none;
+   int       sub;
+   if ( bnd_thread< 1 >( v, v.frec, seg, int( blockIdx.x * blockDim.x + threadIdx.x ), low, sub, none ) != BND_LOW ) return;
+   constexpr bool CARRIES = OP == OP_JAC || OP == OP_CHEB0 || OP == OP_CHEBI;
+   const bool     flagged = ( low.bc & flag ) != 0;
+   if ( !flagged && !( CARRIES && copy_unflagged ) ) low.count = 0;
+   A val = A( 0 ), second = A( 0 ), s = A( 0 );
+   if ( flagged )
+      for ( int q = sub; q < low.count; q += 8 ) s += part( v.irec[low.begin + q] );
+#pragma unroll
+   for ( int m = 4; m > 0; m >>= 1 ) s += __shfl_xor_sync( 0xffffffffu, s, m, 8 );
+   if ( low.count > 0 )
+   {
+      if ( flagged ) val = owner_value< T, A >( OP, low.owner, s, invd[low.owner], src, v1, v2, dst, a0, a1, second );
+      else if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) val = A( ldv( src + low.owner ) );
+      else if constexpr ( OP == OP_CHEBI ) val = A( ldc( v2 + low.owner ) );
+   }
+   __syncwarp();  // every thread of a task has read the owner before any writes it
+   put_low( v, low, sub, OP == OP_CHEBL ? v2 : dst, val );
+   if constexpr ( OP == OP_CHEBI )
+      if ( flagged ) put_low( v, low, sub, v2, second );
+}
+
+template < typename T, typename A, int OP >
+__global__ void __launch_bounds__( 256 ) k_var_low( LevelView v, BndSegments seg, uint32_t flag, int copy_unflagged, const A* __restrict__ S,
+                                                     int64_t ssize, const A* __restrict__ invd, const T* src, const T* v1, T* v2, T* dst,
+                                                     A a0, A a1 )
+{
+   low_owner< T, A, OP >( v, seg, flag, copy_unflagged, invd, src, v1, v2, dst, a0, a1, [&]( const IncRec& I ) {
+      return var_sum< T, A >( S + I.slot, ssize, src + I.slot, v.n, I.x, I.y, I.z, false, std::make_integer_sequence< int, 15 >() );
+   } );
+}
+
+// P2 level 0: a macro-cell is one micro-cell, and a node's row its ten nodes (component: blockIdx.y)
+template < typename T, typename A, int OP >
+__global__ void __launch_bounds__( 256 ) k_p2_stored_low( LevelView v, BndSegments seg, P2StoredView sv, uint32_t flag, int copy_unflagged,
+                                                           const A* __restrict__ S, const A* __restrict__ invd, AccVecs< T, A > vec, A a0,
+                                                           A a1 )
+{
+   const T* src = component( vec.src, blockIdx.y );
+   low_owner< T, A, OP >( v, seg, flag, copy_unflagged, invd, src, component( vec.v1, blockIdx.y ), component( vec.v2, blockIdx.y ),
+                          component( vec.dst, blockIdx.y ), a0, a1, [&]( const IncRec& I ) {
+                             int64_t       skip;
+                             const int64_t w = p2_weight_at( sv, I.cell, I.x, I.y, I.z, skip );
+                             const int     i = c_p2_node0[I.x + 3 * I.y + 9 * I.z];
+                             const int64_t c = v.cell_off[I.cell];
+                             A             sum = A( 0 );
+#pragma unroll
+                             for ( int j = 0; j < 10; ++j )
+                             {
+                                const int l = c_p2_loc[0][j];
+                                sum += __ldg( S + w + c_p2s_ent[10 * i + j] * skip ) * A( ldv( src + c + cidx( 2, l % 3, ( l / 3 ) % 3, l / 9 ) ) );
+                             }
+                             return sum;
+                          } );
+}
+
 template < typename A >
 __global__ void k_cell_invert( int n, int nrows, const int2* __restrict__ rows, const int64_t* __restrict__ cell_off, const A* acc,
                                A* invd )
@@ -2130,6 +2201,18 @@ static void run_var( Context* ctx, Mesh* m, Operator* op, int L, int dtype, cons
    A*         acc = acc_buffer< A >( op, L, P.size );
    const A*   S   = assembled_stencils< A >( op, L );
    const A*   inv = reinterpret_cast< const A* >( e.d_invd[dtype] );
+   if ( P.n <= 2 )
+   {
+      const LevelView   v   = make_view( m, L );
+      const BndSegments seg = bnd_segments( v, a.flag, a.copy_unflagged );
+      if ( seg.threads == 0 ) return;
+      k_var_low< T, A, OP ><<< ( seg.threads + 255 ) / 256, 256, 0, ctx->stream >>>( v, seg, a.flag, a.copy_unflagged, S, P.size, inv,
+                                                                                     (const T*) a.src, (const T*) a.v1, (T*) a.v2,
+                                                                                     (T*) a.dst, A( a.a0 ), A( a.a1 ) );
+      ++ctx->launches;
+      check_cuda( cudaGetLastError(), "assembled stencil launch" );
+      return;
+   }
    const int  np = int( tet_size( P.n + 1 ) ), stride = ( np + 31 ) / 32 * 32, nC = m->topo.nC;
    k_var_sweep< T, A, OP ><<< unsigned( ( int64_t( nC ) * stride + 255 ) / 256 ), 256, 0, ctx->stream >>>(
        P.n, nC, np, stride, reinterpret_cast< const ushort4* >( e.d_pts ), P.d_off + P.nB, P.d_bc + P.nB, a.flag, S, P.size, inv, acc,
@@ -2137,6 +2220,20 @@ static void run_var( Context* ctx, Mesh* m, Operator* op, int L, int dtype, cons
    ++ctx->launches;
    launch_bnd_acc< T, A, OP >( ctx, ctx->stream, P, a.flag, a.copy_unflagged, acc_vecs< T, A >( acc, a ), 1, inv, nullptr, A( a.a0 ), A( a.a1 ) );
    check_cuda( cudaGetLastError(), "assembled stencil launch" );
+}
+
+// P2 level 0 with stored matrices, up to three components in one launch
+template < typename T, typename A, int OP >
+static void run_stored_low( Context* ctx, Mesh* m, Operator* op, int L, const A* S, const A* inv, const AccVecs< T, A >& vec, int ncomp,
+                            const StencilArgs& a )
+{
+   const LevelView   v   = make_view( m, L );
+   const BndSegments seg = bnd_segments( v, a.flag, a.copy_unflagged );
+   if ( seg.threads == 0 ) return;
+   k_p2_stored_low< T, A, OP ><<< dim3( ( seg.threads + 255 ) / 256, ncomp ), 256, 0, ctx->stream >>>(
+       v, seg, *op->el[L].p2s, a.flag, a.copy_unflagged, S, inv, vec, A( a.a0 ), A( a.a1 ) );
+   ++ctx->launches;
+   check_cuda( cudaGetLastError(), "stored P2 launch" );
 }
 
 template < typename T, typename A, int OP >
@@ -2148,6 +2245,7 @@ static void run_elem( Context* ctx, Mesh* m, Operator* op, int L, int dtype, con
    const A* inv = reinterpret_cast< const A* >( op->el[L].d_invd[dtype] );
    if ( const A* S = assembled_stencils< A >( op, L ) )
    {
+      if ( P.n == 2 ) return run_stored_low< T, A, OP >( ctx, m, op, L, S, inv, acc_vecs< T, A >( acc, a ), 1, a );
       launch_p2_stored_sweep( ctx, P, dtype, *op->el[L].p2s, S, inv, acc, &a, 1 );
       launch_bnd_acc< T, A, OP >( ctx, ctx->stream, P, a.flag, a.copy_unflagged, acc_vecs< T, A >( acc, a ), 1, inv, nullptr, A( a.a0 ),
                                   A( a.a1 ) );
@@ -2489,13 +2587,14 @@ static void run_stored3( Context* ctx, Mesh* m, Operator* op, int L, int dtype, 
    const A*   inv = reinterpret_cast< const A* >( e.d_invd[dtype] );
    if ( !e.d_sacc ) check_cuda( cudaMalloc( &e.d_sacc, size_t( 3 * P.size ) * sizeof( double ) ), "cudaMalloc(component scratch)" );
    A* acc = reinterpret_cast< A* >( e.d_sacc );
-   launch_p2_stored_sweep( ctx, P, dtype, *e.p2s, S, inv, acc, a, 3 );
    AccVecs< T, A > vec{};
    for ( int k = 0; k < 3; ++k )
    {
       const AccVecs< T, A > v = acc_vecs< T, A >( acc + k * P.size, a[k] );
       vec.acc[k] = v.acc[0], vec.src[k] = v.src[0], vec.v1[k] = v.v1[0], vec.v2[k] = v.v2[0], vec.dst[k] = v.dst[0];
    }
+   if ( P.n == 2 ) return run_stored_low< T, A, OP >( ctx, m, op, L, S, inv, vec, 3, a[0] );
+   launch_p2_stored_sweep( ctx, P, dtype, *e.p2s, S, inv, acc, a, 3 );
    launch_bnd_acc< T, A, OP >( ctx, ctx->stream, P, a[0].flag, a[0].copy_unflagged, vec, 3, inv, nullptr, A( a[0].a0 ), A( a[0].a1 ) );
    check_cuda( cudaGetLastError(), "stored P2 combine launch" );
 }
