@@ -1431,8 +1431,9 @@ __global__ void __launch_bounds__( 256 ) k_var_sweep( int n, int nC, int np, int
 
 // Stored stencils on levels whose tasks are edges and vertices alone: P1 levels 0 and 1, P2 level 0 (two
 // storage points per edge).  A sweep would only fill partial sums, and its launch and the wait for it are most of
-// the time there (shell of 240 cells: P1 apply, level 1 12.7 us with a sweep and the owners' combine and 8.8 us so,
-// P2 level 0 19.3 and 8.8), so the owners gather from their cells at once, eight threads each.  part( I ): the sum of incidence I's cell.
+// the time there (shell of 240 cells: P1 apply on level 0, all vertices on the boundary, 12.6 us with a sweep and
+// the owners' combine and 2.9 us so, P2 level 0 19.3 and 8.8), so the owners gather from their cells at once, eight
+// threads each.  part( I ): the sum of incidence I's cell.
 template < typename T, typename A, int OP, typename F >
 __device__ __forceinline__ void low_owner( const LevelView& v, const BndSegments& seg, uint32_t flag, int copy_unflagged, const A* invd,
                                            const T* src, const T* v1, T* v2, T* dst, A a0, A a1, F part )

@@ -830,6 +830,7 @@ __device__ __forceinline__ A face_stencil( const T* c, const A* W, int cls, int 
    }
 }
 
+// (copy_unflagged: only set for the operations that carry a value to unflagged owners)
 // One boundary task: the sum over its neighbour cells of the stencil of its position class in each, the
 // operation's epilogue, and the write to the owner and every copy in the neighbouring cell arrays.  Every
 // index comes from the task's records, so the values wait on one dependent load for a face and on two for
@@ -844,11 +845,10 @@ __device__ __forceinline__ void bnd_point( const LevelView& v, const OpView< A >
    int       sub;
    const int kind = bnd_thread< 1 >( v, v.frec, seg, t, low, sub, r );
    if ( kind == BND_NONE ) return;
-   constexpr bool CARRIES = OP == OP_JAC || OP == OP_CHEB0 || OP == OP_CHEBI;  // only these write unflagged owners
    if ( kind == BND_LOW )
    {
       const bool flagged = ( low.bc & flag ) != 0;
-      if ( !flagged && !( CARRIES && copy_unflagged ) ) low.count = 0;
+      if ( !flagged && !copy_unflagged ) low.count = 0;
       A val = A( 0 ), second = A( 0 ), s = A( 0 );
       if ( flagged )
          for ( int q = sub; q < low.count; q += 8 )
@@ -874,7 +874,7 @@ __device__ __forceinline__ void bnd_point( const LevelView& v, const OpView< A >
    auto put = [&]( T* vec, A x ) { put_face( r, vec, x ); };
    if ( !( r.bc & flag ) )
    {
-      if ( !CARRIES || !copy_unflagged ) return;
+      if ( !copy_unflagged ) return;
       if constexpr ( OP == OP_JAC || OP == OP_CHEB0 ) put( dst, A( ldv( src + r.owner ) ) );
       else if constexpr ( OP == OP_CHEBI ) put( dst, A( ldc( v2 + r.owner ) ) );
       return;
@@ -971,13 +971,16 @@ static void run_stencil( Context* ctx, const LevelView& v, const OpView< A >& o,
    using Cfg = SwCfg< T, OP >;
    // cell interiors and boundary owners write disjoint slots and read only src (and their own
    // slots of the second vector), so the two kernels may run in either order
-   const BndSegments seg = bnd_segments( v, a.flag, a.copy_unflagged );
+   // the other operations leave unflagged owners alone (decided here: inside the kernel it changed the code of the
+   // last Chebyshev step, FP64 cycles on small levels 4 to 9 % slower)
+   const int         copy = OP == OP_JAC || OP == OP_CHEB0 || OP == OP_CHEBI ? a.copy_unflagged : 0;
+   const BndSegments seg  = bnd_segments( v, a.flag, copy );
    const int         nt  = seg.threads, nbnd = ( nt + kBndThreads - 1 ) / kBndThreads;
    if ( flat_cells< T, sweep_aux< OP >() >( v.n, int64_t( nC ) * v.nipts ) )
    {
       const int blocks = nbnd + int( ( int64_t( nC ) * v.nipts + kBndThreads - 1 ) / kBndThreads );
       if ( blocks == 0 ) return;
-      k_flat_stencil< T, A, OP ><<< blocks, kBndThreads, 0, ctx->stream >>>( v, o, seg, nbnd, nC, a.flag, a.copy_unflagged, src, v1, v2, dst,
+      k_flat_stencil< T, A, OP ><<< blocks, kBndThreads, 0, ctx->stream >>>( v, o, seg, nbnd, nC, a.flag, copy, src, v1, v2, dst,
                                                                             A( a.a0 ), A( a.a1 ) );
       ++ctx->launches;
       check_cuda( cudaGetLastError(), "stencil launch" );
@@ -1009,7 +1012,7 @@ static void run_stencil( Context* ctx, const LevelView& v, const OpView< A >& o,
       // branches, and the boundary kernel fills the SMs the sweep's last blocks leave idle.
       if ( nt > 0 )
       {
-         k_bnd_stencil< T, A, OP ><<< nbnd, kBndThreads, 0, ctx->stream >>>( v, o, seg, a.flag, a.copy_unflagged, src, v1, v2, dst,
+         k_bnd_stencil< T, A, OP ><<< nbnd, kBndThreads, 0, ctx->stream >>>( v, o, seg, a.flag, copy, src, v1, v2, dst,
                                                                                    A( a.a0 ), A( a.a1 ) );
          ++ctx->launches;
       }
@@ -1022,7 +1025,7 @@ static void run_stencil( Context* ctx, const LevelView& v, const OpView< A >& o,
    if ( big ) cell();
    if ( nt > 0 )
    {
-      k_bnd_stencil< T, A, OP ><<< nbnd, kBndThreads, 0, fk.aux() >>>( v, o, seg, a.flag, a.copy_unflagged, src, v1, v2, dst,
+      k_bnd_stencil< T, A, OP ><<< nbnd, kBndThreads, 0, fk.aux() >>>( v, o, seg, a.flag, copy, src, v1, v2, dst,
                                                                              A( a.a0 ), A( a.a1 ) );
       ++ctx->launches;
    }
