@@ -613,7 +613,7 @@ def p2_constant_leg(H, ctx, level=7, cycle_level=7):
     out = {"mesh": "unit cube, 6 macro-tets", "level": level, "inner_dofs": ndof, "dtype": "f64",
            "apply_ms": ms, "mdofs": ndof / (ms * 1e-3) / 1e6,
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                        "peak_kind": peak_kind, "kernel": "k_p2c_sweep<double,double,OP_APPLY> + k_p2c_bnd"}}
+                        "peak_kind": peak_kind, "kernel": "k_p2c_sweep<double,double,OP_APPLY> + k_p2c_flat"}}
     del x, y
     g = H.GeometricMultigridSolver(ctx, A, 0, cycle_level, 3, 3, smoother="chebyshev", chebyshev_order=3,
                                    power_iterations=20)
